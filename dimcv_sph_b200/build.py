@@ -2,8 +2,8 @@
 
 The SPH translation units are compiled with ``-fmad=false`` (no FMA
 contraction) and IEEE division / square root so that every per-pair
-expression rounds exactly as written; the N-body unit (dv_vvpe.cu) keeps FMA
-contraction on.  Objects go to ``dimcv_sph_b200/_build``; the shared library
+expression rounds exactly as written; the N-body units (dv_vvpe.cu,
+dv_farbox.cu) keep FMA contraction on.  Objects go to ``dimcv_sph_b200/_build``; the shared library
 lands next to this file so that it travels with the source tree.
 """
 from __future__ import annotations
@@ -30,6 +30,7 @@ UNITS = {
     "dv_sph.cu": ["-fmad=false"],
     "dv_dimcv.cu": ["-fmad=false"],
     "dv_vvpe.cu": [],
+    "dv_farbox.cu": [],
     "dv_noalloc.cu": ["-fmad=false"],
     "dv_vpm.cu": [],
     "dv_batch.cu": ["-fmad=false"],

@@ -65,6 +65,7 @@ static int build_morton(dv_ctx* c) {
   if (total > 26)
     return dv_fail(c, DV_EUNSUPPORTED, "cell grid needs %d Morton bits (max 26): domain/h too large",
                    total);
+  for (int d = 0; d < 3; ++d) c->axis_bits[d] = bits[d];
   int pos[3][21];
   int next = 0;
   int maxb = bits[0] > bits[1] ? bits[0] : bits[1];
@@ -110,6 +111,7 @@ static cudaError_t alloc(T** p, int64_t count) {
 DV_API void dv_destroy(dv_ctx* c) {
   if (!c) return;
   dv_batch_free(c);
+  dv_farbox_free(c);
   void* ptrs[] = {c->d_cnt,   c->d_flag,    c->keys[0],   c->keys[1],   c->vals[0], c->vals[1],
                   c->hist,    c->cell_start, c->cell_end, c->mt[0],     c->mt[1],   c->mt[2],
                   c->scan_part, c->dscan_part, c->red_part, c->ired_part, c->flags, c->offs,
@@ -205,7 +207,7 @@ DV_API dv_ctx* dv_create(const dv_params* params, int64_t capacity, void* stream
   c->nbr_cap = cap * (params->dim == 3 ? 48 : 24);
   A(c->nbr_off, cap + 1);
   A(c->nbr_idx, c->nbr_cap);
-  A(c->d_nbr_ok, 2);  // [0]: lists valid, [1]: a material other than fluid / solid seen by the build
+  A(c->d_nbr_ok, 3);  // [0]: lists valid, [1]: keys valid, [2]: a material other than fluid / solid seen by the build
   // the 3-D build's first pass stores up to 64 neighbours per particle in
   // fixed rows (a settled lattice has at most 36); 2-D builds have none
   c->nbr_slots = params->dim == 3 ? 64 : 0;
@@ -217,12 +219,17 @@ DV_API dv_ctx* dv_create(const dv_params* params, int64_t capacity, void* stream
   if (e == cudaSuccess) e = cudaMemset(c->d_cnt, 0, sizeof(dv_counters));
   if (e == cudaSuccess) e = cudaMemset(c->d_flag, 0, sizeof(int32_t) * 4);
   if (e == cudaSuccess) e = cudaMemset(c->d_prof, 0, sizeof(double) * 4);
-  if (e == cudaSuccess) e = cudaMemset(c->d_nbr_ok, 0, 2 * sizeof(int32_t));
+  if (e == cudaSuccess) e = cudaMemset(c->d_nbr_ok, 0, 3 * sizeof(int32_t));
   if (e == cudaSuccess) e = cudaMemset(c->cell_start, 0, sizeof(int32_t) * c->ncells);
   if (e == cudaSuccess) e = cudaMemset(c->cell_end, 0, sizeof(int32_t) * c->ncells);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e != cudaSuccess) {
     dv_cuda_check(c, e, "dv_create allocation");
+    g_create_error = c->err;
+    dv_destroy(c);
+    return nullptr;
+  }
+  if (dv_farbox_create(c) != DV_OK) {
     g_create_error = c->err;
     dv_destroy(c);
     return nullptr;

@@ -215,13 +215,19 @@ __global__ void k_flag_samples(const dv_fields F, const dv_counters* __restrict_
   flags[i] = (i < C->n && F.is_sample[i] == 1) ? 1u : 0u;
 }
 
-template <int D>
+// CHECK: also tell the far field on boxes of a target outside its sorted box
+template <int D, bool CHECK>
 __global__ void k_flag_targets(dv_params P, const dv_fields F, const dv_counters* __restrict__ C,
-                               int m, uint32_t* __restrict__ flags) {
+                               int m, uint32_t* __restrict__ flags, DevGrid G, const uint32_t* __restrict__ keys,
+                               dv_farbox B) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
   uint32_t f = 0;
-  if (i < C->n && F.material[i] == DV_MATERIAL_FLUID) f = in_vortex_domain<D>(P, ldv<D>(F.x, i)) ? 1u : 0u;
+  if (i < C->n && F.material[i] == DV_MATERIAL_FLUID) {
+    const V3 x = ldv<D>(F.x, i);
+    f = in_vortex_domain<D>(P, x) ? 1u : 0u;
+    if (CHECK && f && !in_sorted_box(P, G, x, keys[i], B.lowbits)) B.meta[0] = 1u;
+  }
   flags[i] = f;
 }
 
@@ -243,13 +249,17 @@ __global__ void k_store_count(const uint32_t* __restrict__ offs, dv_counters* C,
 
 // Fills c->targets with the slots of fluid particles inside the vortex
 // domain, in ascending slot order; count in C->n_targets.
-int dv_build_targets(dv_ctx* c, const dv_fields* f) {
+int dv_build_targets(dv_ctx* c, const dv_fields* f, bool check) {
   const int m = (int)std::min<int64_t>(c->n_upper, c->cap) + 1;
   const int nb = dv_blocks(m);
+  const DevGrid G = dv_grid_cells(c);
+  const uint32_t* keys = c->keys[c->perm_buf];
   if (c->p.dim == 2)
-    k_flag_targets<2><<<nb, DV_THREADS, 0, c->stream>>>(c->p, *f, c->d_cnt, m, c->flags);
+    k_flag_targets<2, false><<<nb, DV_THREADS, 0, c->stream>>>(c->p, *f, c->d_cnt, m, c->flags, G, keys, c->farbox);
+  else if (check)
+    k_flag_targets<3, true><<<nb, DV_THREADS, 0, c->stream>>>(c->p, *f, c->d_cnt, m, c->flags, G, keys, c->farbox);
   else
-    k_flag_targets<3><<<nb, DV_THREADS, 0, c->stream>>>(c->p, *f, c->d_cnt, m, c->flags);
+    k_flag_targets<3, false><<<nb, DV_THREADS, 0, c->stream>>>(c->p, *f, c->d_cnt, m, c->flags, G, keys, c->farbox);
   DV_LAUNCHED(c);
   int rc = dv_scan_u32(c, c->flags, c->offs, m);
   if (rc) return rc;
@@ -604,6 +614,7 @@ DV_API int dv_kvn_sample(dv_ctx* c, const dv_fields* f, const dv_solver_fields* 
 DV_API int dv_record_samples(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s) {
   if (!c || !f) return DV_EINVAL;
   if (int rc = check_solver(c, s)) return rc;
+  c->host_samples = -1;
   const int m = (int)std::min<int64_t>(c->n_upper, c->cap) + 1;
   const int nb = dv_blocks(m);
   k_flag_samples<<<nb, DV_THREADS, 0, c->stream>>>(*f, c->d_cnt, m, c->flags);
@@ -644,7 +655,9 @@ DV_API int dv_sample(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s, i
   if (M < 0 || M > c->cap) return dv_fail(c, DV_EINVAL, "dv_sample: M=%d outside [0, capacity]", M);
   if (mode == DV_SAMPLE_BERNOULLI) {
     return dv_record_samples(c, f, s);
-  } else if (mode == DV_SAMPLE_INJECTED) {
+  }
+  if (mode == DV_SAMPLE_INJECTED || mode == DV_SAMPLE_INVERSE_CDF || mode == DV_SAMPLE_STRATIFIED) c->host_samples = M;
+  if (mode == DV_SAMPLE_INJECTED) {
     k_set_num_samples<<<1, 1, 0, c->stream>>>(c->d_cnt, M);
     DV_LAUNCHED(c);
     return DV_OK;

@@ -317,7 +317,7 @@ __global__ void k_csr_fill(dv_params P, DevGrid G, const float* __restrict__ x,
   if (i >= C->n || !ok[0] || !nbr_row_built(mat, dyn, i)) return;
   uint32_t k = off[i];
   for_each_neighbor_m<D>(P, G, x, mat, i, ldv<D>(x, i),
-                         [&](int j, V3, float, int mj) { out[k++] = nbr_entry(j, mj, ok + 1); });
+                         [&](int j, V3, float, int mj) { out[k++] = nbr_entry(j, mj, ok + 2); });
 }
 
 template <int D>
@@ -357,12 +357,12 @@ __global__ void k_csr_compact(dv_params P, DevGrid G, const float* __restrict__ 
       const int32_t* row = rows + (int64_t)i * slots;
       for (uint32_t k = lane; k < cnt; k += 32) {
         const int j = row[k];
-        out[k0 + k] = nbr_entry(j, __ldg(mat + j), ok + 1);
+        out[k0 + k] = nbr_entry(j, __ldg(mat + j), ok + 2);
       }
     } else if (lane == (i & 31)) {
       uint32_t k = k0;
       for_each_neighbor_m<D>(P, G, x, mat, i, ldv<D>(x, i),
-                             [&](int j, V3, float, int mj) { out[k++] = nbr_entry(j, mj, ok + 1); });
+                             [&](int j, V3, float, int mj) { out[k++] = nbr_entry(j, mj, ok + 2); });
     }
   }
 }
@@ -370,12 +370,13 @@ __global__ void k_csr_compact(dv_params P, DevGrid G, const float* __restrict__ 
 __global__ void k_csr_ok(const uint32_t* __restrict__ off, const dv_counters* __restrict__ C, int64_t cap,
                          int32_t* __restrict__ ok) {
   ok[0] = (int64_t)off[C->n] <= cap ? 1 : 0;
+  ok[1] = 1;  // the sorted keys are those of the current slots
 }
 
 // after the fill: lists that met a material other than fluid or solid are
 // not used (their entries cannot encode it)
 __global__ void k_csr_material_check(int32_t* __restrict__ ok) {
-  if (ok[1]) ok[0] = 0;
+  if (ok[2]) ok[0] = 0;
 }
 
 static int build_csr(dv_ctx* c, const dv_fields* f) {
@@ -383,7 +384,7 @@ static int build_csr(dv_ctx* c, const dv_fields* f) {
   const int nb = dv_blocks(m);
   DevGrid G = dv_grid_cells(c);
   const bool rows = c->p.dim == 3;
-  DV_CK(c, cudaMemsetAsync(c->d_nbr_ok + 1, 0, sizeof(int32_t), c->stream));
+  DV_CK(c, cudaMemsetAsync(c->d_nbr_ok + 2, 0, sizeof(int32_t), c->stream));
   if (rows)
     k_csr_rows<3><<<nb, DV_THREADS, 0, c->stream>>>(c->p, G, f->x, f->material, f->is_dynamic, c->d_cnt, m,
                                                     c->nbr_slots, c->flags, c->nbr_rows);
@@ -409,7 +410,7 @@ static int build_csr(dv_ctx* c, const dv_fields* f) {
 
 // positions or the particle count changed: sweeps go back to the cell scan
 int dv_invalidate_lists(dv_ctx* c) {
-  DV_CK(c, cudaMemsetAsync(c->d_nbr_ok, 0, sizeof(int32_t), c->stream));
+  DV_CK(c, cudaMemsetAsync(c->d_nbr_ok, 0, 2 * sizeof(int32_t), c->stream));
   return DV_OK;
 }
 

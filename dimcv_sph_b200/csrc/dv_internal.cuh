@@ -18,6 +18,26 @@
 #define DV_THREADS 256
 #define DV_MAX_FAR_CHUNKS 8
 
+// ------------------------------------------------- far field on boxes (3-D)
+// Device buffers of dv_farbox.cu; enabled = 0 where the grid or the size is
+// none that they are built for.  A box is 8 cells on a side (whole axes of
+// fewer cells): the cell keys that agree above `lowbits`.
+struct dv_farbox {
+  int enabled = 0;
+  int nbox = 0, lowbits = 0, max_boxes = 0, stripe_mul = 1;
+  // [0] a position or weight that needs the direct loop; [1] boxes with
+  // targets, [2] boxes with samples, [3] near tiles; [4..5] pair evaluations (u64)
+  uint32_t* meta = nullptr;
+  int32_t *bt = nullptr, *bs = nullptr;     // [nbox + 1] first target / sample of a box
+  int4* tbox = nullptr;                     // [max_boxes] boxes with targets: coordinates, first target
+  int32_t *tcnt = nullptr, *tile0 = nullptr;  // [max_boxes] their targets and first near tile
+  int4* sbox = nullptr;                     // [nbox] boxes with samples: coordinates, first sample
+  int32_t* scnt = nullptr;
+  float* nodes = nullptr;                   // node sums
+  float4* coef = nullptr;                   // polynomial coefficients
+  float4 *pos = nullptr, *w = nullptr;      // [cap] the distinct samples in slot order
+};
+
 // ------------------------------------------------------------------ context
 struct dv_ctx {
   dv_params p;
@@ -44,6 +64,7 @@ struct dv_ctx {
   int64_t ncells = 0;  // padded Morton cell count
   int kbits = 0;       // sort key bits (Morton bits + 1 for the inactive key)
   int npasses = 0;
+  int axis_bits[3] = {0, 0, 0};  // cell-coordinate bits of each axis in the key
   int perm_buf = 0;    // which vals[] holds the last permutation
   uint32_t* mt[3] = {nullptr, nullptr, nullptr};  // per-axis Morton tables
 
@@ -77,9 +98,13 @@ struct dv_ctx {
   uint32_t* nbr_off = nullptr;  // cap + 1
   int32_t* nbr_idx = nullptr;   // nbr_cap
   int64_t nbr_cap = 0;
-  int32_t* d_nbr_ok = nullptr;  // [0]: 1 while the lists match the current positions; [1]: build scratch
+  int32_t* d_nbr_ok = nullptr;  // [0]: 1 while the lists match the current positions; [1]: 1 while keys[perm_buf]
+                                // are the sorted slots' cell keys; [2]: build scratch
   int32_t* nbr_rows = nullptr;  // 3-D: cap * nbr_slots, the first pass's fixed row of particle i at i * nbr_slots
   int nbr_slots = 0;
+
+  dv_farbox farbox;
+  int64_t host_samples = -1;  // sample count of the last draw where the host knows it
 
   // scene batch (n_scenes > 1): cell keys carry the scene id above
   // scene_shift bits; scene_ptr is the scene id of each slot of the sorted
@@ -184,7 +209,19 @@ int dv_batch_draw(dv_ctx* c, const dv_solver_fields* s);
 int dv_batch_vvpe(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s);
 int dv_far_tile_width(const dv_ctx* c);
 int dv_far_min_tile_width();  // the narrowest far-field tile (threads per CTA x 2 targets)
-int dv_build_targets(dv_ctx* c, const dv_fields* f);
+// check: also raise farbox.meta[0] where a target has left the box of its sorted cell
+int dv_build_targets(dv_ctx* c, const dv_fields* f, bool check = false);
+// dv_farbox.cu: the 3-D far field by interpolation on boxes.  wanted: host-side
+// rule; begin (before dv_build_targets), pack (instead of the slot list), plan,
+// run; the device decides with farbox_on whether the result is used
+int dv_farbox_create(dv_ctx* c);
+void dv_farbox_free(dv_ctx* c);
+bool dv_farbox_wanted(const dv_ctx* c);
+int dv_farbox_near_parts(const dv_ctx* c);
+int dv_farbox_begin(dv_ctx* c);
+int dv_farbox_pack(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s, int nu);
+int dv_farbox_plan(dv_ctx* c);
+int dv_farbox_run(dv_ctx* c, const dv_fields* f);
 
 // ------------------------------------------------------------- scan helpers
 // Exclusive scan of uint32 / double arrays on the context stream
@@ -451,6 +488,35 @@ __device__ __forceinline__ void for_each_neighbor_m(const dv_params& P, const De
                                                     const float* __restrict__ x, const int32_t* __restrict__ mat,
                                                     int i, V3 xi, F&& f) {
   for_each_neighbor_impl<D, true>(P, G, x, mat, i, xi, f);
+}
+
+// ------------------------------------------------- far field on boxes (3-D)
+// Whether the boxes carry this call's far field: every position in its sorted
+// box and every weight of ordinary size (meta[0]), and fewer pair evaluations
+// than the direct loop: the node sums and near pairs, 250 a target for reading
+// the polynomial, 5e7 (about 25 us) for the extra launches, and a tenth of
+// slack.  The same answer in every thread of every kernel that asks.
+__device__ __forceinline__ bool farbox_on(const dv_farbox& B, const dv_counters* __restrict__ C) {
+  if (!B.enabled) return false;
+  const uint32_t na = B.meta[1];
+  if (B.meta[0] || na == 0 || na > (uint32_t)B.max_boxes) return false;
+  const unsigned long long nt = (unsigned long long)C->n_targets, M = (unsigned long long)C->num_samples;
+  const unsigned long long cost =
+      *reinterpret_cast<const unsigned long long*>(B.meta + 4) + 250ull * nt + 50000000ull;
+  return cost < nt * M / 10ull * 9ull;
+}
+
+// x lies inside the cell grid and its box is that of the sorted cell `key`
+__device__ __forceinline__ bool in_sorted_box(const dv_params& P, const DevGrid& G, V3 x, uint32_t key, int lowbits) {
+  const float t[3] = {P.cell_origin_offset ? x.x - P.domain_start[0] : x.x,
+                      P.cell_origin_offset ? x.y - P.domain_start[1] : x.y,
+                      P.cell_origin_offset ? x.z - P.domain_start[2] : x.z};
+  const int c[3] = {cell_coord(P, x.x, 0), cell_coord(P, x.y, 1), cell_coord(P, x.z, 2)};
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+    if (!(t[d] >= 0.0f) || c[d] >= P.grid_num[d]) return false;
+  const uint32_t k = __ldg(G.mt0 + c[0]) | __ldg(G.mt1 + c[1]) | __ldg(G.mt2 + c[2]);
+  return ((k ^ key) >> lowbits) == 0u;
 }
 
 // ---------------------------------------------------------------- Philox

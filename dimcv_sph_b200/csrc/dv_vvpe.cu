@@ -13,9 +13,9 @@
 // This file is compiled with FMA contraction on.
 #include <algorithm>
 
+#include "dv_far.cuh"
 #include "dv_internal.cuh"
 
-int dv_build_targets(dv_ctx* c, const dv_fields* f);
 int dv_launch_vvpe_near(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s);
 
 #define FT 256  // threads per CTA
@@ -217,35 +217,6 @@ static bool fast_kernel_ok(const dv_params& P) {
 // bit for bit as the main loop computed them) and removes them from the far
 // count.  Per pair this leaves ~14 issue slots instead of ~28.
 
-__device__ __forceinline__ float rcp_approx(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-
-// 1/sqrt(x) in one MUFU operation.  The blob kernel's argument |r|² + δ² is
-// at least δ² > 0 and never subnormal, so flushing subnormals changes no
-// result; without .ftz the approximate rsqrt also carries the code that
-// rescales subnormal inputs, which every pair would pay for.
-__device__ __forceinline__ float rsqrt_approx(float x) {
-  float r;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-
-// The blob kernel's (|r|² + δ²)^(-3/2): s = δ² + dx² + dy² + dz² by three
-// fma (δ² enters first, saving an add), then 1/s · 1/sqrt(s) from two MUFU
-// operations and one multiply instead of the cube of 1/sqrt(s) (two
-// multiplies): 16 FP32-pipe operations per pair instead of 18 in a loop the
-// FP32 pipe bounds, one more on the otherwise idle MUFU.  The scalar loop,
-// the paired loop and the near-sample correction all use this one form.
-__device__ __forceinline__ float blob_k(float dx, float dy, float dz, float d2) {
-  float s = __fmaf_rn(dx, dx, d2);
-  s = __fmaf_rn(dy, dy, s);
-  s = __fmaf_rn(dz, dz, s);
-  return __fmul_rn(rcp_approx(s), rsqrt_approx(s));
-}
-
 // coordinate difference, minimum image on a periodic box
 template <bool PER>
 __device__ __forceinline__ float wrapd(float d, float L) {
@@ -328,11 +299,6 @@ __device__ __forceinline__ void far_accum(float px, float py, float pz, float4 s
 // more of the rcp -> mul -> fma latency than 16: sphere3d far field 57.5 ->
 // 54.6 ms per step), 2 for 6 and 8 (their wider register tiles spill at 80)
 #define DV_FAR_MINB(TT) (((TT) <= 4 ? 3 : 2) * (256 / FT2))
-#ifndef DV_FAR_QUNROLL
-#define DV_FAR_QUNROLL 2  // samples per unrolled step of the paired loop
-#endif
-constexpr int kFarQUnroll = DV_FAR_QUNROLL;
-
 // sample chunk blockIdx.y of nchunk: [m0, m0 + M) of the M_total samples;
 // the chunk's partial sums go to far_acc[chunk * stride + t]
 __device__ __forceinline__ void sample_chunk(int M_total, int nchunk, int& m0, int& M) {
@@ -347,9 +313,11 @@ __global__ void __launch_bounds__(FT2) k_far_main(dv_params P, const float* __re
                                                   const int32_t* __restrict__ targets,
                                                   const float4* __restrict__ spos,
                                                   const float4* __restrict__ sw,
-                                                  float4* __restrict__ far_acc, int nchunk, int64_t stride) {
+                                                  float4* __restrict__ far_acc, int nchunk, int64_t stride,
+                                                  dv_farbox B) {
   __shared__ float4 s_p[FTILE2];
   __shared__ float4 s_w[FTILE2];
+  if (D == 3 && !COMP && !PER && farbox_on(B, C)) return;
   const int nt = C->n_targets;
   int m0, M;
   sample_chunk(C->num_samples, nchunk, m0, M);
@@ -421,12 +389,14 @@ __global__ void k_sample_slots(const int32_t* __restrict__ mult, int nu, const u
     if (mult[j] > 0) slot[rank[j]] = j;
 }
 
-static int sample_slots(dv_ctx* c) {
+// boxed: the slot list comes with the packed samples of the far field on boxes
+static int sample_slots(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s, bool boxed = false) {
   const int nu = (int)std::min<int64_t>(c->n_upper, c->cap);
   k_sample_flags<<<c->num_sms * 4, DV_THREADS, 0, c->stream>>>(c->mult, nu, c->sflag);
   DV_LAUNCHED(c);
   int rc = dv_scan_u32(c, c->sflag, c->srank, (int64_t)nu + 1);
   if (rc) return rc;
+  if (boxed) return dv_farbox_pack(c, f, s, nu);
   k_sample_slots<<<c->num_sms * 4, DV_THREADS, 0, c->stream>>>(c->mult, nu, c->srank, c->sslot);
   DV_LAUNCHED(c);
   return DV_OK;
@@ -544,9 +514,10 @@ __global__ void k_far_fix(dv_params P, DevGrid G, dv_fields F, dv_solver_fields 
                           const int32_t* __restrict__ mult, const uint32_t* __restrict__ srank,
                           const int32_t* __restrict__ sslot, const float4* __restrict__ far_acc,
                           const float4* __restrict__ near_v, const float* __restrict__ near_S, int nchunk,
-                          int64_t stride) {
+                          int64_t stride, dv_farbox B, int box_parts) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= C->n_targets) return;
+  if (D == 3 && farbox_on(B, C)) nchunk = box_parts;
   far_fix_one<D, BLOB, PER>(P, G, F, S, t, targets[t], C->num_samples, C->kden_sum_f32, 0u, mult, srank, sslot,
                             far_acc, near_v, near_S, nchunk, stride);
 }
@@ -645,38 +616,8 @@ __global__ void __launch_bounds__(FT2) k_far_main_b(dv_params P, const float* __
 // loop's own IEEE operation in the same order, so far_acc is bit-identical;
 // the pairs halve the issue slots of a loop that is issue-bound, not
 // FP32-pipe-bound.  Samples are staged in shared memory pre-duplicated
-// ({s, s} pairs, ω̃/kden components negated where the loop subtracts).
-typedef unsigned long long f2_t;
-__device__ __forceinline__ f2_t f2_pack(float a, float b) {
-  f2_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void f2_unpack(f2_t v, float& a, float& b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ f2_t f2_sub(f2_t a, f2_t b) {
-  f2_t d;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ f2_t f2_mul(f2_t a, f2_t b) {
-  f2_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ f2_t f2_fma(f2_t a, f2_t b, f2_t c) {
-  f2_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-
-// float4 words per staged sample of the paired loops: the reference kernel
-// needs {x, y, (z,) ω̂z, -ω̂z, (ω̂y, -ω̂x)}, the blob kernel {x, y, z, ω̂, -ω̂}
-template <int D, bool BLOB>
-constexpr int far_x2_words() {
-  return BLOB ? 5 : (D == 3 ? 4 : 2);
-}
+// ({s, s} pairs, ω̃/kden components negated where the loop subtracts); the
+// inner loop is far_x2_loop (dv_far.cuh).
 
 // targets [tbase + k·FT2 + tid] (k < TT) of targets[0, nt) against samples
 // [m0, m0 + M); writes far_acc[t] for t < nt.  Block-uniform bounds.
@@ -694,7 +635,6 @@ __device__ __forceinline__ void far_x2_run(const dv_params& P, const float* __re
                                            int M, float4* __restrict__ far_acc, float4* s4, int n_valid = -1) {
   static_assert(!BLOB || D == 3, "the paired blob loop is 3-D");
   constexpr int NP = TT / 2;
-  constexpr int NQ = far_x2_words<D, BLOB>();  // duplicated float4 per sample
   f2_t PX[NP], PY[NP], PZ[NP], AX[NP], AY[NP], AZ[NP];
   bool OK[2 * NP];
 #pragma unroll
@@ -722,87 +662,10 @@ __device__ __forceinline__ void far_x2_run(const dv_params& P, const float* __re
     for (int q = threadIdx.x; q < m; q += FT2) {
       const float4 sp = spos[m0 + base + q];
       const float4 w = sw[m0 + base + q];
-      if (BLOB) {
-        s4[5 * q] = make_float4(sp.x, sp.x, sp.y, sp.y);
-        s4[5 * q + 1] = make_float4(sp.z, sp.z, w.z, w.z);
-        s4[5 * q + 2] = make_float4(-w.y, -w.y, w.x, w.x);
-        s4[5 * q + 3] = make_float4(-w.z, -w.z, w.y, w.y);
-        s4[5 * q + 4] = make_float4(-w.x, -w.x, 0.0f, 0.0f);
-      } else if (D == 3) {
-        s4[4 * q] = make_float4(sp.x, sp.x, sp.y, sp.y);
-        s4[4 * q + 1] = make_float4(sp.z, sp.z, w.z, w.z);
-        s4[4 * q + 2] = make_float4(-w.z, -w.z, w.y, w.y);
-        s4[4 * q + 3] = make_float4(-w.x, -w.x, 0.0f, 0.0f);
-      } else {
-        s4[2 * q] = make_float4(sp.x, sp.x, sp.y, sp.y);
-        s4[2 * q + 1] = make_float4(w.z, w.z, -w.z, -w.z);
-      }
+      far_x2_stage<D, BLOB>(s4, q, sp, w);
     }
     __syncthreads();
-    if (BLOB) {
-      const float d2v = P.blob_delta2;
-      const f2_t D2 = f2_pack(d2v, d2v);
-#pragma unroll kFarQUnroll
-      for (int q = 0; q < m; ++q) {
-        const ulonglong2 v0 = s2[NQ * q], v1 = s2[NQ * q + 1], v2 = s2[NQ * q + 2], v3 = s2[NQ * q + 3];
-        const ulonglong2 v4 = s2[NQ * q + 4];
-        const f2_t SZ = v1.x, WZ = v1.y, NWY = v2.x, WX = v2.y, NWZ = v3.x, WY = v3.y, NWX = v4.x;
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-          const f2_t DX = f2_sub(PX[p], v0.x), DY = f2_sub(PY[p], v0.y), DZ = f2_sub(PZ[p], SZ);
-          f2_t S2 = f2_fma(DX, DX, D2);
-          S2 = f2_fma(DY, DY, S2);
-          S2 = f2_fma(DZ, DZ, S2);
-          float sa, sb;
-          f2_unpack(S2, sa, sb);
-          const f2_t KK = f2_mul(f2_pack(rcp_approx(sa), rcp_approx(sb)), f2_pack(rsqrt_approx(sa), rsqrt_approx(sb)));
-          const f2_t A = f2_mul(KK, DX), B = f2_mul(KK, DY), E = f2_mul(KK, DZ);
-          AX[p] = f2_fma(B, WZ, AX[p]);
-          AX[p] = f2_fma(E, NWY, AX[p]);
-          AY[p] = f2_fma(E, WX, AY[p]);
-          AY[p] = f2_fma(A, NWZ, AY[p]);
-          AZ[p] = f2_fma(A, WY, AZ[p]);
-          AZ[p] = f2_fma(B, NWX, AZ[p]);
-        }
-      }
-      continue;
-    }
-#pragma unroll kFarQUnroll
-    for (int q = 0; q < m; ++q) {
-      const ulonglong2 v0 = s2[NQ * q], v1 = s2[NQ * q + 1];
-      f2_t SZ = 0ull, WZ, NWZ, WY = 0ull, NWX = 0ull;
-      if (D == 3) {
-        const ulonglong2 v2 = s2[NQ * q + 2], v3 = s2[NQ * q + 3];
-        SZ = v1.x;
-        WZ = v1.y;
-        NWZ = v2.x;
-        WY = v2.y;
-        NWX = v3.x;
-      } else {
-        WZ = v1.x;
-        NWZ = v1.y;
-      }
-#pragma unroll
-      for (int p = 0; p < NP; ++p) {
-        const f2_t DX = f2_sub(PX[p], v0.x), DY = f2_sub(PY[p], v0.y);
-        f2_t R2 = f2_mul(DX, DX);
-        R2 = f2_fma(DY, DY, R2);
-        if (D == 3) {
-          const f2_t DZ = f2_sub(PZ[p], SZ);
-          R2 = f2_fma(DZ, DZ, R2);
-        }
-        float ra, rb;
-        f2_unpack(R2, ra, rb);
-        const f2_t KK = f2_pack(rcp_approx(fmaxf(ra, lim)), rcp_approx(fmaxf(rb, lim)));
-        const f2_t A = f2_mul(KK, DX), B = f2_mul(KK, DY);
-        AX[p] = f2_fma(B, WZ, AX[p]);
-        AY[p] = f2_fma(A, NWZ, AY[p]);
-        if (D == 3) {
-          AZ[p] = f2_fma(A, WY, AZ[p]);
-          AZ[p] = f2_fma(B, NWX, AZ[p]);
-        }
-      }
-    }
+    far_x2_loop<D, NP, BLOB, true>(s2, 0, 1, m, PX, PY, PZ, AX, AY, AZ, lim, P.blob_delta2);
   }
 #pragma unroll
   for (int p = 0; p < NP; ++p) {
@@ -822,8 +685,9 @@ __global__ void __launch_bounds__(FT2, DV_FAR_MINB(TT)) k_far_main_x2(dv_params 
                                                      const int32_t* __restrict__ targets,
                                                      const float4* __restrict__ spos,
                                                      const float4* __restrict__ sw, float4* __restrict__ far_acc,
-                                                     int nchunk, int64_t stride) {
+                                                     int nchunk, int64_t stride, dv_farbox B) {
   __shared__ float4 s4[far_x2_words<D, BLOB>() * FTILE2];
+  if (D == 3 && farbox_on(B, C)) return;
   const int nt = C->n_targets;
   const int tbase = blockIdx.x * FT2 * TT;
   if (tbase >= nt) return;  // uniform per CTA
@@ -857,7 +721,7 @@ static inline int far_tile_run(int tt, bool paired) {
 }
 
 template <int D, bool BLOB, bool COMP, bool PER>
-static void launch_main_tt(dv_ctx* c, const dv_fields* f, int tt_req) {
+static void launch_main_tt(dv_ctx* c, const dv_fields* f, int tt_req, const dv_farbox& B) {
   // the plain (uncompensated, non-periodic) loops: the reference kernel, and
   // the blob kernel in 3-D
   constexpr bool paired = !COMP && !PER && (!BLOB || D == 3);
@@ -867,10 +731,10 @@ static void launch_main_tt(dv_ctx* c, const dv_fields* f, int tt_req) {
   const dim3 grid(nb, c->far_chunks);
 #define L(TTV)                                                                                                 \
   k_far_main<D, TTV, BLOB, COMP, PER><<<grid, FT2, 0, c->stream>>>(c->p, f->x, c->d_cnt, c->targets, c->spos, \
-                                                                   c->sw, c->far_acc, c->far_chunks, c->cap)
+                                                                   c->sw, c->far_acc, c->far_chunks, c->cap, B)
 #define L2(TTV)                                                                                              \
   k_far_main_x2<D, TTV, BLOB && D == 3><<<grid, FT2, 0, c->stream>>>(c->p, f->x, c->d_cnt, c->targets, c->spos, \
-                                                                     c->sw, c->far_acc, c->far_chunks, c->cap)
+                                                                     c->sw, c->far_acc, c->far_chunks, c->cap, B)
   if (tt == 2)
     L(2);
   else if (tt == 4) {
@@ -891,30 +755,32 @@ static void launch_main_tt(dv_ctx* c, const dv_fields* f, int tt_req) {
 }
 
 template <int D, bool PER>
-static void launch_main_p(dv_ctx* c, const dv_fields* f, int tt) {
+static void launch_main_p(dv_ctx* c, const dv_fields* f, int tt, const dv_farbox& B) {
   const bool blob = c->p.kernel_mode == DV_KERNEL_BLOB3D;
   const bool comp = c->p.compensated != 0;
   if (blob)
-    comp ? launch_main_tt<D, true, true, PER>(c, f, tt) : launch_main_tt<D, true, false, PER>(c, f, tt);
+    comp ? launch_main_tt<D, true, true, PER>(c, f, tt, B) : launch_main_tt<D, true, false, PER>(c, f, tt, B);
   else
-    comp ? launch_main_tt<D, false, true, PER>(c, f, tt) : launch_main_tt<D, false, false, PER>(c, f, tt);
+    comp ? launch_main_tt<D, false, true, PER>(c, f, tt, B) : launch_main_tt<D, false, false, PER>(c, f, tt, B);
 }
 
+// B: the boxes that may carry this call's far field instead (the loop then
+// returns at once); a disabled dv_farbox where they were not planned
 template <int D>
-static void launch_main(dv_ctx* c, const dv_fields* f, int tt) {
+static void launch_main(dv_ctx* c, const dv_fields* f, int tt, const dv_farbox& B) {
   if (c->p.periodic)
-    launch_main_p<D, true>(c, f, tt);
+    launch_main_p<D, true>(c, f, tt, B);
   else
-    launch_main_p<D, false>(c, f, tt);
+    launch_main_p<D, false>(c, f, tt, B);
 }
 
 template <int D>
-static void launch_fix(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s) {
+static void launch_fix(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s, const dv_farbox& B) {
   const int nb = dv_blocks(std::min<int64_t>(c->n_upper, c->cap), 128);
-#define LF(B, PR)                                                                                      \
-  k_far_fix<D, B, PR><<<nb, 128, 0, c->stream>>>(c->p, dv_grid(c), *f, *s, c->d_cnt, c->targets, c->mult, \
+#define LF(BL, PR)                                                                                     \
+  k_far_fix<D, BL, PR><<<nb, 128, 0, c->stream>>>(c->p, dv_grid(c), *f, *s, c->d_cnt, c->targets, c->mult, \
                                                  c->srank, c->sslot, c->far_acc, c->near_v, c->near_S,    \
-                                                 c->far_chunks, c->cap)
+                                                 c->far_chunks, c->cap, B, dv_farbox_near_parts(c))
   const bool blob = c->p.kernel_mode == DV_KERNEL_BLOB3D;
   if (c->p.periodic)
     blob ? LF(true, true) : LF(false, true);
@@ -923,8 +789,11 @@ static void launch_fix(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s)
 #undef LF
 }
 
-__global__ void k_prof_pairs(const dv_counters* __restrict__ C, double* acc) {
-  acc[0] += (double)C->n_targets * (double)C->num_samples;
+// pair evaluations of the far field: every target with every sample, or those
+// of the boxes
+__global__ void k_prof_pairs(const dv_counters* __restrict__ C, double* acc, dv_farbox B) {
+  acc[0] += farbox_on(B, C) ? (double)*reinterpret_cast<const unsigned long long*>(B.meta + 4)
+                            : (double)C->n_targets * (double)C->num_samples;
 }
 
 static int prof_fold(dv_ctx* c) {
@@ -964,6 +833,30 @@ DV_API int dv_profile_read(dv_ctx* c, double* far_ms, int64_t* launches, double*
   return DV_OK;
 }
 
+// Packs the samples for the direct loop and, in the split form, their
+// multiplicities and slots for the correction kernel; where the boxes may
+// carry the far field, their plan too.
+static int prepare_far(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s, bool split, bool boxed) {
+  const int packb = c->num_sms * 4;
+  if (c->p.dim == 2)
+    k_pack_samples<2><<<packb, DV_THREADS, 0, c->stream>>>(*f, *s, c->d_cnt, c->spos, c->sw, c->p.kden_eps);
+  else
+    k_pack_samples<3><<<packb, DV_THREADS, 0, c->stream>>>(*f, *s, c->d_cnt, c->spos, c->sw, c->p.kden_eps);
+  DV_LAUNCHED(c);
+  if (!split) return DV_OK;
+  const int64_t nu = std::min<int64_t>(c->n_upper, c->cap);
+  DV_CK(c, cudaMemsetAsync(c->mult, 0, sizeof(int32_t) * nu, c->stream));
+  k_mult<<<c->num_sms * 4, DV_THREADS, 0, c->stream>>>(s->sample_idx, c->d_cnt, c->mult);
+  DV_LAUNCHED(c);
+  int rc = sample_slots(c, f, s, boxed);
+  if (rc || !boxed) return rc;
+  return dv_farbox_plan(c);
+}
+
+__global__ void k_farbox_on(dv_farbox B, const dv_counters* __restrict__ C, int32_t* out) {
+  *out = farbox_on(B, C) ? 1 : 0;
+}
+
 // Times the far-field main loop for 2, 4, 6 and 8 targets per thread on the
 // current targets and samples (CUDA events, best of two launches after one
 // warm-up) and keeps the fastest for this context.
@@ -971,14 +864,30 @@ DV_API int dv_autotune(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s,
                        float* best_ms) {
   if (!c || !f || !s || !s->sample_idx) return DV_EINVAL;
   if (!fast_kernel_ok(c->p) && c->p.kernel_mode != DV_KERNEL_BLOB3D) return DV_OK;
-  int rc = dv_build_targets(c, f);
+  const bool boxed = dv_farbox_wanted(c);
+  int rc = boxed ? dv_farbox_begin(c) : DV_OK;
   if (rc) return rc;
-  const int packb = c->num_sms * 4;
-  if (c->p.dim == 2)
-    k_pack_samples<2><<<packb, DV_THREADS, 0, c->stream>>>(*f, *s, c->d_cnt, c->spos, c->sw, c->p.kden_eps);
-  else
-    k_pack_samples<3><<<packb, DV_THREADS, 0, c->stream>>>(*f, *s, c->d_cnt, c->spos, c->sw, c->p.kden_eps);
-  DV_LAUNCHED(c);
+  rc = dv_build_targets(c, f, boxed);
+  if (rc) return rc;
+  rc = prepare_far(c, f, s, boxed, boxed);
+  if (rc) return rc;
+  if (boxed) {
+    // the boxes carry this state's far field: the tile of the direct loop is
+    // not timed, but set to the shape that wins at such sizes
+    int32_t* on = c->d_flag + 1;
+    k_farbox_on<<<1, 1, 0, c->stream>>>(c->farbox, c->d_cnt, on);
+    DV_LAUNCHED(c);
+    DV_CK(c, cudaMemcpyAsync(c->h_flag, on, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
+    DV_CK(c, cudaStreamSynchronize(c->stream));
+    if (*c->h_flag) {
+      c->far_tt = 8;
+      c->far_chunks = DV_MAX_FAR_CHUNKS;
+      if (best_tt) *best_tt = c->far_tt;
+      if (best_ms) *best_ms = 0.0f;
+      return DV_OK;
+    }
+  }
+  const dv_farbox none{};
   cudaEvent_t e0, e1;
   DV_CK(c, cudaEventCreate(&e0));
   DV_CK(c, cudaEventCreate(&e1));
@@ -991,9 +900,9 @@ DV_API int dv_autotune(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s,
       for (int rep = 0; rep < 3; ++rep) {
         DV_CK(c, cudaEventRecord(e0, c->stream));
         if (c->p.dim == 2)
-          launch_main<2>(c, f, tt);
+          launch_main<2>(c, f, tt, none);
         else
-          launch_main<3>(c, f, tt);
+          launch_main<3>(c, f, tt, none);
         DV_LAUNCHED(c);
         DV_CK(c, cudaEventRecord(e1, c->stream));
         DV_CK(c, cudaEventSynchronize(e1));
@@ -1033,29 +942,20 @@ DV_API int32_t dv_get_far_chunks(dv_ctx* c) { return c ? c->far_chunks : DV_EINV
 DV_API int dv_vvpe_mc(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s) {
   if (!c || !f || !s || !s->sample_idx || !s->kden || !s->d_vort_smoothed)
     return c ? dv_fail(c, DV_EINVAL, "dv_vvpe_mc: NULL field") : DV_EINVAL;
-  int rc = dv_build_targets(c, f);
+  const bool fastk = fast_kernel_ok(c->p) || c->p.kernel_mode == DV_KERNEL_BLOB3D;
+  const bool boxed = fastk && dv_farbox_wanted(c);
+  int rc = boxed ? dv_farbox_begin(c) : DV_OK;
+  if (rc) return rc;
+  rc = dv_build_targets(c, f, boxed);
   if (rc) return rc;
   rc = dv_launch_vvpe_near(c, f, s);
   if (rc) return rc;
-  const int packb = c->num_sms * 4;
-  if (c->p.dim == 2)
-    k_pack_samples<2><<<packb, DV_THREADS, 0, c->stream>>>(*f, *s, c->d_cnt, c->spos, c->sw,
-                                                          c->p.kden_eps);
-  else
-    k_pack_samples<3><<<packb, DV_THREADS, 0, c->stream>>>(*f, *s, c->d_cnt, c->spos, c->sw,
-                                                          c->p.kden_eps);
-  DV_LAUNCHED(c);
   const int64_t nu = std::min<int64_t>(c->n_upper, c->cap);
-  const bool fastk = fast_kernel_ok(c->p) || c->p.kernel_mode == DV_KERNEL_BLOB3D;
   if (!fastk && c->p.periodic)
     return dv_fail(c, DV_EUNSUPPORTED, "dv_vvpe_mc: periodic boxes need h > 1.05e-4 (reference kernel)");
-  if (fastk) {  // split form: sample multiplicities for the correction kernel
-    DV_CK(c, cudaMemsetAsync(c->mult, 0, sizeof(int32_t) * nu, c->stream));
-    k_mult<<<c->num_sms * 4, DV_THREADS, 0, c->stream>>>(s->sample_idx, c->d_cnt, c->mult);
-    DV_LAUNCHED(c);
-    rc = sample_slots(c);
-    if (rc) return rc;
-  }
+  rc = prepare_far(c, f, s, fastk, boxed);
+  if (rc) return rc;
+  const dv_farbox B = boxed ? c->farbox : dv_farbox{};
   if (c->prof) {
     if (c->prof_used == dv_ctx::kProfPool) {
       int rc2 = prof_fold(c);
@@ -1064,10 +964,14 @@ DV_API int dv_vvpe_mc(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s) 
     DV_CK(c, cudaEventRecord(c->prof_ev[2 * c->prof_used], c->stream));
   }
   if (fastk) {
+    if (boxed) {
+      rc = dv_farbox_run(c, f);
+      if (rc) return rc;
+    }
     if (c->p.dim == 2)
-      launch_main<2>(c, f, c->far_tt);
+      launch_main<2>(c, f, c->far_tt, B);
     else
-      launch_main<3>(c, f, c->far_tt);
+      launch_main<3>(c, f, c->far_tt, B);
   } else {  // |r| > h may not underflow exp(-|r|/ε): per-pair exact kernel
     const int nb = (int)std::max<int64_t>(1, (nu + FT * 2 - 1) / (FT * 2));
     if (c->p.dim == 2)
@@ -1081,15 +985,15 @@ DV_API int dv_vvpe_mc(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s) 
   }
   if (fastk) {
     if (c->p.dim == 2)
-      launch_fix<2>(c, f, s);
+      launch_fix<2>(c, f, s, B);
     else
-      launch_fix<3>(c, f, s);
+      launch_fix<3>(c, f, s, B);
     DV_LAUNCHED(c);
   }
   if (c->prof) {
     c->prof_used++;
     c->prof_launches++;
-    k_prof_pairs<<<1, 1, 0, c->stream>>>(c->d_cnt, c->d_prof);
+    k_prof_pairs<<<1, 1, 0, c->stream>>>(c->d_cnt, c->d_prof, B);
     DV_LAUNCHED(c);
   }
   return DV_OK;
@@ -1153,7 +1057,7 @@ int dv_batch_vvpe(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s) {
   DV_CK(c, cudaMemsetAsync(c->mult, 0, sizeof(int32_t) * c->cap, c->stream));
   k_mult<<<c->num_sms * 4, DV_THREADS, 0, c->stream>>>(s->sample_idx, c->d_cnt, c->mult);
   DV_LAUNCHED(c);
-  rc = sample_slots(c);
+  rc = sample_slots(c, f, s);
   if (rc) return rc;
   const bool blob = c->p.kernel_mode == DV_KERNEL_BLOB3D, comp = c->p.compensated != 0;
 #define LB(DD)                                                                             \

@@ -384,12 +384,18 @@ DV_API int dv_smooth_akde(dv_ctx* ctx, const dv_fields* f, const dv_solver_field
 DV_API int dv_sample(dv_ctx* ctx, const dv_fields* f, const dv_solver_fields* s, int32_t mode,
                      uint64_t seed, uint64_t step, int32_t M);
 /* vort2vel (dimcv_sph.py:649-719): near-field neighbour sum, Monte-Carlo
- * far field over sample_idx[0:num_samples], the ‖v_vort‖ < ‖v‖ gate. */
+ * far field over sample_idx[0:num_samples], the ‖v_vort‖ < ‖v‖ gate.  In 3-D,
+ * uncompensated, non-periodic and from 65,536 particles on, the far field of
+ * targets and samples that lie in the boxes of the last grid build is
+ * interpolated on those boxes where that takes fewer pair evaluations (chosen
+ * on the device; same accuracy); every other call sums all pairs. */
 DV_API int dv_vvpe_mc(dv_ctx* ctx, const dv_fields* f, const dv_solver_fields* s);
 /* New (tuning): times the far-field main loop of dv_vvpe_mc for 2, 4, 6 and 8
  * targets per thread (6 runs as 8 where the loop is not the paired one) and
  * 1-8 sample chunks on the current targets / samples and keeps the fastest
- * for this context (synchronises; *best_tt / *best_ms may be NULL).
+ * for this context (synchronises; *best_tt / *best_ms may be NULL).  Where
+ * boxes carry the far field the loop does not run: tile 8 and 8 chunks are
+ * kept without timing (*best_ms = 0).
  * dv_set_far_tile sets the tile directly (2, 4, 6 or 8). */
 DV_API int dv_autotune(dv_ctx* ctx, const dv_fields* f, const dv_solver_fields* s, int32_t* best_tt,
                        float* best_ms);
@@ -406,10 +412,10 @@ DV_API int dv_vis(dv_ctx* ctx, const dv_fields* f, const dv_solver_fields* s);
 DV_API int dv_bs_full(dv_ctx* ctx, const dv_fields* f, const float* omega, const int32_t* targets,
                       int32_t nt, void* out, int32_t precision);
 
-/* Kernel timing of the Monte-Carlo far-field kernel (the FP32-bound hot
- * loop of dv_vvpe_mc): when enabled, CUDA events bracket every far-field
- * launch on the context stream and a device counter accumulates the pair
- * count n_targets × num_samples.  dv_profile resets; dv_profile_read
+/* Kernel timing of the Monte-Carlo far field (the FP32-bound hot part of
+ * dv_vvpe_mc): when enabled, CUDA events bracket its launches on the context
+ * stream and a device counter accumulates the pair evaluations: n_targets ×
+ * num_samples, or fewer where boxes carry the far field (3-D, large calls).  dv_profile resets; dv_profile_read
  * synchronises and returns the totals since the reset. */
 DV_API int dv_profile(dv_ctx* ctx, int32_t enable);
 DV_API int dv_profile_read(dv_ctx* ctx, double* far_ms, int64_t* launches, double* pairs);
