@@ -117,7 +117,8 @@ DV_API void dv_destroy(dv_ctx* c) {
                   c->scan_part, c->dscan_part, c->red_part, c->ired_part, c->flags, c->offs,
                   c->targets, c->cdf,       c->spos,      c->sw,        c->near_v,  c->near_S,
                   c->far_acc, c->mult,      c->nbr_off,   c->nbr_idx,   c->d_nbr_ok,
-                  c->nbr_rows, c->sflag,   c->srank,     c->sslot};
+                  c->nbr_rows, c->sflag,   c->srank,     c->sslot,   c->nbr_len,   c->pk_a,    c->pk_b,
+                  c->pk_k};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (int k = 0; k < 2 * dv_ctx::kProfPool; ++k)
@@ -202,10 +203,16 @@ DV_API dv_ctx* dv_create(const dv_params* params, int64_t capacity, void* stream
   A(c->sflag, cap + 1);
   A(c->srank, cap + 1);
   A(c->sslot, cap);
-  // neighbour lists: 48 (3-D) / 24 (2-D) entries per particle on average,
-  // beyond which the sweeps keep scanning cells
-  c->nbr_cap = cap * (params->dim == 3 ? 48 : 24);
+  // neighbour lists: 48 (3-D, and 3 of padding) / 24 (2-D) entries per
+  // particle on average, beyond which the sweeps keep scanning cells
+  c->nbr_cap = cap * (params->dim == 3 ? 51 : 24);
   A(c->nbr_off, cap + 1);
+  if (params->dim == 3) {
+    A(c->nbr_len, cap);
+    A(c->pk_a, cap);
+    A(c->pk_b, cap);
+    A(c->pk_k, cap);
+  }
   A(c->nbr_idx, c->nbr_cap);
   A(c->d_nbr_ok, 3);  // [0]: lists valid, [1]: keys valid, [2]: a material other than fluid / solid seen by the build
   // the 3-D build's first pass stores up to 64 neighbours per particle in

@@ -89,8 +89,9 @@ __global__ void k_d_vorticity(dv_params P, DevGrid G, dv_fields F, dv_solver_fie
 // stores v*_j with, so every sum (ω, ∇v, ∇×v*) and Δω are bit-identical to
 // the two separate sweeps, without re-reading the list, positions and
 // materials or storing and gathering v*.
+// 3-D: K.a = (x, m_V).
 template <int D>
-__global__ void k_vorticity_dvort(dv_params P, DevGrid G, dv_fields F, dv_solver_fields S,
+__global__ void k_vorticity_dvort(dv_params P, DevGrid G, dv_fields F, dv_solver_fields S, DevPack K,
                                   const dv_counters* __restrict__ C) {
   FOR_I;
   const int DD = D * D;
@@ -109,13 +110,13 @@ __global__ void k_vorticity_dvort(dv_params P, DevGrid G, dv_fields F, dv_solver
   V3 w{0.f, 0.f, 0.f};
   V3 curl{0.f, 0.f, 0.f};
   float g[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  for_each_neighbor_m<D>(P, G, F.x, F.material, i, xi, [&](int j, V3 r, float r2, int mj) {
+  for_each_neighbor_p<D>(P, G, F.x, K.a, F.material, i, xi, [&](int j, V3 r, float r2, int mj, float pw) {
     if (mj != DV_MATERIAL_FLUID) return;
     V3 vj = ldv<D>(F.v, j);
     V3 aj = ldv<D>(F.acceleration, j);
     V3 vsj{vj.x + aj.x * P.dt, vj.y + aj.y * P.dt, D == 3 ? vj.z + aj.z * P.dt : 0.0f};
     V3 gw = cubic_gradW<D>(P, r, r2);
-    float mv = F.m_V[j];
+    float mv = D == 3 ? pw : F.m_V[j];
     V3 c = cross3(sub3(vj, vi), gw);
     w.x += mv * c.x;
     w.y += mv * c.y;
@@ -314,8 +315,9 @@ __global__ void k_akde(dv_params P, DevGrid G, dv_fields F, dv_solver_fields S,
 // the FP64 block partials of kden_sum come out bit-identical to the two
 // separate sweeps.  KVN must be current (k_kvn_sample first); the smoothing
 // does not read it.
+// 3-D: K.a = (x, m_V), K.b = (Δω, KVN).
 template <int D>
-__global__ void k_smooth_akde(dv_params P, DevGrid G, dv_fields F, dv_solver_fields S,
+__global__ void k_smooth_akde(dv_params P, DevGrid G, dv_fields F, dv_solver_fields S, DevPack K,
                               const dv_counters* __restrict__ C, double* __restrict__ part) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   double contrib = 0.0;
@@ -327,15 +329,24 @@ __global__ void k_smooth_akde(dv_params P, DevGrid G, dv_fields F, dv_solver_fie
       float w0 = cubic_W(P, 0.0f);
       V3 acc{mvi * di.x * w0, mvi * di.y * w0, mvi * di.z * w0};
       float kd = S.kvn[i] * epan<D>(P, V3{0.f, 0.f, 0.f});
-      for_each_neighbor_m<D>(P, G, F.x, F.material, i, xi, [&](int j, V3 r, float r2, int mj) {
+      for_each_neighbor_p<D>(P, G, F.x, K.a, F.material, i, xi, [&](int j, V3 r, float r2, int mj, float pw) {
         if (mj != DV_MATERIAL_FLUID) return;
-        float mv = F.m_V[j];
-        V3 dj = ld4(S.d_vort, j);
+        float mv = pw, kj;
+        V3 dj;
+        if (D == 3) {
+          const float4 q = __ldg(K.b + j);
+          dj = V3{q.x, q.y, q.z};
+          kj = q.w;
+        } else {
+          mv = F.m_V[j];
+          dj = ld4(S.d_vort, j);
+          kj = S.kvn[j];
+        }
         float wk = cubic_W(P, sqrtf(r2));
         acc.x += mv * dj.x * wk;
         acc.y += mv * dj.y * wk;
         acc.z += mv * dj.z * wk;
-        kd += S.kvn[j] * epan<D>(P, r);
+        kd += kj * epan<D>(P, r);
       });
       st4(S.d_vort_smoothed, i, acc);
       S.kden[i] = kd;
@@ -468,8 +479,9 @@ int dv_batch_draw(dv_ctx* c, const dv_solver_fields* s) {
 // vort2vel_neighbors_2d_task (dimcv_sph.py:649-658) for each target:
 // near_v = 0.1592 V Σ_fluid Kε(|r_xy|) (r_xy × ω̃_j) and
 // S_i = kden_i + Σ_fluid kden_j.  DV_KERNEL_BLOB3D uses the blob kernel.
+// 3-D: K.b = (ω̃, kden).
 template <int D>
-__global__ void k_vvpe_near(dv_params P, DevGrid G, dv_fields F, dv_solver_fields S,
+__global__ void k_vvpe_near(dv_params P, DevGrid G, dv_fields F, dv_solver_fields S, DevPack K,
                             const dv_counters* __restrict__ C, const int32_t* __restrict__ targets,
                             float4* __restrict__ near_v, float* __restrict__ near_S) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -481,7 +493,16 @@ __global__ void k_vvpe_near(dv_params P, DevGrid G, dv_fields F, dv_solver_field
   const bool blob = P.kernel_mode == DV_KERNEL_BLOB3D;
   for_each_neighbor_m<D>(P, G, F.x, F.material, i, xi, [&](int j, V3 r, float r2, int mj) {
     if (mj != DV_MATERIAL_FLUID) return;
-    V3 w = ld4(S.d_vort_smoothed, j);
+    V3 w;
+    float kj;
+    if (D == 3) {
+      const float4 q = __ldg(K.b + j);
+      w = V3{q.x, q.y, q.z};
+      kj = q.w;
+    } else {
+      w = ld4(S.d_vort_smoothed, j);
+      kj = S.kden[j];
+    }
     if (!blob) {
       V3 rp{r.x, r.y, 0.0f};
       float rn = sqrtf(__fadd_rn(__fadd_rn(__fmul_rn(rp.x, rp.x), __fmul_rn(rp.y, rp.y)), 0.0f * 0.0f));
@@ -499,7 +520,7 @@ __global__ void k_vvpe_near(dv_params P, DevGrid G, dv_fields F, dv_solver_field
       acc.y += inv * c.y;
       acc.z += inv * c.z;
     }
-    Ssum += S.kden[j];
+    Ssum += kj;
   });
   float coef = blob ? P.blob_coef : P.vvpe_coef;
   near_v[t] = make_float4(acc.x * coef, acc.y * coef, acc.z * coef, 0.0f);
@@ -508,11 +529,12 @@ __global__ void k_vvpe_near(dv_params P, DevGrid G, dv_fields F, dv_solver_field
 
 int dv_launch_vvpe_near(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s) {
   const int nb = dv_blocks(std::min<int64_t>(c->n_upper, c->cap));
+  if (int rc = dv_pack(c, f, s, DV_PK_SW)) return rc;
   if (c->p.dim == 2)
-    k_vvpe_near<2><<<nb, DV_THREADS, 0, c->stream>>>(c->p, dv_grid(c), *f, *s, c->d_cnt, c->targets,
+    k_vvpe_near<2><<<nb, DV_THREADS, 0, c->stream>>>(c->p, dv_grid(c), *f, *s, dv_packs(c), c->d_cnt, c->targets,
                                                      c->near_v, c->near_S);
   else
-    k_vvpe_near<3><<<nb, DV_THREADS, 0, c->stream>>>(c->p, dv_grid(c), *f, *s, c->d_cnt, c->targets,
+    k_vvpe_near<3><<<nb, DV_THREADS, 0, c->stream>>>(c->p, dv_grid(c), *f, *s, dv_packs(c), c->d_cnt, c->targets,
                                                      c->near_v, c->near_S);
   DV_LAUNCHED(c);
   return DV_OK;
@@ -584,7 +606,8 @@ DV_API int dv_dimcv_vorticity(dv_ctx* c, const dv_fields* f, const dv_solver_fie
 DV_API int dv_vorticity_dvort(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s) {
   if (!c || !f) return DV_EINVAL;
   if (int rc = check_solver(c, s)) return rc;
-  LAUNCH_D(k_vorticity_dvort, nblk(c), c->p, dv_grid(c), *f, *s, c->d_cnt);
+  if (int rc = dv_pack(c, f, s, DV_PK_XV)) return rc;
+  LAUNCH_D(k_vorticity_dvort, nblk(c), c->p, dv_grid(c), *f, *s, dv_packs(c), c->d_cnt);
   return DV_OK;
 }
 
@@ -642,7 +665,8 @@ DV_API int dv_smooth_akde(dv_ctx* c, const dv_fields* f, const dv_solver_fields*
   if (!c || !f) return DV_EINVAL;
   if (int rc = check_solver(c, s)) return rc;
   const int nb = nblk(c);
-  LAUNCH_D(k_smooth_akde, nb, c->p, dv_grid(c), *f, *s, c->d_cnt, c->red_part);
+  if (int rc = dv_pack(c, f, s, DV_PK_XV | DV_PK_DW)) return rc;
+  LAUNCH_D(k_smooth_akde, nb, c->p, dv_grid(c), *f, *s, dv_packs(c), c->d_cnt, c->red_part);
   k_akde_finalize<<<1, 1024, 0, c->stream>>>(c->red_part, nb, c->d_cnt);
   DV_LAUNCHED(c);
   return DV_OK;

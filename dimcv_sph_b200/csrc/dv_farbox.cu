@@ -89,7 +89,7 @@ struct Sets {
   static constexpr int K = Cheb<deg<BLOB>(0)>::K;
   // floats of the node sums of one box, for stripe_mul 1
   static constexpr int FLOATS = 3 * (stripes(0) * P0 + stripes(1) * P1 + stripes(2) * P2 + stripes(3) * P3);
-  static constexpr int WARPS = BLOB ? 8 : 6;  // of a node block: class 0 fills 7 (BLOB) or 6 with 4 nodes a thread
+  static constexpr int WARPS = BLOB ? 8 : 6;  // of a node block: two groups of 3 for class 0, blob: one of 7
 };
 constexpr int kCoefMax = Sets<true>::K;
 constexpr int kFloatsMax = Sets<true>::FLOATS;

@@ -282,8 +282,9 @@ __global__ void k_finalize_counts(const int32_t* __restrict__ part, int nparts,
 //
 // 3-D (27 cells, ~8 candidates each): one cell-scan pass stores each
 // particle's first `slots` neighbours in its own fixed row and its count; a
-// warp-wide copy then moves the rows into CSR (a particle with more
-// neighbours than slots scans its cells again there).  This saves a second
+// copy then moves the rows into CSR (a particle with more neighbours than
+// slots scans its cells again there).  CSR rows start and end on 16 bytes, so
+// that the sweeps read four entries a load.  This saves a second
 // 27-cell scan.  2-D (9 cells): counting is cheap and the fixed rows cost
 // more write traffic than they save, so a count pass and a fill pass.
 __device__ __forceinline__ bool nbr_row_built(const int32_t* __restrict__ mat, const uint8_t* __restrict__ dyn,
@@ -323,7 +324,7 @@ __global__ void k_csr_fill(dv_params P, DevGrid G, const float* __restrict__ x,
 template <int D>
 __global__ void k_csr_rows(dv_params P, DevGrid G, const float* __restrict__ x, const int32_t* __restrict__ mat,
                            const uint8_t* __restrict__ dyn, const dv_counters* __restrict__ C, int m, int slots,
-                           uint32_t* __restrict__ cnt, int32_t* __restrict__ rows) {
+                           uint32_t* __restrict__ room, uint32_t* __restrict__ len, int32_t* __restrict__ rows) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
   uint32_t k = 0;
@@ -334,35 +335,46 @@ __global__ void k_csr_rows(dv_params P, DevGrid G, const float* __restrict__ x, 
       ++k;
     });
   }
-  cnt[i] = k;
+  room[i] = (k + 3u) & ~3u;  // rows start on 16 bytes
+  if (i < m - 1) len[i] = k;
 }
 
-// one warp per group of 32 particles; each row is copied by the whole warp
-// (coalesced reads of the row, coalesced writes of the CSR segment), and the
-// neighbours' materials are gathered here, 32 independent loads at a time,
-// rather than in the row scan's dependent chain
+// one warp per group of 32 particles; eight lanes copy a row, four entries a
+// lane (16-byte loads of the row and stores of the CSR segment: four rows of
+// up to 32 entries at a time), and the neighbours' materials are gathered
+// here, independent loads, rather than in the row scan's dependent chain.
+// 0.75M particles: 77 -> 56 us against a row per warp and 4-byte copies.
 template <int D>
 __global__ void k_csr_compact(dv_params P, DevGrid G, const float* __restrict__ x, const int32_t* __restrict__ mat,
                               const dv_counters* __restrict__ C, int slots, const int32_t* __restrict__ rows,
-                              const uint32_t* __restrict__ off, int32_t* __restrict__ ok,
-                              int32_t* __restrict__ out) {
+                              const uint32_t* __restrict__ off, const uint32_t* __restrict__ len,
+                              int32_t* __restrict__ ok, int32_t* __restrict__ out) {
   if (!ok[0]) return;
   const int n = C->n;
   const int lane = threadIdx.x & 31;
   const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31;
-  const int iend = min(i0 + 32, n);
-  for (int i = i0; i < iend; ++i) {
-    const uint32_t k0 = off[i], cnt = off[i + 1] - k0;
+  const uint32_t l4 = 4u * (lane & 7);
+#pragma unroll 2
+  for (int g = 0; g < 32; g += 4) {
+    const int i = i0 + g + (lane >> 3);
+    if (i >= n) break;
+    const uint32_t k0 = off[i], cnt = len[i];
     if (cnt <= (uint32_t)slots) {
-      const int32_t* row = rows + (int64_t)i * slots;
-      for (uint32_t k = lane; k < cnt; k += 32) {
-        const int j = row[k];
-        out[k0 + k] = nbr_entry(j, __ldg(mat + j), ok + 2);
+      const int4* row = reinterpret_cast<const int4*>(rows + (int64_t)i * slots);
+      for (uint32_t k = l4; k < cnt; k += 32) {
+        const int4 q = row[k >> 2];
+        int4 e;  // past the row's end: padding with a valid slot
+        e.x = nbr_entry(q.x, __ldg(mat + q.x), ok + 2);
+        e.y = k + 1 < cnt ? nbr_entry(q.y, __ldg(mat + q.y), ok + 2) : i;
+        e.z = k + 2 < cnt ? nbr_entry(q.z, __ldg(mat + q.z), ok + 2) : i;
+        e.w = k + 3 < cnt ? nbr_entry(q.w, __ldg(mat + q.w), ok + 2) : i;
+        *reinterpret_cast<int4*>(out + k0 + k) = e;
       }
-    } else if (lane == (i & 31)) {
+    } else if ((lane & 7) == 0) {
       uint32_t k = k0;
       for_each_neighbor_m<D>(P, G, x, mat, i, ldv<D>(x, i),
                              [&](int j, V3, float, int mj) { out[k++] = nbr_entry(j, mj, ok + 2); });
+      while (k & 3u) out[k++] = i;
     }
   }
 }
@@ -387,7 +399,7 @@ static int build_csr(dv_ctx* c, const dv_fields* f) {
   DV_CK(c, cudaMemsetAsync(c->d_nbr_ok + 2, 0, sizeof(int32_t), c->stream));
   if (rows)
     k_csr_rows<3><<<nb, DV_THREADS, 0, c->stream>>>(c->p, G, f->x, f->material, f->is_dynamic, c->d_cnt, m,
-                                                    c->nbr_slots, c->flags, c->nbr_rows);
+                                                    c->nbr_slots, c->flags, c->nbr_len, c->nbr_rows);
   else
     k_csr_count<2><<<nb, DV_THREADS, 0, c->stream>>>(c->p, G, f->x, f->material, f->is_dynamic, c->d_cnt, m,
                                                      c->flags);
@@ -398,7 +410,7 @@ static int build_csr(dv_ctx* c, const dv_fields* f) {
   DV_LAUNCHED(c);
   if (rows)
     k_csr_compact<3><<<nb, DV_THREADS, 0, c->stream>>>(c->p, G, f->x, f->material, c->d_cnt, c->nbr_slots,
-                                                       c->nbr_rows, c->nbr_off, c->d_nbr_ok, c->nbr_idx);
+                                                       c->nbr_rows, c->nbr_off, c->nbr_len, c->d_nbr_ok, c->nbr_idx);
   else
     k_csr_fill<2><<<nb, DV_THREADS, 0, c->stream>>>(c->p, G, f->x, f->material, c->d_cnt, c->nbr_off,
                                                     c->d_nbr_ok, c->nbr_idx, f->is_dynamic);
@@ -591,9 +603,14 @@ __global__ void k_u32_to_i64(const uint32_t* __restrict__ a, int64_t* __restrict
   if (i < m) b[i] = a[i];
 }
 
-__global__ void k_nbr_slots(const int32_t* __restrict__ in, int64_t m, int32_t* __restrict__ out) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < m) out[k] = nbr_slot((uint32_t)in[k]);
+// the slots of row i, without the material bit and the padding
+__global__ void k_nbr_slots(const uint32_t* __restrict__ off, const uint32_t* __restrict__ len,
+                            const int32_t* __restrict__ in, int n, const uint32_t* __restrict__ out_off,
+                            int32_t* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t a = off[i], m = len ? len[i] : off[i + 1] - a, o = out_off[i];
+  for (uint32_t k = 0; k < m; ++k) out[o + k] = nbr_slot((uint32_t)in[a + k]);
 }
 
 DV_API int64_t dv_stored_lists(dv_ctx* c, uint32_t* dev_offsets, int32_t* dev_nbrs, int64_t max_entries) {
@@ -604,20 +621,30 @@ DV_API int64_t dv_stored_lists(dv_ctx* c, uint32_t* dev_offsets, int32_t* dev_nb
   int32_t ok = 0;
   uint32_t total32 = 0;
   const int n = cnt.n;
+  // offsets without the padding of the 3-D rows
+  const uint32_t* off = c->nbr_off;
+  if (c->nbr_len) {
+    DV_CK(c, cudaMemsetAsync(c->flags + n, 0, sizeof(uint32_t), c->stream));
+    if (n > 0)
+      DV_CK(c, cudaMemcpyAsync(c->flags, c->nbr_len, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, c->stream));
+    rc = dv_scan_u32(c, c->flags, c->offs, (int64_t)n + 1);
+    if (rc) return rc;
+    off = c->offs;
+  }
   DV_CK(c, cudaMemcpyAsync(&ok, c->d_nbr_ok, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-  DV_CK(c, cudaMemcpyAsync(&total32, c->nbr_off + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
+  DV_CK(c, cudaMemcpyAsync(&total32, off + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
   DV_CK(c, cudaStreamSynchronize(c->stream));
   if (!ok) return dv_fail(c, DV_EINVAL, "dv_stored_lists: no valid lists (positions changed since the grid build)");
   const int64_t total = total32;
   if (dev_offsets)
-    DV_CK(c, cudaMemcpyAsync(dev_offsets, c->nbr_off, sizeof(uint32_t) * ((size_t)n + 1), cudaMemcpyDeviceToDevice,
+    DV_CK(c, cudaMemcpyAsync(dev_offsets, off, sizeof(uint32_t) * ((size_t)n + 1), cudaMemcpyDeviceToDevice,
                              c->stream));
   if (dev_nbrs) {
     if (total > max_entries)
       return dv_fail(c, DV_ECAPACITY, "dv_stored_lists: %lld entries > max_entries %lld", (long long)total,
                      (long long)max_entries);
-    if (total > 0) {  // the slots, without the material bit
-      k_nbr_slots<<<dv_blocks(total), DV_THREADS, 0, c->stream>>>(c->nbr_idx, total, dev_nbrs);
+    if (total > 0) {
+      k_nbr_slots<<<dv_blocks(n), DV_THREADS, 0, c->stream>>>(c->nbr_off, c->nbr_len, c->nbr_idx, n, off, dev_nbrs);
       DV_LAUNCHED(c);
     }
   }

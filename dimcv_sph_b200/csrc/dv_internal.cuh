@@ -76,6 +76,12 @@ struct dv_ctx {
   int32_t* ired_part = nullptr;   // int per-block partials
   int64_t red_cap = 0;
 
+  // 3-D: per-sweep copies of the fields a neighbour walk gathers, packed so
+  // that a neighbour costs one or two 16-byte loads (dv_pack)
+  float4* pk_a = nullptr;  // cap: (x, m_V)
+  float4* pk_b = nullptr;  // cap: (v, m), (Δω, KVN) or (smoothed Δω, kden)
+  float2* pk_k = nullptr;  // cap: (k, m) of the Jacobi solves
+
   // DIMCV scratch
   uint32_t* flags = nullptr;   // cap+1
   uint32_t* offs = nullptr;    // cap+1
@@ -94,8 +100,11 @@ struct dv_ctx {
   int far_chunks = 1;          // sample chunks of the far-field grid (autotuned, <= DV_MAX_FAR_CHUNKS)
   bool dyn_rigid = false;      // dynamic rigid particles present: pressure iterations add their reaction
 
-  // per-step neighbour lists (CSR, visit order) built by dv_grid_build
+  // per-step neighbour lists (CSR, visit order) built by dv_grid_build; in 3-D
+  // every row starts at a multiple of 4 entries (16 bytes), is padded to one
+  // with entries of its own slot, and has its length in nbr_len
   uint32_t* nbr_off = nullptr;  // cap + 1
+  uint32_t* nbr_len = nullptr;  // 3-D: cap
   int32_t* nbr_idx = nullptr;   // nbr_cap
   int64_t nbr_cap = 0;
   int32_t* d_nbr_ok = nullptr;  // [0]: 1 while the lists match the current positions; [1]: 1 while keys[perm_buf]
@@ -153,6 +162,7 @@ struct DevGrid {
   // neighbour lists of the last grid build (CSR in visit order); used while
   // *nok != 0, i.e. until positions move or particles are added
   const uint32_t* noff;
+  const uint32_t* nlen;  // 3-D: row lengths (rows are padded to 16 bytes)
   const int32_t* nidx;
   const int32_t* nok;
   // scene batch: the cell key of slot i is (scene[i] << scene_shift) | Morton
@@ -160,12 +170,19 @@ struct DevGrid {
   int scene_shift;
 };
 static inline DevGrid dv_grid(const dv_ctx* c) {
-  return DevGrid{c->cell_start, c->cell_end, c->mt[0], c->mt[1], c->mt[2], c->nbr_off, c->nbr_idx,
+  return DevGrid{c->cell_start, c->cell_end, c->mt[0], c->mt[1], c->mt[2], c->nbr_off, c->nbr_len, c->nbr_idx,
                  c->d_nbr_ok, c->scene_ptr, c->scene_shift};
 }
+// the packed copies, as kernel arguments
+struct DevPack {
+  const float4* a;
+  float4* b;
+  float2* k;
+};
+static inline DevPack dv_packs(const dv_ctx* c) { return DevPack{c->pk_a, c->pk_b, c->pk_k}; }
 // the cell-scan form only (used to build the neighbour lists)
 static inline DevGrid dv_grid_cells(const dv_ctx* c) {
-  return DevGrid{c->cell_start, c->cell_end, c->mt[0], c->mt[1], c->mt[2], nullptr, nullptr, nullptr,
+  return DevGrid{c->cell_start, c->cell_end, c->mt[0], c->mt[1], c->mt[2], nullptr, nullptr, nullptr, nullptr,
                  c->scene_ptr, c->scene_shift};
 }
 
@@ -194,6 +211,17 @@ struct dv_batch_state {
   cudaStream_t bstream = nullptr;     // captures the Jacobi loop bodies
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 };
+// dv_sph.cu: fills the packed copies a 3-D walk gathers from (no-op in 2-D);
+// what: OR of DV_PK_*
+enum {
+  DV_PK_XV = 1,    // pk_a = (x, m_V)
+  DV_PK_VM = 2,    // pk_b = (v, m)
+  DV_PK_DIV = 4,   // pk_k = (density_adv · factor · density, m) (divergence solve)
+  DV_PK_P = 8,     // pk_k = ((density_adv - density0) · factor, m) (pressure solve)
+  DV_PK_DW = 16,   // pk_b = (d_vort, kvn)
+  DV_PK_SW = 32    // pk_b = (d_vort_smoothed, kden)
+};
+int dv_pack(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s, int what);
 // dv_batch.cu
 void dv_batch_free(dv_ctx* c);
 int dv_batch_solve_reset(dv_ctx* c, int which);
@@ -400,38 +428,87 @@ __device__ __forceinline__ float transit_weight(const dv_params& P, float x0) {
 __device__ __forceinline__ int nbr_slot(uint32_t e) { return (int)(e & DV_NBR_SLOT); }
 __device__ __forceinline__ int nbr_mat(uint32_t e) { return (e & DV_NBR_SOLID) ? DV_MATERIAL_SOLID : DV_MATERIAL_FLUID; }
 
-template <int D, bool MAT, typename F>
+// Packed walks (3-D): pk[j] = (x_j, w_j) replaces the position gather and
+// brings one more field along; f also gets w_j.  Each gather of 32 scattered
+// lanes costs the L1 data pipe about six passes whatever its width, and that
+// pipe was 70% busy with the five gathers of a density sweep, so fields are
+// packed before the sweep (dv_pack).  0.75M particles, before -> with the packed
+// copies and the four-entry list loads: densities + factor + change 146 -> 95
+// us, divergence iteration 147 -> 102, residual + forces 135 -> 124,
+// vorticity + Δω 171 -> 140, smoothing + AKDE 142 -> 92; a packing pass takes
+// 5 to 9.  2-D walks ignore pk and pass w = 0: their scenes are small, and
+// one more launch costs what the gathers would save.
+template <int D, bool PK>
+__device__ __forceinline__ float4 ld_pos(const float* __restrict__ x, const float4* __restrict__ pk, int j) {
+  if (PK && D == 3) return __ldg(pk + j);
+  const V3 t = ldv<D>(x, j);
+  return make_float4(t.x, t.y, t.z, 0.0f);
+}
+
+template <int D, bool MAT, bool PK, typename F>
 __device__ __forceinline__ void for_each_neighbor_impl(const dv_params& P, const DevGrid& G,
                                                        const float* __restrict__ x,
+                                                       const float4* __restrict__ pk,
                                                        const int32_t* __restrict__ mat, int i, V3 xi, F&& f) {
+  auto call = [&](uint32_t e, float4 p) {
+    const V3 r = rel<D>(P, xi, V3{p.x, p.y, p.z});
+    if constexpr (PK)
+      f(nbr_slot(e), r, sqnorm<D>(r), nbr_mat(e), p.w);
+    else if constexpr (MAT)
+      f(nbr_slot(e), r, sqnorm<D>(r), nbr_mat(e));
+    else
+      f(nbr_slot(e), r, sqnorm<D>(r));
+  };
   if (G.nok && __ldg(G.nok)) {  // the lists hold exactly these j, in this order
-    uint32_t k = __ldg(G.noff + i);
-    const uint32_t k1 = __ldg(G.noff + i + 1);
-    if (k >= k1) return;
-    // one-deep software pipeline: the next neighbour's entry and position
-    // are loaded before f runs on the current one (f still runs in list
-    // order).  Sweeps -5% at 2.37M particles; a two-deep pipeline was slower.
-    const uint32_t* __restrict__ nl = reinterpret_cast<const uint32_t*>(G.nidx);
-    uint32_t e = __ldg(nl + k);
-    int j = nbr_slot(e);
-    V3 xj = ldv<D>(x, j);
-    int mj = nbr_mat(e);
+    const uint32_t k0 = __ldg(G.noff + i);
+    const uint32_t* __restrict__ nl = reinterpret_cast<const uint32_t*>(G.nidx) + k0;
+    if constexpr (D == 3) {
+      // four entries a load; the next entry's position is loaded before f
+      // runs on the current one (a two-deep pipeline was slower)
+      const int len = (int)__ldg(G.nlen + i);
+      if (len == 0) return;
+      const uint4* __restrict__ n4 = reinterpret_cast<const uint4*>(nl);
+      uint4 q = __ldg(n4);
+      float4 p = ld_pos<D, PK>(x, pk, nbr_slot(q.x));
 #pragma unroll 1
-    while (true) {
-      const bool more = ++k < k1;
-      const uint32_t en = more ? __ldg(nl + k) : e;
-      const int jn = nbr_slot(en);
-      const V3 xn = ldv<D>(x, jn);
-      const int mn = nbr_mat(en);
-      V3 r = rel<D>(P, xi, xj);
-      if constexpr (MAT)
-        f(j, r, sqnorm<D>(r), mj);
-      else
-        f(j, r, sqnorm<D>(r));
-      if (!more) break;
-      j = jn;
-      xj = xn;
-      mj = mn;
+      for (int k = 0; k < len; k += 4) {
+        const uint4 qn = k + 4 < len ? __ldg(n4 + (k >> 2) + 1) : q;
+        float4 pn = ld_pos<D, PK>(x, pk, nbr_slot(q.y));
+        call(q.x, p);
+        p = pn;
+        if (k + 1 >= len) break;
+        pn = ld_pos<D, PK>(x, pk, nbr_slot(q.z));
+        call(q.y, p);
+        p = pn;
+        if (k + 2 >= len) break;
+        pn = ld_pos<D, PK>(x, pk, nbr_slot(q.w));
+        call(q.z, p);
+        p = pn;
+        if (k + 3 >= len) break;
+        pn = ld_pos<D, PK>(x, pk, nbr_slot(qn.x));
+        call(q.w, p);
+        p = pn;
+        q = qn;
+      }
+    } else {
+      const uint32_t len = __ldg(G.noff + i + 1) - k0;
+      if (len == 0) return;
+      // one-deep software pipeline: the next neighbour's entry and position
+      // are loaded before f runs on the current one (f still runs in list
+      // order).  Sweeps -5% at 2.37M particles; a two-deep pipeline was slower.
+      uint32_t e = __ldg(nl);
+      float4 p = ld_pos<D, PK>(x, pk, nbr_slot(e));
+      uint32_t k = 0;
+#pragma unroll 1
+      while (true) {
+        const bool more = ++k < len;
+        const uint32_t en = more ? __ldg(nl + k) : e;
+        const float4 pn = ld_pos<D, PK>(x, pk, nbr_slot(en));
+        call(e, p);
+        if (!more) break;
+        e = en;
+        p = pn;
+      }
     }
     return;
   }
@@ -463,10 +540,13 @@ __device__ __forceinline__ void for_each_neighbor_impl(const dv_params& P, const
 #pragma unroll 1
         for (int j = s; j < e; ++j) {
           if (j == i) continue;
-          V3 r = rel<D>(P, xi, ldv<D>(x, j));
+          const float4 p = ld_pos<D, PK>(x, pk, j);
+          V3 r = rel<D>(P, xi, V3{p.x, p.y, p.z});
           float r2 = sqnorm<D>(r);
           if (r2 < lim) {
-            if constexpr (MAT)
+            if constexpr (PK)
+              f(j, r, r2, __ldg(mat + j), p.w);
+            else if constexpr (MAT)
               f(j, r, r2, __ldg(mat + j));
             else
               f(j, r, r2);
@@ -480,14 +560,22 @@ __device__ __forceinline__ void for_each_neighbor_impl(const dv_params& P, const
 template <int D, typename F>
 __device__ __forceinline__ void for_each_neighbor(const dv_params& P, const DevGrid& G,
                                                   const float* __restrict__ x, int i, V3 xi, F&& f) {
-  for_each_neighbor_impl<D, false>(P, G, x, nullptr, i, xi, f);
+  for_each_neighbor_impl<D, false, false>(P, G, x, nullptr, nullptr, i, xi, f);
 }
 
 template <int D, typename F>
 __device__ __forceinline__ void for_each_neighbor_m(const dv_params& P, const DevGrid& G,
                                                     const float* __restrict__ x, const int32_t* __restrict__ mat,
                                                     int i, V3 xi, F&& f) {
-  for_each_neighbor_impl<D, true>(P, G, x, mat, i, xi, f);
+  for_each_neighbor_impl<D, true, false>(P, G, x, nullptr, mat, i, xi, f);
+}
+
+// packed walk: f(j, r, r2, mj, w)
+template <int D, typename F>
+__device__ __forceinline__ void for_each_neighbor_p(const dv_params& P, const DevGrid& G,
+                                                    const float* __restrict__ x, const float4* __restrict__ pk,
+                                                    const int32_t* __restrict__ mat, int i, V3 xi, F&& f) {
+  for_each_neighbor_impl<D, true, true>(P, G, x, pk, mat, i, xi, f);
 }
 
 // ------------------------------------------------- far field on boxes (3-D)

@@ -13,6 +13,61 @@
   int i = blockIdx.x * blockDim.x + threadIdx.x;   \
   if (i >= C->n) return;
 
+// ------------------------------------------------------------ packed copies
+// One pass over the particles before a 3-D sweep (36 to 72 bytes each, 10 to
+// 25 us at 2.4M particles), against a gather of 32 scattered lanes per saved
+// field and neighbour.  Written anew by every call that reads them, since the
+// caller may change any field between calls.
+template <int WHAT>
+__global__ void k_pack_fields(dv_params P, dv_fields F, dv_solver_fields S, const dv_counters* __restrict__ C,
+                              float4* __restrict__ a, float4* __restrict__ b, float2* __restrict__ k) {
+  FOR_I;
+  if (WHAT & DV_PK_XV) {
+    const V3 x = ldv<3>(F.x, i);
+    a[i] = make_float4(x.x, x.y, x.z, F.m_V[i]);
+  }
+  if (WHAT & DV_PK_VM) {
+    const V3 v = ldv<3>(F.v, i);
+    b[i] = make_float4(v.x, v.y, v.z, F.m[i]);
+  }
+  if (WHAT & DV_PK_DW) {
+    const V3 w = ld4(S.d_vort, i);
+    b[i] = make_float4(w.x, w.y, w.z, S.kvn[i]);
+  }
+  if (WHAT & DV_PK_SW) {
+    const V3 w = ld4(S.d_vort_smoothed, i);
+    b[i] = make_float4(w.x, w.y, w.z, S.kden[i]);
+  }
+  if (WHAT & DV_PK_DIV) k[i] = make_float2(F.density_adv[i] * F.dfsph_factor[i] * F.density[i], F.m[i]);
+  if (WHAT & DV_PK_P) k[i] = make_float2((F.density_adv[i] - P.density0) * F.dfsph_factor[i], F.m[i]);
+}
+
+int dv_pack(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s, int what) {
+  if (c->p.dim != 3) return DV_OK;
+  const int nb = dv_blocks(std::min<int64_t>(c->n_upper, c->cap));
+  const dv_solver_fields sv = s ? *s : dv_solver_fields{};
+#define DV_PK(W)                                                                                            \
+  case (W):                                                                                                 \
+    k_pack_fields<(W)><<<nb, DV_THREADS, 0, c->stream>>>(c->p, *f, sv, c->d_cnt, c->pk_a, c->pk_b, c->pk_k); \
+    break
+  switch (what) {
+    DV_PK(DV_PK_XV);
+    DV_PK(DV_PK_P);
+    DV_PK(DV_PK_SW);
+    DV_PK(DV_PK_XV | DV_PK_VM);
+    DV_PK(DV_PK_XV | DV_PK_DIV);
+    DV_PK(DV_PK_XV | DV_PK_P);
+    DV_PK(DV_PK_XV | DV_PK_DW);
+    default:
+      return dv_fail(c, DV_EINVAL, "dv_pack: no kernel for %d", what);
+  }
+#undef DV_PK
+  // counted with the sweep that it prepares (dv_launch_count)
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return dv_cuda_check(c, e, "kernel launch");
+  return DV_OK;
+}
+
 // --------------------------------------------------------- boundary volume
 // compute_static_boundary_volume (sph_base.py:91-103) for the static solids,
 // compute_moving_boundary_volume (:105-112) for the dynamic ones
@@ -85,9 +140,10 @@ __global__ void k_dfsph_factor(dv_params P, DevGrid G, dv_fields F, const dv_cou
 // solve (dimcv_sph.py:337-374): it reads only v, x and m_V, which neither of
 // the two sweeps changes, and shares their ∇W; density_adv is bit-identical
 // to k_density_change's.
+// 3-D: K.a = (x, m_V), with DC also K.b = (v, m).
 template <int D, bool DC>
 __device__ __forceinline__ void densities_factor_body(const dv_params& P, const DevGrid& G, const dv_fields& F,
-                                                      const dv_counters* __restrict__ C) {
+                                                      const DevPack& K, const dv_counters* __restrict__ C) {
   FOR_I;
   if (F.material[i] != DV_MATERIAL_FLUID) return;
   V3 xi = ldv<D>(F.x, i);
@@ -98,13 +154,15 @@ __device__ __forceinline__ void densities_factor_body(const dv_params& P, const 
   float sum_k = 0.0f;
   float adv = 0.0f;
   int nn = 0;
-  for_each_neighbor_m<D>(P, G, F.x, F.material, i, xi, [&](int j, V3 r, float r2, int mj) {
+  for_each_neighbor_p<D>(P, G, F.x, K.a, F.material, i, xi, [&](int j, V3 r, float r2, int mj, float w) {
     if (mj == DV_MATERIAL_FLUID || mj == DV_MATERIAL_SOLID) {
-      const float mvj = F.m_V[j];
+      const float mvj = D == 3 ? w : F.m_V[j];
+      float4 vm = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (D == 3 && DC) vm = __ldg(K.b + j);
       den += mvj * cubic_W(P, sqrtf(r2));
       V3 gw = cubic_gradW<D>(P, r, r2);
       if (mj == DV_MATERIAL_FLUID) {
-        float mm = F.m[j];
+        float mm = (D == 3 && DC) ? vm.w : F.m[j];
         V3 g{mm * gw.x, mm * gw.y, mm * gw.z};
         sum_k += sqnorm<D>(g);
         gi.x += g.x;
@@ -117,7 +175,7 @@ __device__ __forceinline__ void densities_factor_body(const dv_params& P, const 
         if (D == 3) gi.z += s * gw.z;
       }
       if (DC) {
-        V3 vj = ldv<D>(F.v, j);
+        V3 vj = D == 3 ? V3{vm.x, vm.y, vm.z} : ldv<D>(F.v, j);
         V3 dv{vi.x - vj.x, vi.y - vj.y, vi.z - vj.z};
         adv += mvj * dot<D>(dv, gw);
       }
@@ -145,25 +203,28 @@ __global__ void k_scale_factor(dv_fields F, float s, const dv_counters* __restri
 // ------------------------------------------------------- density change
 // compute_density_change (dimcv_sph.py:337-374) of slot i; returns the
 // compute_density_error(0) term (dimcv_sph.py:407-419), 0 for non-fluid.
-template <int D>
+// 3-D: K.a = (x, m_V), and with NEXT (the Jacobi loop) slot i's k of the next
+// iteration goes to K.k.
+template <int D, bool NEXT>
 __device__ __forceinline__ double density_change_one(const dv_params& P, const DevGrid& G, const dv_fields& F,
-                                                     int i) {
+                                                     const DevPack& K, int i) {
   if (F.material[i] != DV_MATERIAL_FLUID) return 0.0;
   V3 xi = ldv<D>(F.x, i);
   V3 vi = ldv<D>(F.v, i);
   float adv = 0.0f;
   int nn = 0;
-  for_each_neighbor_m<D>(P, G, F.x, F.material, i, xi, [&](int j, V3 r, float r2, int mj) {
+  for_each_neighbor_p<D>(P, G, F.x, K.a, F.material, i, xi, [&](int j, V3 r, float r2, int mj, float w) {
     if (mj == DV_MATERIAL_FLUID || mj == DV_MATERIAL_SOLID) {
       V3 vj = ldv<D>(F.v, j);
       V3 dv{vi.x - vj.x, vi.y - vj.y, vi.z - vj.z};
-      adv += F.m_V[j] * dot<D>(dv, cubic_gradW<D>(P, r, r2));
+      adv += (D == 3 ? w : F.m_V[j]) * dot<D>(dv, cubic_gradW<D>(P, r, r2));
     }
     nn += 1;
   });
   float da = fmaxf(adv, 0.0f);
   if (nn < P.neighbor_min) da = 0.0f;
   F.density_adv[i] = da;
+  if (D == 3 && NEXT) K.k[i].x = da * F.dfsph_factor[i] * F.density[i];
   float term = P.has_transit ? transit_weight(P, xi.x) * (da - 0.0f) : (da - 0.0f);
   return (double)term;
 }
@@ -177,7 +238,7 @@ __device__ __forceinline__ double density_change_one(const dv_params& P, const D
 // slots gravity).
 template <int D>
 __device__ __forceinline__ double density_change_np_one(const dv_params& P, const DevGrid& G, const dv_fields& F,
-                                                        int i) {
+                                                        const DevPack& K, int i) {
   const int mi = F.material[i];
   const V3 g{P.gravity[0], P.gravity[1], D == 3 ? P.gravity[2] : 0.0f};
   if (mi != DV_MATERIAL_FLUID) {
@@ -189,11 +250,11 @@ __device__ __forceinline__ double density_change_np_one(const dv_params& P, cons
   float adv = 0.0f;
   int nn = 0;
   V3 acc = g;
-  for_each_neighbor_m<D>(P, G, F.x, F.material, i, xi, [&](int j, V3 r, float r2, int mj) {
+  for_each_neighbor_p<D>(P, G, F.x, K.a, F.material, i, xi, [&](int j, V3 r, float r2, int mj, float w) {
     if (mj == DV_MATERIAL_FLUID || mj == DV_MATERIAL_SOLID) {
       V3 vj = ldv<D>(F.v, j);
       V3 dv{vi.x - vj.x, vi.y - vj.y, vi.z - vj.z};
-      const float mvj = F.m_V[j];
+      const float mvj = D == 3 ? w : F.m_V[j];
       V3 gw = cubic_gradW<D>(P, r, r2);
       adv += mvj * dot<D>(dv, gw);
       if (mj == DV_MATERIAL_FLUID) {
@@ -211,19 +272,20 @@ __device__ __forceinline__ double density_change_np_one(const dv_params& P, cons
   float da = fmaxf(adv, 0.0f);
   if (nn < P.neighbor_min) da = 0.0f;
   F.density_adv[i] = da;
+  if (D == 3) K.k[i].x = da * F.dfsph_factor[i] * F.density[i];
   float term = P.has_transit ? transit_weight(P, xi.x) * (da - 0.0f) : (da - 0.0f);
   return (double)term;
 }
 
-// optionally the FP64 block partial of the error terms
-template <int D>
-__global__ void k_density_change(dv_params P, DevGrid G, dv_fields F, const dv_counters* __restrict__ C,
+// NEXT: in the Jacobi loop, with the FP64 block partial of the error terms
+template <int D, bool NEXT>
+__global__ void k_density_change(dv_params P, DevGrid G, dv_fields F, DevPack K, const dv_counters* __restrict__ C,
                                  const int32_t* __restrict__ done, double* __restrict__ part) {
   if (done && *done) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   double err = 0.0;
-  if (i < C->n) err = density_change_one<D>(P, G, F, i);
-  if (part) {
+  if (i < C->n) err = density_change_one<D, NEXT>(P, G, F, K, i);
+  if (NEXT) {
     double s = block_sum<double>(err);
     if (threadIdx.x == 0) part[blockIdx.x] = s;
   }
@@ -231,52 +293,60 @@ __global__ void k_density_change(dv_params P, DevGrid G, dv_fields F, const dv_c
 
 // the divergence Jacobi loop's residual sweep with the non-pressure forces
 template <int D>
-__global__ void k_density_change_np(dv_params P, DevGrid G, dv_fields F, const dv_counters* __restrict__ C,
+__global__ void k_density_change_np(dv_params P, DevGrid G, dv_fields F, DevPack K,
+                                    const dv_counters* __restrict__ C,
                                     const int32_t* __restrict__ done, double* __restrict__ part) {
   if (*done) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   double err = 0.0;
-  if (i < C->n) err = density_change_np_one<D>(P, G, F, i);
+  if (i < C->n) err = density_change_np_one<D>(P, G, F, K, i);
   double s = block_sum<double>(err);
   if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
 // ------------------------------------------------------------ density adv
 // compute_density_adv (dimcv_sph.py:470-493) of slot i; returns the
-// compute_density_error(density0) term, 0 for non-fluid.
-template <int D>
+// compute_density_error(density0) term, 0 for non-fluid.  3-D: K.a = (x, m_V),
+// K.b = (v, m); NEXT as in density_change_one.
+template <int D, bool NEXT>
 __device__ __forceinline__ double density_adv_one(const dv_params& P, const DevGrid& G, const dv_fields& F,
-                                                  int i) {
+                                                  const DevPack& K, int i) {
   if (F.material[i] != DV_MATERIAL_FLUID) return 0.0;
   V3 xi = ldv<D>(F.x, i);
   V3 vi = ldv<D>(F.v, i);
   float delta = 0.0f;
-  for_each_neighbor_m<D>(P, G, F.x, F.material, i, xi, [&](int j, V3 r, float r2, int mj) {
-    if (mj == DV_MATERIAL_FLUID) {
-      V3 vj = ldv<D>(F.v, j);
+  for_each_neighbor_p<D>(P, G, F.x, K.a, F.material, i, xi, [&](int j, V3 r, float r2, int mj, float w) {
+    if (mj == DV_MATERIAL_FLUID || mj == DV_MATERIAL_SOLID) {
+      V3 vj;
+      float mj_;
+      if (D == 3) {
+        const float4 vm = K.b[j];
+        vj = V3{vm.x, vm.y, vm.z};
+        mj_ = mj == DV_MATERIAL_FLUID ? vm.w : w * P.density0;
+      } else {
+        vj = ldv<D>(F.v, j);
+        mj_ = mj == DV_MATERIAL_FLUID ? F.m[j] : F.m_V[j] * P.density0;
+      }
       V3 dv{vi.x - vj.x, vi.y - vj.y, vi.z - vj.z};
-      delta += F.m[j] * dot<D>(dv, cubic_gradW<D>(P, r, r2));
-    } else if (mj == DV_MATERIAL_SOLID) {
-      V3 vj = ldv<D>(F.v, j);
-      V3 dv{vi.x - vj.x, vi.y - vj.y, vi.z - vj.z};
-      delta += F.m_V[j] * P.density0 * dot<D>(dv, cubic_gradW<D>(P, r, r2));
+      delta += mj_ * dot<D>(dv, cubic_gradW<D>(P, r, r2));
     }
   });
   float da = F.density[i] + P.dt * delta;
   da = fmaxf(da, P.density0);
   F.density_adv[i] = da;
+  if (D == 3 && NEXT) K.k[i].x = (da - P.density0) * F.dfsph_factor[i];
   float term = P.has_transit ? transit_weight(P, xi.x) * (da - P.density0) : (da - P.density0);
   return (double)term;
 }
 
-template <int D>
-__global__ void k_density_adv(dv_params P, DevGrid G, dv_fields F, const dv_counters* __restrict__ C,
+template <int D, bool NEXT>
+__global__ void k_density_adv(dv_params P, DevGrid G, dv_fields F, DevPack K, const dv_counters* __restrict__ C,
                               const int32_t* __restrict__ done, double* __restrict__ part) {
   if (done && *done) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   double err = 0.0;
-  if (i < C->n) err = density_adv_one<D>(P, G, F, i);
-  if (part) {
+  if (i < C->n) err = density_adv_one<D, NEXT>(P, G, F, K, i);
+  if (NEXT) {
     double s = block_sum<double>(err);
     if (threadIdx.x == 0) part[blockIdx.x] = s;
   }
@@ -288,7 +358,7 @@ __global__ void k_density_adv(dv_params P, DevGrid G, dv_fields F, const dv_coun
 // vorticity, which the pressure iterations (they write v) leave unchanged, so
 // the solve's first sweep gives what the vis sweep after the solve would.
 template <int D>
-__global__ void k_density_adv_vis(dv_params P, DevGrid G, dv_fields F, dv_solver_fields S,
+__global__ void k_density_adv_vis(dv_params P, DevGrid G, dv_fields F, dv_solver_fields S, DevPack K,
                                   const dv_counters* __restrict__ C) {
   FOR_I;
   const V3 xi = ldv<D>(F.x, i);
@@ -303,16 +373,21 @@ __global__ void k_density_adv_vis(dv_params P, DevGrid G, dv_fields F, dv_solver
   const V3 wi = ld4(F.vorticity, i);
   V3 vort{w * wi.x, w * wi.y, w * wi.z};
   float ws = w;
-  for_each_neighbor_m<D>(P, G, F.x, F.material, i, xi, [&](int j, V3 r, float r2, int mj) {
-    const float mvj = F.m_V[j];
-    if (mj == DV_MATERIAL_FLUID) {
-      V3 vj = ldv<D>(F.v, j);
+  for_each_neighbor_p<D>(P, G, F.x, K.a, F.material, i, xi, [&](int j, V3 r, float r2, int mj, float pw) {
+    const float mvj = D == 3 ? pw : F.m_V[j];
+    if (mj == DV_MATERIAL_FLUID || mj == DV_MATERIAL_SOLID) {
+      V3 vj;
+      float mj_;
+      if (D == 3) {
+        const float4 vm = __ldg(K.b + j);
+        vj = V3{vm.x, vm.y, vm.z};
+        mj_ = mj == DV_MATERIAL_FLUID ? vm.w : mvj * P.density0;
+      } else {
+        vj = ldv<D>(F.v, j);
+        mj_ = mj == DV_MATERIAL_FLUID ? F.m[j] : mvj * P.density0;
+      }
       V3 dv{vi.x - vj.x, vi.y - vj.y, vi.z - vj.z};
-      delta += F.m[j] * dot<D>(dv, cubic_gradW<D>(P, r, r2));
-    } else if (mj == DV_MATERIAL_SOLID) {
-      V3 vj = ldv<D>(F.v, j);
-      V3 dv{vi.x - vj.x, vi.y - vj.y, vi.z - vj.z};
-      delta += mvj * P.density0 * dot<D>(dv, cubic_gradW<D>(P, r, r2));
+      delta += mj_ * dot<D>(dv, cubic_gradW<D>(P, r, r2));
     }
     const float wj = mvj * cubic_W(P, sqrtf(r2));
     const V3 oj = ld4(F.vorticity, j);
@@ -351,23 +426,30 @@ __global__ void k_density_error(dv_params P, dv_fields F, const dv_counters* __r
 
 // ---------------------------------------------------- Jacobi iterations
 // divergence_solver_iteration_kernel (dimcv_sph.py:421-468)
+// 3-D: K.a = (x, m_V), K.k = (k, m).
 template <int D>
 __device__ __forceinline__ void divergence_iter_one(const dv_params& P, const DevGrid& G, const dv_fields& F,
-                                                    int i) {
+                                                    const DevPack& K, int i) {
   if (F.material[i] != DV_MATERIAL_FLUID) return;
   V3 xi = ldv<D>(F.x, i);
   float b_i = F.density_adv[i];
   float k_i = b_i * F.dfsph_factor[i] * F.density[i];
   V3 dv{0.f, 0.f, 0.f};
   const float dt = P.dt;
-  for_each_neighbor_m<D>(P, G, F.x, F.material, i, xi, [&](int j, V3 r, float r2, int mj) {
+  for_each_neighbor_p<D>(P, G, F.x, K.a, F.material, i, xi, [&](int j, V3 r, float r2, int mj, float w) {
     if (mj == DV_MATERIAL_FLUID) {
-      float b_j = F.density_adv[j];
-      float k_j = b_j * F.dfsph_factor[j] * F.density[j];
+      float k_j, mm = 0.0f;
+      if (D == 3) {
+        const float2 km = K.k[j];
+        k_j = km.x;
+        mm = km.y;
+      } else {
+        k_j = F.density_adv[j] * F.dfsph_factor[j] * F.density[j];
+      }
       float k_sum = k_i + k_j;
       if (fabsf(k_sum) > P.m_eps) {
         V3 gw = cubic_gradW<D>(P, r, r2);
-        float mm = F.m[j];
+        if (D != 3) mm = F.m[j];
         float s = dt * k_sum;
         dv.x -= s * (mm * gw.x);
         dv.y -= s * (mm * gw.y);
@@ -376,7 +458,7 @@ __device__ __forceinline__ void divergence_iter_one(const dv_params& P, const De
     } else if (mj == DV_MATERIAL_SOLID) {
       if (fabsf(k_i) > P.m_eps) {
         V3 gw = cubic_gradW<D>(P, r, r2);
-        float sm = F.m_V[j] * P.density0;
+        float sm = (D == 3 ? w : F.m_V[j]) * P.density0;
         float s = -dt * 1.0f * k_i;
         dv.x += s * (sm * gw.x);
         dv.y += s * (sm * gw.y);
@@ -399,10 +481,11 @@ __device__ __forceinline__ void divergence_iter_one(const dv_params& P, const De
 }
 
 // pressure_solve_iteration_kernel (dimcv_sph.py:495-549): the velocity is
-// updated pair by pair (the reference writes v[p_i] inside the task).
+// updated pair by pair (the reference writes v[p_i] inside the task).  3-D:
+// K.a = (x, m_V), K.k = (k, m), and the new (v, m) goes to K.b.
 template <int D>
 __device__ __forceinline__ void pressure_iter_one(const dv_params& P, const DevGrid& G, const dv_fields& F,
-                                                  int i) {
+                                                  const DevPack& K, int i) {
   if (F.material[i] != DV_MATERIAL_FLUID) return;
   V3 xi = ldv<D>(F.x, i);
   V3 vi = ldv<D>(F.v, i);
@@ -410,14 +493,20 @@ __device__ __forceinline__ void pressure_iter_one(const dv_params& P, const DevG
   float k_i = b_i * F.dfsph_factor[i];
   const float dt = P.dt;
   const float w = P.has_transit ? transit_weight(P, xi.x) : 1.0f;
-  for_each_neighbor_m<D>(P, G, F.x, F.material, i, xi, [&](int j, V3 r, float r2, int mj) {
+  for_each_neighbor_p<D>(P, G, F.x, K.a, F.material, i, xi, [&](int j, V3 r, float r2, int mj, float pw) {
     if (mj == DV_MATERIAL_FLUID) {
-      float b_j = F.density_adv[j] - P.density0;
-      float k_j = b_j * F.dfsph_factor[j];
+      float k_j, mm = 0.0f;
+      if (D == 3) {
+        const float2 km = K.k[j];
+        k_j = km.x;
+        mm = km.y;
+      } else {
+        k_j = (F.density_adv[j] - P.density0) * F.dfsph_factor[j];
+      }
       float k_sum = k_i + k_j;
       if (fabsf(k_sum) > P.m_eps) {
         V3 gw = cubic_gradW<D>(P, r, r2);
-        float mm = F.m[j];
+        if (D != 3) mm = F.m[j];
         float s = P.has_transit ? (w * dt) * k_sum : dt * k_sum;
         vi.x -= s * (mm * gw.x);
         vi.y -= s * (mm * gw.y);
@@ -426,7 +515,7 @@ __device__ __forceinline__ void pressure_iter_one(const dv_params& P, const DevG
     } else if (mj == DV_MATERIAL_SOLID) {
       if (fabsf(k_i) > P.m_eps) {
         V3 gw = cubic_gradW<D>(P, r, r2);
-        float sm = F.m_V[j] * P.density0;
+        float sm = (D == 3 ? pw : F.m_V[j]) * P.density0;
         float s = -dt * 1.0f * k_i;
         V3 vc{s * (sm * gw.x), s * (sm * gw.y), D == 3 ? s * (sm * gw.z) : 0.0f};
         if (P.has_transit) {
@@ -442,6 +531,7 @@ __device__ __forceinline__ void pressure_iter_one(const dv_params& P, const DevG
     }
   });
   stv<D>(F.v, i, vi);
+  if (D == 3) K.b[i] = make_float4(vi.x, vi.y, vi.z, F.m[i]);
 }
 
 // The reaction on dynamic rigid particles of one pressure iteration
@@ -481,19 +571,21 @@ __global__ void k_rigid_reaction(dv_params P, DevGrid G, dv_fields F, const dv_c
 }
 
 template <int D>
-__global__ void k_divergence_iter(dv_params P, DevGrid G, dv_fields F, const dv_counters* __restrict__ C,
+__global__ void k_divergence_iter(dv_params P, DevGrid G, dv_fields F, DevPack K,
+                                const dv_counters* __restrict__ C,
                                   const int32_t* __restrict__ done) {
   if (done && *done) return;
   FOR_I;
-  divergence_iter_one<D>(P, G, F, i);
+  divergence_iter_one<D>(P, G, F, K, i);
 }
 
 template <int D>
-__global__ void k_pressure_iter(dv_params P, DevGrid G, dv_fields F, const dv_counters* __restrict__ C,
+__global__ void k_pressure_iter(dv_params P, DevGrid G, dv_fields F, DevPack K,
+                                const dv_counters* __restrict__ C,
                                 const int32_t* __restrict__ done) {
   if (done && *done) return;
   FOR_I;
-  pressure_iter_one<D>(P, G, F, i);
+  pressure_iter_one<D>(P, G, F, K, i);
 }
 
 // Scene batch forms: a grid of a few blocks per SM walks the work list of
@@ -512,7 +604,7 @@ __device__ __forceinline__ int wl_scene(const int32_t* __restrict__ wl, int S, i
 }
 
 template <int D, int WHICH>
-__global__ void k_batch_iter(dv_params P, DevGrid G, dv_fields F, const dv_scene_state* __restrict__ st,
+__global__ void k_batch_iter(dv_params P, DevGrid G, dv_fields F, DevPack K, const dv_scene_state* __restrict__ st,
                              const int32_t* __restrict__ wl, int S) {
   const int tot = wl[S];
   for (int b = blockIdx.x; b < tot; b += gridDim.x) {
@@ -520,9 +612,9 @@ __global__ void k_batch_iter(dv_params P, DevGrid G, dv_fields F, const dv_scene
     const int i = st[s].start + (b - wl[s]) * DV_THREADS + threadIdx.x;
     if (i >= st[s].end) continue;
     if (WHICH == 0)
-      divergence_iter_one<D>(P, G, F, i);
+      divergence_iter_one<D>(P, G, F, K, i);
     else
-      pressure_iter_one<D>(P, G, F, i);
+      pressure_iter_one<D>(P, G, F, K, i);
   }
 }
 
@@ -530,7 +622,8 @@ __global__ void k_batch_iter(dv_params P, DevGrid G, dv_fields F, const dv_scene
 // (a block never spans two scenes) into part[b]; WHICH 2 is the divergence
 // residual with the non-pressure forces (density_change_np_one)
 template <int D, int WHICH>
-__global__ void k_batch_residual(dv_params P, DevGrid G, dv_fields F, const dv_scene_state* __restrict__ st,
+__global__ void k_batch_residual(dv_params P, DevGrid G, dv_fields F, DevPack K,
+                                 const dv_scene_state* __restrict__ st,
                                  const int32_t* __restrict__ wl, int S, double* __restrict__ part) {
   const int tot = wl[S];
   for (int b = blockIdx.x; b < tot; b += gridDim.x) {  // block-uniform bounds
@@ -538,9 +631,9 @@ __global__ void k_batch_residual(dv_params P, DevGrid G, dv_fields F, const dv_s
     const int i = st[s].start + (b - wl[s]) * DV_THREADS + threadIdx.x;
     double e = 0.0;
     if (i < st[s].end)
-      e = WHICH == 0   ? density_change_one<D>(P, G, F, i)
-          : WHICH == 1 ? density_adv_one<D>(P, G, F, i)
-                       : density_change_np_one<D>(P, G, F, i);
+      e = WHICH == 0   ? density_change_one<D, true>(P, G, F, K, i)
+          : WHICH == 1 ? density_adv_one<D, true>(P, G, F, K, i)
+                       : density_change_np_one<D>(P, G, F, K, i);
     e = block_sum<double>(e);
     if (threadIdx.x == 0) part[b] = e;
   }
@@ -701,23 +794,27 @@ DV_API int dv_dfsph_factor(dv_ctx* c, const dv_fields* f) {
 }
 
 template <int D>
-__global__ void k_densities_factor_only(dv_params P, DevGrid G, dv_fields F, const dv_counters* __restrict__ C) {
-  densities_factor_body<D, false>(P, G, F, C);
+__global__ void k_densities_factor_only(dv_params P, DevGrid G, dv_fields F, DevPack K,
+                                        const dv_counters* __restrict__ C) {
+  densities_factor_body<D, false>(P, G, F, K, C);
 }
 template <int D>
-__global__ void k_densities_factor_change(dv_params P, DevGrid G, dv_fields F, const dv_counters* __restrict__ C) {
-  densities_factor_body<D, true>(P, G, F, C);
+__global__ void k_densities_factor_change(dv_params P, DevGrid G, dv_fields F, DevPack K,
+                                          const dv_counters* __restrict__ C) {
+  densities_factor_body<D, true>(P, G, F, K, C);
 }
 
 DV_API int dv_densities_factor(dv_ctx* c, const dv_fields* f) {
   if (!c || !f) return DV_EINVAL;
-  LAUNCH_D(k_densities_factor_only, nblk(c), c->p, dv_grid(c), *f, c->d_cnt);
+  if (int rc = dv_pack(c, f, nullptr, DV_PK_XV)) return rc;
+  LAUNCH_D(k_densities_factor_only, nblk(c), c->p, dv_grid(c), *f, dv_packs(c), c->d_cnt);
   return DV_OK;
 }
 
 DV_API int dv_densities_factor_change(dv_ctx* c, const dv_fields* f) {
   if (!c || !f) return DV_EINVAL;
-  LAUNCH_D(k_densities_factor_change, nblk(c), c->p, dv_grid(c), *f, c->d_cnt);
+  if (int rc = dv_pack(c, f, nullptr, DV_PK_XV | DV_PK_VM)) return rc;
+  LAUNCH_D(k_densities_factor_change, nblk(c), c->p, dv_grid(c), *f, dv_packs(c), c->d_cnt);
   return DV_OK;
 }
 
@@ -728,17 +825,29 @@ DV_API int dv_scale_factor(dv_ctx* c, const dv_fields* f, float s) {
   return DV_OK;
 }
 
+// LAUNCH_D for the kernels of template <D, NEXT>
+#define LAUNCH_DN(kern, nx, nb, ...)                                                     \
+  do {                                                                                   \
+    if (c->p.dim == 2)                                                                   \
+      kern<2, nx><<<(nb), DV_THREADS, 0, c->stream>>>(__VA_ARGS__);                      \
+    else                                                                                 \
+      kern<3, nx><<<(nb), DV_THREADS, 0, c->stream>>>(__VA_ARGS__);                      \
+    DV_LAUNCHED(c);                                                                      \
+  } while (0)
+
 DV_API int dv_density_change(dv_ctx* c, const dv_fields* f) {
   if (!c || !f) return DV_EINVAL;
-  LAUNCH_D(k_density_change, nblk(c), c->p, dv_grid(c), *f, c->d_cnt, (const int32_t*)nullptr,
-           (double*)nullptr);
+  if (int rc = dv_pack(c, f, nullptr, DV_PK_XV)) return rc;
+  LAUNCH_DN(k_density_change, false, nblk(c), c->p, dv_grid(c), *f, dv_packs(c), c->d_cnt, (const int32_t*)nullptr,
+            (double*)nullptr);
   return DV_OK;
 }
 
 DV_API int dv_density_adv(dv_ctx* c, const dv_fields* f) {
   if (!c || !f) return DV_EINVAL;
-  LAUNCH_D(k_density_adv, nblk(c), c->p, dv_grid(c), *f, c->d_cnt, (const int32_t*)nullptr,
-           (double*)nullptr);
+  if (int rc = dv_pack(c, f, nullptr, DV_PK_XV | DV_PK_VM)) return rc;
+  LAUNCH_DN(k_density_adv, false, nblk(c), c->p, dv_grid(c), *f, dv_packs(c), c->d_cnt, (const int32_t*)nullptr,
+            (double*)nullptr);
   return DV_OK;
 }
 
@@ -756,20 +865,24 @@ DV_API int dv_density_error(dv_ctx* c, const dv_fields* f, float offset, double*
 
 DV_API int dv_divergence_iteration(dv_ctx* c, const dv_fields* f) {
   if (!c || !f) return DV_EINVAL;
-  LAUNCH_D(k_divergence_iter, nblk(c), c->p, dv_grid(c), *f, c->d_cnt, (const int32_t*)nullptr);
+  if (int rc = dv_pack(c, f, nullptr, DV_PK_XV | DV_PK_DIV)) return rc;
+  LAUNCH_D(k_divergence_iter, nblk(c), c->p, dv_grid(c), *f, dv_packs(c), c->d_cnt, (const int32_t*)nullptr);
   return DV_OK;
 }
 
 DV_API int dv_pressure_iteration(dv_ctx* c, const dv_fields* f) {
   if (!c || !f) return DV_EINVAL;
-  LAUNCH_D(k_pressure_iter, nblk(c), c->p, dv_grid(c), *f, c->d_cnt, (const int32_t*)nullptr);
+  if (int rc = dv_pack(c, f, nullptr, DV_PK_XV | DV_PK_P)) return rc;
+  LAUNCH_D(k_pressure_iter, nblk(c), c->p, dv_grid(c), *f, dv_packs(c), c->d_cnt, (const int32_t*)nullptr);
   if (c->dyn_rigid) LAUNCH_D(k_rigid_reaction, nblk(c), c->p, dv_grid(c), *f, c->d_cnt, (const int32_t*)nullptr);
   return DV_OK;
 }
 
 // Runs Jacobi iterations in chunks of 2, 4, 8, ... launches; every iteration
 // is (update sweep, residual sweep + FP64 block partials, finalize) and all
-// three return at once once the done flag is set.
+// three return at once once the done flag is set.  3-D: the packed copies are
+// made here (pressure: the caller's opening sweep left K.a and K.b), and the
+// residual sweeps keep K.k and the pressure updates K.b current.
 static int jacobi_loop(dv_ctx* c, const dv_fields* f, int which, bool nonpressure = false) {
   const int nb = nblk(c);
   const int max_iter = which == 0 ? c->p.max_iter_div : c->p.max_iter_p;
@@ -777,23 +890,25 @@ static int jacobi_loop(dv_ctx* c, const dv_fields* f, int which, bool nonpressur
   int32_t* done = c->d_flag;
   k_solve_reset<<<1, 1, 0, c->stream>>>(c->d_cnt, done, which);
   DV_LAUNCHED(c);
+  const DevPack K = dv_packs(c);
+  if (int rc = dv_pack(c, f, nullptr, which == 0 ? DV_PK_XV | DV_PK_DIV : DV_PK_P)) return rc;
   int launched = 0, chunk = 2;
   while (launched < max_iter) {
     int m = std::min(chunk, max_iter - launched);
     for (int k = 0; k < m; ++k) {
       if (which == 0) {
-        LAUNCH_D(k_divergence_iter, nb, c->p, dv_grid(c), *f, c->d_cnt, (const int32_t*)done);
+        LAUNCH_D(k_divergence_iter, nb, c->p, dv_grid(c), *f, K, c->d_cnt, (const int32_t*)done);
         if (nonpressure)
-          LAUNCH_D(k_density_change_np, nb, c->p, dv_grid(c), *f, c->d_cnt, (const int32_t*)done,
+          LAUNCH_D(k_density_change_np, nb, c->p, dv_grid(c), *f, K, c->d_cnt, (const int32_t*)done,
                    c->red_part);
         else
-          LAUNCH_D(k_density_change, nb, c->p, dv_grid(c), *f, c->d_cnt, (const int32_t*)done,
-                   c->red_part);
+          LAUNCH_DN(k_density_change, true, nb, c->p, dv_grid(c), *f, K, c->d_cnt, (const int32_t*)done,
+                    c->red_part);
       } else {
-        LAUNCH_D(k_pressure_iter, nb, c->p, dv_grid(c), *f, c->d_cnt, (const int32_t*)done);
+        LAUNCH_D(k_pressure_iter, nb, c->p, dv_grid(c), *f, K, c->d_cnt, (const int32_t*)done);
         if (c->dyn_rigid) LAUNCH_D(k_rigid_reaction, nb, c->p, dv_grid(c), *f, c->d_cnt, (const int32_t*)done);
-        LAUNCH_D(k_density_adv, nb, c->p, dv_grid(c), *f, c->d_cnt, (const int32_t*)done,
-                 c->red_part);
+        LAUNCH_DN(k_density_adv, true, nb, c->p, dv_grid(c), *f, K, c->d_cnt, (const int32_t*)done,
+                  c->red_part);
       }
       k_solve_finalize<<<1, 1024, 0, c->stream>>>(c->red_part, nb, c->d_cnt, done, eta, max_iter,
                                                   which);
@@ -830,15 +945,16 @@ static int batch_iteration(dv_ctx* c, const dv_fields* f, int which, bool nonpre
                  : K<3, 1><<<grid, DV_THREADS, 0, c->stream>>>(__VA_ARGS__);                \
     DV_LAUNCHED(c);                                                                          \
   } while (0)
-  LB(k_batch_iter, c->p, G, *f, b->d_state, b->d_wl, b->S);
+  const DevPack K = dv_packs(c);
+  LB(k_batch_iter, c->p, G, *f, K, b->d_state, b->d_wl, b->S);
   if (which == 0 && nonpressure) {
     if (c->p.dim == 2)
-      k_batch_residual<2, 2><<<grid, DV_THREADS, 0, c->stream>>>(c->p, G, *f, b->d_state, b->d_wl, b->S, b->d_err);
+      k_batch_residual<2, 2><<<grid, DV_THREADS, 0, c->stream>>>(c->p, G, *f, K, b->d_state, b->d_wl, b->S, b->d_err);
     else
-      k_batch_residual<3, 2><<<grid, DV_THREADS, 0, c->stream>>>(c->p, G, *f, b->d_state, b->d_wl, b->S, b->d_err);
+      k_batch_residual<3, 2><<<grid, DV_THREADS, 0, c->stream>>>(c->p, G, *f, K, b->d_state, b->d_wl, b->S, b->d_err);
     DV_LAUNCHED(c);
   } else {
-    LB(k_batch_residual, c->p, G, *f, b->d_state, b->d_wl, b->S, b->d_err);
+    LB(k_batch_residual, c->p, G, *f, K, b->d_state, b->d_wl, b->S, b->d_err);
   }
 #undef LB
   return dv_batch_solve_finalize(c, which);
@@ -848,6 +964,9 @@ int dv_batch_solve(dv_ctx* c, const dv_fields* f, int which, bool nonpressure) {
   dv_batch_state* b = c->batch;
   const int max_iter = which == 0 ? c->p.max_iter_div : c->p.max_iter_p;
   int rc = dv_batch_solve_reset(c, which);
+  if (rc) return rc;
+  // 3-D: as in jacobi_loop (the step's density_adv sweep left K.a and K.b)
+  rc = dv_pack(c, f, nullptr, which == 0 ? DV_PK_XV | DV_PK_DIV : DV_PK_P);
   if (rc) return rc;
   if (b->capturing) {
     cudaStream_t st = c->stream;
@@ -953,8 +1072,9 @@ DV_API int dv_pressure_solve_ex(dv_ctx* c, const dv_fields* f, const dv_solver_f
   if (flags & DV_SOLVE_VIS) {
     if (!s || !s->x_temp || !s->vorticity_vis)
       return dv_fail(c, DV_EINVAL, "dv_pressure_solve_ex: DV_SOLVE_VIS needs x_temp and vorticity_vis");
-    LAUNCH_D(k_density_adv_vis, nblk(c), c->p, dv_grid(c), *f, *s, c->d_cnt);
-    rc = DV_OK;
+    rc = dv_pack(c, f, s, DV_PK_XV | DV_PK_VM);
+    if (rc) return rc;
+    LAUNCH_D(k_density_adv_vis, nblk(c), c->p, dv_grid(c), *f, *s, dv_packs(c), c->d_cnt);
   } else {
     rc = dv_density_adv(c, f);
   }

@@ -209,7 +209,8 @@ DV_API int dv_set_stream(dv_ctx* ctx, void* stream);
  * `solver.dt[None] = ...` (dimcv_sph.py:13). */
 DV_API int dv_set_params(dv_ctx* ctx, const dv_params* params);
 /* Library version string and the number of kernels launched so far by this
- * context (used by benchmarks to report launch counts). */
+ * context (used by benchmarks to report launch counts; a 3-D sweep and the
+ * pass that packs its gathered fields count as one). */
 DV_API const char* dv_version(void);
 DV_API int64_t dv_launch_count(const dv_ctx* ctx);
 
