@@ -27,17 +27,25 @@
 // runs as a 2-D grid (target blocks × source chunks) with per-chunk partials
 // summed in fixed order, so every result is deterministic.  Its VJP computes
 // the target-side and the source-side gradient in one pass over the pairs:
-// the target side in registers, the source side by a butterfly warp
-// reduction per source and a fixed-order sum over warps and target blocks.
+// the target side in registers, the source side by a warp reduction per
+// source and a fixed-order sum over warps and target blocks.  The FP32 pair
+// kernels hold two targets in each 64-bit register (k_far_x2, k_far_bwd_x2).
 #include <algorithm>
 
+#include "dv_far.cuh"
 #include "dv_internal.cuh"
 
 namespace {
 
 constexpr int VT = 256;  // threads per block of the pair kernels
-constexpr int VTT = 2;   // targets per thread
+constexpr int VTT = 2;   // targets per thread (FP64)
 constexpr int VTS = 128; // sources per shared-memory tile
+// targets per thread of the FP32 kernels: wide where there are targets enough
+// for it (the source side's warp reduction is shared by them), narrow for
+// small clouds, which need the blocks
+constexpr int kWideN = 8192;
+__host__ inline int fwd_tt(int n) { return n >= kWideN ? 4 : 2; }
+__host__ inline int bwd_tt(int n) { return n >= kWideN ? 8 : 2; }
 
 template <typename T>
 struct Geo {
@@ -283,18 +291,29 @@ __global__ void k_curl_bwd(Geo<T> g, dv_vpm_plan p, const T* __restrict__ x, con
 
 // ------------------------------------------------------------ velocity
 struct Layout {
-  int ntb, nch, chunk;
+  int ntb, nch, chunk;     // forward: target blocks, source chunks, sources per chunk
+  int bntb, bnch, bchunk;  // backward
   int64_t sp, spb, part, tpart, spart, sg, total;  // byte offsets / total
 };
+
+// Chunks for about `waves` waves of two blocks per SM, in FP32 of 32 sources
+// at least (part-full tiles cost little there), in FP64 of one tile.
+template <typename T>
+void split(int n, int src_cap, int num_sms, int tt, int& ntb, int& nch, int& chunk) {
+  const bool f32 = sizeof(T) == 4;
+  const int per = VT * tt, least = f32 ? 32 : VTS, waves = f32 ? 4 : 1;
+  ntb = std::max(1, (n + per - 1) / per);
+  const int want = (2 * waves * num_sms) / ntb;
+  const int maxch = std::max(1, (src_cap + least - 1) / least);
+  nch = std::max(1, std::min(f32 ? want : (2 * num_sms + ntb - 1) / ntb, maxch));
+  chunk = std::max(1, (src_cap + nch - 1) / nch);
+}
 
 template <typename T>
 Layout layout(int n, int src_cap, int num_sms) {
   Layout L;
-  L.ntb = std::max(1, (n + VT * VTT - 1) / (VT * VTT));
-  const int want = (2 * num_sms + L.ntb - 1) / L.ntb;
-  const int maxch = std::max(1, (src_cap + VTS - 1) / VTS);
-  L.nch = std::max(1, std::min(want, maxch));
-  L.chunk = std::max(1, (src_cap + L.nch - 1) / L.nch);
+  split<T>(n, src_cap, num_sms, sizeof(T) == 4 ? fwd_tt(n) : VTT, L.ntb, L.nch, L.chunk);
+  split<T>(n, src_cap, num_sms, sizeof(T) == 4 ? bwd_tt(n) : VTT, L.bntb, L.bnch, L.bchunk);
   auto al = [](int64_t b) { return (b + 255) & ~int64_t(255); };
   const int64_t t = sizeof(T);
   int64_t o = 0;
@@ -305,9 +324,9 @@ Layout layout(int n, int src_cap, int num_sms) {
   L.part = o;
   o += al(t * 2 * (int64_t)L.nch * n);
   L.tpart = o;
-  o += al(t * 3 * (int64_t)L.nch * n);
+  o += al(t * 3 * (int64_t)L.bnch * n);
   L.spart = o;
-  o += al(t * 5 * (int64_t)L.ntb * std::max(src_cap, 1));
+  o += al(t * 5 * (int64_t)L.bntb * std::max(src_cap, 1));
   L.sg = o;
   o += al(t * 3 * (int64_t)std::max(src_cap, 1));
   L.total = o;
@@ -385,6 +404,240 @@ __global__ void __launch_bounds__(VT) k_far(Geo<T> g, dv_vpm_plan p, const T* __
     if (t < n) {
       part[2 * ((int64_t)ch * n + t)] = ax[k];
       part[2 * ((int64_t)ch * n + t) + 1] = ay[k];
+    }
+  }
+}
+
+// ------------------------------------------- FP32 pairs, two targets a lane
+// pd<float, IMG> of two targets at once, the same operations.  rint is taken
+// as (t + 1.5·2^23) − 1.5·2^23, which is rint(t) for |t| < 2^22 (positions of
+// fewer than four million box lengths): rintf runs on the unit of the
+// reciprocals at a quarter of the FP32 rate, twice a pair, and bounded the loop.
+struct Geo2 {
+  f2_t nLx, nLy, iLx, iLy, magic;
+};
+__device__ __forceinline__ Geo2 make_geo2(const Geo<float>& g) {
+  return Geo2{f2_pack(-g.Lx, -g.Lx), f2_pack(-g.Ly, -g.Ly), f2_pack(g.iLx, g.iLx), f2_pack(g.iLy, g.iLy),
+              f2_pack(12582912.0f, 12582912.0f)};
+}
+template <int IMG>
+__device__ __forceinline__ f2_t pd2(f2_t a, f2_t b, f2_t abar, f2_t bbar, f2_t nL, f2_t iL, f2_t magic) {
+  const f2_t d = f2_sub(a, b);
+  if (IMG == 0) return d;
+  const f2_t t = f2_mul(IMG == 2 ? f2_sub(abar, bbar) : d, iL);
+  return f2_fma(f2_sub(f2_add(t, magic), magic), nL, d);
+}
+// inv_r2<float> of two values
+__device__ __forceinline__ f2_t inv_r2_2(f2_t r2, float tiny) {
+  float a, b;
+  f2_unpack(r2, a, b);
+  return f2_pack(inv_r2<float>(a, tiny), inv_r2<float>(b, tiny));
+}
+
+// sources staged twice each: (x, x, y, y), (b, b, 0, 0) and for IMG 2 the
+// nominal position (x̄, x̄, ȳ, ȳ)
+template <int IMG>
+constexpr int src_words() { return IMG == 2 ? 3 : 2; }
+template <int IMG>
+__device__ __forceinline__ void stage_sources(float4* s4, const float* __restrict__ sp, const float* __restrict__ spb,
+                                              int base, int cnt) {
+  constexpr int NW = src_words<IMG>();
+  for (int q = threadIdx.x; q < cnt; q += VT) {
+    const float x = sp[3 * (base + q)], y = sp[3 * (base + q) + 1], b = sp[3 * (base + q) + 2];
+    s4[NW * q] = make_float4(x, x, y, y);
+    s4[NW * q + 1] = make_float4(b, b, 0.0f, 0.0f);
+    if (IMG == 2) {
+      const float u = spb[2 * (base + q)], v = spb[2 * (base + q) + 1];
+      s4[NW * q + 2] = make_float4(u, u, v, v);
+    }
+  }
+}
+
+// Targets 2p and 2p + 1 of a thread are the lanes of pair p.  Bound by the
+// FP32 pipe, 15 lane operations a pair with the periodic image; 65,536
+// targets x 4,096 sources: 245 -> 139 us (0.74 of the pipe).
+template <int IMG, int TT>
+__global__ void __launch_bounds__(VT) k_far_x2(Geo<float> g, dv_vpm_plan p, const float* __restrict__ x,
+                                               const float* __restrict__ xb, const float* __restrict__ sp,
+                                               const float* __restrict__ spb, int chunk, float* __restrict__ part) {
+  constexpr int NP = TT / 2, NW = src_words<IMG>();
+  __shared__ float4 s4[NW * VTS];
+  const int n = p.n, ns = *p.n_src, tid = threadIdx.x, ch = blockIdx.y;
+  const int s0 = ch * chunk, s1 = min(ns, s0 + chunk);
+  const Geo2 G = make_geo2(g);
+  f2_t PX[NP], PY[NP], BX[NP], BY[NP], AX[NP], AY[NP];
+#pragma unroll
+  for (int k = 0; k < NP; ++k) {
+    float v[2][4];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int t = min(blockIdx.x * VT * TT + (2 * k + u) * VT + tid, n - 1);
+      v[u][0] = x[2 * t];
+      v[u][1] = x[2 * t + 1];
+      v[u][2] = IMG == 2 ? xb[2 * t] : 0.0f;
+      v[u][3] = IMG == 2 ? xb[2 * t + 1] : 0.0f;
+    }
+    PX[k] = f2_pack(v[0][0], v[1][0]);
+    PY[k] = f2_pack(v[0][1], v[1][1]);
+    BX[k] = f2_pack(v[0][2], v[1][2]);
+    BY[k] = f2_pack(v[0][3], v[1][3]);
+    AX[k] = AY[k] = 0ull;
+  }
+  const ulonglong2* s2 = reinterpret_cast<const ulonglong2*>(s4);
+  for (int base = s0; base < s1; base += VTS) {
+    const int cnt = min(VTS, s1 - base);
+    __syncthreads();
+    stage_sources<IMG>(s4, sp, spb, base, cnt);
+    __syncthreads();
+#pragma unroll 2
+    for (int q = 0; q < cnt; ++q) {
+      const ulonglong2 v0 = s2[NW * q], v1 = s2[NW * q + 1];
+      ulonglong2 vb{0ull, 0ull};
+      if (IMG == 2) vb = s2[NW * q + 2];
+#pragma unroll
+      for (int k = 0; k < NP; ++k) {
+        const f2_t dx = pd2<IMG>(PX[k], v0.x, BX[k], vb.x, G.nLx, G.iLx, G.magic);
+        const f2_t dy = pd2<IMG>(PY[k], v0.y, BY[k], vb.y, G.nLy, G.iLy, G.magic);
+        const f2_t bs = f2_mul(v1.x, inv_r2_2(f2_fma(dy, dy, f2_mul(dx, dx)), g.tiny));
+        AX[k] = f2_fma(bs, dy, AX[k]);
+        AY[k] = f2_fma(bs, dx, AY[k]);  // the sum with the sign of −u_y
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < NP; ++k) {
+    float a[2], b[2];
+    f2_unpack(AX[k], a[0], a[1]);
+    f2_unpack(AY[k], b[0], b[1]);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int t = blockIdx.x * VT * TT + (2 * k + u) * VT + tid;
+      if (t < n) reinterpret_cast<float2*>(part)[(int64_t)ch * n + t] = make_float2(a[u], -b[u]);
+    }
+  }
+}
+
+// Sums five values over a warp with 8 shuffles instead of 25: while values
+// are left to pair up, the two halves of the warp each keep one of a pair.
+// Lane 0, 16, 8, 24, 4 end up with v0, v1, v2, v3, v4.
+__device__ __forceinline__ float warp_sum5(float v0, float v1, float v2, float v3, float v4, int lane) {
+  const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+  const unsigned m = 0xffffffffu;
+  float a = (b4 ? v1 : v0) + __shfl_xor_sync(m, b4 ? v0 : v1, 16);
+  float b = (b4 ? v3 : v2) + __shfl_xor_sync(m, b4 ? v2 : v3, 16);
+  float c = v4 + __shfl_xor_sync(m, v4, 16);
+  a = (b3 ? b : a) + __shfl_xor_sync(m, b3 ? a : b, 8);
+  c += __shfl_xor_sync(m, c, 8);
+  a = (b2 ? c : a) + __shfl_xor_sync(m, b2 ? a : c, 4);
+  a += __shfl_xor_sync(m, a, 2);
+  a += __shfl_xor_sync(m, a, 1);
+  return a;
+}
+
+// k_far_bwd for FP32, 25 lane operations a pair; the source side's five sums
+// are added over the thread's targets before the warp reduction, so a wide
+// tile (8 targets) spends a tenth of its issue slots there instead of half.
+// 65,536 targets x 4,096 sources: 675 -> 281 us (6 targets: 310).
+template <int IMG, int TT>
+__global__ void __launch_bounds__(VT) k_far_bwd_x2(Geo<float> g, dv_vpm_plan p, const float* __restrict__ x,
+                                                   const float* __restrict__ xb, const float* __restrict__ sp,
+                                                   const float* __restrict__ spb, const float* __restrict__ gu,
+                                                   int chunk, float* __restrict__ tpart, float* __restrict__ spart) {
+  constexpr int NP = TT / 2, NW = src_words<IMG>();
+  __shared__ float4 s4[NW * VTS];
+  __shared__ float s_r[(VT / 32) * VTS * 5];
+  const int n = p.n, ns = *p.n_src;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ch = blockIdx.y;
+  const int s0 = ch * chunk, s1 = min(ns, s0 + chunk);
+  const Geo2 G = make_geo2(g);
+  f2_t PX[NP], PY[NP], BX[NP], BY[NP], GX[NP], GY[NP], NGY[NP], AP[NP], AQX[NP], AQY[NP];
+#pragma unroll
+  for (int k = 0; k < NP; ++k) {
+    float v[2][6];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int t = blockIdx.x * VT * TT + (2 * k + u) * VT + tid, tc = min(t, n - 1);
+      const float f = t < n ? p.f[tc] : 0.0f;  // a lane past the end adds zeros to the source side
+      v[u][0] = x[2 * tc];
+      v[u][1] = x[2 * tc + 1];
+      v[u][2] = IMG == 2 ? xb[2 * tc] : 0.0f;
+      v[u][3] = IMG == 2 ? xb[2 * tc + 1] : 0.0f;
+      v[u][4] = t < n ? f * gu[2 * tc] : 0.0f;
+      v[u][5] = t < n ? f * gu[2 * tc + 1] : 0.0f;
+    }
+    PX[k] = f2_pack(v[0][0], v[1][0]);
+    PY[k] = f2_pack(v[0][1], v[1][1]);
+    BX[k] = f2_pack(v[0][2], v[1][2]);
+    BY[k] = f2_pack(v[0][3], v[1][3]);
+    GX[k] = f2_pack(v[0][4], v[1][4]);
+    GY[k] = f2_pack(v[0][5], v[1][5]);
+    NGY[k] = f2_pack(-v[0][5], -v[1][5]);
+    AP[k] = AQX[k] = AQY[k] = 0ull;
+  }
+  const ulonglong2* s2 = reinterpret_cast<const ulonglong2*>(s4);
+  const int slot = lane == 0 ? 0 : lane == 16 ? 1 : lane == 8 ? 2 : lane == 24 ? 3 : 4;
+  const bool writes = lane == 0 || lane == 16 || lane == 8 || lane == 24 || lane == 4;
+  for (int base = s0; base < s1; base += VTS) {
+    const int cnt = min(VTS, s1 - base);
+    __syncthreads();
+    stage_sources<IMG>(s4, sp, spb, base, cnt);
+    __syncthreads();
+#pragma unroll 1
+    for (int q = 0; q < cnt; ++q) {
+      const ulonglong2 v0 = s2[NW * q], v1 = s2[NW * q + 1];
+      ulonglong2 vb{0ull, 0ull};
+      if (IMG == 2) vb = s2[NW * q + 2];
+      f2_t BW = 0ull, BGX = 0ull, BGY = 0ull, CX = 0ull, CY = 0ull;
+#pragma unroll
+      for (int k = 0; k < NP; ++k) {
+        const f2_t dx = pd2<IMG>(PX[k], v0.x, BX[k], vb.x, G.nLx, G.iLx, G.magic);
+        const f2_t dy = pd2<IMG>(PY[k], v0.y, BY[k], vb.y, G.nLy, G.iLy, G.magic);
+        const f2_t s = inv_r2_2(f2_fma(dy, dy, f2_mul(dx, dx)), g.tiny);
+        const f2_t sc = f2_mul(s, f2_fma(GX[k], dy, f2_mul(NGY[k], dx)));
+        const f2_t u = f2_mul(s, sc);
+        AP[k] = f2_fma(v1.x, s, AP[k]);
+        const f2_t bu = f2_mul(v1.x, u);
+        AQX[k] = f2_fma(bu, dx, AQX[k]);
+        AQY[k] = f2_fma(bu, dy, AQY[k]);
+        BW = f2_add(BW, sc);
+        BGX = f2_fma(s, GX[k], BGX);
+        BGY = f2_fma(s, GY[k], BGY);
+        CX = f2_fma(u, dx, CX);
+        CY = f2_fma(u, dy, CY);
+      }
+      float h[5][2];
+      f2_unpack(BW, h[0][0], h[0][1]);
+      f2_unpack(BGX, h[1][0], h[1][1]);
+      f2_unpack(BGY, h[2][0], h[2][1]);
+      f2_unpack(CX, h[3][0], h[3][1]);
+      f2_unpack(CY, h[4][0], h[4][1]);
+      const float r = warp_sum5(h[0][0] + h[0][1], h[1][0] + h[1][1], h[2][0] + h[2][1], h[3][0] + h[3][1],
+                                h[4][0] + h[4][1], lane);
+      if (writes) s_r[(warp * VTS + q) * 5 + slot] = r;
+    }
+    __syncthreads();
+    for (int e = tid; e < 5 * cnt; e += VT) {
+      float acc = 0.0f;
+#pragma unroll
+      for (int w = 0; w < VT / 32; ++w) acc += s_r[w * VTS * 5 + e];
+      spart[((int64_t)blockIdx.x * p.src_cap + base) * 5 + e] = acc;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < NP; ++k) {
+    float a[2][3];
+    f2_unpack(AP[k], a[0][0], a[1][0]);
+    f2_unpack(AQX[k], a[0][1], a[1][1]);
+    f2_unpack(AQY[k], a[0][2], a[1][2]);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int t = blockIdx.x * VT * TT + (2 * k + u) * VT + tid;
+      if (t < n) {
+        float* o = tpart + 3 * ((int64_t)ch * n + t);
+        o[0] = a[u][0];
+        o[1] = a[u][1];
+        o[2] = a[u][2];
+      }
     }
   }
 }
@@ -770,8 +1023,17 @@ int velocity_t(dv_ctx* c, const dv_vpm_plan* p, const void* x, const void* wt, v
   }
   if (p->n > 0) {
     const dim3 grid(L.ntb, L.nch);
-    DV_IMG_DISPATCH(img, (k_far<T, IMG><<<grid, VT, 0, c->stream>>>(g, *p, (const T*)x, xb, sp, spb, L.chunk,
-                                                                     part)));
+    if constexpr (sizeof(T) == 4) {
+      if (fwd_tt(p->n) == 4)
+        DV_IMG_DISPATCH(img, (k_far_x2<IMG, 4><<<grid, VT, 0, c->stream>>>(g, *p, (const T*)x, xb, sp, spb, L.chunk,
+                                                                           part)));
+      else
+        DV_IMG_DISPATCH(img, (k_far_x2<IMG, 2><<<grid, VT, 0, c->stream>>>(g, *p, (const T*)x, xb, sp, spb, L.chunk,
+                                                                           part)));
+    } else {
+      DV_IMG_DISPATCH(img, (k_far<T, IMG><<<grid, VT, 0, c->stream>>>(g, *p, (const T*)x, xb, sp, spb, L.chunk,
+                                                                       part)));
+    }
     DV_LAUNCHED(c);
     DV_IMG_DISPATCH(img, (k_vel_fin<T, IMG><<<dv_blocks(p->n), DV_THREADS, 0, c->stream>>>(
                              g, *p, (const T*)x, xb, (const T*)wt, part, L.nch, (T*)u)));
@@ -800,16 +1062,25 @@ int velocity_bwd_t(dv_ctx* c, const dv_vpm_plan* p, const void* x, const void* w
     k_pack<T><<<dv_blocks(p->src_cap), DV_THREADS, 0, c->stream>>>(*p, (const T*)x, xb, (const T*)wt, sp, spb);
     DV_LAUNCHED(c);
   }
-  const dim3 grid(L.ntb, L.nch);
-  DV_IMG_DISPATCH(img, (k_far_bwd<T, IMG><<<grid, VT, 0, c->stream>>>(g, *p, (const T*)x, xb, sp, spb,
-                                                                       (const T*)gu, L.chunk, tpart, spart)));
+  const dim3 grid(L.bntb, L.bnch);
+  if constexpr (sizeof(T) == 4) {
+    if (bwd_tt(p->n) == 8)
+      DV_IMG_DISPATCH(img, (k_far_bwd_x2<IMG, 8><<<grid, VT, 0, c->stream>>>(
+                               g, *p, (const T*)x, xb, sp, spb, (const T*)gu, L.bchunk, tpart, spart)));
+    else
+      DV_IMG_DISPATCH(img, (k_far_bwd_x2<IMG, 2><<<grid, VT, 0, c->stream>>>(
+                               g, *p, (const T*)x, xb, sp, spb, (const T*)gu, L.bchunk, tpart, spart)));
+  } else {
+    DV_IMG_DISPATCH(img, (k_far_bwd<T, IMG><<<grid, VT, 0, c->stream>>>(g, *p, (const T*)x, xb, sp, spb,
+                                                                         (const T*)gu, L.bchunk, tpart, spart)));
+  }
   DV_LAUNCHED(c);
   if (p->src_cap > 0) {
-    k_src_fin<T><<<dv_blocks(p->src_cap), DV_THREADS, 0, c->stream>>>(*p, sp, spart, L.ntb, sg);
+    k_src_fin<T><<<dv_blocks(p->src_cap), DV_THREADS, 0, c->stream>>>(*p, sp, spart, L.bntb, sg);
     DV_LAUNCHED(c);
   }
   DV_IMG_DISPATCH(img, (k_vel_bwd_fin<T, IMG><<<dv_blocks(p->n), DV_THREADS, 0, c->stream>>>(
-                           g, *p, (const T*)x, xb, (const T*)wt, (const T*)gu, tpart, L.nch, sg, (T*)gwt,
+                           g, *p, (const T*)x, xb, (const T*)wt, (const T*)gu, tpart, L.bnch, sg, (T*)gwt,
                            (T*)gx)));
   DV_LAUNCHED(c);
   return DV_OK;
