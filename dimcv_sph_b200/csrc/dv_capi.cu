@@ -6,6 +6,7 @@
 #include <algorithm>
 
 #include "dv_internal.cuh"
+#include "dv_lookback.cuh"
 
 static thread_local std::string g_create_error;
 
@@ -113,11 +114,11 @@ DV_API void dv_destroy(dv_ctx* c) {
   dv_batch_free(c);
   dv_farbox_free(c);
   void* ptrs[] = {c->d_cnt,   c->d_flag,    c->keys[0],   c->keys[1],   c->vals[0], c->vals[1],
-                  c->hist,    c->cell_start, c->cell_end, c->mt[0],     c->mt[1],   c->mt[2],
-                  c->scan_part, c->dscan_part, c->red_part, c->ired_part, c->flags, c->offs,
+                  c->sort_state, c->cell_start, c->cell_end, c->mt[0],     c->mt[1],   c->mt[2],
+                  c->look_state, c->look_ctl, c->dscan_part, c->red_part, c->ired_part, c->flags, c->offs,
                   c->targets, c->cdf,       c->spos,      c->sw,        c->near_v,  c->near_S,
                   c->far_acc, c->mult,      c->nbr_off,   c->nbr_idx,   c->d_nbr_ok,
-                  c->nbr_rows, c->sflag,   c->srank,     c->sslot,   c->nbr_len,   c->pk_a,    c->pk_b,
+                  c->nbr_rows, c->srank,     c->sslot,   c->nbr_len,   c->pk_a,    c->pk_b,
                   c->pk_k};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -173,7 +174,8 @@ DV_API dv_ctx* dv_create(const dv_params* params, int64_t capacity, void* stream
   const int64_t cap = capacity;
   c->max_tiles = (cap + 2047) / 2048 + 1;
   c->red_cap = (cap + 127) / 128 + 1024;
-  c->scan_part_cap = (std::max<int64_t>(cap + 1, 256 * c->max_tiles) + 4095) / 4096 + 1024;
+  c->scan_part_cap = (cap + 1 + 4095) / 4096 + 1024;
+  const int64_t look_tiles = (cap + 1 + 255) / 256 + 64;  // tiles of 256 elements at least
   cudaError_t e = cudaSuccess;
 #define A(ptr, cnt) \
   if (e == cudaSuccess) e = alloc(&(ptr), (cnt));
@@ -183,10 +185,12 @@ DV_API dv_ctx* dv_create(const dv_params* params, int64_t capacity, void* stream
   A(c->keys[1], cap);
   A(c->vals[0], cap);
   A(c->vals[1], cap);
-  A(c->hist, 256 * c->max_tiles);
+  const int64_t sort_words = 256 * c->npasses * (c->max_tiles + 1) + 64;
+  A(c->sort_state, sort_words);
   A(c->cell_start, c->ncells);
   A(c->cell_end, c->ncells);
-  A(c->scan_part, c->scan_part_cap);
+  A(c->look_state, look_tiles);
+  A(c->look_ctl, 4);
   A(c->dscan_part, c->scan_part_cap);
   A(c->red_part, c->red_cap);
   A(c->ired_part, c->red_cap);
@@ -200,7 +204,6 @@ DV_API dv_ctx* dv_create(const dv_params* params, int64_t capacity, void* stream
   A(c->near_S, cap);
   A(c->far_acc, cap * DV_MAX_FAR_CHUNKS);
   A(c->mult, cap);
-  A(c->sflag, cap + 1);
   A(c->srank, cap + 1);
   A(c->sslot, cap);
   // neighbour lists: 48 (3-D, and 3 of padding) / 24 (2-D) entries per
@@ -225,6 +228,8 @@ DV_API dv_ctx* dv_create(const dv_params* params, int64_t capacity, void* stream
   if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_flag, sizeof(int32_t) * 4);
   if (e == cudaSuccess) e = cudaMemset(c->d_cnt, 0, sizeof(dv_counters));
   if (e == cudaSuccess) e = cudaMemset(c->d_flag, 0, sizeof(int32_t) * 4);
+  if (e == cudaSuccess) e = cudaMemset(c->look_state, 0, sizeof(unsigned long long) * look_tiles);
+  if (e == cudaSuccess) e = cudaMemset(c->look_ctl, 0, 4 * sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMemset(c->d_prof, 0, sizeof(double) * 4);
   if (e == cudaSuccess) e = cudaMemset(c->d_nbr_ok, 0, 3 * sizeof(int32_t));
   if (e == cudaSuccess) e = cudaMemset(c->cell_start, 0, sizeof(int32_t) * c->ncells);
@@ -376,25 +381,84 @@ __global__ void k_scan_down(const T* __restrict__ in, T* __restrict__ out, int64
   }
 }
 
-template <typename T>
-static int scan_impl(dv_ctx* c, const T* in, T* out, int64_t m, T* part) {
+int dv_scan_f64(dv_ctx* c, const double* in, double* out, int64_t m) {
   if (m <= 0) return DV_OK;
   int64_t nb = (m + SCAN_TILE - 1) / SCAN_TILE;
   if (nb > c->scan_part_cap) return dv_fail(c, DV_ECAPACITY, "scan of %lld elements too large", (long long)m);
-  k_scan_reduce<T><<<(unsigned)nb, SCAN_T, 0, c->stream>>>(in, m, part);
+  k_scan_reduce<double><<<(unsigned)nb, SCAN_T, 0, c->stream>>>(in, m, c->dscan_part);
   DV_LAUNCHED(c);
-  k_scan_top<T><<<1, SCAN_T, 0, c->stream>>>(part, (int)nb);
+  k_scan_top<double><<<1, SCAN_T, 0, c->stream>>>(c->dscan_part, (int)nb);
   DV_LAUNCHED(c);
-  k_scan_down<T><<<(unsigned)nb, SCAN_T, 0, c->stream>>>(in, out, m, part);
+  k_scan_down<double><<<(unsigned)nb, SCAN_T, 0, c->stream>>>(in, out, m, c->dscan_part);
   DV_LAUNCHED(c);
   return DV_OK;
 }
 
-int dv_scan_u32(dv_ctx* c, const uint32_t* in, uint32_t* out, int64_t m) {
-  return scan_impl<uint32_t>(c, in, out, m, c->scan_part);
+// uint32: one launch, 8 consecutive elements a thread.
+template <int T>
+__global__ void __launch_bounds__(T) k_scan_u32(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, int m,
+                                                  unsigned long long* state, uint32_t* ctl, dv_counters* C) {
+  constexpr int W = T / 32;
+  __shared__ uint32_t s_w[W];
+  const int tile = look_tile(ctl), tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int64_t e0 = (int64_t)tile * (8 * T) + 8 * tid;
+  uint32_t v[8];
+  uint32_t sum = 0;
+  if (e0 + 8 <= m) {
+    const uint4 a = reinterpret_cast<const uint4*>(in + e0)[0], b = reinterpret_cast<const uint4*>(in + e0)[1];
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+  } else {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = e0 + k < m ? in[e0 + k] : 0u;
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) sum += v[k];
+  uint32_t inc = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
+  }
+  if (lane == 31) s_w[w] = inc;
+  __syncthreads();
+  uint32_t before = 0, total = 0;
+#pragma unroll
+  for (int k = 0; k < W; ++k) {
+    before += k < w ? s_w[k] : 0u;
+    total += s_w[k];
+  }
+  uint32_t run = look_prefix<T>(state, tile, total, &C->status) + before + inc - sum;
+  if (e0 + 8 <= m) {
+    uint32_t o[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      o[k] = run;
+      run += v[k];
+    }
+    reinterpret_cast<uint4*>(out + e0)[0] = make_uint4(o[0], o[1], o[2], o[3]);
+    reinterpret_cast<uint4*>(out + e0)[1] = make_uint4(o[4], o[5], o[6], o[7]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (e0 + k < m) out[e0 + k] = run;
+      run += v[k];
+    }
+  }
+  look_end(state, ctl);
 }
-int dv_scan_f64(dv_ctx* c, const double* in, double* out, int64_t m) {
-  return scan_impl<double>(c, in, out, m, c->dscan_part);
+
+// in and out start on 16 bytes (both are whole allocations here)
+int dv_scan_u32(dv_ctx* c, const uint32_t* in, uint32_t* out, int64_t m) {
+  if (m <= 0) return DV_OK;
+  if (m > c->cap + 1) return dv_fail(c, DV_ECAPACITY, "scan of %lld elements too large", (long long)m);
+  if (look_wide(m))
+    k_scan_u32<1024><<<(unsigned)((m + 8191) / 8192), 1024, 0, c->stream>>>(in, out, (int)m, c->look_state,
+                                                                           c->look_ctl, c->d_cnt);
+  else
+    k_scan_u32<256><<<(unsigned)((m + 2047) / 2048), 256, 0, c->stream>>>(in, out, (int)m, c->look_state, c->look_ctl,
+                                                                         c->d_cnt);
+  DV_LAUNCHED(c);
+  return DV_OK;
 }
 
 __global__ void k_finalize_sum(const double* __restrict__ parts, int nparts, double* dst) {

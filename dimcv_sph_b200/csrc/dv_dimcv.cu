@@ -7,6 +7,7 @@
 #include <algorithm>
 
 #include "dv_internal.cuh"
+#include "dv_lookback.cuh"
 
 #define FOR_I                                    \
   int i = blockIdx.x * blockDim.x + threadIdx.x; \
@@ -209,64 +210,58 @@ __global__ void k_kvn_sample(dv_params P, dv_fields F, dv_solver_fields S,
 }
 
 // ------------------------------------------------------ compaction helpers
-__global__ void k_flag_samples(const dv_fields F, const dv_counters* __restrict__ C, int m,
-                               uint32_t* __restrict__ flags) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  flags[i] = (i < C->n && F.is_sample[i] == 1) ? 1u : 0u;
+// Lists of slots in ascending order, one launch each (look_compact); flags,
+// a scan of three launches, a compaction and a count before.
+template <int T>
+__global__ void __launch_bounds__(T) k_sample_list(const dv_fields F, dv_counters* C, int m,
+                                                     unsigned long long* state, uint32_t* ctl,
+                                                     int32_t* __restrict__ out) {
+  const int n = C->n;
+  look_compact<T, false>(
+      m, state, ctl, &C->status, nullptr, &C->num_samples, [&](int i) { return i < n && F.is_sample[i] == 1; },
+      [&](int i, uint32_t pos) { out[pos] = i; });
 }
 
-// CHECK: also tell the far field on boxes of a target outside its sorted box
-template <int D, bool CHECK>
-__global__ void k_flag_targets(dv_params P, const dv_fields F, const dv_counters* __restrict__ C,
-                               int m, uint32_t* __restrict__ flags, DevGrid G, const uint32_t* __restrict__ keys,
-                               dv_farbox B) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  uint32_t f = 0;
-  if (i < C->n && F.material[i] == DV_MATERIAL_FLUID) {
-    const V3 x = ldv<D>(F.x, i);
-    f = in_vortex_domain<D>(P, x) ? 1u : 0u;
-    if (CHECK && f && !in_sorted_box(P, G, x, keys[i], B.lowbits)) B.meta[0] = 1u;
-  }
-  flags[i] = f;
-}
-
-__global__ void k_compact(const uint32_t* __restrict__ flags, const uint32_t* __restrict__ offs,
-                          int m, int32_t* __restrict__ out) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  if (flags[i]) out[offs[i]] = i;
-}
-
-// count = offs[n] (the scan covers [0, m) with flags[n..m) = 0)
-__global__ void k_store_count(const uint32_t* __restrict__ offs, dv_counters* C, int which) {
-  int c = (int)offs[C->n];
-  if (which == 0)
-    C->num_samples = c;
-  else
-    C->n_targets = c;
+// CHECK: also tell the far field on boxes of a target outside its sorted box,
+// and keep every slot's place (offs)
+template <int D, bool CHECK, int T>
+__global__ void __launch_bounds__(T) k_target_list(dv_params P, const dv_fields F, dv_counters* C, int m,
+                                                     unsigned long long* state, uint32_t* ctl,
+                                                     int32_t* __restrict__ out, uint32_t* __restrict__ offs, DevGrid G,
+                                                     const uint32_t* __restrict__ keys, dv_farbox B) {
+  const int n = C->n;
+  look_compact<T, CHECK>(
+      m, state, ctl, &C->status, offs, &C->n_targets,
+      [&](int i) {
+        if (i >= n || F.material[i] != DV_MATERIAL_FLUID) return false;
+        if (!CHECK && !P.has_vortex_domain) return true;
+        const V3 x = ldv<D>(F.x, i);
+        if (!in_vortex_domain<D>(P, x)) return false;
+        if (CHECK && !in_sorted_box(P, G, x, keys[i], B.lowbits)) B.meta[0] = 1u;
+        return true;
+      },
+      [&](int i, uint32_t pos) { out[pos] = i; });
 }
 
 // Fills c->targets with the slots of fluid particles inside the vortex
 // domain, in ascending slot order; count in C->n_targets.
 int dv_build_targets(dv_ctx* c, const dv_fields* f, bool check) {
   const int m = (int)std::min<int64_t>(c->n_upper, c->cap) + 1;
-  const int nb = dv_blocks(m);
+  const int nb = look_blocks(m);
   const DevGrid G = dv_grid_cells(c);
   const uint32_t* keys = c->keys[c->perm_buf];
+#define TLT(DD, CH, T)                                                                                          \
+  k_target_list<DD, CH, T><<<nb, T, 0, c->stream>>>(c->p, *f, c->d_cnt, m, c->look_state, c->look_ctl, c->targets, \
+                                                    c->offs, G, keys, c->farbox)
+#define TL(DD, CH) look_wide(m) ? TLT(DD, CH, 1024) : TLT(DD, CH, 256)
   if (c->p.dim == 2)
-    k_flag_targets<2, false><<<nb, DV_THREADS, 0, c->stream>>>(c->p, *f, c->d_cnt, m, c->flags, G, keys, c->farbox);
+    TL(2, false);
   else if (check)
-    k_flag_targets<3, true><<<nb, DV_THREADS, 0, c->stream>>>(c->p, *f, c->d_cnt, m, c->flags, G, keys, c->farbox);
+    TL(3, true);
   else
-    k_flag_targets<3, false><<<nb, DV_THREADS, 0, c->stream>>>(c->p, *f, c->d_cnt, m, c->flags, G, keys, c->farbox);
-  DV_LAUNCHED(c);
-  int rc = dv_scan_u32(c, c->flags, c->offs, m);
-  if (rc) return rc;
-  k_compact<<<nb, DV_THREADS, 0, c->stream>>>(c->flags, c->offs, m, c->targets);
-  DV_LAUNCHED(c);
-  k_store_count<<<1, 1, 0, c->stream>>>(c->offs, c->d_cnt, 1);
+    TL(3, false);
+#undef TL
+#undef TLT
   DV_LAUNCHED(c);
   return DV_OK;
 }
@@ -638,15 +633,13 @@ DV_API int dv_record_samples(dv_ctx* c, const dv_fields* f, const dv_solver_fiel
   if (!c || !f) return DV_EINVAL;
   if (int rc = check_solver(c, s)) return rc;
   c->host_samples = -1;
-  const int m = (int)std::min<int64_t>(c->n_upper, c->cap) + 1;
-  const int nb = dv_blocks(m);
-  k_flag_samples<<<nb, DV_THREADS, 0, c->stream>>>(*f, c->d_cnt, m, c->flags);
-  DV_LAUNCHED(c);
-  int rc = dv_scan_u32(c, c->flags, c->offs, m);
-  if (rc) return rc;
-  k_compact<<<nb, DV_THREADS, 0, c->stream>>>(c->flags, c->offs, m, s->sample_idx);
-  DV_LAUNCHED(c);
-  k_store_count<<<1, 1, 0, c->stream>>>(c->offs, c->d_cnt, 0);
+  const int m = (int)std::min<int64_t>(c->n_upper, c->cap);
+  if (look_wide(m))
+    k_sample_list<1024><<<look_blocks(m), 1024, 0, c->stream>>>(*f, c->d_cnt, m, c->look_state, c->look_ctl,
+                                                               s->sample_idx);
+  else
+    k_sample_list<256><<<look_blocks(m), 256, 0, c->stream>>>(*f, c->d_cnt, m, c->look_state, c->look_ctl,
+                                                             s->sample_idx);
   DV_LAUNCHED(c);
   return DV_OK;
 }

@@ -651,17 +651,15 @@ __global__ void __launch_bounds__(kNearT, 2) k_box_near(dv_params P, dv_farbox B
 }
 
 // The distinct samples in slot order with their multiplicity folded into the
-// weight, and the slot list that k_far_fix reads.  A sample that has left the
+// weight.  A sample that has left the
 // box of its sorted cell, or a weight that is not of ordinary size, sends the
 // call to the direct loop.
 __global__ void k_box_pack(dv_params P, dv_fields F, dv_solver_fields S, DevGrid G, const uint32_t* __restrict__ keys,
                            const int32_t* __restrict__ mult, int nu, const uint32_t* __restrict__ rank, int lowbits,
-                           int32_t* __restrict__ slot, dv_farbox B) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nu; j += gridDim.x * blockDim.x) {
-    const int m = mult[j];
-    if (m <= 0) continue;
-    const uint32_t r = rank[j];
-    slot[r] = j;
+                           const int32_t* __restrict__ slot, dv_farbox B) {
+  const int ns = (int)rank[nu];
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < ns; r += gridDim.x * blockDim.x) {
+    const int j = slot[r], m = mult[j];
     const V3 x = ldv<3>(F.x, j);
     const V3 w = ld4(S.d_vort_smoothed, j);
     const float inv = 1.0f / (S.kden[j] + P.kden_eps);

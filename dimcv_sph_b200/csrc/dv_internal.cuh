@@ -57,7 +57,9 @@ struct dv_ctx {
   // grid / sort
   uint32_t* keys[2] = {nullptr, nullptr};
   uint32_t* vals[2] = {nullptr, nullptr};
-  uint32_t* hist = nullptr;  // 256 * max_tiles
+  // radix sort: [0, 256 * npasses) digit counts of every pass, then a ticket
+  // per pass (padded to 64 words), then per pass the (tile, digit) states
+  uint32_t* sort_state = nullptr;
   int64_t max_tiles = 0;
   int32_t* cell_start = nullptr;
   int32_t* cell_end = nullptr;
@@ -69,7 +71,8 @@ struct dv_ctx {
   uint32_t* mt[3] = {nullptr, nullptr, nullptr};  // per-axis Morton tables
 
   // scans and reductions
-  uint32_t* scan_part = nullptr;  // uint32 block partials
+  unsigned long long* look_state = nullptr;  // one-launch scans (dv_lookback.cuh): a word per tile, zero between launches
+  uint32_t* look_ctl = nullptr;              // [0] ticket, [1] blocks done
   double* dscan_part = nullptr;   // double block partials
   int64_t scan_part_cap = 0;
   double* red_part = nullptr;     // FP64 per-block partials of sweeps
@@ -93,8 +96,7 @@ struct dv_ctx {
   float* near_S = nullptr;     // cap
   float4* far_acc = nullptr;   // cap: far-field sums of the main loop, per target
   int32_t* mult = nullptr;     // cap: sample multiplicity per slot
-  uint32_t* sflag = nullptr;   // cap + 1: 1 where mult > 0
-  uint32_t* srank = nullptr;   // cap + 1: exclusive scan of sflag (sampled slots before a slot)
+  uint32_t* srank = nullptr;   // cap + 1: sampled slots before a slot
   int32_t* sslot = nullptr;    // cap: the sampled slots in slot order, srank[j] -> j
   int far_tt = 4;              // targets per thread of the far-field main loop (autotuned)
   int far_chunks = 1;          // sample chunks of the far-field grid (autotuned, <= DV_MAX_FAR_CHUNKS)
@@ -252,8 +254,9 @@ int dv_farbox_plan(dv_ctx* c);
 int dv_farbox_run(dv_ctx* c, const dv_fields* f);
 
 // ------------------------------------------------------------- scan helpers
-// Exclusive scan of uint32 / double arrays on the context stream
-// (deterministic three-phase: block reduce, scan of partials, block scan).
+// Exclusive scan of uint32 / double arrays on the context stream (uint32: one
+// launch, dv_lookback.cuh; double: deterministic three-phase block reduce,
+// scan of partials, block scan).
 int dv_scan_u32(dv_ctx* c, const uint32_t* in, uint32_t* out, int64_t m);
 int dv_scan_f64(dv_ctx* c, const double* in, double* out, int64_t m);
 // Sum of `nparts` FP64 partials into *dst (device), one block, fixed order.

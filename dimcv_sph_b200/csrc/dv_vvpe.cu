@@ -15,6 +15,7 @@
 
 #include "dv_far.cuh"
 #include "dv_internal.cuh"
+#include "dv_lookback.cuh"
 
 int dv_launch_vvpe_near(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s);
 
@@ -378,28 +379,26 @@ __global__ void k_mult(const int32_t* __restrict__ sample_idx, const dv_counters
 // [s, e) of a cell are sslot[srank[s] .. srank[e]), in slot order, so the
 // correction kernel reads a cell's few samples instead of testing every
 // particle's multiplicity.
-__global__ void k_sample_flags(const int32_t* __restrict__ mult, int nu, uint32_t* __restrict__ flag) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j <= nu; j += gridDim.x * blockDim.x)
-    flag[j] = (j < nu && mult[j] > 0) ? 1u : 0u;
+template <int T>
+__global__ void __launch_bounds__(T) k_sample_slots(const int32_t* __restrict__ mult, int nu, dv_counters* C,
+                                                      unsigned long long* state, uint32_t* ctl,
+                                                      uint32_t* __restrict__ rank, int32_t* __restrict__ slot) {
+  look_compact<T, true>(
+      nu + 1, state, ctl, &C->status, rank, nullptr, [&](int j) { return j < nu && mult[j] > 0; },
+      [&](int j, uint32_t pos) { slot[pos] = j; });
 }
 
-__global__ void k_sample_slots(const int32_t* __restrict__ mult, int nu, const uint32_t* __restrict__ rank,
-                               int32_t* __restrict__ slot) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nu; j += gridDim.x * blockDim.x)
-    if (mult[j] > 0) slot[rank[j]] = j;
-}
-
-// boxed: the slot list comes with the packed samples of the far field on boxes
+// boxed: also the packed samples of the far field on boxes
 static int sample_slots(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s, bool boxed = false) {
   const int nu = (int)std::min<int64_t>(c->n_upper, c->cap);
-  k_sample_flags<<<c->num_sms * 4, DV_THREADS, 0, c->stream>>>(c->mult, nu, c->sflag);
+  if (look_wide(nu + 1))
+    k_sample_slots<1024><<<look_blocks(nu + 1), 1024, 0, c->stream>>>(c->mult, nu, c->d_cnt, c->look_state,
+                                                                      c->look_ctl, c->srank, c->sslot);
+  else
+    k_sample_slots<256><<<look_blocks(nu + 1), 256, 0, c->stream>>>(c->mult, nu, c->d_cnt, c->look_state,
+                                                                    c->look_ctl, c->srank, c->sslot);
   DV_LAUNCHED(c);
-  int rc = dv_scan_u32(c, c->sflag, c->srank, (int64_t)nu + 1);
-  if (rc) return rc;
-  if (boxed) return dv_farbox_pack(c, f, s, nu);
-  k_sample_slots<<<c->num_sms * 4, DV_THREADS, 0, c->stream>>>(c->mult, nu, c->srank, c->sslot);
-  DV_LAUNCHED(c);
-  return DV_OK;
+  return boxed ? dv_farbox_pack(c, f, s, nu) : DV_OK;
 }
 
 // cell window of a target that contains every particle within h: the 3^d

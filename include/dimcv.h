@@ -64,6 +64,7 @@ enum dv_status {
 #define DV_WARN_CAPACITY (1 << 3)          /* emission clamped at capacity (particle_system.py:361) */
 #define DV_WARN_NAN (1 << 4)               /* a non-finite error norm was seen in a solve */
 #define DV_WARN_BAD_INDEX (1 << 5)         /* an injected sample index was outside [0, n): ignored */
+#define DV_WARN_WAIT (1 << 6)              /* a bounded wait between blocks ran out (never expected) */
 
 /* Sampling modes of dv_sample (new: the reference only has the Bernoulli
  * birth/death process of dimcv_sph.py:305-335). */
