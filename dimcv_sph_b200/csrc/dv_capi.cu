@@ -118,7 +118,7 @@ DV_API void dv_destroy(dv_ctx* c) {
                   c->look_state, c->look_ctl, c->dscan_part, c->red_part, c->ired_part, c->flags, c->offs,
                   c->targets, c->cdf,       c->spos,      c->sw,        c->near_v,  c->near_S,
                   c->far_acc, c->mult,      c->nbr_off,   c->nbr_idx,   c->d_nbr_ok,
-                  c->nbr_rows, c->srank,     c->sslot,   c->nbr_len,   c->pk_a,    c->pk_b,
+                  c->srank,     c->sslot,   c->nbr_len,   c->pk_a,    c->pk_b,
                   c->pk_k};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -175,7 +175,7 @@ DV_API dv_ctx* dv_create(const dv_params* params, int64_t capacity, void* stream
   c->max_tiles = (cap + 2047) / 2048 + 1;
   c->red_cap = (cap + 127) / 128 + 1024;
   c->scan_part_cap = (cap + 1 + 4095) / 4096 + 1024;
-  const int64_t look_tiles = (cap + 1 + 255) / 256 + 64;  // tiles of 256 elements at least
+  const int64_t look_tiles = (cap + 1 + 63) / 64 + 64;  // tiles of 64 elements at least
   cudaError_t e = cudaSuccess;
 #define A(ptr, cnt) \
   if (e == cudaSuccess) e = alloc(&(ptr), (cnt));
@@ -206,9 +206,10 @@ DV_API dv_ctx* dv_create(const dv_params* params, int64_t capacity, void* stream
   A(c->mult, cap);
   A(c->srank, cap + 1);
   A(c->sslot, cap);
-  // neighbour lists: 48 (3-D, and 3 of padding) / 24 (2-D) entries per
-  // particle on average, beyond which the sweeps keep scanning cells
-  c->nbr_cap = cap * (params->dim == 3 ? 51 : 24);
+  // neighbour lists: 24 entries per particle on average in 2-D; a row per
+  // particle and 51 entries per particle on average for the longer rows in
+  // 3-D; beyond that the sweeps keep scanning cells
+  c->nbr_cap = params->dim == 3 ? 4 * nbr_row0(cap + 31 & ~(int64_t)31) + (51 * cap & ~(int64_t)3) : cap * 24;
   A(c->nbr_off, cap + 1);
   if (params->dim == 3) {
     A(c->nbr_len, cap);
@@ -217,11 +218,7 @@ DV_API dv_ctx* dv_create(const dv_params* params, int64_t capacity, void* stream
     A(c->pk_k, cap);
   }
   A(c->nbr_idx, c->nbr_cap);
-  A(c->d_nbr_ok, 3);  // [0]: lists valid, [1]: keys valid, [2]: a material other than fluid / solid seen by the build
-  // the 3-D build's first pass stores up to 64 neighbours per particle in
-  // fixed rows (a settled lattice has at most 36); 2-D builds have none
-  c->nbr_slots = params->dim == 3 ? 64 : 0;
-  if (c->nbr_slots) A(c->nbr_rows, cap * c->nbr_slots);
+  A(c->d_nbr_ok, 2);  // [0]: lists valid, [1]: keys valid
   A(c->d_prof, 4);
 #undef A
   if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_cnt, sizeof(dv_counters));
@@ -231,7 +228,7 @@ DV_API dv_ctx* dv_create(const dv_params* params, int64_t capacity, void* stream
   if (e == cudaSuccess) e = cudaMemset(c->look_state, 0, sizeof(unsigned long long) * look_tiles);
   if (e == cudaSuccess) e = cudaMemset(c->look_ctl, 0, 4 * sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMemset(c->d_prof, 0, sizeof(double) * 4);
-  if (e == cudaSuccess) e = cudaMemset(c->d_nbr_ok, 0, 3 * sizeof(int32_t));
+  if (e == cudaSuccess) e = cudaMemset(c->d_nbr_ok, 0, 2 * sizeof(int32_t));
   if (e == cudaSuccess) e = cudaMemset(c->cell_start, 0, sizeof(int32_t) * c->ncells);
   if (e == cudaSuccess) e = cudaMemset(c->cell_end, 0, sizeof(int32_t) * c->ncells);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();

@@ -6,6 +6,7 @@
 // and CSR neighbour lists.
 #include <algorithm>
 
+#include "dv_far.cuh"
 #include "dv_internal.cuh"
 #include "dv_lookback.cuh"
 
@@ -306,7 +307,8 @@ __global__ void k_permute(dv_fields S, dv_fields T, const uint32_t* __restrict__
 }
 
 __global__ void k_finalize_counts(const int32_t* __restrict__ part, int nparts,
-                                  const int32_t* __restrict__ n_new_p, dv_counters* C) {
+                                  const int32_t* __restrict__ n_new_p, dv_counters* C, int32_t* ok,
+                                  uint32_t* far_used) {
   int fl = 0, so = 0;
   for (int k = threadIdx.x; k < nparts; k += blockDim.x) {
     fl += part[2 * k];
@@ -318,6 +320,9 @@ __global__ void k_finalize_counts(const int32_t* __restrict__ part, int nparts,
     C->n = *n_new_p;
     C->n_fluid = fl;
     C->n_solid = so;
+    ok[0] = 1;  // until the list build finds otherwise
+    ok[1] = 1;  // the sorted keys are those of the current slots
+    *far_used = 0u;
   }
 }
 
@@ -327,149 +332,274 @@ __global__ void k_finalize_counts(const int32_t* __restrict__ part, int nparts,
 // sweeps read the lists as CSR (offsets = exclusive scan of the counts).
 //
 // Each entry carries the neighbour's material in its top bit (DV_NBR_SOLID),
-// so the sweeps do not gather it; a material other than fluid or solid sets
-// bad[0] and the lists are not used.
+// so the sweeps do not gather it; a material other than fluid or solid makes
+// the lists invalid.
 //
 // Rows of static solids stay empty: every neighbour walk of the step has a
 // fluid particle (or, for the rigid coupling, a dynamic solid) at its centre,
 // and the static boundary volume (once, at initialisation) scans cells.
 //
-// 3-D (27 cells, ~8 candidates each): one cell-scan pass stores each
-// particle's first `slots` neighbours in its own fixed row and its count; a
-// copy then moves the rows into CSR (a particle with more neighbours than
-// slots scans its cells again there).  CSR rows start and end on 16 bytes, so
-// that the sweeps read four entries a load.  This saves a second
-// 27-cell scan.  2-D (9 cells): counting is cheap and the fixed rows cost
-// more write traffic than they save, so a count pass and a fill pass.
+// One launch: k_csr_rows (3-D), k_csr_build (2-D).  k_finalize_counts has set
+// the lists valid before it; a build that cannot store them takes that back.
 __device__ __forceinline__ bool nbr_row_built(const int32_t* __restrict__ mat, const uint8_t* __restrict__ dyn,
                                               int i) {
   return !(mat[i] == DV_MATERIAL_SOLID && !dyn[i]);
 }
 
-__device__ __forceinline__ int32_t nbr_entry(int j, int mj, int32_t* bad) {
-  if (mj != DV_MATERIAL_FLUID && mj != DV_MATERIAL_SOLID) *bad = 1;
+__device__ __forceinline__ int32_t nbr_entry(int j, int mj, int32_t* ok) {
+  if (mj != DV_MATERIAL_FLUID && mj != DV_MATERIAL_SOLID) *ok = 0;
   return (int32_t)((uint32_t)j | (mj == DV_MATERIAL_SOLID ? DV_NBR_SOLID : 0u));
 }
 
-template <int D>
-__global__ void k_csr_count(dv_params P, DevGrid G, const float* __restrict__ x, const int32_t* __restrict__ mat,
-                            const uint8_t* __restrict__ dyn, const dv_counters* __restrict__ C, int m,
-                            uint32_t* __restrict__ cnt) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  uint32_t k = 0;
-  if (i < C->n && nbr_row_built(mat, dyn, i))
-    for_each_neighbor<D>(P, G, x, i, ldv<D>(x, i), [&](int, V3, float) { ++k; });
-  cnt[i] = k;
+// 3-D: a warp takes 32 slots, which lie in about five cells.  For each of these
+// cells, 27 lanes look up the neighbouring cells' ranges at once, the lanes
+// take the concatenated candidates 32 at a time (coalesced loads), and every
+// particle of the cell is tested against all 32 in one go, two particles per
+// f32x2 instruction; the ballot gives each accepted candidate its place, so
+// rows keep the visit order.  A thread per particle that tested candidate after
+// candidate was bound by the L1's passes over scattered loads and stores, and
+// needed a scan and a compaction of its rows: 0.75M particles 306 us in four
+// launches, now 193 in one; 2.02M 836, now 590.  Issue slots are 79% busy;
+// groups of 8 or 10 particles and fewer or more registers were level or slower.
+// Any material other than fluid or solid in the window of a built row makes
+// the lists invalid.
+constexpr int kCsrWarps = 8;  // of a block
+//
+// `one` is 1: the squares are added by an fma with it, which rounds as the
+// reference's addition does.  ptxas turned mul.rn.f32x2 and add.rn.f32x2 into
+// one fma, so that a pair at the support radius was missed.
+constexpr int kCsrGroup = 12;  // particles of a cell tested together (8 a cell on a lattice)
+__global__ void __launch_bounds__(kCsrWarps * 32) k_csr_rows(dv_params P, DevGrid G, const float* __restrict__ x,
+                                                             const int32_t* __restrict__ mat,
+                                                             const uint8_t* __restrict__ dyn,
+                                                             const dv_counters* __restrict__ C, float one,
+                                                             uint32_t far0,
+                                                             uint32_t far_cap, uint32_t* far_used,
+                                                             uint32_t* __restrict__ off, uint32_t* __restrict__ len,
+                                                             int32_t* ok, int32_t* __restrict__ out) {
+  __shared__ float4 s_t[kCsrWarps][kCsrGroup];  // pairs of particles: {x, x, y, y}, {z, z, row, row}
+  __shared__ int2 s_r[kCsrWarps][32];           // ranges that are not empty: {first candidate, slot - candidate}
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i = (blockIdx.x * kCsrWarps + w) * 32 + lane, n = C->n;
+  if (i - lane >= n) return;
+  const unsigned lt = (1u << lane) - 1u;
+  const bool live = i < n;
+  const V3 xi = live ? ldv<3>(x, i) : V3{0.f, 0.f, 0.f};
+  const unsigned built = __ballot_sync(0xffffffffu, live && nbr_row_built(mat, dyn, i));
+  const int c0 = cell_coord(P, xi.x, 0), c1 = cell_coord(P, xi.y, 1), c2 = cell_coord(P, xi.z, 2);
+  const uint32_t sk = G.scene && live ? ((uint32_t)__ldg(G.scene + i) << G.scene_shift) : 0u;
+  const int q0 = __shfl_up_sync(0xffffffffu, c0, 1), q1 = __shfl_up_sync(0xffffffffu, c1, 1);
+  const int q2 = __shfl_up_sync(0xffffffffu, c2, 1);
+  const uint32_t qs = __shfl_up_sync(0xffffffffu, sk, 1);
+  unsigned heads = __ballot_sync(0xffffffffu, q0 != c0 || q1 != c1 || q2 != c2 || qs != sk || lane == 0);
+  const float lim = P.nbr_r2_limit;
+  const f2_t ONE = f2_pack(one, one);
+  uint32_t mylen = 0;
+  bool bad = false;
+  while (heads) {
+    const int h = __ffs(heads) - 1;
+    heads &= heads - 1;
+    unsigned todo = built & (heads ? (1u << (__ffs(heads) - 1)) - 1u : 0xffffffffu) & ~((1u << h) - 1u);
+    if (!todo) continue;
+    const int g0 = __shfl_sync(0xffffffffu, c0, h), g1 = __shfl_sync(0xffffffffu, c1, h);
+    const int g2 = __shfl_sync(0xffffffffu, c2, h);
+    const uint32_t gs = __shfl_sync(0xffffffffu, sk, h);
+    int start = 0, cnt = 0;
+    if (lane < 27) {
+      const int gx = cell_step(P, g0, lane / 9 - 1, P.grid_num[0]);
+      const int gy = cell_step(P, g1, (lane / 3) % 3 - 1, P.grid_num[1]);
+      const int gz = cell_step(P, g2, lane % 3 - 1, P.grid_num[2]);
+      if (gx >= 0 && gy >= 0 && gz >= 0) {
+        const uint32_t key = __ldg(G.mt0 + gx) | __ldg(G.mt1 + gy) | __ldg(G.mt2 + gz);
+        if (!(P.skip_cell0 && key == 0u)) {  // the scene's own flat cell 0
+          start = __ldg(G.start + (key | gs));
+          cnt = __ldg(G.end + (key | gs)) - start;
+        }
+      }
+    }
+    int inc = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += u;
+    }
+    const int total = __shfl_sync(0xffffffffu, inc, 31);
+    const unsigned some = __ballot_sync(0xffffffffu, cnt > 0);
+    __syncwarp();
+    if (cnt > 0) s_r[w][__popc(some & lt)] = make_int2(inc - cnt, start - (inc - cnt));
+    __syncwarp();
+    const int2 rng = lane < __popc(some) ? s_r[w][lane] : make_int2(0x7fffffff, 0);
+    do {
+      const int rank = __popc(todo & lt);
+      const bool mine = ((todo >> lane) & 1u) && rank < kCsrGroup;
+      const int nt = min(__popc(todo), kCsrGroup);
+      todo &= ~__ballot_sync(0xffffffffu, mine);
+      if (mine) {
+        float* t = reinterpret_cast<float*>(&s_t[w][rank & ~1]) + (rank & 1);
+        t[0] = xi.x;
+        t[2] = xi.y;
+        t[4] = xi.z;
+        t[6] = __int_as_float((int)nbr_row0(i));
+      }
+      if (lane == 0 && (nt & 1)) reinterpret_cast<float*>(&s_t[w][nt - 1])[1] = INFINITY;  // no partner: never near
+      __syncwarp();
+      uint32_t k[kCsrGroup];
+#pragma unroll
+      for (int t = 0; t < kCsrGroup; ++t) k[t] = 0;
+      int before = 0;  // ranges that start before the 32 candidates
+#pragma unroll 1
+      for (int e0 = 0; e0 < total; e0 += 32) {
+        const int e = e0 + lane;
+        const unsigned starts =
+            __reduce_or_sync(0xffffffffu, rng.x >= e0 && rng.x < e0 + 32 ? 1u << (rng.x - e0) : 0u);
+        const int own = before + __popc(starts & (lt | (1u << lane))) - 1;
+        before += __popc(starts);
+        const int j = e + __shfl_sync(0xffffffffu, rng.y, own);
+        const bool valid = e < total;
+        V3 xj{INFINITY, INFINITY, INFINITY};
+        int mj = DV_MATERIAL_FLUID;
+        if (valid) {
+          xj = ldv<3>(x, j);
+          mj = __ldg(mat + j);
+        }
+        const int rj = (int)nbr_row0(j);  // tells j from the particle as well as the slot does
+        const int32_t entry = (int32_t)((uint32_t)j | (mj == DV_MATERIAL_SOLID ? DV_NBR_SOLID : 0u));
+        bad |= mj != DV_MATERIAL_FLUID && mj != DV_MATERIAL_SOLID;
+        const f2_t CX = f2_pack(xj.x, xj.x), CY = f2_pack(xj.y, xj.y), CZ = f2_pack(xj.z, xj.z);
+#pragma unroll
+        for (int p = 0; p < kCsrGroup; p += 2) {
+          if (p < nt) {
+            const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(&s_t[w][p]);
+            const float4 zs = s_t[w][p + 1];
+            const f2_t DX = f2_sub(u.x, CX), DY = f2_sub(u.y, CY), DZ = f2_sub(f2_pack(zs.x, zs.y), CZ);
+            float r2[2];
+            if (!P.periodic) {
+              f2_unpack(f2_fma(f2_mul(DZ, DZ), ONE, f2_fma(f2_mul(DY, DY), ONE, f2_mul(DX, DX))), r2[0], r2[1]);
+            } else {
+              V3 a, b;
+              f2_unpack(DX, a.x, b.x);
+              f2_unpack(DY, a.y, b.y);
+              f2_unpack(DZ, a.z, b.z);
+              r2[0] = sqnorm<3>(V3{min_image(a.x, P.box[0]), min_image(a.y, P.box[1]), min_image(a.z, P.box[2])});
+              r2[1] = sqnorm<3>(V3{min_image(b.x, P.box[0]), min_image(b.y, P.box[1]), min_image(b.z, P.box[2])});
+            }
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              const int row = __float_as_int(q ? zs.w : zs.z);
+              const bool acc = r2[q] < lim && rj != row;
+              const unsigned hit = __ballot_sync(0xffffffffu, acc);
+              const uint32_t at = k[p + q] + __popc(hit & lt);
+              if (acc && at < kNbrRow) (out + 4 * (int64_t)(uint32_t)row)[at + 124u * (at >> 2)] = entry;
+              k[p + q] += __popc(hit);
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < kCsrGroup; ++t)
+        if (mine && rank == t) mylen = k[t];
+      __syncwarp();  // s_t is read
+    } while (todo);
+  }
+  if (!live) return;
+  uint32_t at = (uint32_t)nbr_row0(i);
+  if (mylen <= kNbrRow) {
+    for (uint32_t e = mylen; e & 3u; ++e) out[4 * ((int64_t)at + 32 * (e >> 2)) + (e & 3u)] = i;
+  } else {
+    const uint32_t room = (mylen + 3u) / 4u, a = atomicAdd(far_used, room);
+    if (a + room <= far_cap) {
+      at = far0 + a;
+      int64_t e = 4 * (int64_t)at;
+      for_each_neighbor_m<3>(P, G, x, mat, i, xi,
+                             [&](int j, V3, float, int mj) { out[e++] = nbr_entry(j, mj, ok); });
+      while (e & 3) out[e++] = i;
+    } else {
+      bad = true;  // no room: the sweeps scan cells
+    }
+  }
+  off[i] = at;
+  len[i] = mylen;
+  if (bad) ok[0] = 0;
 }
 
-template <int D>
-__global__ void k_csr_fill(dv_params P, DevGrid G, const float* __restrict__ x,
-                           const int32_t* __restrict__ mat, const dv_counters* __restrict__ C,
-                           const uint32_t* __restrict__ off, int32_t* __restrict__ ok,
-                           int32_t* __restrict__ out, const uint8_t* __restrict__ dyn) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= C->n || !ok[0] || !nbr_row_built(mat, dyn, i)) return;
-  uint32_t k = off[i];
-  for_each_neighbor_m<D>(P, G, x, mat, i, ldv<D>(x, i),
-                         [&](int j, V3, float, int mj) { out[k++] = nbr_entry(j, mj, ok + 2); });
-}
-
-template <int D>
-__global__ void k_csr_rows(dv_params P, DevGrid G, const float* __restrict__ x, const int32_t* __restrict__ mat,
-                           const uint8_t* __restrict__ dyn, const dv_counters* __restrict__ C, int m, int slots,
-                           uint32_t* __restrict__ room, uint32_t* __restrict__ len, int32_t* __restrict__ rows) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m) return;
+// 2-D: a block scans the cells of its particles (a thread each) into rows of
+// up to kCsrSlots entries in shared memory, scans the lengths (look-back over
+// the blocks before) and copies the rows out, eight lanes a row, the
+// neighbours' materials gathered on the way; a particle with more neighbours
+// (a settled lattice has at most 20) scans its cells again.  Counting, a scan
+// and filling, with two more launches for the checks, before: 10,000 particles
+// 33 -> 21 us, a batch of 340,000 70 -> 66.
+constexpr int kCsrSlots = 32;
+template <int T>
+__global__ void __launch_bounds__(T) k_csr_build(dv_params P, DevGrid G, const float* __restrict__ x,
+                                                 const int32_t* __restrict__ mat, const uint8_t* __restrict__ dyn,
+                                                 dv_counters* C, int m, int64_t cap, unsigned long long* state,
+                                                 uint32_t* ctl, uint32_t* __restrict__ off, int32_t* ok,
+                                                 int32_t* __restrict__ out) {
+  constexpr int ST = kCsrSlots + 1, W = T / 32;
+  __shared__ int32_t s_rows[T * ST];
+  __shared__ uint32_t s_w[W];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int tile = look_tile(ctl), i = tile * T + tid, n = C->n;
   uint32_t k = 0;
-  if (i < C->n && nbr_row_built(mat, dyn, i)) {
-    int32_t* row = rows + (int64_t)i * slots;
-    for_each_neighbor<D>(P, G, x, i, ldv<D>(x, i), [&](int j, V3, float) {
-      if (k < (uint32_t)slots) row[k] = j;
+  if (i < n && nbr_row_built(mat, dyn, i)) {
+    int32_t* row = s_rows + tid * ST;
+    for_each_neighbor<2>(P, G, x, i, ldv<2>(x, i), [&](int j, V3, float) {
+      if (k < (uint32_t)kCsrSlots) row[k] = j;
       ++k;
     });
   }
-  room[i] = (k + 3u) & ~3u;  // rows start on 16 bytes
-  if (i < m - 1) len[i] = k;
-}
-
-// one warp per group of 32 particles; eight lanes copy a row, four entries a
-// lane (16-byte loads of the row and stores of the CSR segment: four rows of
-// up to 32 entries at a time), and the neighbours' materials are gathered
-// here, independent loads, rather than in the row scan's dependent chain.
-// 0.75M particles: 77 -> 56 us against a row per warp and 4-byte copies.
-template <int D>
-__global__ void k_csr_compact(dv_params P, DevGrid G, const float* __restrict__ x, const int32_t* __restrict__ mat,
-                              const dv_counters* __restrict__ C, int slots, const int32_t* __restrict__ rows,
-                              const uint32_t* __restrict__ off, const uint32_t* __restrict__ len,
-                              int32_t* __restrict__ ok, int32_t* __restrict__ out) {
-  if (!ok[0]) return;
-  const int n = C->n;
-  const int lane = threadIdx.x & 31;
-  const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31;
-  const uint32_t l4 = 4u * (lane & 7);
-#pragma unroll 2
+  uint32_t inc = k;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
+  }
+  if (lane == 31) s_w[w] = inc;
+  __syncthreads();
+  uint32_t before = 0, total = 0;
+#pragma unroll
+  for (int q = 0; q < W; ++q) {
+    before += q < w ? s_w[q] : 0u;
+    total += s_w[q];
+  }
+  const uint32_t at = look_prefix<T>(state, tile, total, &C->status) + before + inc - k;
+  if (i < m) off[i] = at;
+  if (i == n && (int64_t)at > cap) ok[0] = 0;  // too long for the buffer: the sweeps scan cells
+  __syncwarp();
   for (int g = 0; g < 32; g += 4) {
-    const int i = i0 + g + (lane >> 3);
-    if (i >= n) break;
-    const uint32_t k0 = off[i], cnt = len[i];
-    if (cnt <= (uint32_t)slots) {
-      const int4* row = reinterpret_cast<const int4*>(rows + (int64_t)i * slots);
-      for (uint32_t k = l4; k < cnt; k += 32) {
-        const int4 q = row[k >> 2];
-        int4 e;  // past the row's end: padding with a valid slot
-        e.x = nbr_entry(q.x, __ldg(mat + q.x), ok + 2);
-        e.y = k + 1 < cnt ? nbr_entry(q.y, __ldg(mat + q.y), ok + 2) : i;
-        e.z = k + 2 < cnt ? nbr_entry(q.z, __ldg(mat + q.z), ok + 2) : i;
-        e.w = k + 3 < cnt ? nbr_entry(q.w, __ldg(mat + q.w), ok + 2) : i;
-        *reinterpret_cast<int4*>(out + k0 + k) = e;
-      }
+    const int r = g + (lane >> 3), ir = tile * T + 32 * w + r;
+    const uint32_t cnt = __shfl_sync(0xffffffffu, k, r), o = __shfl_sync(0xffffffffu, at, r);
+    if (cnt == 0 || (int64_t)o + cnt > cap) continue;
+    const int32_t* row = s_rows + (32 * w + r) * ST;
+    if (cnt <= (uint32_t)kCsrSlots) {
+      for (uint32_t e = lane & 7; e < cnt; e += 8) out[o + e] = nbr_entry(row[e], __ldg(mat + row[e]), ok);
     } else if ((lane & 7) == 0) {
-      uint32_t k = k0;
-      for_each_neighbor_m<D>(P, G, x, mat, i, ldv<D>(x, i),
-                             [&](int j, V3, float, int mj) { out[k++] = nbr_entry(j, mj, ok + 2); });
-      while (k & 3u) out[k++] = i;
+      uint32_t e = o;
+      for_each_neighbor_m<2>(P, G, x, mat, ir, ldv<2>(x, ir),
+                             [&](int j, V3, float, int mj) { out[e++] = nbr_entry(j, mj, ok); });
     }
   }
-}
-
-__global__ void k_csr_ok(const uint32_t* __restrict__ off, const dv_counters* __restrict__ C, int64_t cap,
-                         int32_t* __restrict__ ok) {
-  ok[0] = (int64_t)off[C->n] <= cap ? 1 : 0;
-  ok[1] = 1;  // the sorted keys are those of the current slots
-}
-
-// after the fill: lists that met a material other than fluid or solid are
-// not used (their entries cannot encode it)
-__global__ void k_csr_material_check(int32_t* __restrict__ ok) {
-  if (ok[2]) ok[0] = 0;
+  look_end(state, ctl);
 }
 
 static int build_csr(dv_ctx* c, const dv_fields* f) {
   const int m = (int)std::min<int64_t>(c->n_upper, c->cap) + 1;
-  const int nb = dv_blocks(m);
   DevGrid G = dv_grid_cells(c);
-  const bool rows = c->p.dim == 3;
-  DV_CK(c, cudaMemsetAsync(c->d_nbr_ok + 2, 0, sizeof(int32_t), c->stream));
-  if (rows)
-    k_csr_rows<3><<<nb, DV_THREADS, 0, c->stream>>>(c->p, G, f->x, f->material, f->is_dynamic, c->d_cnt, m,
-                                                    c->nbr_slots, c->flags, c->nbr_len, c->nbr_rows);
+#define CSR2(T)                                                                                                     \
+  k_csr_build<T><<<dv_blocks(m, T), T, 0, c->stream>>>(c->p, G, f->x, f->material, f->is_dynamic, c->d_cnt, m,       \
+                                                       c->nbr_cap, c->look_state, c->look_ctl, c->nbr_off, c->d_nbr_ok, \
+                                                       c->nbr_idx)
+  if (c->p.dim == 3)
+    k_csr_rows<<<dv_blocks(m, kCsrWarps * 32), kCsrWarps * 32, 0, c->stream>>>(
+        c->p, G, f->x, f->material, f->is_dynamic, c->d_cnt, 1.0f, (uint32_t)nbr_row0(c->cap + 31 & ~(int64_t)31),
+        (uint32_t)(c->nbr_cap / 4 - nbr_row0(c->cap + 31 & ~(int64_t)31)), c->look_ctl + 2, c->nbr_off, c->nbr_len,
+        c->d_nbr_ok, c->nbr_idx);
+  else if (m <= 256 * c->num_sms)
+    CSR2(64);
   else
-    k_csr_count<2><<<nb, DV_THREADS, 0, c->stream>>>(c->p, G, f->x, f->material, f->is_dynamic, c->d_cnt, m,
-                                                     c->flags);
-  DV_LAUNCHED(c);
-  int rc = dv_scan_u32(c, c->flags, c->nbr_off, m);
-  if (rc) return rc;
-  k_csr_ok<<<1, 1, 0, c->stream>>>(c->nbr_off, c->d_cnt, c->nbr_cap, c->d_nbr_ok);
-  DV_LAUNCHED(c);
-  if (rows)
-    k_csr_compact<3><<<nb, DV_THREADS, 0, c->stream>>>(c->p, G, f->x, f->material, c->d_cnt, c->nbr_slots,
-                                                       c->nbr_rows, c->nbr_off, c->nbr_len, c->d_nbr_ok, c->nbr_idx);
-  else
-    k_csr_fill<2><<<nb, DV_THREADS, 0, c->stream>>>(c->p, G, f->x, f->material, c->d_cnt, c->nbr_off,
-                                                    c->d_nbr_ok, c->nbr_idx, f->is_dynamic);
-  DV_LAUNCHED(c);
-  k_csr_material_check<<<1, 1, 0, c->stream>>>(c->d_nbr_ok);
+    CSR2(256);
+#undef CSR2
   DV_LAUNCHED(c);
   return DV_OK;
 }
@@ -555,7 +685,8 @@ DV_API int dv_grid_build(dv_ctx* c, const dv_fields* src, const dv_fields* dst) 
     k_permute<3><<<nb, DV_THREADS, 0, c->stream>>>(*src, *dst, c->vals[cur], c->keys[cur],
                                                    c->d_flag + 1, (int)c->cap, c->d_cnt, c->ired_part);
   DV_LAUNCHED(c);
-  k_finalize_counts<<<1, 1024, 0, c->stream>>>(c->ired_part, nb, c->d_flag + 1, c->d_cnt);
+  k_finalize_counts<<<1, 1024, 0, c->stream>>>(c->ired_part, nb, c->d_flag + 1, c->d_cnt, c->d_nbr_ok,
+                                               c->look_ctl + 2);
   DV_LAUNCHED(c);
   c->scene_ptr = batch ? dst->object_id : nullptr;  // scene of each sorted slot
   return build_csr(c, dst);
@@ -675,8 +806,11 @@ __global__ void k_nbr_slots(const uint32_t* __restrict__ off, const uint32_t* __
                             int32_t* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const uint32_t a = off[i], m = len ? len[i] : off[i + 1] - a, o = out_off[i];
-  for (uint32_t k = 0; k < m; ++k) out[o + k] = nbr_slot((uint32_t)in[a + k]);
+  const uint32_t m = len ? len[i] : off[i + 1] - off[i], o = out_off[i];
+  const uint32_t a = off[i];
+  const int st = nbr_stride(m);
+  for (uint32_t k = 0; k < m; ++k)
+    out[o + k] = nbr_slot((uint32_t)in[len ? 4 * ((int64_t)a + st * (k >> 2)) + (k & 3u) : (int64_t)a + k]);
 }
 
 DV_API int64_t dv_stored_lists(dv_ctx* c, uint32_t* dev_offsets, int32_t* dev_nbrs, int64_t max_entries) {

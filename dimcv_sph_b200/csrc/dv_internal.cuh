@@ -102,17 +102,14 @@ struct dv_ctx {
   int far_chunks = 1;          // sample chunks of the far-field grid (autotuned, <= DV_MAX_FAR_CHUNKS)
   bool dyn_rigid = false;      // dynamic rigid particles present: pressure iterations add their reaction
 
-  // per-step neighbour lists (CSR, visit order) built by dv_grid_build; in 3-D
-  // every row starts at a multiple of 4 entries (16 bytes), is padded to one
-  // with entries of its own slot, and has its length in nbr_len
-  uint32_t* nbr_off = nullptr;  // cap + 1
+  // per-step neighbour lists (visit order) built by dv_grid_build: CSR in 2-D,
+  // nbr_at rows in 3-D with their lengths in nbr_len
+  uint32_t* nbr_off = nullptr;  // cap + 1: first entry of a row; 3-D: first quad
   uint32_t* nbr_len = nullptr;  // 3-D: cap
   int32_t* nbr_idx = nullptr;   // nbr_cap
   int64_t nbr_cap = 0;
   int32_t* d_nbr_ok = nullptr;  // [0]: 1 while the lists match the current positions; [1]: 1 while keys[perm_buf]
-                                // are the sorted slots' cell keys; [2]: build scratch
-  int32_t* nbr_rows = nullptr;  // 3-D: cap * nbr_slots, the first pass's fixed row of particle i at i * nbr_slots
-  int nbr_slots = 0;
+                                // are the sorted slots' cell keys
 
   dv_farbox farbox;
   int64_t host_samples = -1;  // sample count of the last draw where the host knows it
@@ -161,10 +158,10 @@ struct DevGrid {
   const uint32_t* mt0;
   const uint32_t* mt1;
   const uint32_t* mt2;
-  // neighbour lists of the last grid build (CSR in visit order); used while
+  // neighbour lists of the last grid build (visit order); used while
   // *nok != 0, i.e. until positions move or particles are added
   const uint32_t* noff;
-  const uint32_t* nlen;  // 3-D: row lengths (rows are padded to 16 bytes)
+  const uint32_t* nlen;  // 3-D: row lengths
   const int32_t* nidx;
   const int32_t* nok;
   // scene batch: the cell key of slot i is (scene[i] << scene_shift) | Morton
@@ -428,6 +425,15 @@ __device__ __forceinline__ float transit_weight(const dv_params& P, float x0) {
 // meets a material other than fluid or solid, so the sweeps then scan cells.
 #define DV_NBR_SOLID 0x80000000u
 #define DV_NBR_SLOT 0x7fffffffu
+// 3-D rows: quads of entries (16 bytes, the last one padded with the particle's
+// own slot), interleaved by 32 particles, so that the quads that a warp's
+// lanes read together are next to each other: quad c of particle i is
+// (i / 32 * 16 + c) * 32 + i % 32.  A row of more than kNbrRow entries lies by
+// itself behind those of all particles.  One row after the other, a load of 32
+// lanes touched 32 lines, and that was half of the L1's work in a sweep.
+constexpr uint32_t kNbrRow = 64;
+__host__ __device__ __forceinline__ int64_t nbr_row0(int64_t i) { return (i >> 5) * (kNbrRow * 8) + (i & 31); }
+__device__ __forceinline__ int nbr_stride(uint32_t len) { return len <= kNbrRow ? 32 : 1; }  // quads
 __device__ __forceinline__ int nbr_slot(uint32_t e) { return (int)(e & DV_NBR_SLOT); }
 __device__ __forceinline__ int nbr_mat(uint32_t e) { return (e & DV_NBR_SOLID) ? DV_MATERIAL_SOLID : DV_MATERIAL_FLUID; }
 
@@ -464,18 +470,19 @@ __device__ __forceinline__ void for_each_neighbor_impl(const dv_params& P, const
   };
   if (G.nok && __ldg(G.nok)) {  // the lists hold exactly these j, in this order
     const uint32_t k0 = __ldg(G.noff + i);
-    const uint32_t* __restrict__ nl = reinterpret_cast<const uint32_t*>(G.nidx) + k0;
     if constexpr (D == 3) {
       // four entries a load; the next entry's position is loaded before f
       // runs on the current one (a two-deep pipeline was slower)
       const int len = (int)__ldg(G.nlen + i);
       if (len == 0) return;
-      const uint4* __restrict__ n4 = reinterpret_cast<const uint4*>(nl);
+      const uint4* __restrict__ n4 = reinterpret_cast<const uint4*>(G.nidx) + k0;
+      const int st = nbr_stride(len);
       uint4 q = __ldg(n4);
       float4 p = ld_pos<D, PK>(x, pk, nbr_slot(q.x));
 #pragma unroll 1
       for (int k = 0; k < len; k += 4) {
-        const uint4 qn = k + 4 < len ? __ldg(n4 + (k >> 2) + 1) : q;
+        n4 += st;
+        const uint4 qn = k + 4 < len ? __ldg(n4) : q;
         float4 pn = ld_pos<D, PK>(x, pk, nbr_slot(q.y));
         call(q.x, p);
         p = pn;
@@ -495,6 +502,7 @@ __device__ __forceinline__ void for_each_neighbor_impl(const dv_params& P, const
       }
     } else {
       const uint32_t len = __ldg(G.noff + i + 1) - k0;
+      const uint32_t* __restrict__ nl = reinterpret_cast<const uint32_t*>(G.nidx) + k0;
       if (len == 0) return;
       // one-deep software pipeline: the next neighbour's entry and position
       // are loaded before f runs on the current one (f still runs in list
