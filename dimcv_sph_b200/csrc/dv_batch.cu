@@ -258,7 +258,7 @@ __global__ void k_batch_solve_reset(dv_scene_state* st, int32_t* done, int S, in
   }
 }
 
-// k_solve_finalize per scene: FP64 sum of the scene's residual block sums
+// solve_end per scene: FP64 sum of the scene's residual block sums
 // (part[wl[s] .. wl[s+1]) of the iteration's work list), average over its
 // fluid count, convergence test against eta or the iteration cap
 __global__ void k_batch_solve_finalize(const double* __restrict__ part, const int32_t* __restrict__ wl,

@@ -283,11 +283,22 @@ __device__ __forceinline__ float epan(const dv_params& P, V3 r) {
   return ret;
 }
 
-// compute_kernel_density (dimcv_sph.py:732-751) + FP64 block partials of
-// kden_sum (the reference accumulates it with an f32 atomic add)
+// kden_sum from the FP64 block sums (the reference accumulates it with an f32
+// atomic add)
+__device__ __forceinline__ void akde_end(dv_counters* C, double* part, uint32_t* ctr, double block_kden) {
+  if (threadIdx.x == 0) part[blockIdx.x] = block_kden;
+  if (!last_block(ctr)) return;
+  const double s = sum_partials(part, gridDim.x);
+  if (threadIdx.x == 0) {
+    C->kden_sum = s;
+    C->kden_sum_f32 = (float)s;
+  }
+}
+
+// compute_kernel_density (dimcv_sph.py:732-751) and kden_sum
 template <int D>
 __global__ void k_akde(dv_params P, DevGrid G, dv_fields F, dv_solver_fields S,
-                       const dv_counters* __restrict__ C, double* __restrict__ part) {
+                       dv_counters* C, double* __restrict__ part, uint32_t* ctr) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   double contrib = 0.0;
   if (i < C->n && F.material[i] == DV_MATERIAL_FLUID) {
@@ -301,8 +312,7 @@ __global__ void k_akde(dv_params P, DevGrid G, dv_fields F, dv_solver_fields S,
       contrib = (double)kd;
     }
   }
-  double s = block_sum<double>(contrib);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
+  akde_end(C, part, ctr, block_sum<double>(contrib));
 }
 
 // k_smooth and k_akde in one neighbour walk (both over the fluid neighbours
@@ -313,7 +323,7 @@ __global__ void k_akde(dv_params P, DevGrid G, dv_fields F, dv_solver_fields S,
 // 3-D: K.a = (x, m_V), K.b = (Δω, KVN).
 template <int D>
 __global__ void k_smooth_akde(dv_params P, DevGrid G, dv_fields F, dv_solver_fields S, DevPack K,
-                              const dv_counters* __restrict__ C, double* __restrict__ part) {
+                              dv_counters* C, double* __restrict__ part, uint32_t* ctr) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   double contrib = 0.0;
   if (i < C->n && F.material[i] == DV_MATERIAL_FLUID) {
@@ -348,28 +358,10 @@ __global__ void k_smooth_akde(dv_params P, DevGrid G, dv_fields F, dv_solver_fie
       contrib = (double)kd;
     }
   }
-  double s = block_sum<double>(contrib);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
-}
-
-__global__ void k_akde_finalize(const double* __restrict__ part, int nparts, dv_counters* C) {
-  double s = 0.0;
-  for (int k = threadIdx.x; k < nparts; k += blockDim.x) s += part[k];
-  s = block_sum<double>(s);
-  if (threadIdx.x == 0) {
-    C->kden_sum = s;
-    C->kden_sum_f32 = (float)s;
-  }
+  akde_end(C, part, ctr, block_sum<double>(contrib));
 }
 
 // ------------------------------------------------------- inverse-CDF draws
-__global__ void k_cdf_weights(const int32_t* __restrict__ targets, const float* __restrict__ kden,
-                              const dv_counters* __restrict__ C, int m, double* __restrict__ w) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= m) return;
-  w[k] = k < C->n_targets ? (double)kden[targets[k]] : 0.0;
-}
-
 // draw s: u ~ U[0,1) (53 bits, Philox keyed by (s, 2, step, seed)), or in
 // stratified mode u = (s + ξ)/M with ξ that draw; the target k with
 // cdf_ex[k] <= u·total < cdf_ex[k] + w_k (w_k > 0)
@@ -458,10 +450,7 @@ __global__ void k_batch_draw(const double* __restrict__ cdf_ex, const int32_t* _
 int dv_batch_draw(dv_ctx* c, const dv_solver_fields* s) {
   dv_batch_state* b = c->batch;
   const int m = (int)std::min<int64_t>(c->n_upper, c->cap);
-  k_cdf_weights<<<dv_blocks(m), DV_THREADS, 0, c->stream>>>(c->targets, s->kden, c->d_cnt, m,
-                                                          reinterpret_cast<double*>(c->near_v));
-  DV_LAUNCHED(c);
-  int rc = dv_scan_f64(c, reinterpret_cast<double*>(c->near_v), c->cdf, m);
+  int rc = dv_scan_cdf(c, c->targets, s->kden, c->cdf, m);
   if (rc) return rc;
   k_batch_draw<<<dv_blocks(b->m_cap), DV_THREADS, 0, c->stream>>>(c->cdf, c->targets, s->kden, b->d_state,
                                                                   b->d_scenes, b->S, b->d_step, c->d_cnt,
@@ -648,9 +637,7 @@ DV_API int dv_akde(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s) {
   if (!c || !f) return DV_EINVAL;
   if (int rc = check_solver(c, s)) return rc;
   const int nb = nblk(c);
-  LAUNCH_D(k_akde, nb, c->p, dv_grid(c), *f, *s, c->d_cnt, c->red_part);
-  k_akde_finalize<<<1, 1024, 0, c->stream>>>(c->red_part, nb, c->d_cnt);
-  DV_LAUNCHED(c);
+  LAUNCH_D(k_akde, nb, c->p, dv_grid(c), *f, *s, c->d_cnt, c->red_part, c->look_ctl + 3);
   return DV_OK;
 }
 
@@ -659,9 +646,7 @@ DV_API int dv_smooth_akde(dv_ctx* c, const dv_fields* f, const dv_solver_fields*
   if (int rc = check_solver(c, s)) return rc;
   const int nb = nblk(c);
   if (int rc = dv_pack(c, f, s, DV_PK_XV | DV_PK_DW)) return rc;
-  LAUNCH_D(k_smooth_akde, nb, c->p, dv_grid(c), *f, *s, dv_packs(c), c->d_cnt, c->red_part);
-  k_akde_finalize<<<1, 1024, 0, c->stream>>>(c->red_part, nb, c->d_cnt);
-  DV_LAUNCHED(c);
+  LAUNCH_D(k_smooth_akde, nb, c->p, dv_grid(c), *f, *s, dv_packs(c), c->d_cnt, c->red_part, c->look_ctl + 3);
   return DV_OK;
 }
 
@@ -684,11 +669,7 @@ DV_API int dv_sample(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s, i
   int rc = dv_build_targets(c, f);
   if (rc) return rc;
   const int m = (int)std::min<int64_t>(c->n_upper, c->cap);
-  k_cdf_weights<<<dv_blocks(m), DV_THREADS, 0, c->stream>>>(c->targets, s->kden, c->d_cnt, m,
-                                                          reinterpret_cast<double*>(c->near_v));
-  DV_LAUNCHED(c);
-  // near_v (16 B per slot) is free scratch here: it holds the FP64 weights
-  rc = dv_scan_f64(c, reinterpret_cast<double*>(c->near_v), c->cdf, m);
+  rc = dv_scan_cdf(c, c->targets, s->kden, c->cdf, m);
   if (rc) return rc;
   k_cdf_draw<<<dv_blocks(std::max(M, 1)), DV_THREADS, 0, c->stream>>>(
       c->cdf, c->targets, s->kden, c->d_cnt, M, (uint32_t)seed, (uint32_t)(seed >> 32),

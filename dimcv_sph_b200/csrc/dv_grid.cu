@@ -215,36 +215,25 @@ __global__ void __launch_bounds__(RS_T) k_rs_pass(const uint32_t* __restrict__ k
   }
 }
 
-// cell table from sorted keys; n_new = number of valid keys
-__global__ void k_cell_ranges(const uint32_t* __restrict__ keys, const dv_counters* __restrict__ C,
-                              uint32_t invalid, int32_t* __restrict__ cstart,
-                              int32_t* __restrict__ cend, int32_t* __restrict__ n_new_out) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  const int n_old = C->n;  // the sorted range; keys past it are stale
-  if (p >= n_old) return;
-  uint32_t k = keys[p];
-  if (k == invalid) return;
-  uint32_t kp = p > 0 ? keys[p - 1] : 0xffffffffu;
-  uint32_t kn = p + 1 < n_old ? keys[p + 1] : invalid;
-  if (p == 0 || kp != k) cstart[k] = p;
-  if (kn != k) cend[k] = p + 1;
-  if (kn == invalid) *n_new_out = p + 1;
-}
-
-// Gathers every dv_fields array into the new order; counts fluid / solid
-// per block (deterministic partials).  Slots in [n_new, n_old) receive the
+// The cell table from the sorted keys, every dv_fields array gathered into the
+// new order, and the new counts, in the last block.  Slots in [n_new, n_old) receive the
 // reference's partition fill values (particle_system.py:455-465) for the
 // filled fields and keep their own values for the others.
 template <int D>
 __global__ void k_permute(dv_fields S, dv_fields T, const uint32_t* __restrict__ perm,
-                          const uint32_t* __restrict__ keys, const int32_t* __restrict__ n_new_p,
-                          int n_old_cap, const dv_counters* __restrict__ C,
-                          int32_t* __restrict__ part) {
+                          const uint32_t* __restrict__ keys, uint32_t invalid, int n_old_cap, dv_counters* C,
+                          int32_t* __restrict__ cstart, int32_t* __restrict__ cend, int32_t* part, uint32_t* ctl,
+                          int32_t* __restrict__ ok) {
   const int VS = D == 2 ? 2 : 4;
   int p = blockIdx.x * blockDim.x + threadIdx.x;
-  int n_old = C->n, n_new = *n_new_p;
+  const int n_old = C->n;  // the sorted range; keys past it are stale
+  const uint32_t key = p < n_old ? keys[p] : invalid;
   int fl = 0, so = 0;
-  if (p < n_new) {
+  if (key != invalid) {
+    const uint32_t next = p + 1 < n_old ? keys[p + 1] : invalid;
+    if (p == 0 || keys[p - 1] != key) cstart[key] = p;
+    if (next != key) cend[key] = p + 1;
+    if (next == invalid) ctl[4] = (uint32_t)p + 1u;
     int j = (int)perm[p];
     if (D == 2) {
       reinterpret_cast<float2*>(T.x)[p] = reinterpret_cast<const float2*>(S.x)[j];
@@ -269,7 +258,7 @@ __global__ void k_permute(dv_fields S, dv_fields T, const uint32_t* __restrict__
     int mat = S.material[j];
     T.material[p] = mat;
     T.object_id[p] = S.object_id[j];
-    T.grid_ids[p] = (int32_t)keys[p];
+    T.grid_ids[p] = (int32_t)key;
     T.is_dynamic[p] = S.is_dynamic[j];
     T.is_active[p] = S.is_active[j];
     T.is_sample[p] = S.is_sample[j];
@@ -304,25 +293,22 @@ __global__ void k_permute(dv_fields S, dv_fields T, const uint32_t* __restrict__
     part[2 * blockIdx.x] = sfl;
     part[2 * blockIdx.x + 1] = sso;
   }
-}
-
-__global__ void k_finalize_counts(const int32_t* __restrict__ part, int nparts,
-                                  const int32_t* __restrict__ n_new_p, dv_counters* C, int32_t* ok,
-                                  uint32_t* far_used) {
-  int fl = 0, so = 0;
-  for (int k = threadIdx.x; k < nparts; k += blockDim.x) {
-    fl += part[2 * k];
-    so += part[2 * k + 1];
+  if (!last_block(ctl + 3)) return;
+  fl = so = 0;
+  for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) {
+    fl += __ldcg(part + 2 * k);
+    so += __ldcg(part + 2 * k + 1);
   }
   fl = block_sum<int>(fl);
   so = block_sum<int>(so);
   if (threadIdx.x == 0) {
-    C->n = *n_new_p;
+    C->n = (int)__ldcg(ctl + 4);
     C->n_fluid = fl;
     C->n_solid = so;
-    ok[0] = 1;  // until the list build finds otherwise
-    ok[1] = 1;  // the sorted keys are those of the current slots
-    *far_used = 0u;
+    ctl[4] = 0u;
+    ctl[2] = 0u;  // entries of long rows used by the list build
+    ok[0] = 1;    // until the list build finds otherwise
+    ok[1] = 1;    // the sorted keys are those of the current slots
   }
 }
 
@@ -339,7 +325,7 @@ __global__ void k_finalize_counts(const int32_t* __restrict__ part, int nparts,
 // fluid particle (or, for the rigid coupling, a dynamic solid) at its centre,
 // and the static boundary volume (once, at initialisation) scans cells.
 //
-// One launch: k_csr_rows (3-D), k_csr_build (2-D).  k_finalize_counts has set
+// One launch: k_csr_rows (3-D), k_csr_build (2-D).  k_permute has set
 // the lists valid before it; a build that cannot store them takes that back.
 __device__ __forceinline__ bool nbr_row_built(const int32_t* __restrict__ mat, const uint8_t* __restrict__ dyn,
                                               int i) {
@@ -645,8 +631,9 @@ DV_API int dv_grid_build(dv_ctx* c, const dv_fields* src, const dv_fields* dst) 
   uint32_t* count = c->sort_state;
   uint32_t* ticket = count + 256 * c->npasses;
   uint32_t* state = ticket + 64;
-  DV_CK(c, cudaMemsetAsync(c->sort_state, 0,
-                           sizeof(uint32_t) * (256 * (size_t)c->npasses * (size_t)(tiles + 1) + 64), c->stream));
+  // the cell tables lie before the sort's state
+  const size_t zeroed = 2 * (size_t)c->ncells + 256 * (size_t)c->npasses * (size_t)(tiles + 1) + 64;
+  DV_CK(c, cudaMemsetAsync(c->cell_start, 0, sizeof(uint32_t) * zeroed, c->stream));
   const int kr = ntiles < 2 * c->num_sms ? 1 : 8;
 #define CK(DD, RR)                                                                                                  \
   k_cell_keys<DD, RR><<<dv_blocks(nu, RS_T * RR), RS_T, 0, c->stream>>>(c->p, *src, G, c->d_cnt, c->keys[0], invalid, \
@@ -672,21 +659,15 @@ DV_API int dv_grid_build(dv_ctx* c, const dv_fields* src, const dv_fields* dst) 
   }
   c->perm_buf = cur;
   // cell table
-  DV_CK(c, cudaMemsetAsync(c->cell_start, 0, sizeof(int32_t) * c->ncells, c->stream));
-  DV_CK(c, cudaMemsetAsync(c->cell_end, 0, sizeof(int32_t) * c->ncells, c->stream));
-  DV_CK(c, cudaMemsetAsync(c->d_flag + 1, 0, sizeof(int32_t), c->stream));
-  k_cell_ranges<<<nb, DV_THREADS, 0, c->stream>>>(c->keys[cur], c->d_cnt, invalid, c->cell_start,
-                                                  c->cell_end, c->d_flag + 1);
-  DV_LAUNCHED(c);
+#define PERM(DD)                                                                                                     \
+  k_permute<DD><<<nb, DV_THREADS, 0, c->stream>>>(*src, *dst, c->vals[cur], c->keys[cur], invalid, (int)c->cap,      \
+                                                  c->d_cnt, c->cell_start, c->cell_end, c->ired_part, c->look_ctl, \
+                                                  c->d_nbr_ok)
   if (c->p.dim == 2)
-    k_permute<2><<<nb, DV_THREADS, 0, c->stream>>>(*src, *dst, c->vals[cur], c->keys[cur],
-                                                   c->d_flag + 1, (int)c->cap, c->d_cnt, c->ired_part);
+    PERM(2);
   else
-    k_permute<3><<<nb, DV_THREADS, 0, c->stream>>>(*src, *dst, c->vals[cur], c->keys[cur],
-                                                   c->d_flag + 1, (int)c->cap, c->d_cnt, c->ired_part);
-  DV_LAUNCHED(c);
-  k_finalize_counts<<<1, 1024, 0, c->stream>>>(c->ired_part, nb, c->d_flag + 1, c->d_cnt, c->d_nbr_ok,
-                                               c->look_ctl + 2);
+    PERM(3);
+#undef PERM
   DV_LAUNCHED(c);
   c->scene_ptr = batch ? dst->object_id : nullptr;  // scene of each sorted slot
   return build_csr(c, dst);

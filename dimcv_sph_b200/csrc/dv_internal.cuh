@@ -72,7 +72,8 @@ struct dv_ctx {
 
   // scans and reductions
   unsigned long long* look_state = nullptr;  // one-launch scans (dv_lookback.cuh): a word per tile, zero between launches
-  uint32_t* look_ctl = nullptr;              // [0] ticket, [1] blocks done
+  // [0] ticket, [1] blocks done; [2] long list rows; [3] blocks done (last_block); [4] valid keys
+  uint32_t* look_ctl = nullptr;
   double* dscan_part = nullptr;   // double block partials
   int64_t scan_part_cap = 0;
   double* red_part = nullptr;     // FP64 per-block partials of sweeps
@@ -255,7 +256,8 @@ int dv_farbox_run(dv_ctx* c, const dv_fields* f);
 // launch, dv_lookback.cuh; double: deterministic three-phase block reduce,
 // scan of partials, block scan).
 int dv_scan_u32(dv_ctx* c, const uint32_t* in, uint32_t* out, int64_t m);
-int dv_scan_f64(dv_ctx* c, const double* in, double* out, int64_t m);
+// out[k] = sum of kden[targets[q]], q < k (0 past the target count), k < m
+int dv_scan_cdf(dv_ctx* c, const int32_t* targets, const float* kden, double* out, int64_t m);
 // Sum of `nparts` FP64 partials into *dst (device), one block, fixed order.
 int dv_finalize_sum(dv_ctx* c, const double* parts, int nparts, double* dst);
 // Marks the per-step neighbour lists stale (positions or counts changed).
@@ -673,5 +675,46 @@ __device__ __forceinline__ T block_sum(T v) {
   int nw = (blockDim.x + 31) >> 5;
   T t = (threadIdx.x < nw) ? s_ws[threadIdx.x] : T(0);
   if (w == 0) t = warp_sum(t);
+  return t;
+}
+
+// ------------------------------------------------- last block of a launch
+// True in every thread of the block that finishes last, which sees what the
+// others wrote; *ctr is zero before and after.  A sum of block partials ends in
+// the kernel that makes them: a launch of one block for it cost 2 us, and as
+// much again between the launches.
+__device__ __forceinline__ bool last_block(uint32_t* ctr) {
+  __shared__ bool s_last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(ctr, 1u) == gridDim.x - 1;
+    if (s_last) *ctr = 0u;
+    __threadfence();
+  }
+  __syncthreads();
+  return s_last;
+}
+// Sum of n block partials in thread 0 of a block of DV_THREADS, in the order of
+// a block of 1,024 (thread k adds k, k + 1,024, ...; then the tree).
+__device__ __forceinline__ double sum_partials(const double* part, int n) {
+  constexpr int Q = 1024 / DV_THREADS;
+  __shared__ double s_q[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double a[Q];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) a[q] = 0.0;
+  for (int k = threadIdx.x; k < n; k += 1024)
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+      if (k + q * DV_THREADS < n) a[q] += __ldcg(part + k + q * DV_THREADS);
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    a[q] = warp_sum(a[q]);
+    if (lane == 0) s_q[q * (DV_THREADS / 32) + w] = a[q];
+  }
+  __syncthreads();
+  double t = 0.0;
+  if (w == 0) t = warp_sum(s_q[lane]);
   return t;
 }

@@ -195,9 +195,52 @@ __device__ __forceinline__ void densities_factor_body(const dv_params& P, const 
 }
 
 // multiply_time_step (dimcv_sph.py:395-399)
-__global__ void k_scale_factor(dv_fields F, float s, const dv_counters* __restrict__ C) {
+__device__ __forceinline__ void solve_reset(dv_counters* C, int32_t* done, int which) {
+  *done = 0;
+  if (which == 0)
+    C->iters_div = 0;
+  else
+    C->iters_p = 0;
+}
+// done: also starts the solve `which`
+__global__ void k_scale_factor(dv_fields F, float s, dv_counters* C, int32_t* done, int which) {
+  if (done && blockIdx.x == 0 && threadIdx.x == 0) solve_reset(C, done, which);
   FOR_I;
   if (F.material[i] == DV_MATERIAL_FLUID) F.dfsph_factor[i] *= s;
+}
+
+// The convergence test of one Jacobi iteration, in the last block of its
+// residual sweep: average error over the fluid count against eta; sets the
+// done flag at convergence or at max_iter.
+struct SolveEnd {
+  double* part;  // block partials of the error
+  dv_counters* C;
+  int32_t* done;
+  uint32_t* ctr;
+  double eta;
+  int max_iter, which;
+};
+__device__ __forceinline__ void solve_end(const SolveEnd& E, double block_err) {
+  if (threadIdx.x == 0) E.part[blockIdx.x] = block_err;
+  if (!last_block(E.ctr)) return;
+  const double s = sum_partials(E.part, gridDim.x);
+  if (threadIdx.x == 0) {
+    dv_counters* C = E.C;
+    const int nf = C->n_fluid;
+    const double avg = nf > 0 ? s / (double)nf : 0.0;
+    const int it = (E.which == 0 ? ++C->iters_div : ++C->iters_p);
+    if (E.which == 0)
+      C->err_div = avg;
+    else
+      C->err_p = avg;
+    if (!isfinite(avg)) C->status |= DV_WARN_NAN;
+    if (avg <= E.eta || nf == 0) {
+      *E.done = 1;
+    } else if (it >= E.max_iter) {
+      *E.done = 1;
+      C->status |= (E.which == 0 ? DV_WARN_DIV_NOT_CONVERGED : DV_WARN_P_NOT_CONVERGED);
+    }
+  }
 }
 
 // ------------------------------------------------------- density change
@@ -280,28 +323,24 @@ __device__ __forceinline__ double density_change_np_one(const dv_params& P, cons
 // NEXT: in the Jacobi loop, with the FP64 block partial of the error terms
 template <int D, bool NEXT>
 __global__ void k_density_change(dv_params P, DevGrid G, dv_fields F, DevPack K, const dv_counters* __restrict__ C,
-                                 const int32_t* __restrict__ done, double* __restrict__ part) {
-  if (done && *done) return;
+                                 SolveEnd E) {
+  if (NEXT && *E.done) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   double err = 0.0;
   if (i < C->n) err = density_change_one<D, NEXT>(P, G, F, K, i);
-  if (NEXT) {
-    double s = block_sum<double>(err);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
-  }
+  if (NEXT) solve_end(E, block_sum<double>(err));
 }
 
 // the divergence Jacobi loop's residual sweep with the non-pressure forces
 template <int D>
 __global__ void k_density_change_np(dv_params P, DevGrid G, dv_fields F, DevPack K,
                                     const dv_counters* __restrict__ C,
-                                    const int32_t* __restrict__ done, double* __restrict__ part) {
-  if (*done) return;
+                                    SolveEnd E) {
+  if (*E.done) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   double err = 0.0;
   if (i < C->n) err = density_change_np_one<D>(P, G, F, K, i);
-  double s = block_sum<double>(err);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
+  solve_end(E, block_sum<double>(err));
 }
 
 // ------------------------------------------------------------ density adv
@@ -341,25 +380,25 @@ __device__ __forceinline__ double density_adv_one(const dv_params& P, const DevG
 
 template <int D, bool NEXT>
 __global__ void k_density_adv(dv_params P, DevGrid G, dv_fields F, DevPack K, const dv_counters* __restrict__ C,
-                              const int32_t* __restrict__ done, double* __restrict__ part) {
-  if (done && *done) return;
+                              SolveEnd E) {
+  if (NEXT && *E.done) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   double err = 0.0;
   if (i < C->n) err = density_adv_one<D, NEXT>(P, G, F, K, i);
-  if (NEXT) {
-    double s = block_sum<double>(err);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
-  }
+  if (NEXT) solve_end(E, block_sum<double>(err));
 }
 
 // The pressure solve's opening density_adv sweep and, in the same walk,
 // copy_x_temp + compute_vorticity_vis (dimcv_sph.py:778-801), with the
 // operations and order of k_vis: the vis sweep reads x, m_V, material and
 // vorticity, which the pressure iterations (they write v) leave unchanged, so
-// the solve's first sweep gives what the vis sweep after the solve would.
+// the solve's first sweep gives what the vis sweep after the solve would.  It
+// also scales the factors for the solve (multiply_time_step), which the sweep
+// does not read, and starts it.
 template <int D>
 __global__ void k_density_adv_vis(dv_params P, DevGrid G, dv_fields F, dv_solver_fields S, DevPack K,
-                                  const dv_counters* __restrict__ C) {
+                                  dv_counters* C, float scale, int32_t* done) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) solve_reset(C, done, 1);
   FOR_I;
   const V3 xi = ldv<D>(F.x, i);
   stv<D>(S.x_temp, i, xi);
@@ -367,6 +406,7 @@ __global__ void k_density_adv_vis(dv_params P, DevGrid G, dv_fields F, dv_solver
     st4(S.vorticity_vis, i, V3{0.f, 0.f, 0.f});
     return;
   }
+  F.dfsph_factor[i] *= scale;
   const V3 vi = ldv<D>(F.v, i);
   float delta = 0.0f;
   const float w = F.m_V[i] * cubic_W(P, 0.0f);
@@ -639,40 +679,6 @@ __global__ void k_batch_residual(dv_params P, DevGrid G, dv_fields F, DevPack K,
   }
 }
 
-// convergence test of one Jacobi iteration: average error over the fluid
-// count against eta; sets the done flag at convergence or at max_iter
-__global__ void k_solve_finalize(const double* __restrict__ part, int nparts, dv_counters* C,
-                                 int32_t* done, double eta, int max_iter, int which) {
-  if (*done) return;
-  double s = 0.0;
-  for (int k = threadIdx.x; k < nparts; k += blockDim.x) s += part[k];
-  s = block_sum<double>(s);
-  if (threadIdx.x == 0) {
-    int nf = C->n_fluid;
-    double avg = nf > 0 ? s / (double)nf : 0.0;
-    int it = (which == 0 ? ++C->iters_div : ++C->iters_p);
-    if (which == 0)
-      C->err_div = avg;
-    else
-      C->err_p = avg;
-    if (!isfinite(avg)) C->status |= DV_WARN_NAN;
-    if (avg <= eta || nf == 0) {
-      *done = 1;
-    } else if (it >= max_iter) {
-      *done = 1;
-      C->status |= (which == 0 ? DV_WARN_DIV_NOT_CONVERGED : DV_WARN_P_NOT_CONVERGED);
-    }
-  }
-}
-
-__global__ void k_solve_reset(dv_counters* C, int32_t* done, int which) {
-  *done = 0;
-  if (which == 0)
-    C->iters_div = 0;
-  else
-    C->iters_p = 0;
-}
-
 // ------------------------------------------------------- non-pressure forces
 // compute_non_pressure_forces (dimcv_sph.py:150-208).  The surface tension
 // coefficient is 0 in the reference (dimcv_sph.py:12) and boundary viscosity
@@ -720,7 +726,8 @@ __global__ void k_predict_velocity(dv_params P, dv_fields F, const dv_counters* 
 
 // advect (dimcv_sph.py:210-218)
 template <int D>
-__global__ void k_advect(dv_params P, dv_fields F, const dv_counters* __restrict__ C) {
+__global__ void k_advect(dv_params P, dv_fields F, const dv_counters* __restrict__ C, int32_t* __restrict__ ok) {
+  if (blockIdx.x == 0 && threadIdx.x < 2) ok[threadIdx.x] = 0;  // the lists and sorted keys, as dv_invalidate_lists
   FOR_I;
   if (!F.is_dynamic[i]) return;
   V3 v = ldv<D>(F.v, i);
@@ -818,11 +825,15 @@ DV_API int dv_densities_factor_change(dv_ctx* c, const dv_fields* f) {
   return DV_OK;
 }
 
-DV_API int dv_scale_factor(dv_ctx* c, const dv_fields* f, float s) {
-  if (!c || !f) return DV_EINVAL;
-  k_scale_factor<<<nblk(c), DV_THREADS, 0, c->stream>>>(*f, s, c->d_cnt);
+static int scale_factor(dv_ctx* c, const dv_fields* f, float s, int32_t* done, int which) {
+  k_scale_factor<<<nblk(c), DV_THREADS, 0, c->stream>>>(*f, s, c->d_cnt, done, which);
   DV_LAUNCHED(c);
   return DV_OK;
+}
+
+DV_API int dv_scale_factor(dv_ctx* c, const dv_fields* f, float s) {
+  if (!c || !f) return DV_EINVAL;
+  return scale_factor(c, f, s, nullptr, 0);
 }
 
 // LAUNCH_D for the kernels of template <D, NEXT>
@@ -838,16 +849,14 @@ DV_API int dv_scale_factor(dv_ctx* c, const dv_fields* f, float s) {
 DV_API int dv_density_change(dv_ctx* c, const dv_fields* f) {
   if (!c || !f) return DV_EINVAL;
   if (int rc = dv_pack(c, f, nullptr, DV_PK_XV)) return rc;
-  LAUNCH_DN(k_density_change, false, nblk(c), c->p, dv_grid(c), *f, dv_packs(c), c->d_cnt, (const int32_t*)nullptr,
-            (double*)nullptr);
+  LAUNCH_DN(k_density_change, false, nblk(c), c->p, dv_grid(c), *f, dv_packs(c), c->d_cnt, SolveEnd{});
   return DV_OK;
 }
 
 DV_API int dv_density_adv(dv_ctx* c, const dv_fields* f) {
   if (!c || !f) return DV_EINVAL;
   if (int rc = dv_pack(c, f, nullptr, DV_PK_XV | DV_PK_VM)) return rc;
-  LAUNCH_DN(k_density_adv, false, nblk(c), c->p, dv_grid(c), *f, dv_packs(c), c->d_cnt, (const int32_t*)nullptr,
-            (double*)nullptr);
+  LAUNCH_DN(k_density_adv, false, nblk(c), c->p, dv_grid(c), *f, dv_packs(c), c->d_cnt, SolveEnd{});
   return DV_OK;
 }
 
@@ -879,8 +888,9 @@ DV_API int dv_pressure_iteration(dv_ctx* c, const dv_fields* f) {
 }
 
 // Runs Jacobi iterations in chunks of 2, 4, 8, ... launches; every iteration
-// is (update sweep, residual sweep + FP64 block partials, finalize) and all
-// three return at once once the done flag is set.  3-D: the packed copies are
+// is an update sweep and a residual sweep, whose last block tests for
+// convergence; both return at once when the done flag is set.  The caller's
+// scaling of the factors has reset the flag.  3-D: the packed copies are
 // made here (pressure: the caller's opening sweep left K.a and K.b), and the
 // residual sweeps keep K.k and the pressure updates K.b current.
 static int jacobi_loop(dv_ctx* c, const dv_fields* f, int which, bool nonpressure = false) {
@@ -888,8 +898,7 @@ static int jacobi_loop(dv_ctx* c, const dv_fields* f, int which, bool nonpressur
   const int max_iter = which == 0 ? c->p.max_iter_div : c->p.max_iter_p;
   const double eta = which == 0 ? c->p.eta_div : c->p.eta_p;
   int32_t* done = c->d_flag;
-  k_solve_reset<<<1, 1, 0, c->stream>>>(c->d_cnt, done, which);
-  DV_LAUNCHED(c);
+  const SolveEnd E{c->red_part, c->d_cnt, done, c->look_ctl + 3, eta, max_iter, which};
   const DevPack K = dv_packs(c);
   if (int rc = dv_pack(c, f, nullptr, which == 0 ? DV_PK_XV | DV_PK_DIV : DV_PK_P)) return rc;
   int launched = 0, chunk = 2;
@@ -899,20 +908,14 @@ static int jacobi_loop(dv_ctx* c, const dv_fields* f, int which, bool nonpressur
       if (which == 0) {
         LAUNCH_D(k_divergence_iter, nb, c->p, dv_grid(c), *f, K, c->d_cnt, (const int32_t*)done);
         if (nonpressure)
-          LAUNCH_D(k_density_change_np, nb, c->p, dv_grid(c), *f, K, c->d_cnt, (const int32_t*)done,
-                   c->red_part);
+          LAUNCH_D(k_density_change_np, nb, c->p, dv_grid(c), *f, K, c->d_cnt, E);
         else
-          LAUNCH_DN(k_density_change, true, nb, c->p, dv_grid(c), *f, K, c->d_cnt, (const int32_t*)done,
-                    c->red_part);
+          LAUNCH_DN(k_density_change, true, nb, c->p, dv_grid(c), *f, K, c->d_cnt, E);
       } else {
         LAUNCH_D(k_pressure_iter, nb, c->p, dv_grid(c), *f, K, c->d_cnt, (const int32_t*)done);
         if (c->dyn_rigid) LAUNCH_D(k_rigid_reaction, nb, c->p, dv_grid(c), *f, c->d_cnt, (const int32_t*)done);
-        LAUNCH_DN(k_density_adv, true, nb, c->p, dv_grid(c), *f, K, c->d_cnt, (const int32_t*)done,
-                  c->red_part);
+        LAUNCH_DN(k_density_adv, true, nb, c->p, dv_grid(c), *f, K, c->d_cnt, E);
       }
-      k_solve_finalize<<<1, 1024, 0, c->stream>>>(c->red_part, nb, c->d_cnt, done, eta, max_iter,
-                                                  which);
-      DV_LAUNCHED(c);
     }
     launched += m;
     if (launched >= max_iter) break;
@@ -1033,7 +1036,7 @@ static int divergence_solve(dv_ctx* c, const dv_fields* f, int32_t* iters, int32
   const bool nonpressure = (flags & DV_SOLVE_NONPRESSURE) != 0;
   int rc = (flags & DV_SOLVE_PREPARED) ? DV_OK : dv_density_change(c, f);
   if (rc) return rc;
-  rc = dv_scale_factor(c, f, c->p.inv_dt);
+  rc = scale_factor(c, f, c->p.inv_dt, c->d_flag, 0);
   if (rc) return rc;
   rc = jacobi_loop(c, f, 0, nonpressure);
   if (rc) return rc;
@@ -1074,13 +1077,13 @@ DV_API int dv_pressure_solve_ex(dv_ctx* c, const dv_fields* f, const dv_solver_f
       return dv_fail(c, DV_EINVAL, "dv_pressure_solve_ex: DV_SOLVE_VIS needs x_temp and vorticity_vis");
     rc = dv_pack(c, f, s, DV_PK_XV | DV_PK_VM);
     if (rc) return rc;
-    LAUNCH_D(k_density_adv_vis, nblk(c), c->p, dv_grid(c), *f, *s, dv_packs(c), c->d_cnt);
+    LAUNCH_D(k_density_adv_vis, nblk(c), c->p, dv_grid(c), *f, *s, dv_packs(c), c->d_cnt, c->p.inv_dt2, c->d_flag);
   } else {
     rc = dv_density_adv(c, f);
+    if (rc) return rc;
+    rc = scale_factor(c, f, c->p.inv_dt2, c->d_flag, 1);
+    if (rc) return rc;
   }
-  if (rc) return rc;
-  rc = dv_scale_factor(c, f, c->p.inv_dt2);
-  if (rc) return rc;
   rc = jacobi_loop(c, f, 1);
   if (rc) return rc;
   return read_iters(c, 1, iters);
@@ -1090,7 +1093,7 @@ DV_API int dv_pressure_solve(dv_ctx* c, const dv_fields* f, int32_t* iters) {
   if (!c || !f) return DV_EINVAL;
   int rc = dv_density_adv(c, f);
   if (rc) return rc;
-  rc = dv_scale_factor(c, f, c->p.inv_dt2);
+  rc = scale_factor(c, f, c->p.inv_dt2, c->d_flag, 1);
   if (rc) return rc;
   rc = jacobi_loop(c, f, 1);
   if (rc) return rc;
@@ -1166,6 +1169,6 @@ DV_API int dv_enforce_boundary(dv_ctx* c, const dv_fields* f, int32_t material, 
 
 DV_API int dv_advect(dv_ctx* c, const dv_fields* f) {
   if (!c || !f) return DV_EINVAL;
-  LAUNCH_D(k_advect, nblk(c), c->p, *f, c->d_cnt);
-  return dv_invalidate_lists(c);  // positions moved
+  LAUNCH_D(k_advect, nblk(c), c->p, *f, c->d_cnt, c->d_nbr_ok);
+  return DV_OK;
 }
