@@ -356,11 +356,10 @@ __device__ __forceinline__ void node_sums(const dv_params& P, const dv_farbox& B
     AX[p] = AY[p] = AZ[p] = 0ull;
   }
   const float3 org = make_float3(box_centre(P, me.x, 0), box_centre(P, me.y, 1), box_centre(P, me.z, 2));
-  const ulonglong2* s2 = reinterpret_cast<const ulonglong2*>(s4);
   const bool run = grp < G;
   staged_samples<BLOB, NT>(B, me, part, stripes(S) * B.stripe_mul, S + 2, S == kSets - 1 ? 0x7fffffff : S + 2, org,
                            s4, s_start, s_pref, [&](int m) {
-                             if (run) far_x2_loop<3, NP, BLOB, false>(s2, grp, G, m, PX, PY, PZ, AX, AY, AZ, 0.0f,
+                             if (run) far_x2_loop<3, NP, BLOB, false>(s4, grp, G, m, PX, PY, PZ, AX, AY, AZ, 0.0f,
                                                                       P.blob_delta2);
                            });
   float* red = reinterpret_cast<float*>(s4);  // [3][P]
@@ -595,12 +594,11 @@ __global__ void __launch_bounds__(kNearT, 2) k_box_near(dv_params P, dv_farbox B
     PZ[p] = f2_pack(u.z, v.z);
     AX[p] = AY[p] = AZ[p] = 0ull;
   }
-  const ulonglong2* s2 = reinterpret_cast<const ulonglong2*>(s4);
   const bool run = tw < nt;
   const float lim = P.far_r2_limit;
   staged_samples<BLOB, kNearT>(B, me, blockIdx.y, gridDim.y, 0, 1, make_float3(0.f, 0.f, 0.f), s4, s_start, s_pref,
                                [&](int m) {
-                                 if (run) far_x2_loop<3, NP, BLOB, true>(s2, 0, 1, m, PX, PY, PZ, AX, AY, AZ, lim,
+                                 if (run) far_x2_loop<3, NP, BLOB, true>(s4, 0, 1, m, PX, PY, PZ, AX, AY, AZ, lim,
                                                                         P.blob_delta2);
                                });
   if (blockIdx.y == 0) {

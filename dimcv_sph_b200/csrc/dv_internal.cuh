@@ -100,6 +100,7 @@ struct dv_ctx {
   uint32_t* srank = nullptr;   // cap + 1: sampled slots before a slot
   int32_t* sslot = nullptr;    // cap: the sampled slots in slot order, srank[j] -> j
   int far_tt = 4;              // targets per thread of the far-field main loop (autotuned)
+  bool far_tt_set = false;     // by dv_set_far_tile or dv_autotune
   int far_chunks = 1;          // sample chunks of the far-field grid (autotuned, <= DV_MAX_FAR_CHUNKS)
   bool dyn_rigid = false;      // dynamic rigid particles present: pressure iterations add their reaction
 

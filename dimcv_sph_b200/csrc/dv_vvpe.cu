@@ -614,9 +614,9 @@ __global__ void __launch_bounds__(FT2) k_far_main_b(dv_params P, const float* __
 // (Blackwell's sub/mul/fma.rn.f32x2): every lane operation is the scalar
 // loop's own IEEE operation in the same order, so far_acc is bit-identical;
 // the pairs halve the issue slots of a loop that is issue-bound, not
-// FP32-pipe-bound.  Samples are staged in shared memory pre-duplicated
-// ({s, s} pairs, ω̃/kden components negated where the loop subtracts); the
-// inner loop is far_x2_loop (dv_far.cuh).
+// FP32-pipe-bound.  Samples are staged in shared memory with the ω̃/kden
+// components negated where the loop subtracts (far_x2_stage); the inner loop is
+// far_x2_loop (dv_far.cuh).
 
 // targets [tbase + k·FT2 + tid] (k < TT) of targets[0, nt) against samples
 // [m0, m0 + M); writes far_acc[t] for t < nt.  Block-uniform bounds.
@@ -654,7 +654,6 @@ __device__ __forceinline__ void far_x2_run(const dv_params& P, const float* __re
     AX[p] = AY[p] = AZ[p] = 0ull;
   }
   const float lim = P.far_r2_limit;
-  const ulonglong2* s2 = reinterpret_cast<const ulonglong2*>(s4);
   for (int base = 0; base < M; base += FTILE2) {
     const int m = min(FTILE2, M - base);
     __syncthreads();
@@ -664,7 +663,7 @@ __device__ __forceinline__ void far_x2_run(const dv_params& P, const float* __re
       far_x2_stage<D, BLOB>(s4, q, sp, w);
     }
     __syncthreads();
-    far_x2_loop<D, NP, BLOB, true>(s2, 0, 1, m, PX, PY, PZ, AX, AY, AZ, lim, P.blob_delta2);
+    far_x2_loop<D, NP, BLOB, true>(s4, 0, 1, m, PX, PY, PZ, AX, AY, AZ, lim, P.blob_delta2);
   }
 #pragma unroll
   for (int p = 0; p < NP; ++p) {
@@ -704,7 +703,7 @@ __global__ void __launch_bounds__(FT2, DV_FAR_MINB(TT)) k_far_main_x2_b(dv_param
                                                        const int32_t* __restrict__ order, int S,
                                                        const int32_t* __restrict__ ntiles,
                                                        float4* __restrict__ far_acc) {
-  __shared__ float4 s4[(D == 3 ? 4 : 2) * FTILE2];
+  __shared__ float4 s4[far_x2_words<D, false>() * FTILE2];
   const int blk = blockIdx.x;
   if (blk >= *ntiles) return;  // uniform per CTA
   const int sc = batch_block_scene(st, order, S, blk);
@@ -880,6 +879,7 @@ DV_API int dv_autotune(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s,
     DV_CK(c, cudaStreamSynchronize(c->stream));
     if (*c->h_flag) {
       c->far_tt = 8;
+      c->far_tt_set = true;
       c->far_chunks = DV_MAX_FAR_CHUNKS;
       if (best_tt) *best_tt = c->far_tt;
       if (best_ms) *best_ms = 0.0f;
@@ -918,6 +918,7 @@ DV_API int dv_autotune(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s,
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   c->far_tt = best_t;
+  c->far_tt_set = true;
   c->far_chunks = best_c;
   if (best_tt) *best_tt = best_t;
   if (best_ms) *best_ms = best;
@@ -927,6 +928,7 @@ DV_API int dv_autotune(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s,
 DV_API int dv_set_far_tile(dv_ctx* c, int32_t tt) {
   if (!c || (tt != 2 && tt != 4 && tt != 6 && tt != 8)) return DV_EINVAL;
   c->far_tt = tt;
+  c->far_tt_set = true;
   return DV_OK;
 }
 
@@ -1316,9 +1318,13 @@ static int bs_dispatch(dv_ctx* c, const dv_fields* f, const int32_t* targets, in
   const bool blob = c->p.kernel_mode == DV_KERNEL_BLOB3D;
   const int32_t* ns = c->d_flag + 2;
   if (precision == 32 && blob && !c->p.periodic && !c->p.compensated && D == 3 && c->far_tt > 2) {
-    // the paired loop (a tile of 2 keeps the scalar loop below)
-    if (c->far_tt <= 4) return launch_bs_x2<4>(c, f, targets, nt, ns, (float*)out);
-    if (c->far_tt <= 6) return launch_bs_x2<6>(c, f, targets, nt, ns, (float*)out);
+    // the paired loop (a tile of 2 keeps the scalar loop below); while no tile
+    // has been chosen, 8 targets a thread unless rounding nt up to its tiles
+    // costs more than it gives (65,536 x 65,536: 2.84 ms with 4, 2.67 with 8)
+    auto padded = [&](int64_t tt) { return (nt + FT2 * tt - 1) / (FT2 * tt) * (FT2 * tt); };
+    const int tt = c->far_tt_set ? c->far_tt : 100 * padded(8) <= 109 * padded(4) ? 8 : 4;
+    if (tt <= 4) return launch_bs_x2<4>(c, f, targets, nt, ns, (float*)out);
+    if (tt <= 6) return launch_bs_x2<6>(c, f, targets, nt, ns, (float*)out);
     return launch_bs_x2<8>(c, f, targets, nt, ns, (float*)out);
   }
   if (precision == 32 && blob && !c->p.periodic) {

@@ -398,7 +398,8 @@ DV_API int dv_vvpe_mc(dv_ctx* ctx, const dv_fields* f, const dv_solver_fields* s
  * for this context (synchronises; *best_tt / *best_ms may be NULL).  Where
  * boxes carry the far field the loop does not run: tile 8 and 8 chunks are
  * kept without timing (*best_ms = 0).
- * dv_set_far_tile sets the tile directly (2, 4, 6 or 8). */
+ * dv_set_far_tile sets the tile directly (2, 4, 6 or 8); until either call
+ * dv_vvpe_mc runs 4 and dv_bs_full 4 or 8 by the target count. */
 DV_API int dv_autotune(dv_ctx* ctx, const dv_fields* f, const dv_solver_fields* s, int32_t* best_tt,
                        float* best_ms);
 DV_API int dv_set_far_tile(dv_ctx* ctx, int32_t tt);
