@@ -15,25 +15,31 @@
 // (cos iπ/m, cos jπ/m, cos kπ/m) with i, j, k all even or all odd, about
 // (N + 2)^3 / 4 of them; the weighted sum over the points with the products
 // T_a T_b T_c, a + b + c <= N, gives the coefficients, exactly for
-// polynomials of degree N.  The degree falls with the distance of the sample
-// box (Chebyshev distance Δ in boxes).  Truncation error of a shell relative
-// to the whole sum, random-sign weights (the worst case), measured in FP64
-// for the reference / the blob kernel:
-//   Δ = 2: degree 12, 686 points 1e-7 / 3e-7; degree 13, 855 points 5e-8 / 1e-7
-//   Δ = 3: degree 9, 341 points 4e-8 / 3e-8
-//   Δ = 4: degree 7, 189 points 7e-8 / 3e-8
-//   Δ >= 5: degree 6, 128 points 5e-8 / 3e-8
+// polynomials of degree N.  The degree falls with the gap between the boxes
+// (g² = the squared distance of their nearest points, in boxes): a box two
+// steps away along one axis only is as near as 53 others, one two steps away
+// along two axes already converges three degrees faster.  Truncation error of
+// a class relative to the whole sum, random-sign weights (the worst case),
+// measured in FP64 for the reference / the blob kernel:
+//   g² = 1:        degree 12, 686 points 1e-7 / 3e-7; degree 13, 855 points 4e-8 / 1e-7
+//   g² = 2 .. 4:   degree 9, 341 points 9e-8 / 2e-7; degree 10, 432 points 2e-8 / 6e-8
+//   g² = 5 .. 13:  degree 8, 250 points 3e-8 / 4e-8
+//   g² = 14 .. 99: degree 6, 128 points 7e-8 / 5e-8
+//   g² >= 100:     degree 4, 54 points 6e-8 / 3e-8
+// (reference: 12, 9, 8, 6, 4; blob: 13, 10, 8, 6, 4).  Classes by the steps
+// along the farthest axis (2, 3, 4 and more, degrees 12 or 13, 9, 7, 6) took a
+// fifth more node sums.  Classes that a grid is too small for are not run.
 // The direct FP32 sum of some ten thousand samples is 2e-7 to 4e-7 off; the
-// whole scheme measured 1.6e-7 against 2.3e-7 of the direct loop (205,379
-// targets, 6,418 samples, reference kernel), 2.0e-7 against 3.1e-7 (12,836
-// samples) and 2.8e-7 against 3.9e-7 (ring, blob kernel, 262,144 x 16,384).
+// whole scheme measured 1.8e-7 against 2.3e-7 of the direct loop (205,379
+// targets, 6,418 samples, reference kernel) and 2.7e-7 against 3.9e-7 (ring,
+// blob kernel, 262,144 x 16,384).
 //
 // Far field on one B200, direct loop and boxes:
-//   2.02M targets x 63k samples, reference kernel   51.8 -> 8.0 ms (6,690 of 63,225 pairs a target)
-//   262,144 x 16,384, blob kernel                   2.57 -> 1.21 ms (5,755 of 16,384)
-//   205,379 x 6,418, reference kernel               0.60 -> 0.36 ms (2,516 of 6,418)
+//   2.02M targets x 63k samples, reference kernel   51.8 -> 6.9 ms
+//   262,144 x 16,384, blob kernel                   2.57 -> 1.07 ms
+//   205,379 x 6,418, reference kernel               0.60 -> 0.33 ms
 // The node sums and near pairs are bound by the FP32 pipe as the direct loop
-// is (two f32x2 lanes an instruction, far_x2_loop): 4.8 and 2.5 ms of the 8.0;
+// is (two f32x2 lanes an instruction, far_x2_loop): 3.9 and 2.3 ms of the 6.9;
 // reading the polynomial 0.3, staging the samples 0.2, the projection 0.1.
 // 16 cells on a side would make 8 times larger near parts, 4 cells (512
 // targets) no longer pay for 686 nodes.
@@ -49,7 +55,7 @@
 namespace {
 
 constexpr int kLeafLog = 3;     // 2^3 cells per axis and box
-constexpr int kSets = 4;        // distance classes Δ = 2, 3, 4, >= 5
+constexpr int kSets = 5;        // distance classes
 constexpr int kNearT = 256;     // threads of the near kernel
 constexpr int kNearTT = 4;      // targets per thread: 4 at 114 registers; 6 and 8 were level or slower (a box
                                 // has too few tiles of 1,536 or 2,048), 4 at 80 registers 5% slower (spills)
@@ -70,31 +76,45 @@ struct Cheb {
 // degree of the distance class s
 template <bool BLOB>
 __host__ __device__ constexpr int deg(int s) {
-  return s == 0 ? (BLOB ? 13 : 12) : s == 1 ? 9 : s == 2 ? 7 : 6;
+  return s == 0 ? (BLOB ? 13 : 12) : s == 1 ? (BLOB ? 10 : 9) : s == 2 ? 8 : s == 3 ? 6 : 4;
+}
+template <bool BLOB>
+__host__ __device__ constexpr int pts(int s) {
+  const int ne = (deg<BLOB>(s) + 1) / 2 + 1, no = (deg<BLOB>(s) + 2) / 2;
+  return ne * ne * ne + no * no * no;
 }
 // nodes a thread holds: the even number whose warps are filled best (0.89,
-// 0.89, 0.98 and 1.0 of the lanes; blob class 0: 0.95), and enough independent
-// chains for the FP32 pipe
+// 0.89, 0.98, 1.0 and 0.84 of the lanes; blob: 0.95 and 0.84 in classes 0 and
+// 1), and enough independent chains for the FP32 pipe
 template <bool BLOB>
 __host__ __device__ constexpr int node_tt(int s) {
-  return s == 0 ? (BLOB ? 4 : 8) : s <= 2 ? 6 : 4;
+  return s == 0 ? (BLOB ? 4 : 8) : s == 1 ? (BLOB ? 8 : 6) : s == 2 ? 8 : s == 3 ? 4 : 2;
 }
 // sample stripes (blocks) per box and class where there are many boxes:
-// about two thousand samples each; times dv_farbox::stripe_mul
-__host__ __device__ constexpr int stripes(int s) { return s <= 1 ? 4 : 2; }
+// about a million pairs each; times dv_farbox::stripe_mul
+__host__ __device__ constexpr int stripes(int s) { return s <= 1 ? 4 : s == 2 ? 5 : 3; }
+__host__ __device__ constexpr int all_stripes(int sets) {
+  int n = 0;
+  for (int s = 0; s < sets; ++s) n += stripes(s);
+  return n;
+}
+template <bool BLOB>
+__host__ __device__ constexpr int node_floats() {  // of one box, for stripe_mul 1
+  int n = 0;
+  for (int s = 0; s < kSets; ++s) n += 3 * stripes(s) * pts<BLOB>(s);
+  return n;
+}
 template <bool BLOB>
 struct Sets {
-  static constexpr int P0 = Cheb<deg<BLOB>(0)>::P, P1 = Cheb<deg<BLOB>(1)>::P, P2 = Cheb<deg<BLOB>(2)>::P,
-                       P3 = Cheb<deg<BLOB>(3)>::P;
+  static constexpr int P0 = pts<BLOB>(0);
   static constexpr int K = Cheb<deg<BLOB>(0)>::K;
-  // floats of the node sums of one box, for stripe_mul 1
-  static constexpr int FLOATS = 3 * (stripes(0) * P0 + stripes(1) * P1 + stripes(2) * P2 + stripes(3) * P3);
+  static constexpr int FLOATS = node_floats<BLOB>();
   static constexpr int WARPS = BLOB ? 8 : 6;  // of a node block: two groups of 3 for class 0, blob: one of 7
 };
 constexpr int kCoefMax = Sets<true>::K;
 constexpr int kFloatsMax = Sets<true>::FLOATS;
 
-// node coordinates cos(iπ/m) of the four degrees
+// node coordinates cos(iπ/m) of the degrees
 struct Nodes {
   float c[kSets][16];
 };
@@ -108,8 +128,13 @@ Nodes make_nodes() {
   return t;
 }
 
-__device__ __forceinline__ int box_class(int4 a, int4 b) {  // Δ of two boxes
-  return max(max(abs(a.x - b.x), abs(a.y - b.y)), abs(a.z - b.z));
+// distance class of two boxes, -1 for the 27 near ones
+__host__ __device__ __forceinline__ int gap_class(int g2) {
+  return g2 < 2 ? g2 - 1 : g2 < 5 ? 1 : g2 < 14 ? 2 : g2 < 100 ? 3 : 4;
+}
+__device__ __forceinline__ int box_class(int4 a, int4 b) {
+  const int x = max(abs(a.x - b.x) - 1, 0), y = max(abs(a.y - b.y) - 1, 0), z = max(abs(a.z - b.z) - 1, 0);
+  return gap_class(x * x + y * y + z * z);
 }
 
 // centre of box b and half its edge (eight cells)
@@ -236,18 +261,18 @@ __global__ void __launch_bounds__(128) k_box_cost(dv_farbox B) {
   for (int q = threadIdx.x; q < ns; q += 128) {
     const int d = box_class(me, B.sbox[q]);
     const unsigned long long m = (unsigned long long)B.scnt[q];
-    c += m * (d <= 1   ? nt
-              : d == 2 ? (unsigned long long)Sets<BLOB>::P0
-              : d == 3 ? (unsigned long long)Sets<BLOB>::P1
-              : d == 4 ? (unsigned long long)Sets<BLOB>::P2
-                       : (unsigned long long)Sets<BLOB>::P3);
+    unsigned long long per = nt;
+#pragma unroll
+    for (int s = 0; s < kSets; ++s)
+      if (d == s) per = (unsigned long long)pts<BLOB>(s);
+    c += m * per;
   }
   c = block_sum<unsigned long long>(c);
   if (threadIdx.x == 0) atomicAdd(reinterpret_cast<unsigned long long*>(B.meta + 4), c);
 }
 
 // ---------------------------------------------------------- sample staging
-// Samples of the boxes whose distance class lies in [dlo, dhi], every np-th one
+// Samples of the boxes of distance class `cls`, every np-th one
 // from the part-th on, staged kStage at a time (relative to `org`) as the
 // paired loop reads them; f(m) runs on each staged tile.  They come in turn
 // from 64 equal parts of the list of boxes, so that every running sum is a
@@ -256,8 +281,8 @@ __global__ void __launch_bounds__(128) k_box_cost(dv_farbox B) {
 // (ring of 262,144 targets, blob kernel, stripes of boxes: 7.0e-7 off the
 // FP64 sum against 3.9e-7 of the direct loop, whose draws are in random order).
 template <bool BLOB, int NT, typename F>
-__device__ __forceinline__ void staged_samples(const dv_farbox& B, int4 me, int part, int np, int dlo, int dhi,
-                                               float3 org, float4* s4, int* s_start, int* s_pref, F&& f) {
+__device__ __forceinline__ void staged_samples(const dv_farbox& B, int4 me, int part, int np, int cls, float3 org,
+                                               float4* s4, int* s_start, int* s_pref, F&& f) {
   __shared__ int s_ws[NT / 32];
   const int ns = (int)B.meta[2], tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   for (int base = 0; base < ns; base += NT) {
@@ -265,8 +290,7 @@ __device__ __forceinline__ void staged_samples(const dv_farbox& B, int4 me, int 
     int len = 0, start = 0;
     if (q < ns) {
       const int4 sb = B.sbox[q];
-      const int d = box_class(me, sb);
-      if (d >= dlo && d <= dhi) {
+      if (box_class(me, sb) == cls) {
         len = B.scnt[q];
         start = sb.w;
       }
@@ -357,8 +381,7 @@ __device__ __forceinline__ void node_sums(const dv_params& P, const dv_farbox& B
   }
   const float3 org = make_float3(box_centre(P, me.x, 0), box_centre(P, me.y, 1), box_centre(P, me.z, 2));
   const bool run = grp < G;
-  staged_samples<BLOB, NT>(B, me, part, stripes(S) * B.stripe_mul, S + 2, S == kSets - 1 ? 0x7fffffff : S + 2, org,
-                           s4, s_start, s_pref, [&](int m) {
+  staged_samples<BLOB, NT>(B, me, part, stripes(S) * B.stripe_mul, S, org, s4, s_start, s_pref, [&](int m) {
                              if (run) far_x2_loop<3, NP, BLOB, false>(s4, grp, G, m, PX, PY, PZ, AX, AY, AZ, 0.0f,
                                                                       P.blob_delta2);
                            });
@@ -389,6 +412,18 @@ __device__ __forceinline__ void node_sums(const dv_params& P, const dv_farbox& B
   for (int k = threadIdx.x; k < 3 * Ch::P; k += NT) out[k] = red[k];
 }
 
+// the class and stripe of block row y
+template <bool BLOB, int S>
+__device__ __forceinline__ void node_class(const dv_params& P, const dv_farbox& B, const Nodes& nd, int4 me, int y,
+                                           float* __restrict__ out, float4* s4, int* s_start, int* s_pref) {
+  const int n = B.stripe_mul * stripes(S);
+  if (y < n) {
+    node_sums<BLOB, S>(P, B, nd, me, y, out + 3 * y * pts<BLOB>(S), s4, s_start, s_pref);
+  } else if constexpr (S + 1 < kSets) {
+    node_class<BLOB, S + 1>(P, B, nd, me, y - n, out + 3 * n * pts<BLOB>(S), s4, s_start, s_pref);
+  }
+}
+
 template <bool BLOB>
 __global__ void __launch_bounds__(Sets<BLOB>::WARPS * 32) k_box_nodes(dv_params P, dv_farbox B, Nodes nd,
                                                                       const dv_counters* __restrict__ C) {
@@ -398,20 +433,8 @@ __global__ void __launch_bounds__(Sets<BLOB>::WARPS * 32) k_box_nodes(dv_params 
   static_assert(sizeof(s4) >= sizeof(float) * 3 * St::P0, "node sums fit the staging buffer");
   const int a = blockIdx.x;
   if (!farbox_on(B, C) || a >= (int)B.meta[1]) return;  // uniform per CTA
-  const int4 me = B.tbox[a];
-  const int r = B.stripe_mul;
-  float* out = B.nodes + (int64_t)a * St::FLOATS * r;
-  int y = blockIdx.y;
-  if (y < r * stripes(0)) return node_sums<BLOB, 0>(P, B, nd, me, y, out + 3 * y * St::P0, s4, s_start, s_pref);
-  y -= r * stripes(0);
-  out += 3 * r * stripes(0) * St::P0;
-  if (y < r * stripes(1)) return node_sums<BLOB, 1>(P, B, nd, me, y, out + 3 * y * St::P1, s4, s_start, s_pref);
-  y -= r * stripes(1);
-  out += 3 * r * stripes(1) * St::P1;
-  if (y < r * stripes(2)) return node_sums<BLOB, 2>(P, B, nd, me, y, out + 3 * y * St::P2, s4, s_start, s_pref);
-  y -= r * stripes(2);
-  out += 3 * r * stripes(2) * St::P2;
-  node_sums<BLOB, 3>(P, B, nd, me, y, out + 3 * y * St::P3, s4, s_start, s_pref);
+  node_class<BLOB, 0>(P, B, nd, B.tbox[a], blockIdx.y, B.nodes + (int64_t)a * St::FLOATS * B.stripe_mul, s4, s_start,
+                      s_pref);
 }
 
 // ------------------------------------------------------------ coefficients
@@ -478,6 +501,14 @@ __device__ void project(const float* __restrict__ sums, int np, double* s_coef, 
 }
 
 constexpr int kProjT = 256;
+template <bool BLOB, int S>
+__device__ __forceinline__ void project_all(const float* __restrict__ sums, int sets, int e, int r, double* s_coef, double* s_f,
+                                            double* s_g1, double* s_g2, double* s_A) {
+  if (S >= sets) return;
+  project<BLOB, S, kProjT>(sums + e * pts<BLOB>(S), r * stripes(S), s_coef, s_f, s_g1, s_g2, s_A);
+  if constexpr (S + 1 < kSets)
+    project_all<BLOB, S + 1>(sums + 3 * r * stripes(S) * pts<BLOB>(S), sets, e, r, s_coef, s_f, s_g1, s_g2, s_A);
+}
 // block (box, component)
 template <bool BLOB>
 __global__ void __launch_bounds__(kProjT) k_box_coefs(dv_farbox B, const dv_counters* __restrict__ C) {
@@ -488,13 +519,7 @@ __global__ void __launch_bounds__(kProjT) k_box_coefs(dv_farbox B, const dv_coun
   if (!farbox_on(B, C) || a >= (int)B.meta[1]) return;
   for (int k = threadIdx.x; k < St::K; k += kProjT) s_coef[k] = 0.0;
   const float* sums = B.nodes + (int64_t)a * St::FLOATS * r;
-  project<BLOB, 0, kProjT>(sums + e * St::P0, r * stripes(0), s_coef, s_f, s_g1, s_g2, s_A);
-  sums += 3 * r * stripes(0) * St::P0;
-  project<BLOB, 1, kProjT>(sums + e * St::P1, r * stripes(1), s_coef, s_f, s_g1, s_g2, s_A);
-  sums += 3 * r * stripes(1) * St::P1;
-  project<BLOB, 2, kProjT>(sums + e * St::P2, r * stripes(2), s_coef, s_f, s_g1, s_g2, s_A);
-  sums += 3 * r * stripes(2) * St::P2;
-  project<BLOB, 3, kProjT>(sums + e * St::P3, r * stripes(3), s_coef, s_f, s_g1, s_g2, s_A);
+  project_all<BLOB, 0>(sums, B.sets, e, r, s_coef, s_f, s_g1, s_g2, s_A);
   float* out = reinterpret_cast<float*>(B.coef + (int64_t)a * St::K) + e;
   for (int k = threadIdx.x; k < St::K; k += kProjT) out[4 * k] = (float)s_coef[k];
 }
@@ -596,7 +621,7 @@ __global__ void __launch_bounds__(kNearT, 2) k_box_near(dv_params P, dv_farbox B
   }
   const bool run = tw < nt;
   const float lim = P.far_r2_limit;
-  staged_samples<BLOB, kNearT>(B, me, blockIdx.y, gridDim.y, 0, 1, make_float3(0.f, 0.f, 0.f), s4, s_start, s_pref,
+  staged_samples<BLOB, kNearT>(B, me, blockIdx.y, gridDim.y, -1, make_float3(0.f, 0.f, 0.f), s4, s_start, s_pref,
                                [&](int m) {
                                  if (run) far_x2_loop<3, NP, BLOB, true>(s4, 0, 1, m, PX, PY, PZ, AX, AY, AZ, lim,
                                                                         P.blob_delta2);
@@ -698,6 +723,12 @@ int dv_farbox_create(dv_ctx* c) {
   al(&B.tile0, B.max_boxes);
   al(&B.sbox, nbox);
   al(&B.scnt, nbox);
+  int g2 = 0;  // the farthest boxes of this grid
+  for (int d = 0; d < 3; ++d) {
+    const int gap = std::max((P.grid_num[d] + (1 << kLeafLog) - 1 >> kLeafLog) - 2, 0);
+    g2 += gap * gap;
+  }
+  B.sets = std::max(gap_class(g2) + 1, 1);
   // few boxes: more stripes, so that the node sums fill the chip
   B.stripe_mul = B.max_boxes <= 96 ? 4 : B.max_boxes <= 256 ? 2 : 1;
   al(&B.nodes, (int64_t)B.max_boxes * kFloatsMax * B.stripe_mul);
@@ -770,7 +801,7 @@ template <bool BLOB>
 static int run(dv_ctx* c, const dv_fields* f) {
   dv_farbox& B = c->farbox;
   const Nodes nd = make_nodes<BLOB>();
-  const dim3 gn(B.max_boxes, B.stripe_mul * (stripes(0) + stripes(1) + stripes(2) + stripes(3)));
+  const dim3 gn(B.max_boxes, B.stripe_mul * all_stripes(B.sets));
   k_box_nodes<BLOB><<<gn, Sets<BLOB>::WARPS * 32, 0, c->stream>>>(c->p, B, nd, c->d_cnt);
   DV_LAUNCHED(c);
   k_box_coefs<BLOB><<<dim3(B.max_boxes, 3), kProjT, 0, c->stream>>>(B, c->d_cnt);

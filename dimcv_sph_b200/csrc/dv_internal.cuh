@@ -25,6 +25,7 @@
 struct dv_farbox {
   int enabled = 0;
   int nbox = 0, lowbits = 0, max_boxes = 0, stripe_mul = 1;
+  int sets = 1;  // distance classes that the grid is large enough for
   // [0] a position or weight that needs the direct loop; [1] boxes with
   // targets, [2] boxes with samples, [3] near tiles; [4..5] pair evaluations (u64)
   uint32_t* meta = nullptr;
