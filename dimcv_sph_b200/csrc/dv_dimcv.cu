@@ -285,14 +285,20 @@ __device__ __forceinline__ float epan(const dv_params& P, V3 r) {
 
 // kden_sum from the FP64 block sums (the reference accumulates it with an f32
 // atomic add)
-__device__ __forceinline__ void akde_end(dv_counters* C, double* part, uint32_t* ctr, double block_kden) {
-  if (threadIdx.x == 0) part[blockIdx.x] = block_kden;
-  if (!last_block(ctr)) return;
-  const double s = sum_partials(part, gridDim.x);
+__device__ __forceinline__ void akde_sum(dv_counters* C, const double* part, int nparts) {
+  const double s = sum_partials(part, nparts);
   if (threadIdx.x == 0) {
     C->kden_sum = s;
     C->kden_sum_f32 = (float)s;
   }
+}
+// ctr: in the last block, null: in k_akde_end
+__device__ __forceinline__ void akde_end(dv_counters* C, double* part, uint32_t* ctr, double block_kden) {
+  if (threadIdx.x == 0) part[blockIdx.x] = block_kden;
+  if (ctr && last_block(ctr)) akde_sum(C, part, gridDim.x);
+}
+__global__ void __launch_bounds__(DV_THREADS) k_akde_end(const double* part, int nparts, dv_counters* C) {
+  akde_sum(C, part, nparts);
 }
 
 // compute_kernel_density (dimcv_sph.py:732-751) and kden_sum
@@ -637,7 +643,11 @@ DV_API int dv_akde(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s) {
   if (!c || !f) return DV_EINVAL;
   if (int rc = check_solver(c, s)) return rc;
   const int nb = nblk(c);
-  LAUNCH_D(k_akde, nb, c->p, dv_grid(c), *f, *s, c->d_cnt, c->red_part, c->look_ctl + 3);
+  LAUNCH_D(k_akde, nb, c->p, dv_grid(c), *f, *s, c->d_cnt, c->red_part, fold_end(c, nb) ? c->look_ctl + 3 : nullptr);
+  if (!fold_end(c, nb)) {
+    k_akde_end<<<1, DV_THREADS, 0, c->stream>>>(c->red_part, nb, c->d_cnt);
+    DV_LAUNCHED(c);
+  }
   return DV_OK;
 }
 
@@ -646,7 +656,11 @@ DV_API int dv_smooth_akde(dv_ctx* c, const dv_fields* f, const dv_solver_fields*
   if (int rc = check_solver(c, s)) return rc;
   const int nb = nblk(c);
   if (int rc = dv_pack(c, f, s, DV_PK_XV | DV_PK_DW)) return rc;
-  LAUNCH_D(k_smooth_akde, nb, c->p, dv_grid(c), *f, *s, dv_packs(c), c->d_cnt, c->red_part, c->look_ctl + 3);
+  LAUNCH_D(k_smooth_akde, nb, c->p, dv_grid(c), *f, *s, dv_packs(c), c->d_cnt, c->red_part, fold_end(c, nb) ? c->look_ctl + 3 : nullptr);
+  if (!fold_end(c, nb)) {
+    k_akde_end<<<1, DV_THREADS, 0, c->stream>>>(c->red_part, nb, c->d_cnt);
+    DV_LAUNCHED(c);
+  }
   return DV_OK;
 }
 

@@ -3,7 +3,7 @@
 // stable LSD radix sort on Morton cell keys (one launch a pass: warp-level
 // __match_any_sync ranks, a look-back over the tiles' digit counts, stable
 // scatter), the cell table, the permutation of all particle fields, emission
-// and CSR neighbour lists.
+// and neighbour lists.
 #include <algorithm>
 
 #include "dv_far.cuh"
@@ -215,15 +215,37 @@ __global__ void __launch_bounds__(RS_T) k_rs_pass(const uint32_t* __restrict__ k
   }
 }
 
+// The new counts from the blocks' counts, and the state of the lists.
+__device__ __forceinline__ void permute_end(const int32_t* part, int nparts, dv_counters* C, uint32_t* ctl,
+                                            int32_t* ok) {
+  int fl = 0, so = 0;
+  for (int k = threadIdx.x; k < nparts; k += blockDim.x) {
+    fl += __ldcg(part + 2 * k);
+    so += __ldcg(part + 2 * k + 1);
+  }
+  fl = block_sum<int>(fl);
+  so = block_sum<int>(so);
+  if (threadIdx.x == 0) {
+    C->n = (int)__ldcg(ctl + 4);
+    C->n_fluid = fl;
+    C->n_solid = so;
+    ctl[4] = 0u;
+    ctl[2] = 0u;  // entries of long rows used by the list build
+    ok[0] = 1;    // until the list build finds otherwise
+    ok[1] = 1;    // the sorted keys are those of the current slots
+  }
+}
+
 // The cell table from the sorted keys, every dv_fields array gathered into the
-// new order, and the new counts, in the last block.  Slots in [n_new, n_old) receive the
+// new order, and the new counts (fold: in the last block, else k_permute_end).
+// Slots in [n_new, n_old) receive the
 // reference's partition fill values (particle_system.py:455-465) for the
 // filled fields and keep their own values for the others.
 template <int D>
 __global__ void k_permute(dv_fields S, dv_fields T, const uint32_t* __restrict__ perm,
                           const uint32_t* __restrict__ keys, uint32_t invalid, int n_old_cap, dv_counters* C,
                           int32_t* __restrict__ cstart, int32_t* __restrict__ cend, int32_t* part, uint32_t* ctl,
-                          int32_t* __restrict__ ok) {
+                          int32_t* __restrict__ ok, bool fold) {
   const int VS = D == 2 ? 2 : 4;
   int p = blockIdx.x * blockDim.x + threadIdx.x;
   const int n_old = C->n;  // the sorted range; keys past it are stale
@@ -293,29 +315,18 @@ __global__ void k_permute(dv_fields S, dv_fields T, const uint32_t* __restrict__
     part[2 * blockIdx.x] = sfl;
     part[2 * blockIdx.x + 1] = sso;
   }
-  if (!last_block(ctl + 3)) return;
-  fl = so = 0;
-  for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) {
-    fl += __ldcg(part + 2 * k);
-    so += __ldcg(part + 2 * k + 1);
-  }
-  fl = block_sum<int>(fl);
-  so = block_sum<int>(so);
-  if (threadIdx.x == 0) {
-    C->n = (int)__ldcg(ctl + 4);
-    C->n_fluid = fl;
-    C->n_solid = so;
-    ctl[4] = 0u;
-    ctl[2] = 0u;  // entries of long rows used by the list build
-    ok[0] = 1;    // until the list build finds otherwise
-    ok[1] = 1;    // the sorted keys are those of the current slots
-  }
+  if (fold && last_block(ctl + 3)) permute_end(part, gridDim.x, C, ctl, ok);
+}
+
+__global__ void __launch_bounds__(1024) k_permute_end(const int32_t* part, int nparts, dv_counters* C,
+                                                            uint32_t* ctl, int32_t* ok) {
+  permute_end(part, nparts, C, ctl, ok);
 }
 
 // ------------------------------------------------- per-step neighbour lists
 // After the sort, every sweep of the step visits the same neighbour sets in
 // the same order, so the cell scan (3^d cells) is done once here and the
-// sweeps read the lists as CSR (offsets = exclusive scan of the counts).
+// sweeps read the lists.
 //
 // Each entry carries the neighbour's material in its top bit (DV_NBR_SOLID),
 // so the sweeps do not gather it; a material other than fluid or solid makes
@@ -325,8 +336,8 @@ __global__ void k_permute(dv_fields S, dv_fields T, const uint32_t* __restrict__
 // fluid particle (or, for the rigid coupling, a dynamic solid) at its centre,
 // and the static boundary volume (once, at initialisation) scans cells.
 //
-// One launch: k_csr_rows (3-D), k_csr_build (2-D).  k_permute has set
-// the lists valid before it; a build that cannot store them takes that back.
+// One launch: k_csr_rows (3-D), k_csr_build (2-D).  permute_end has
+// set the lists valid before it; a build that cannot store them takes that back.
 __device__ __forceinline__ bool nbr_row_built(const int32_t* __restrict__ mat, const uint8_t* __restrict__ dyn,
                                               int i) {
   return !(mat[i] == DV_MATERIAL_SOLID && !dyn[i]);
@@ -662,13 +673,17 @@ DV_API int dv_grid_build(dv_ctx* c, const dv_fields* src, const dv_fields* dst) 
 #define PERM(DD)                                                                                                     \
   k_permute<DD><<<nb, DV_THREADS, 0, c->stream>>>(*src, *dst, c->vals[cur], c->keys[cur], invalid, (int)c->cap,      \
                                                   c->d_cnt, c->cell_start, c->cell_end, c->ired_part, c->look_ctl, \
-                                                  c->d_nbr_ok)
+                                                  c->d_nbr_ok, fold_end(c, nb))
   if (c->p.dim == 2)
     PERM(2);
   else
     PERM(3);
 #undef PERM
   DV_LAUNCHED(c);
+  if (!fold_end(c, nb)) {
+    k_permute_end<<<1, 1024, 0, c->stream>>>(c->ired_part, nb, c->d_cnt, c->look_ctl, c->d_nbr_ok);
+    DV_LAUNCHED(c);
+  }
   c->scene_ptr = batch ? dst->object_id : nullptr;  // scene of each sorted slot
   return build_csr(c, dst);
 }

@@ -682,9 +682,12 @@ __device__ __forceinline__ T block_sum(T v) {
 
 // ------------------------------------------------- last block of a launch
 // True in every thread of the block that finishes last, which sees what the
-// others wrote; *ctr is zero before and after.  A sum of block partials ends in
-// the kernel that makes them: a launch of one block for it cost 2 us, and as
-// much again between the launches.
+// others wrote; *ctr is zero before and after.  With few blocks a sum of block
+// partials ends in the kernel that makes them (fold_end): a launch of one block
+// for it cost 2 us, and as much again between the launches (2-D step of 10,000
+// particles 391 -> 353 us).  With many blocks the launch is the cheaper: every
+// block waits at its end until its stores have arrived, which made the residual
+// sweep of 2.37M particles 175 -> 200 us, that of 0.75M 62 -> 64.
 __device__ __forceinline__ bool last_block(uint32_t* ctr) {
   __shared__ bool s_last;
   __syncthreads();
@@ -697,6 +700,8 @@ __device__ __forceinline__ bool last_block(uint32_t* ctr) {
   __syncthreads();
   return s_last;
 }
+static inline bool fold_end(const dv_ctx* c, int blocks) { return blocks <= 4 * c->num_sms; }
+
 // Sum of n block partials in thread 0 of a block of DV_THREADS, in the order of
 // a block of 1,024 (thread k adds k, k + 1,024, ...; then the tree).
 __device__ __forceinline__ double sum_partials(const double* part, int n) {

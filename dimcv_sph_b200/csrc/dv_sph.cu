@@ -210,20 +210,18 @@ __global__ void k_scale_factor(dv_fields F, float s, dv_counters* C, int32_t* do
 }
 
 // The convergence test of one Jacobi iteration, in the last block of its
-// residual sweep: average error over the fluid count against eta; sets the
+// residual sweep (ctr) or in k_solve_end: average error over the fluid count against eta; sets the
 // done flag at convergence or at max_iter.
 struct SolveEnd {
   double* part;  // block partials of the error
   dv_counters* C;
   int32_t* done;
-  uint32_t* ctr;
+  uint32_t* ctr;  // null: a launch of its own
   double eta;
   int max_iter, which;
 };
-__device__ __forceinline__ void solve_end(const SolveEnd& E, double block_err) {
-  if (threadIdx.x == 0) E.part[blockIdx.x] = block_err;
-  if (!last_block(E.ctr)) return;
-  const double s = sum_partials(E.part, gridDim.x);
+__device__ __forceinline__ void solve_test(const SolveEnd& E, int nparts) {
+  const double s = sum_partials(E.part, nparts);
   if (threadIdx.x == 0) {
     dv_counters* C = E.C;
     const int nf = C->n_fluid;
@@ -241,6 +239,13 @@ __device__ __forceinline__ void solve_end(const SolveEnd& E, double block_err) {
       C->status |= (E.which == 0 ? DV_WARN_DIV_NOT_CONVERGED : DV_WARN_P_NOT_CONVERGED);
     }
   }
+}
+__global__ void __launch_bounds__(DV_THREADS) k_solve_end(SolveEnd E, int nparts) {
+  if (!*E.done) solve_test(E, nparts);
+}
+__device__ __forceinline__ void solve_end(const SolveEnd& E, double block_err) {
+  if (threadIdx.x == 0) E.part[blockIdx.x] = block_err;
+  if (E.ctr && last_block(E.ctr)) solve_test(E, gridDim.x);
 }
 
 // ------------------------------------------------------- density change
@@ -888,8 +893,8 @@ DV_API int dv_pressure_iteration(dv_ctx* c, const dv_fields* f) {
 }
 
 // Runs Jacobi iterations in chunks of 2, 4, 8, ... launches; every iteration
-// is an update sweep and a residual sweep, whose last block tests for
-// convergence; both return at once when the done flag is set.  The caller's
+// is an update sweep and a residual sweep with the convergence test (SolveEnd);
+// both return at once when the done flag is set.  The caller's
 // scaling of the factors has reset the flag.  3-D: the packed copies are
 // made here (pressure: the caller's opening sweep left K.a and K.b), and the
 // residual sweeps keep K.k and the pressure updates K.b current.
@@ -898,7 +903,8 @@ static int jacobi_loop(dv_ctx* c, const dv_fields* f, int which, bool nonpressur
   const int max_iter = which == 0 ? c->p.max_iter_div : c->p.max_iter_p;
   const double eta = which == 0 ? c->p.eta_div : c->p.eta_p;
   int32_t* done = c->d_flag;
-  const SolveEnd E{c->red_part, c->d_cnt, done, c->look_ctl + 3, eta, max_iter, which};
+  const bool fold = fold_end(c, nb);
+  const SolveEnd E{c->red_part, c->d_cnt, done, fold ? c->look_ctl + 3 : nullptr, eta, max_iter, which};
   const DevPack K = dv_packs(c);
   if (int rc = dv_pack(c, f, nullptr, which == 0 ? DV_PK_XV | DV_PK_DIV : DV_PK_P)) return rc;
   int launched = 0, chunk = 2;
@@ -915,6 +921,10 @@ static int jacobi_loop(dv_ctx* c, const dv_fields* f, int which, bool nonpressur
         LAUNCH_D(k_pressure_iter, nb, c->p, dv_grid(c), *f, K, c->d_cnt, (const int32_t*)done);
         if (c->dyn_rigid) LAUNCH_D(k_rigid_reaction, nb, c->p, dv_grid(c), *f, c->d_cnt, (const int32_t*)done);
         LAUNCH_DN(k_density_adv, true, nb, c->p, dv_grid(c), *f, K, c->d_cnt, E);
+      }
+      if (!fold) {
+        k_solve_end<<<1, DV_THREADS, 0, c->stream>>>(E, nb);
+        DV_LAUNCHED(c);
       }
     }
     launched += m;
