@@ -127,6 +127,7 @@ DV_API void dv_destroy(dv_ctx* c) {
   if (c->d_prof) cudaFree(c->d_prof);
   if (c->h_cnt) cudaFreeHost(c->h_cnt);
   if (c->h_flag) cudaFreeHost(c->h_flag);
+  if (c->h_solve) cudaFreeHost(c->h_solve);
   delete c;
 }
 
@@ -223,6 +224,8 @@ DV_API dv_ctx* dv_create(const dv_params* params, int64_t capacity, void* stream
 #undef A
   if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_cnt, sizeof(dv_counters));
   if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_flag, sizeof(int32_t) * 4);
+  if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_solve, sizeof(unsigned long long));
+  if (e == cudaSuccess) *c->h_solve = 0;
   if (e == cudaSuccess) e = cudaMemset(c->d_cnt, 0, sizeof(dv_counters));
   if (e == cudaSuccess) e = cudaMemset(c->d_flag, 0, sizeof(int32_t) * 4);
   if (e == cudaSuccess) e = cudaMemset(c->look_state, 0, sizeof(unsigned long long) * look_tiles);

@@ -54,6 +54,8 @@ struct dv_ctx {
   dv_counters* h_cnt = nullptr;  // pinned mirror
   int32_t* d_flag = nullptr;     // [0]: solve done flag, [1]: scratch
   int32_t* h_flag = nullptr;     // pinned mirror
+  unsigned long long* h_solve = nullptr;  // pinned: progress of the Jacobi solve (SolveEnd)
+  uint32_t solve_seq = 0;
 
   // grid / sort
   uint32_t* keys[2] = {nullptr, nullptr};

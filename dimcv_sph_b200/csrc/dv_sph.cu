@@ -219,6 +219,8 @@ struct SolveEnd {
   uint32_t* ctr;  // null: a launch of its own
   double eta;
   int max_iter, which;
+  unsigned long long* host;  // pinned: solve << 32 | done << 31 | iterations, after each test
+  uint32_t solve;
 };
 __device__ __forceinline__ void solve_test(const SolveEnd& E, int nparts) {
   const double s = sum_partials(E.part, nparts);
@@ -238,6 +240,9 @@ __device__ __forceinline__ void solve_test(const SolveEnd& E, int nparts) {
       *E.done = 1;
       C->status |= (E.which == 0 ? DV_WARN_DIV_NOT_CONVERGED : DV_WARN_P_NOT_CONVERGED);
     }
+    __threadfence_system();
+    *reinterpret_cast<volatile unsigned long long*>(E.host) =
+        (unsigned long long)E.solve << 32 | (*E.done ? 1ull << 31 : 0ull) | (unsigned)it;
   }
 }
 __global__ void __launch_bounds__(DV_THREADS) k_solve_end(SolveEnd E, int nparts) {
@@ -892,6 +897,31 @@ DV_API int dv_pressure_iteration(dv_ctx* c, const dv_fields* f) {
   return DV_OK;
 }
 
+// Waits for the test after iteration `launched` of solve E (or an earlier one
+// that ended it).  The tests write their result to pinned memory, which the
+// host reads without a copy and a synchronisation of the stream; a stream that
+// has nothing left, or failed, ends the wait.
+static int solve_poll(dv_ctx* c, const SolveEnd& E, int launched, bool* over) {
+  const volatile unsigned long long* h = c->h_solve;
+  for (int spins = 0;; ++spins) {
+    const unsigned long long v = *h;
+    if ((uint32_t)(v >> 32) == E.solve && ((v >> 31 & 1) || (int)(v & 0x7fffffff) >= launched)) {
+      *over = v >> 31 & 1;
+      return DV_OK;
+    }
+    if (spins % 1024 == 1023) {
+      const cudaError_t e = cudaStreamQuery(c->stream);
+      if (e == cudaErrorNotReady) continue;
+      if (e != cudaSuccess) return dv_cuda_check(c, e, "Jacobi loop");
+      break;
+    }
+  }
+  DV_CK(c, cudaMemcpyAsync(c->h_flag, E.done, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
+  DV_CK(c, cudaStreamSynchronize(c->stream));
+  *over = *c->h_flag != 0;
+  return DV_OK;
+}
+
 // Runs Jacobi iterations in chunks of 2, 4, 8, ... launches; every iteration
 // is an update sweep and a residual sweep with the convergence test (SolveEnd);
 // both return at once when the done flag is set.  The caller's
@@ -904,7 +934,8 @@ static int jacobi_loop(dv_ctx* c, const dv_fields* f, int which, bool nonpressur
   const double eta = which == 0 ? c->p.eta_div : c->p.eta_p;
   int32_t* done = c->d_flag;
   const bool fold = fold_end(c, nb);
-  const SolveEnd E{c->red_part, c->d_cnt, done, fold ? c->look_ctl + 3 : nullptr, eta, max_iter, which};
+  const SolveEnd E{c->red_part, c->d_cnt, done, fold ? c->look_ctl + 3 : nullptr, eta, max_iter, which, c->h_solve,
+                   ++c->solve_seq};
   const DevPack K = dv_packs(c);
   if (int rc = dv_pack(c, f, nullptr, which == 0 ? DV_PK_XV | DV_PK_DIV : DV_PK_P)) return rc;
   int launched = 0, chunk = 2;
@@ -929,9 +960,9 @@ static int jacobi_loop(dv_ctx* c, const dv_fields* f, int which, bool nonpressur
     }
     launched += m;
     if (launched >= max_iter) break;
-    DV_CK(c, cudaMemcpyAsync(c->h_flag, done, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-    DV_CK(c, cudaStreamSynchronize(c->stream));
-    if (*c->h_flag) break;
+    bool over = false;
+    if (int rc = solve_poll(c, E, launched, &over)) return rc;
+    if (over) break;
     chunk *= 2;
   }
   return DV_OK;
