@@ -4,7 +4,7 @@
 // the reference's operation order (compiled with -fmad=false, IEEE div/sqrt).
 // The Jacobi loops run on the device: every iteration kernel returns at once
 // when the solve's done flag is set, so the host launches iterations in
-// chunks and polls the flag once per chunk instead of once per iteration.
+// chunks and waits for their outcome once per chunk instead of once per iteration.
 #include <algorithm>
 
 #include "dv_internal.cuh"
