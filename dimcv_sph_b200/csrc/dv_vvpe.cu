@@ -893,7 +893,10 @@ DV_API int dv_autotune(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s,
   const int cand[4] = {2, 4, 6, 8};
   float best = 1e30f;
   int best_t = c->far_tt, best_c = c->far_chunks;
-  for (int nc = 1; nc <= DV_MAX_FAR_CHUNKS; nc += nc < 4 ? 1 : 2) {  // 1, 2, 3, 4, 6, 8
+  // every chunk count: a grid of two to four waves of blocks can waste most of its
+  // last one (62,500 targets: 41 tiles of 1,536 on 296 resident blocks are one
+  // wave with 7 chunks, 78 us, and 1.1 with 8; 1, 2, 3, 4, 6 and 8 alone gave 92)
+  for (int nc = 1; nc <= DV_MAX_FAR_CHUNKS; ++nc) {
     c->far_chunks = nc;
     for (int tt : cand) {
       for (int rep = 0; rep < 3; ++rep) {
