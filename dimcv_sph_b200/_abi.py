@@ -13,6 +13,7 @@ DV_ECAPACITY = -2
 DV_ECUDA = -3
 DV_ENAN = -4
 DV_EUNSUPPORTED = -5
+DV_EWAIT = -6
 
 DV_WARN_DIV_NOT_CONVERGED = 1 << 0
 DV_WARN_P_NOT_CONVERGED = 1 << 1
@@ -20,6 +21,7 @@ DV_WARN_OUTSIDE_GRID = 1 << 2
 DV_WARN_CAPACITY = 1 << 3
 DV_WARN_NAN = 1 << 4
 DV_WARN_BAD_INDEX = 1 << 5
+DV_WARN_WAIT = 1 << 6
 
 DV_SAMPLE_BERNOULLI = 0
 DV_SAMPLE_INVERSE_CDF = 1

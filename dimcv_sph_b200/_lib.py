@@ -31,6 +31,7 @@ PROTOTYPES = {
     "dv_get_counters": (C.c_int, [_P, C.POINTER(DvCounters)]),
     "dv_set_counts": (C.c_int, [_P, i32, i32, i32]),
     "dv_clear_status": (C.c_int, [_P]),
+    "dv_set_wait_limit": (C.c_int, [_P, i64]),
     "dv_add_particles": (C.c_int, [_P, _FP, _P, _P, i32, i32, f32, f32, i32, i32, i32, i32, i32, f32]),
     "dv_update_activity": (C.c_int, [_P, _FP]),
     "dv_grid_build": (C.c_int, [_P, _FP, _FP]),

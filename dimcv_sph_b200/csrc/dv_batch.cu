@@ -591,7 +591,8 @@ DV_API int dv_batch_read(dv_ctx* c, dv_scene_state* out, int32_t n_scenes, int64
   }
   int64_t st = 0;
   DV_CK(c, cudaMemcpyAsync(&st, b->d_step, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
+  DV_CK(c, cudaMemcpyAsync(c->h_cnt, c->d_cnt, sizeof(dv_counters), cudaMemcpyDeviceToHost, c->stream));
   DV_CK(c, cudaStreamSynchronize(c->stream));
   if (step) *step = st;
-  return DV_OK;
+  return dv_wait_status(c, c->h_cnt->status);
 }

@@ -254,6 +254,18 @@ DV_API int dv_get_counters(dv_ctx* c, dv_counters* out) {
   DV_CK(c, cudaStreamSynchronize(c->stream));
   *out = *c->h_cnt;
   c->n_upper = c->batch ? c->cap : out->n;  // a scene batch keeps capacity-sized launch shapes
+  return dv_wait_status(c, out->status);
+}
+
+int dv_wait_status(dv_ctx* c, int32_t status) {
+  if (!(status & DV_WARN_WAIT)) return DV_OK;
+  return dv_fail(c, DV_EWAIT, "a wait between the blocks of a kernel ran out; results since then are not valid");
+}
+
+DV_API int dv_set_wait_limit(dv_ctx* c, int64_t polls) {
+  if (!c) return DV_EINVAL;
+  if (polls < 0 || polls > (int64_t)1 << 31) return dv_fail(c, DV_EINVAL, "dv_set_wait_limit: %lld polls", (long long)polls);
+  c->look_spins = (uint32_t)polls;
   return DV_OK;
 }
 
@@ -404,10 +416,10 @@ int dv_scan_cdf(dv_ctx* c, const int32_t* targets, const float* kden, double* ou
 // uint32: one launch, 8 consecutive elements a thread.
 template <int T>
 __global__ void __launch_bounds__(T) k_scan_u32(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, int m,
-                                                  unsigned long long* state, uint32_t* ctl, dv_counters* C) {
+                                                  DevLook K) {
   constexpr int W = T / 32;
   __shared__ uint32_t s_w[W];
-  const int tile = look_tile(ctl), tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int tile = look_tile(K.ctl), tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int64_t e0 = (int64_t)tile * (8 * T) + 8 * tid;
   uint32_t v[8];
   uint32_t sum = 0;
@@ -434,7 +446,7 @@ __global__ void __launch_bounds__(T) k_scan_u32(const uint32_t* __restrict__ in,
     before += k < w ? s_w[k] : 0u;
     total += s_w[k];
   }
-  uint32_t run = look_prefix<T>(state, tile, total, &C->status) + before + inc - sum;
+  uint32_t run = look_prefix<T>(K, tile, total) + before + inc - sum;
   if (e0 + 8 <= m) {
     uint32_t o[8];
 #pragma unroll
@@ -451,7 +463,8 @@ __global__ void __launch_bounds__(T) k_scan_u32(const uint32_t* __restrict__ in,
       run += v[k];
     }
   }
-  look_end(state, ctl);
+  if (look_end(K) && look_failed(K.C))
+    for (int e = tid; e < m; e += T) out[e] = 0u;
 }
 
 // in and out start on 16 bytes (both are whole allocations here)
@@ -459,11 +472,9 @@ int dv_scan_u32(dv_ctx* c, const uint32_t* in, uint32_t* out, int64_t m) {
   if (m <= 0) return DV_OK;
   if (m > c->cap + 1) return dv_fail(c, DV_ECAPACITY, "scan of %lld elements too large", (long long)m);
   if (look_wide(m))
-    k_scan_u32<1024><<<(unsigned)((m + 8191) / 8192), 1024, 0, c->stream>>>(in, out, (int)m, c->look_state,
-                                                                           c->look_ctl, c->d_cnt);
+    k_scan_u32<1024><<<(unsigned)((m + 8191) / 8192), 1024, 0, c->stream>>>(in, out, (int)m, dv_look(c));
   else
-    k_scan_u32<256><<<(unsigned)((m + 2047) / 2048), 256, 0, c->stream>>>(in, out, (int)m, c->look_state, c->look_ctl,
-                                                                         c->d_cnt);
+    k_scan_u32<256><<<(unsigned)((m + 2047) / 2048), 256, 0, c->stream>>>(in, out, (int)m, dv_look(c));
   DV_LAUNCHED(c);
   return DV_OK;
 }

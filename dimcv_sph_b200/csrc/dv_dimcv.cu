@@ -213,34 +213,28 @@ __global__ void k_kvn_sample(dv_params P, dv_fields F, dv_solver_fields S,
 // Lists of slots in ascending order, one launch each (look_compact); flags,
 // a scan of three launches, a compaction and a count before.
 template <int T>
-__global__ void __launch_bounds__(T) k_sample_list(const dv_fields F, dv_counters* C, int m,
-                                                     unsigned long long* state, uint32_t* ctl,
-                                                     int32_t* __restrict__ out) {
-  const int n = C->n;
-  look_compact<T, false>(
-      m, state, ctl, &C->status, nullptr, &C->num_samples, [&](int i) { return i < n && F.is_sample[i] == 1; },
-      [&](int i, uint32_t pos) { out[pos] = i; });
+__global__ void __launch_bounds__(T) k_sample_list(const dv_fields F, int m, DevLook K, int32_t* __restrict__ out) {
+  const int n = K.C->n;
+  look_compact<T, false>(m, K, nullptr, &K.C->num_samples, out, m,
+                         [&](int i) { return i < n && F.is_sample[i] == 1; });
 }
 
 // CHECK: also tell the far field on boxes of a target outside its sorted box,
 // and keep every slot's place (offs)
 template <int D, bool CHECK, int T>
-__global__ void __launch_bounds__(T) k_target_list(dv_params P, const dv_fields F, dv_counters* C, int m,
-                                                     unsigned long long* state, uint32_t* ctl,
+__global__ void __launch_bounds__(T) k_target_list(dv_params P, const dv_fields F, int m, DevLook K,
                                                      int32_t* __restrict__ out, uint32_t* __restrict__ offs, DevGrid G,
                                                      const uint32_t* __restrict__ keys, dv_farbox B) {
-  const int n = C->n;
+  const int n = K.C->n;
   look_compact<T, CHECK>(
-      m, state, ctl, &C->status, offs, &C->n_targets,
-      [&](int i) {
+      m, K, offs, &K.C->n_targets, out, m - 1, [&](int i) {
         if (i >= n || F.material[i] != DV_MATERIAL_FLUID) return false;
         if (!CHECK && !P.has_vortex_domain) return true;
         const V3 x = ldv<D>(F.x, i);
         if (!in_vortex_domain<D>(P, x)) return false;
         if (CHECK && !in_sorted_box(P, G, x, keys[i], B.lowbits)) B.meta[0] = 1u;
         return true;
-      },
-      [&](int i, uint32_t pos) { out[pos] = i; });
+      });
 }
 
 // Fills c->targets with the slots of fluid particles inside the vortex
@@ -251,8 +245,7 @@ int dv_build_targets(dv_ctx* c, const dv_fields* f, bool check) {
   const DevGrid G = dv_grid_cells(c);
   const uint32_t* keys = c->keys[c->perm_buf];
 #define TLT(DD, CH, T)                                                                                          \
-  k_target_list<DD, CH, T><<<nb, T, 0, c->stream>>>(c->p, *f, c->d_cnt, m, c->look_state, c->look_ctl, c->targets, \
-                                                    c->offs, G, keys, c->farbox)
+  k_target_list<DD, CH, T><<<nb, T, 0, c->stream>>>(c->p, *f, m, dv_look(c), c->targets, c->offs, G, keys, c->farbox)
 #define TL(DD, CH) look_wide(m) ? TLT(DD, CH, 1024) : TLT(DD, CH, 256)
   if (c->p.dim == 2)
     TL(2, false);
@@ -630,11 +623,9 @@ DV_API int dv_record_samples(dv_ctx* c, const dv_fields* f, const dv_solver_fiel
   c->host_samples = -1;
   const int m = (int)std::min<int64_t>(c->n_upper, c->cap);
   if (look_wide(m))
-    k_sample_list<1024><<<look_blocks(m), 1024, 0, c->stream>>>(*f, c->d_cnt, m, c->look_state, c->look_ctl,
-                                                               s->sample_idx);
+    k_sample_list<1024><<<look_blocks(m), 1024, 0, c->stream>>>(*f, m, dv_look(c), s->sample_idx);
   else
-    k_sample_list<256><<<look_blocks(m), 256, 0, c->stream>>>(*f, c->d_cnt, m, c->look_state, c->look_ctl,
-                                                             s->sample_idx);
+    k_sample_list<256><<<look_blocks(m), 256, 0, c->stream>>>(*f, m, dv_look(c), s->sample_idx);
   DV_LAUNCHED(c);
   return DV_OK;
 }

@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(RS_T) k_rs_pass(const uint32_t* __restrict__ k
                                                   uint32_t* __restrict__ kout, uint32_t* __restrict__ vout,
                                                   dv_counters* __restrict__ C, int shift,
                                                   const uint32_t* __restrict__ count, uint32_t* __restrict__ ticket,
-                                                  uint32_t* __restrict__ state) {
+                                                  uint32_t* __restrict__ state, uint32_t spins) {
   __shared__ uint32_t s_cnt[RS_W][256];
   __shared__ uint32_t s_ws[RS_W];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(RS_T) k_rs_pass(const uint32_t* __restrict__ k
     for (int q = 0; q < 4; ++q) {
       if (done) continue;
       for (uint32_t s = 0; (v[q] >> 30) == 0; ++s) {
-        if (s == kLookSpins) {
+        if (s == spins) {
           atomicOr(&C->status, DV_WARN_WAIT);
           break;
         }
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(RS_T) k_rs_pass(const uint32_t* __restrict__ k
     const int e = e0 + 32 * r;
     if (e >= n) continue;
     const uint32_t pos = s_cnt[warp][(key[r] >> shift) & 255u] + rank[r];
-    if (pos < (uint32_t)n) {  // always, unless a wait ran out
+    if (pos < (uint32_t)n) {  // always, unless a wait ran out (k_permute then drops the order)
       kout[pos] = key[r];
       vout[pos] = vin ? vin[e] : (uint32_t)e;
     }
@@ -226,13 +226,14 @@ __device__ __forceinline__ void permute_end(const int32_t* part, int nparts, dv_
   fl = block_sum<int>(fl);
   so = block_sum<int>(so);
   if (threadIdx.x == 0) {
-    C->n = (int)__ldcg(ctl + 4);
+    const bool sorted = !look_failed(C);
+    if (sorted) C->n = (int)__ldcg(ctl + 4);
     C->n_fluid = fl;
     C->n_solid = so;
     ctl[4] = 0u;
     ctl[2] = 0u;  // entries of long rows used by the list build
-    ok[0] = 1;    // until the list build finds otherwise
-    ok[1] = 1;    // the sorted keys are those of the current slots
+    ok[0] = sorted;  // until the list build finds otherwise
+    ok[1] = sorted;  // the sorted keys are those of the current slots
   }
 }
 
@@ -241,22 +242,32 @@ __device__ __forceinline__ void permute_end(const int32_t* part, int nparts, dv_
 // Slots in [n_new, n_old) receive the
 // reference's partition fill values (particle_system.py:455-465) for the
 // filled fields and keep their own values for the others.
+// Where a wait of the sort ran out, perm and keys have gaps: every slot then
+// keeps its place and its count, no cell holds a particle, and perm and keys
+// are made to say so.
 template <int D>
-__global__ void k_permute(dv_fields S, dv_fields T, const uint32_t* __restrict__ perm,
-                          const uint32_t* __restrict__ keys, uint32_t invalid, int n_old_cap, dv_counters* C,
+__global__ void k_permute(dv_fields S, dv_fields T, uint32_t* __restrict__ perm,
+                          uint32_t* __restrict__ keys, uint32_t invalid, int n_old_cap, dv_counters* C,
                           int32_t* __restrict__ cstart, int32_t* __restrict__ cend, int32_t* part, uint32_t* ctl,
                           int32_t* __restrict__ ok, bool fold) {
   const int VS = D == 2 ? 2 : 4;
   int p = blockIdx.x * blockDim.x + threadIdx.x;
   const int n_old = C->n;  // the sorted range; keys past it are stale
-  const uint32_t key = p < n_old ? keys[p] : invalid;
+  const bool sorted = !look_failed(C);
+  const uint32_t key = sorted && p < n_old ? keys[p] : invalid;
   int fl = 0, so = 0;
-  if (key != invalid) {
-    const uint32_t next = p + 1 < n_old ? keys[p + 1] : invalid;
-    if (p == 0 || keys[p - 1] != key) cstart[key] = p;
-    if (next != key) cend[key] = p + 1;
-    if (next == invalid) ctl[4] = (uint32_t)p + 1u;
-    int j = (int)perm[p];
+  if (key != invalid || (!sorted && p < n_old)) {
+    int j = p;
+    if (sorted) {
+      const uint32_t next = p + 1 < n_old ? keys[p + 1] : invalid;
+      if (p == 0 || keys[p - 1] != key) cstart[key] = p;
+      if (next != key) cend[key] = p + 1;
+      if (next == invalid) ctl[4] = (uint32_t)p + 1u;
+      j = (int)perm[p];
+    } else {
+      perm[p] = (uint32_t)p;
+      keys[p] = invalid;
+    }
     if (D == 2) {
       reinterpret_cast<float2*>(T.x)[p] = reinterpret_cast<const float2*>(S.x)[j];
       reinterpret_cast<float2*>(T.x0)[p] = reinterpret_cast<const float2*>(S.x0)[j];
@@ -530,14 +541,13 @@ constexpr int kCsrSlots = 32;
 template <int T>
 __global__ void __launch_bounds__(T) k_csr_build(dv_params P, DevGrid G, const float* __restrict__ x,
                                                  const int32_t* __restrict__ mat, const uint8_t* __restrict__ dyn,
-                                                 dv_counters* C, int m, int64_t cap, unsigned long long* state,
-                                                 uint32_t* ctl, uint32_t* __restrict__ off, int32_t* ok,
+                                                 int m, int64_t cap, DevLook K, uint32_t* __restrict__ off, int32_t* ok,
                                                  int32_t* __restrict__ out) {
   constexpr int ST = kCsrSlots + 1, W = T / 32;
   __shared__ int32_t s_rows[T * ST];
   __shared__ uint32_t s_w[W];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int tile = look_tile(ctl), i = tile * T + tid, n = C->n;
+  const int tile = look_tile(K.ctl), i = tile * T + tid, n = K.C->n;
   uint32_t k = 0;
   if (i < n && nbr_row_built(mat, dyn, i)) {
     int32_t* row = s_rows + tid * ST;
@@ -560,7 +570,7 @@ __global__ void __launch_bounds__(T) k_csr_build(dv_params P, DevGrid G, const f
     before += q < w ? s_w[q] : 0u;
     total += s_w[q];
   }
-  const uint32_t at = look_prefix<T>(state, tile, total, &C->status) + before + inc - k;
+  const uint32_t at = look_prefix<T>(K, tile, total) + before + inc - k;
   if (i < m) off[i] = at;
   if (i == n && (int64_t)at > cap) ok[0] = 0;  // too long for the buffer: the sweeps scan cells
   __syncwarp();
@@ -577,16 +587,15 @@ __global__ void __launch_bounds__(T) k_csr_build(dv_params P, DevGrid G, const f
                              [&](int j, V3, float, int mj) { out[e++] = nbr_entry(j, mj, ok); });
     }
   }
-  look_end(state, ctl);
+  if (look_end(K) && tid == 0 && look_failed(K.C)) ok[0] = 0;  // offsets that may decrease: the sweeps scan cells
 }
 
 static int build_csr(dv_ctx* c, const dv_fields* f) {
   const int m = (int)std::min<int64_t>(c->n_upper, c->cap) + 1;
   DevGrid G = dv_grid_cells(c);
 #define CSR2(T)                                                                                                     \
-  k_csr_build<T><<<dv_blocks(m, T), T, 0, c->stream>>>(c->p, G, f->x, f->material, f->is_dynamic, c->d_cnt, m,       \
-                                                       c->nbr_cap, c->look_state, c->look_ctl, c->nbr_off, c->d_nbr_ok, \
-                                                       c->nbr_idx)
+  k_csr_build<T><<<dv_blocks(m, T), T, 0, c->stream>>>(c->p, G, f->x, f->material, f->is_dynamic, m, c->nbr_cap,     \
+                                                       dv_look(c), c->nbr_off, c->d_nbr_ok, c->nbr_idx)
   if (c->p.dim == 3)
     k_csr_rows<<<dv_blocks(m, kCsrWarps * 32), kCsrWarps * 32, 0, c->stream>>>(
         c->p, G, f->x, f->material, f->is_dynamic, c->d_cnt, 1.0f, (uint32_t)nbr_row0(c->cap + 31 & ~(int64_t)31),
@@ -661,10 +670,10 @@ DV_API int dv_grid_build(dv_ctx* c, const dv_fields* src, const dv_fields* dst) 
     uint32_t* st = state + (int64_t)256 * tiles * pass;
     if (wide)
       k_rs_pass<16><<<tiles, RS_T, 0, c->stream>>>(c->keys[cur], vin, c->keys[cur ^ 1], c->vals[cur ^ 1], c->d_cnt,
-                                                   8 * pass, count + 256 * pass, ticket + pass, st);
+                                                   8 * pass, count + 256 * pass, ticket + pass, st, c->look_spins);
     else
       k_rs_pass<8><<<tiles, RS_T, 0, c->stream>>>(c->keys[cur], vin, c->keys[cur ^ 1], c->vals[cur ^ 1], c->d_cnt,
-                                                  8 * pass, count + 256 * pass, ticket + pass, st);
+                                                  8 * pass, count + 256 * pass, ticket + pass, st, c->look_spins);
     DV_LAUNCHED(c);
     cur ^= 1;
   }
@@ -829,7 +838,7 @@ DV_API int64_t dv_stored_lists(dv_ctx* c, uint32_t* dev_offsets, int32_t* dev_nb
   }
   DV_CK(c, cudaMemcpyAsync(&ok, c->d_nbr_ok, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
   DV_CK(c, cudaMemcpyAsync(&total32, off + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
-  DV_CK(c, cudaStreamSynchronize(c->stream));
+  if ((rc = dv_get_counters(c, &cnt))) return rc;  // of the scan too; synchronises
   if (!ok) return dv_fail(c, DV_EINVAL, "dv_stored_lists: no valid lists (positions changed since the grid build)");
   const int64_t total = total32;
   if (dev_offsets)
@@ -868,7 +877,7 @@ DV_API int64_t dv_neighbor_lists(dv_ctx* c, const dv_fields* f, int64_t* dev_off
   if (rc) return rc;
   uint32_t total32 = 0;
   DV_CK(c, cudaMemcpyAsync(&total32, c->offs + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
-  DV_CK(c, cudaStreamSynchronize(c->stream));
+  if ((rc = dv_get_counters(c, &cnt))) return rc;  // of the scan too; synchronises
   const int64_t total = total32;
   if (dev_offsets) {
     k_u32_to_i64<<<dv_blocks(n + 1), DV_THREADS, 0, c->stream>>>(c->offs, dev_offsets, n + 1);

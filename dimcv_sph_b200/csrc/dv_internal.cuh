@@ -77,6 +77,7 @@ struct dv_ctx {
   unsigned long long* look_state = nullptr;  // one-launch scans (dv_lookback.cuh): a word per tile, zero between launches
   // [0] ticket, [1] blocks done; [2] long list rows; [3] blocks done (last_block); [4] valid keys
   uint32_t* look_ctl = nullptr;
+  uint32_t look_spins = 1u << 22;  // polls of a wait between blocks (dv_set_wait_limit)
   double* dscan_part = nullptr;   // double block partials
   int64_t scan_part_cap = 0;
   double* red_part = nullptr;     // FP64 per-block partials of sweeps
@@ -139,6 +140,8 @@ struct dv_ctx {
 
 int dv_fail(dv_ctx* c, int code, const char* fmt, ...);
 int dv_cuda_check(dv_ctx* c, cudaError_t e, const char* what);
+// DV_EWAIT where a wait between blocks has run out (status: dv_counters' word, just read)
+int dv_wait_status(dv_ctx* c, int32_t status);
 #define DV_CK(ctx, call)                                    \
   do {                                                      \
     cudaError_t e_ = (call);                                \

@@ -6,14 +6,25 @@
 // Three launches (reduce, scan of the partials, scan) become one, and the data
 // are read once.  Integer sums only: the order of the additions varies.
 //
-// Every wait is bounded (kLookSpins polls); a wait that runs out raises
-// DV_WARN_WAIT and goes on with what it has, so a kernel always ends.  The
-// last block to finish zeroes the state for the next launch.
+// Every wait is bounded (DevLook::spins polls); a wait that runs out raises
+// DV_WARN_WAIT and goes on with what it has, so a kernel always ends.  What
+// it makes is then not to be used as indices: while the bit is set the last
+// block of a scan or compaction replaces its result by an empty one, the lists
+// are off, and k_permute keeps the order; the host gets DV_EWAIT from
+// its next synchronising call.  The last block to finish zeroes the state for
+// the next launch.
 #pragma once
 
 #include "dv_internal.cuh"
 
-constexpr uint32_t kLookSpins = 1u << 22;
+struct DevLook {
+  unsigned long long* state;
+  uint32_t* ctl;
+  dv_counters* C;
+  uint32_t spins;  // polls of a wait (dv_set_wait_limit)
+};
+static inline DevLook dv_look(const dv_ctx* c) { return DevLook{c->look_state, c->look_ctl, c->d_cnt, c->look_spins}; }
+
 // Threads of a scanning block (T below): 1,024 for large arrays, as every
 // block costs two atomic operations on one address (ticket, end): 0.75M
 // elements 13.5 us with 256 threads, 10.4 with 1,024 (three launches: 9.7 and
@@ -38,6 +49,11 @@ __device__ __forceinline__ void look_st32(uint32_t* p, uint32_t v) {
   asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// a wait has run out, in this launch or since dv_clear_status
+__device__ __forceinline__ bool look_failed(const dv_counters* C) {
+  return look_ld32(reinterpret_cast<const uint32_t*>(&C->status)) & DV_WARN_WAIT;
+}
+
 // the block's tile; every thread of the block calls it
 __device__ __forceinline__ int look_tile(uint32_t* ticket) {
   __shared__ int s_tile;
@@ -51,24 +67,24 @@ __device__ __forceinline__ int look_tile(uint32_t* ticket) {
 // prefix with it.  The whole block walks back, T tiles a step: the tiles
 // of a wave publish their sums at about the same time.
 template <int T>
-__device__ __forceinline__ uint32_t look_prefix(unsigned long long* state, int tile, uint32_t total, int32_t* warn) {
+__device__ __forceinline__ uint32_t look_prefix(const DevLook& K, int tile, uint32_t total) {
   constexpr int W = T / 32;
   __shared__ uint32_t s_sum[W];
   __shared__ int s_full[W];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  if (tid == 0) look_st(state + tile, ((tile == 0 ? 2ull : 1ull) << 32) | total);
+  if (tid == 0) look_st(K.state + tile, ((tile == 0 ? 2ull : 1ull) << 32) | total);
   uint32_t ex = 0;
   for (int p = tile - 1; p >= 0; p -= T) {
     const int q = p - tid;
     unsigned long long v = 2ull << 32;  // before the first tile
     if (q >= 0) {
-      v = look_ld(state + q);
+      v = look_ld(K.state + q);
       for (uint32_t s = 0; (v >> 32) == 0; ++s) {
-        if (s == kLookSpins) {
-          atomicOr(warn, DV_WARN_WAIT);
+        if (s == K.spins) {
+          atomicOr(&K.C->status, DV_WARN_WAIT);
           break;
         }
-        v = look_ld(state + q);
+        v = look_ld(K.state + q);
       }
     }
     __syncwarp();
@@ -92,39 +108,40 @@ __device__ __forceinline__ uint32_t look_prefix(unsigned long long* state, int t
       }
     if (done) break;
   }
-  if (tid == 0 && tile > 0) look_st(state + tile, (2ull << 32) | (ex + total));
+  if (tid == 0 && tile > 0) look_st(K.state + tile, (2ull << 32) | (ex + total));
   return ex;
 }
 
 // End of a block; true in the threads of the last block to finish, which has
 // then zeroed the state.  Global writes of all blocks are visible to it.
-__device__ __forceinline__ bool look_end(unsigned long long* state, uint32_t* ctl) {
+__device__ __forceinline__ bool look_end(const DevLook& K) {
   __shared__ bool s_last;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    s_last = atomicAdd(ctl + 1, 1u) == gridDim.x - 1;
+    s_last = atomicAdd(K.ctl + 1, 1u) == gridDim.x - 1;
     __threadfence();
   }
   __syncthreads();
   if (!s_last) return false;
-  for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) state[k] = 0ull;
-  if (threadIdx.x < 2) ctl[threadIdx.x] = 0u;
+  for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) K.state[k] = 0ull;
+  if (threadIdx.x < 2) K.ctl[threadIdx.x] = 0u;
   return true;
 }
 
 // Stable compaction of the elements 0 .. m-1 that pred accepts, R rounds of
-// T a block: out(e, position) for each, and for every element offs(e,
-// number accepted before it) when OFFS; *count gets the total.
+// T a block: list[position] = e for each, and for every element offs[e] =
+// number accepted before it when OFFS; *count gets the total.  After a wait
+// that ran out: no element, and zeros in list[0 .. room) and offs.
 template <int T>
 constexpr int look_rounds() { return T == 256 ? 8 : 4; }
-template <int T, bool OFFS, typename Pred, typename Out>
-__device__ __forceinline__ void look_compact(int m, unsigned long long* state, uint32_t* ctl, int32_t* warn,
-                                             uint32_t* __restrict__ offs, int32_t* count, Pred&& pred, Out&& out) {
+template <int T, bool OFFS, typename Pred>
+__device__ __forceinline__ void look_compact(int m, const DevLook& K, uint32_t* __restrict__ offs, int32_t* count,
+                                             int32_t* __restrict__ list, int room, Pred&& pred) {
   constexpr int R = look_rounds<T>(), W = T / 32, PER = R * W / 32;  // (round, warp) counts a lane scans
   __shared__ uint32_t s_cnt[R * W];
   __shared__ uint32_t s_total;
-  const int tile = look_tile(ctl), tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int tile = look_tile(K.ctl), tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int base = tile * (R * T);
   unsigned ballots[R];
 #pragma unroll
@@ -157,18 +174,24 @@ __device__ __forceinline__ void look_compact(int m, unsigned long long* state, u
     if (lane == 31) s_total = inc;
   }
   __syncthreads();
-  const uint32_t ex = look_prefix<T>(state, tile, s_total, warn);
+  const uint32_t ex = look_prefix<T>(K, tile, s_total);
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int e = base + r * T + tid;
     const uint32_t pos = ex + s_cnt[r * W + w] + __popc(ballots[r] & ((1u << lane) - 1u));
     if (e < m) {
       if (OFFS) offs[e] = pos;
-      if ((ballots[r] >> lane) & 1u) out(e, pos);
+      if ((ballots[r] >> lane) & 1u) list[pos] = e;
     }
   }
   if (count && tid == 0 && tile == (int)gridDim.x - 1) *count = (int32_t)(ex + s_total);
-  look_end(state, ctl);
+  if (look_end(K) && look_failed(K.C)) {
+    for (int e = tid; e < m; e += T) {
+      if (OFFS) offs[e] = 0u;
+      if (e < room) list[e] = 0;
+    }
+    if (count && tid == 0) *count = 0;
+  }
 }
 // blocks of a look_compact launch over m elements
 static inline int look_blocks(int64_t m) {

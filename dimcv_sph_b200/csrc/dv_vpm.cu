@@ -34,6 +34,7 @@
 
 #include "dv_far.cuh"
 #include "dv_internal.cuh"
+#include "dv_lookback.cuh"
 
 namespace {
 
@@ -915,10 +916,10 @@ __global__ void k_plan_slots(dv_params P, DevGrid G, dv_fields F, dv_solver_fiel
 }
 
 __global__ void k_plan_src(dv_vpm_plan p, const uint32_t* __restrict__ flags, const uint32_t* __restrict__ offs,
-                           const int32_t* __restrict__ err) {
+                           const int32_t* __restrict__ err, const dv_counters* __restrict__ C) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int n = p.n;
-  if (i == 0) *p.n_src = (*err || (int64_t)offs[n] > p.src_cap) ? -1 : (int32_t)offs[n];
+  if (i == 0) *p.n_src = (*err || look_failed(C) || (int64_t)offs[n] > p.src_cap) ? -1 : (int32_t)offs[n];
   if (i >= n) return;
   if (flags[i] && (int64_t)offs[i] < p.src_cap) {
     const int s = (int)offs[i];
@@ -1113,7 +1114,7 @@ DV_API int dv_vpm_plan_build(dv_ctx* c, const dv_fields* f, const dv_solver_fiel
                                                                 c->flags, c->d_flag + 1);
   DV_LAUNCHED(c);
   if (int rc = dv_scan_u32(c, c->flags, c->offs, (int64_t)n + 1)) return rc;
-  k_plan_src<<<dv_blocks(n + 1), DV_THREADS, 0, c->stream>>>(*p, c->flags, c->offs, c->d_flag + 1);
+  k_plan_src<<<dv_blocks(n + 1), DV_THREADS, 0, c->stream>>>(*p, c->flags, c->offs, c->d_flag + 1, c->d_cnt);
   DV_LAUNCHED(c);
   return DV_OK;
 }

@@ -380,23 +380,18 @@ __global__ void k_mult(const int32_t* __restrict__ sample_idx, const dv_counters
 // correction kernel reads a cell's few samples instead of testing every
 // particle's multiplicity.
 template <int T>
-__global__ void __launch_bounds__(T) k_sample_slots(const int32_t* __restrict__ mult, int nu, dv_counters* C,
-                                                      unsigned long long* state, uint32_t* ctl,
+__global__ void __launch_bounds__(T) k_sample_slots(const int32_t* __restrict__ mult, int nu, DevLook K,
                                                       uint32_t* __restrict__ rank, int32_t* __restrict__ slot) {
-  look_compact<T, true>(
-      nu + 1, state, ctl, &C->status, rank, nullptr, [&](int j) { return j < nu && mult[j] > 0; },
-      [&](int j, uint32_t pos) { slot[pos] = j; });
+  look_compact<T, true>(nu + 1, K, rank, nullptr, slot, nu, [&](int j) { return j < nu && mult[j] > 0; });
 }
 
 // boxed: also the packed samples of the far field on boxes
 static int sample_slots(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s, bool boxed = false) {
   const int nu = (int)std::min<int64_t>(c->n_upper, c->cap);
   if (look_wide(nu + 1))
-    k_sample_slots<1024><<<look_blocks(nu + 1), 1024, 0, c->stream>>>(c->mult, nu, c->d_cnt, c->look_state,
-                                                                      c->look_ctl, c->srank, c->sslot);
+    k_sample_slots<1024><<<look_blocks(nu + 1), 1024, 0, c->stream>>>(c->mult, nu, dv_look(c), c->srank, c->sslot);
   else
-    k_sample_slots<256><<<look_blocks(nu + 1), 256, 0, c->stream>>>(c->mult, nu, c->d_cnt, c->look_state,
-                                                                    c->look_ctl, c->srank, c->sslot);
+    k_sample_slots<256><<<look_blocks(nu + 1), 256, 0, c->stream>>>(c->mult, nu, dv_look(c), c->srank, c->sslot);
   DV_LAUNCHED(c);
   return boxed ? dv_farbox_pack(c, f, s, nu) : DV_OK;
 }

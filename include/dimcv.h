@@ -54,7 +54,8 @@ enum dv_status {
   DV_ECAPACITY = -2,   /* a size exceeds the context's capacity */
   DV_ECUDA = -3,       /* a CUDA runtime call failed */
   DV_ENAN = -4,        /* a non-finite value was found where one is fatal */
-  DV_EUNSUPPORTED = -5 /* option not built into this library */
+  DV_EUNSUPPORTED = -5, /* option not built into this library */
+  DV_EWAIT = -6        /* a wait between the blocks of a kernel ran out (DV_WARN_WAIT) */
 };
 
 /* device-raised warning bits in dv_counters.status */
@@ -64,7 +65,7 @@ enum dv_status {
 #define DV_WARN_CAPACITY (1 << 3)          /* emission clamped at capacity (particle_system.py:361) */
 #define DV_WARN_NAN (1 << 4)               /* a non-finite error norm was seen in a solve */
 #define DV_WARN_BAD_INDEX (1 << 5)         /* an injected sample index was outside [0, n): ignored */
-#define DV_WARN_WAIT (1 << 6)              /* a bounded wait between blocks ran out (never expected) */
+#define DV_WARN_WAIT (1 << 6)              /* a bounded wait between blocks ran out (dv_set_wait_limit) */
 
 /* Sampling modes of dv_sample (new: the reference only has the Bernoulli
  * birth/death process of dimcv_sph.py:305-335). */
@@ -215,8 +216,18 @@ DV_API int dv_set_params(dv_ctx* ctx, const dv_params* params);
 DV_API const char* dv_version(void);
 DV_API int64_t dv_launch_count(const dv_ctx* ctx);
 
-/* Host view of the device counters (synchronises the stream). */
+/* Host view of the device counters (synchronises the stream).  DV_EWAIT, with
+ * *out filled, while DV_WARN_WAIT is set; so do the other calls that read the
+ * counters (solves with iters, lists, dv_get_permutation, dv_batch_read). */
 DV_API int dv_get_counters(dv_ctx* ctx, dv_counters* out);
+/* New: the scans and the sort of a call wait, block for block, for the tiles
+ * before theirs, at most `polls` reads of a word (default 2^22, some seconds;
+ * 0: the word has to be there at the first read).  A wait that runs out sets
+ * DV_WARN_WAIT, and until dv_clear_status nothing is made of an order or count
+ * that is not known: a grid build keeps every slot's place and leaves the
+ * cells and lists empty, target and sample lists are empty.  The particles
+ * stay whole: clear the status and build again. */
+DV_API int dv_set_wait_limit(dv_ctx* ctx, int64_t polls);
 /* Sets n / n_fluid / n_solid (after the caller filled fields on its own). */
 DV_API int dv_set_counts(dv_ctx* ctx, int32_t n, int32_t n_fluid, int32_t n_solid);
 /* Clears the sticky DV_WARN_* bits of dv_counters.status. */
