@@ -210,7 +210,8 @@ DV_API dv_ctx* dv_create(const dv_params* params, int64_t capacity, void* stream
   // neighbour lists: 24 entries per particle on average in 2-D; a row per
   // particle and 51 entries per particle on average for the longer rows in
   // 3-D; beyond that the sweeps keep scanning cells
-  c->nbr_cap = params->dim == 3 ? 4 * nbr_row0(cap + 31 & ~(int64_t)31) + (51 * cap & ~(int64_t)3) : cap * 24;
+  c->nbr_cap = params->dim == 3 ? 4 * nbr_row0(cap + 31 & ~(int64_t)31) + (51 * cap & ~(int64_t)3)
+                                : std::min<int64_t>(cap * 24, 0xffffffff);  // 32-bit offsets
   A(c->nbr_off, cap + 1);
   if (params->dim == 3) {
     A(c->nbr_len, cap);

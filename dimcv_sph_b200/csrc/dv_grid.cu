@@ -514,8 +514,8 @@ __global__ void __launch_bounds__(kCsrWarps * 32) k_csr_rows(dv_params P, DevGri
   if (mylen <= kNbrRow) {
     for (uint32_t e = mylen; e & 3u; ++e) out[4 * ((int64_t)at + 32 * (e >> 2)) + (e & 3u)] = i;
   } else {
-    const uint32_t room = (mylen + 3u) / 4u, a = atomicAdd(far_used, room);
-    if (a + room <= far_cap) {
+    const uint32_t room = (mylen + 3u) / 4u, a = atomicAdd(far_used, room);  // the sum may wrap: no a + room
+    if (room <= far_cap && a <= far_cap - room) {
       at = far0 + a;
       int64_t e = 4 * (int64_t)at;
       for_each_neighbor_m<3>(P, G, x, mat, i, xi,
@@ -572,12 +572,17 @@ __global__ void __launch_bounds__(T) k_csr_build(dv_params P, DevGrid G, const f
   }
   const uint32_t at = look_prefix<T>(K, tile, total) + before + inc - k;
   if (i < m) off[i] = at;
-  if (i == n && (int64_t)at > cap) ok[0] = 0;  // too long for the buffer: the sweeps scan cells
   __syncwarp();
   for (int g = 0; g < 32; g += 4) {
     const int r = g + (lane >> 3), ir = tile * T + 32 * w + r;
     const uint32_t cnt = __shfl_sync(0xffffffffu, k, r), o = __shfl_sync(0xffffffffu, at, r);
-    if (cnt == 0 || (int64_t)o + cnt > cap) continue;
+    if (cnt == 0) continue;
+    // too long for the buffer: the sweeps scan cells.  Asked of every row, as
+    // the offsets of longer lists wrap (cap < 2^32: the first row past it sees that)
+    if ((int64_t)o + cnt > cap) {
+      ok[0] = 0;
+      continue;
+    }
     const int32_t* row = s_rows + (32 * w + r) * ST;
     if (cnt <= (uint32_t)kCsrSlots) {
       for (uint32_t e = lane & 7; e < cnt; e += 8) out[o + e] = nbr_entry(row[e], __ldg(mat + row[e]), ok);
@@ -782,12 +787,16 @@ DV_API int dv_add_particles(dv_ctx* c, const dv_fields* f, const float* pos, con
 // ----------------------------------------------------------- neighbour CSR
 template <int D>
 __global__ void k_nbr_count(dv_params P, DevGrid G, const float* __restrict__ x,
-                            const dv_counters* __restrict__ C, uint32_t* __restrict__ cnt) {
+                            const dv_counters* __restrict__ C, uint32_t* __restrict__ cnt,
+                            unsigned long long* __restrict__ total) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= C->n) return;
   uint32_t k = 0;
-  for_each_neighbor<D>(P, G, x, i, ldv<D>(x, i), [&](int, V3, float) { ++k; });
-  cnt[i] = k;
+  if (i < C->n) {
+    for_each_neighbor<D>(P, G, x, i, ldv<D>(x, i), [&](int, V3, float) { ++k; });
+    cnt[i] = k;
+  }
+  const unsigned long long s = block_sum<unsigned long long>(k);
+  if (threadIdx.x == 0 && s) atomicAdd(total, s);
 }
 
 template <int D>
@@ -867,18 +876,22 @@ DV_API int64_t dv_neighbor_lists(dv_ctx* c, const dv_fields* f, int64_t* dev_off
   // always the cell scan: this entry point checks the lists the sweeps use
   DevGrid G = dv_grid_cells(c);
   int nb = dv_blocks(n);
+  // all pairs in 64 bits (scratch words): the offsets have 32
+  unsigned long long* sum = reinterpret_cast<unsigned long long*>(c->dscan_part);
+  DV_CK(c, cudaMemsetAsync(sum, 0, sizeof(*sum), c->stream));
   if (c->p.dim == 2)
-    k_nbr_count<2><<<nb, DV_THREADS, 0, c->stream>>>(c->p, G, f->x, c->d_cnt, c->flags);
+    k_nbr_count<2><<<nb, DV_THREADS, 0, c->stream>>>(c->p, G, f->x, c->d_cnt, c->flags, sum);
   else
-    k_nbr_count<3><<<nb, DV_THREADS, 0, c->stream>>>(c->p, G, f->x, c->d_cnt, c->flags);
+    k_nbr_count<3><<<nb, DV_THREADS, 0, c->stream>>>(c->p, G, f->x, c->d_cnt, c->flags, sum);
   DV_LAUNCHED(c);
   DV_CK(c, cudaMemsetAsync(c->flags + n, 0, sizeof(uint32_t), c->stream));
   rc = dv_scan_u32(c, c->flags, c->offs, (int64_t)n + 1);
   if (rc) return rc;
-  uint32_t total32 = 0;
-  DV_CK(c, cudaMemcpyAsync(&total32, c->offs + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
+  int64_t total = 0;
+  DV_CK(c, cudaMemcpyAsync(&total, sum, sizeof(total), cudaMemcpyDeviceToHost, c->stream));
   if ((rc = dv_get_counters(c, &cnt))) return rc;  // of the scan too; synchronises
-  const int64_t total = total32;
+  if (total > (int64_t)0xffffffff)
+    return dv_fail(c, DV_ECAPACITY, "dv_neighbor_lists: %lld pairs, at most 2^32 - 1", (long long)total);
   if (dev_offsets) {
     k_u32_to_i64<<<dv_blocks(n + 1), DV_THREADS, 0, c->stream>>>(c->offs, dev_offsets, n + 1);
     DV_LAUNCHED(c);
