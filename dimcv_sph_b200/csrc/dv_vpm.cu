@@ -52,6 +52,7 @@ template <typename T>
 struct Geo {
   T Lx, Ly, iLx, iLy;  // periodic box and its inverse
   T invh, kW, c, eps, inv_eps, tiny, rmin;
+  T one;  // 1, which the compiler does not know (pd2)
 };
 
 template <typename T>
@@ -68,6 +69,7 @@ Geo<T> make_geo(const dv_params& P) {
   g.inv_eps = (T)P.inv_eps;
   g.tiny = sizeof(T) == 4 ? (T)1e-30 : (T)1e-280;
   g.rmin = (T)P.grad_r_min;
+  g.one = T(1);
   return g;
 }
 
@@ -410,23 +412,27 @@ __global__ void __launch_bounds__(VT) k_far(Geo<T> g, dv_vpm_plan p, const T* __
 }
 
 // ------------------------------------------- FP32 pairs, two targets a lane
-// pd<float, IMG> of two targets at once, the same operations.  rint is taken
-// as (t + 1.5·2^23) − 1.5·2^23, which is rint(t) for |t| < 2^22 (positions of
-// fewer than four million box lengths): rintf runs on the unit of the
-// reciprocals at a quarter of the FP32 rate, twice a pair, and bounded the loop.
+// pd<float, IMG> of two targets at once.  rint is taken
+// as (t + 1.5·2^23) − 1.5·2^23, which is rint(t) for |t| < 2^22, that is for
+// positions less than four million box lengths apart (FP32 positions farther
+// apart are whole half boxes, and a rollout does not wrap them): rintf runs on
+// the unit of the reciprocals at a quarter of the FP32 rate, twice a pair, and
+// bounded the loop.  The sum is an fma with a 1 that is not known at compile
+// time: ptxas makes one fma of mul.rn.f32x2 and add.rn.f32x2, and the rint of
+// the unrounded product takes the other image for pairs half a box apart.
 struct Geo2 {
-  f2_t nLx, nLy, iLx, iLy, magic;
+  f2_t nLx, nLy, iLx, iLy, magic, one;
 };
 __device__ __forceinline__ Geo2 make_geo2(const Geo<float>& g) {
   return Geo2{f2_pack(-g.Lx, -g.Lx), f2_pack(-g.Ly, -g.Ly), f2_pack(g.iLx, g.iLx), f2_pack(g.iLy, g.iLy),
-              f2_pack(12582912.0f, 12582912.0f)};
+              f2_pack(12582912.0f, 12582912.0f), f2_pack(g.one, g.one)};
 }
 template <int IMG>
-__device__ __forceinline__ f2_t pd2(f2_t a, f2_t b, f2_t abar, f2_t bbar, f2_t nL, f2_t iL, f2_t magic) {
+__device__ __forceinline__ f2_t pd2(f2_t a, f2_t b, f2_t abar, f2_t bbar, f2_t nL, f2_t iL, const Geo2& G) {
   const f2_t d = f2_sub(a, b);
   if (IMG == 0) return d;
   const f2_t t = f2_mul(IMG == 2 ? f2_sub(abar, bbar) : d, iL);
-  return f2_fma(f2_sub(f2_add(t, magic), magic), nL, d);
+  return f2_fma(f2_sub(f2_fma(t, G.one, G.magic), G.magic), nL, d);
 }
 // inv_r2<float> of two values
 __device__ __forceinline__ f2_t inv_r2_2(f2_t r2, float tiny) {
@@ -497,8 +503,8 @@ __global__ void __launch_bounds__(VT) k_far_x2(Geo<float> g, dv_vpm_plan p, cons
       if (IMG == 2) vb = s2[NW * q + 2];
 #pragma unroll
       for (int k = 0; k < NP; ++k) {
-        const f2_t dx = pd2<IMG>(PX[k], v0.x, BX[k], vb.x, G.nLx, G.iLx, G.magic);
-        const f2_t dy = pd2<IMG>(PY[k], v0.y, BY[k], vb.y, G.nLy, G.iLy, G.magic);
+        const f2_t dx = pd2<IMG>(PX[k], v0.x, BX[k], vb.x, G.nLx, G.iLx, G);
+        const f2_t dy = pd2<IMG>(PY[k], v0.y, BY[k], vb.y, G.nLy, G.iLy, G);
         const f2_t bs = f2_mul(v1.x, inv_r2_2(f2_fma(dy, dy, f2_mul(dx, dx)), g.tiny));
         AX[k] = f2_fma(bs, dy, AX[k]);
         AY[k] = f2_fma(bs, dx, AY[k]);  // the sum with the sign of −u_y
@@ -591,8 +597,8 @@ __global__ void __launch_bounds__(VT) k_far_bwd_x2(Geo<float> g, dv_vpm_plan p, 
       f2_t BW = 0ull, BGX = 0ull, BGY = 0ull, CX = 0ull, CY = 0ull;
 #pragma unroll
       for (int k = 0; k < NP; ++k) {
-        const f2_t dx = pd2<IMG>(PX[k], v0.x, BX[k], vb.x, G.nLx, G.iLx, G.magic);
-        const f2_t dy = pd2<IMG>(PY[k], v0.y, BY[k], vb.y, G.nLy, G.iLy, G.magic);
+        const f2_t dx = pd2<IMG>(PX[k], v0.x, BX[k], vb.x, G.nLx, G.iLx, G);
+        const f2_t dy = pd2<IMG>(PY[k], v0.y, BY[k], vb.y, G.nLy, G.iLy, G);
         const f2_t s = inv_r2_2(f2_fma(dy, dy, f2_mul(dx, dx)), g.tiny);
         const f2_t sc = f2_mul(s, f2_fma(GX[k], dy, f2_mul(NGY[k], dx)));
         const f2_t u = f2_mul(s, sc);
