@@ -114,8 +114,8 @@ DV_API void dv_destroy(dv_ctx* c) {
   dv_batch_free(c);
   dv_farbox_free(c);
   void* ptrs[] = {c->d_cnt,   c->d_flag,    c->keys[0],   c->keys[1],   c->vals[0], c->vals[1],
-                  c->cell_start, c->mt[0],     c->mt[1],   c->mt[2],
-                  c->look_state, c->look_ctl, c->dscan_part, c->red_part, c->ired_part, c->flags, c->offs,
+                  c->mt[0],     c->mt[1],   c->mt[2],
+                  c->look_state, c->dscan_part, c->red_part, c->ired_part, c->flags, c->offs,
                   c->targets, c->cdf,       c->spos,      c->sw,        c->near_v,  c->near_S,
                   c->far_acc, c->mult,      c->nbr_off,   c->nbr_idx,   c->d_nbr_ok,
                   c->srank,     c->sslot,   c->nbr_len,   c->pk_a,    c->pk_b,
@@ -176,7 +176,7 @@ DV_API dv_ctx* dv_create(const dv_params* params, int64_t capacity, void* stream
   c->max_tiles = (cap + 2047) / 2048 + 1;
   c->red_cap = (cap + 127) / 128 + 1024;
   c->scan_part_cap = (cap + 1 + 4095) / 4096 + 1024;
-  const int64_t look_tiles = (cap + 1 + 63) / 64 + 64;  // tiles of 64 elements at least
+  const int64_t look_tiles = ((cap + 1 + 63) / 64 + 65) & ~(int64_t)1;  // tiles of 64 elements at least
   cudaError_t e = cudaSuccess;
 #define A(ptr, cnt) \
   if (e == cudaSuccess) e = alloc(&(ptr), (cnt));
@@ -187,11 +187,13 @@ DV_API dv_ctx* dv_create(const dv_params* params, int64_t capacity, void* stream
   A(c->vals[0], cap);
   A(c->vals[1], cap);
   const int64_t sort_words = 256 * c->npasses * (c->max_tiles + 1) + 64;
-  A(c->cell_start, 2 * (int64_t)c->ncells + sort_words);
+  // one block, which a grid build clears: scan state, cell tables, sort state
+  c->look_words = 2 * look_tiles + 8;
+  A(c->look_state, (c->look_words + 2 * (int64_t)c->ncells + sort_words + 1) / 2);
+  c->look_ctl = reinterpret_cast<uint32_t*>(c->look_state + look_tiles);
+  c->cell_start = reinterpret_cast<int32_t*>(c->look_ctl + 8);
   c->cell_end = c->cell_start + c->ncells;
   c->sort_state = reinterpret_cast<uint32_t*>(c->cell_end + c->ncells);
-  A(c->look_state, look_tiles);
-  A(c->look_ctl, 8);
   A(c->dscan_part, c->scan_part_cap);
   A(c->red_part, c->red_cap);
   A(c->ired_part, c->red_cap);
@@ -229,11 +231,9 @@ DV_API dv_ctx* dv_create(const dv_params* params, int64_t capacity, void* stream
   if (e == cudaSuccess) *c->h_solve = 0;
   if (e == cudaSuccess) e = cudaMemset(c->d_cnt, 0, sizeof(dv_counters));
   if (e == cudaSuccess) e = cudaMemset(c->d_flag, 0, sizeof(int32_t) * 4);
-  if (e == cudaSuccess) e = cudaMemset(c->look_state, 0, sizeof(unsigned long long) * look_tiles);
-  if (e == cudaSuccess) e = cudaMemset(c->look_ctl, 0, 8 * sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMemset(c->d_prof, 0, sizeof(double) * 4);
   if (e == cudaSuccess) e = cudaMemset(c->d_nbr_ok, 0, 2 * sizeof(int32_t));
-  if (e == cudaSuccess) e = cudaMemset(c->cell_start, 0, sizeof(int32_t) * 2 * c->ncells);
+  if (e == cudaSuccess) e = cudaMemset(c->look_state, 0, sizeof(uint32_t) * (c->look_words + 2 * c->ncells));
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e != cudaSuccess) {
     dv_cuda_check(c, e, "dv_create allocation");

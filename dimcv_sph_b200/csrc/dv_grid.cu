@@ -656,9 +656,12 @@ DV_API int dv_grid_build(dv_ctx* c, const dv_fields* src, const dv_fields* dst) 
   uint32_t* count = c->sort_state;
   uint32_t* ticket = count + 256 * c->npasses;
   uint32_t* state = ticket + 64;
-  // the cell tables lie before the sort's state
-  const size_t zeroed = 2 * (size_t)c->ncells + 256 * (size_t)c->npasses * (size_t)(tiles + 1) + 64;
-  DV_CK(c, cudaMemsetAsync(c->cell_start, 0, sizeof(uint32_t) * zeroed, c->stream));
+  // the scans' words and counters, the cell tables and the sort's state in one
+  // piece: whatever a call left of them (calls that overlapped on two streams)
+  // ends here
+  const size_t zeroed =
+      (size_t)c->look_words + 2 * (size_t)c->ncells + 256 * (size_t)c->npasses * (size_t)(tiles + 1) + 64;
+  DV_CK(c, cudaMemsetAsync(c->look_state, 0, sizeof(uint32_t) * zeroed, c->stream));
   const int kr = ntiles < 2 * c->num_sms ? 1 : 8;
 #define CK(DD, RR)                                                                                                  \
   k_cell_keys<DD, RR><<<dv_blocks(nu, RS_T * RR), RS_T, 0, c->stream>>>(c->p, *src, G, c->d_cnt, c->keys[0], invalid, \

@@ -74,7 +74,11 @@ struct dv_ctx {
   uint32_t* mt[3] = {nullptr, nullptr, nullptr};  // per-axis Morton tables
 
   // scans and reductions
-  unsigned long long* look_state = nullptr;  // one-launch scans (dv_lookback.cuh): a word per tile, zero between launches
+  // one-launch scans (dv_lookback.cuh): a word per tile, zero between launches
+  // and cleared by every grid build; look_ctl, the cell tables and the sort's
+  // state lie behind it
+  unsigned long long* look_state = nullptr;
+  int64_t look_words = 0;  // 32-bit words of look_state and look_ctl
   // [0] ticket, [1] blocks done; [2] long list rows; [3] blocks done (last_block); [4] valid keys
   uint32_t* look_ctl = nullptr;
   uint32_t look_spins = 1u << 22;  // polls of a wait between blocks (dv_set_wait_limit)

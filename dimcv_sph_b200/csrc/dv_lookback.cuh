@@ -54,10 +54,12 @@ __device__ __forceinline__ bool look_failed(const dv_counters* C) {
   return look_ld32(reinterpret_cast<const uint32_t*>(&C->status)) & DV_WARN_WAIT;
 }
 
-// the block's tile; every thread of the block calls it
+// The block's tile; every thread of the block calls it.  Modulo the grid, so
+// that a ticket left by calls that overlapped against the rules names a tile
+// all the same (its waits may then run out).
 __device__ __forceinline__ int look_tile(uint32_t* ticket) {
   __shared__ int s_tile;
-  if (threadIdx.x == 0) s_tile = (int)atomicAdd(ticket, 1u);
+  if (threadIdx.x == 0) s_tile = (int)(atomicAdd(ticket, 1u) % gridDim.x);
   __syncthreads();
   return s_tile;
 }

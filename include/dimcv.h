@@ -203,7 +203,10 @@ DV_API void dv_destroy(dv_ctx* ctx);
 /* Message of the last failed call on ctx; with NULL, of the calling thread's
  * last failed dv_create or context-free call. */
 DV_API const char* dv_last_error(const dv_ctx* ctx);
-/* Later calls on ctx run on `stream` (cudaStream_t, NULL = legacy default). */
+/* Later calls on ctx run on `stream` (cudaStream_t, NULL = legacy default).
+ * All calls on a context share its workspace: order the new stream behind the
+ * old one first (cudaStreamWaitEvent, or a synchronisation).  What calls that
+ * overlapped all the same left in the workspace ends with the next grid build. */
 DV_API int dv_set_stream(dv_ctx* ctx, void* stream);
 /* Replaces the scalar parameters (time step, tolerances, options) of a live
  * context.  The cell grid (dim, grid_num) must stay the same.  Stands in for
