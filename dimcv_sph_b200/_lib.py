@@ -28,6 +28,7 @@ PROTOTYPES = {
     "dv_set_params": (C.c_int, [_P, _PP]),
     "dv_version": (C.c_char_p, []),
     "dv_launch_count": (i64, [_P]),
+    "dv_sweep_count": (i64, [_P]),
     "dv_get_counters": (C.c_int, [_P, C.POINTER(DvCounters)]),
     "dv_set_counts": (C.c_int, [_P, i32, i32, i32]),
     "dv_clear_status": (C.c_int, [_P]),

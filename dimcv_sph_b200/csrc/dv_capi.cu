@@ -35,6 +35,8 @@ DV_API const char* dv_last_error(const dv_ctx* ctx) {
 
 DV_API int64_t dv_launch_count(const dv_ctx* ctx) { return ctx ? ctx->launches : 0; }
 
+DV_API int64_t dv_sweep_count(const dv_ctx* ctx) { return ctx ? ctx->launches - ctx->packs : 0; }
+
 DV_API int dv_set_stream(dv_ctx* ctx, void* stream) {
   if (!ctx) return DV_EINVAL;
   ctx->stream = (cudaStream_t)stream;

@@ -48,6 +48,7 @@ struct dv_ctx {
   int num_sms = 148;
   std::string err;
   int64_t launches = 0;
+  int64_t packs = 0;    // of them passes that pack a sweep's fields (dv_pack)
   int64_t n_upper = 0;  // host-side upper bound of the device particle count
 
   dv_counters* d_cnt = nullptr;  // device counters

@@ -62,9 +62,8 @@ int dv_pack(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s, int what) 
       return dv_fail(c, DV_EINVAL, "dv_pack: no kernel for %d", what);
   }
 #undef DV_PK
-  // counted with the sweep that it prepares (dv_launch_count)
-  const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return dv_cuda_check(c, e, "kernel launch");
+  DV_LAUNCHED(c);
+  c->packs++;
   return DV_OK;
 }
 

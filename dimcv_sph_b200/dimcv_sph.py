@@ -157,7 +157,7 @@ class DIMCVSPHSolver(SPHBase):
     # with the vis sweep, dv_vorticity_dvort): the first
     # method computes all the results and a later one skips its sweep while
     # nothing it reads can have changed: no library kernel has run since
-    # (the context's launch count) and no tensor it reads was written in place
+    # (the context's sweep count) and no tensor it reads was written in place
     # by torch (the tensors' version counters, which views share).
     # compute_densities thereby also writes density_adv, which the reference
     # reads only after divergence_solve's own compute_density_change.
@@ -172,7 +172,9 @@ class DIMCVSPHSolver(SPHBase):
     _fused_dvort = None
 
     def _launches(self):
-        return self.lib.dv_launch_count(self.ctx)
+        # a library (or a stand-in) without packing passes counts the same in both
+        count = getattr(self.lib, "dv_sweep_count", self.lib.dv_launch_count)
+        return count(self.ctx)
 
     def _fusion_mark(self, names, solver_names=()):
         f, sb = self.ps.fields, self._sb

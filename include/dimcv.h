@@ -214,10 +214,13 @@ DV_API int dv_set_stream(dv_ctx* ctx, void* stream);
  * `solver.dt[None] = ...` (dimcv_sph.py:13). */
 DV_API int dv_set_params(dv_ctx* ctx, const dv_params* params);
 /* Library version string and the number of kernels launched so far by this
- * context (used by benchmarks to report launch counts; a 3-D sweep and the
- * pass that packs its gathered fields count as one). */
+ * context (used by benchmarks to report launch counts). */
 DV_API const char* dv_version(void);
 DV_API int64_t dv_launch_count(const dv_ctx* ctx);
+/* New: the same without the passes that pack the fields a 3-D sweep gathers,
+ * so that a sweep counts as one in 2-D and 3-D: a number that moves with every
+ * call that may write a field (the fused sweeps' skips compare it). */
+DV_API int64_t dv_sweep_count(const dv_ctx* ctx);
 
 /* Host view of the device counters (synchronises the stream).  DV_EWAIT, with
  * *out filled, while DV_WARN_WAIT is set; so do the other calls that read the
