@@ -369,8 +369,8 @@ __device__ __forceinline__ int32_t nbr_entry(int j, int mj, int32_t* ok) {
 // needed a scan and a compaction of its rows: 0.75M particles 306 us in four
 // launches, now 193 in one; 2.02M 836, now 590.  Issue slots are 79% busy;
 // groups of 8 or 10 particles and fewer or more registers were level or slower.
-// Any material other than fluid or solid in the window of a built row makes
-// the lists invalid.
+// A neighbour of another material than fluid or solid makes the lists invalid:
+// where one is among 32 candidates they are tested once more, for it alone.
 constexpr int kCsrWarps = 8;  // of a block
 //
 // `one` is 1: the squares are added by an fma with it, which rounds as the
@@ -472,7 +472,14 @@ __global__ void __launch_bounds__(kCsrWarps * 32) k_csr_rows(dv_params P, DevGri
         }
         const int rj = (int)nbr_row0(j);  // tells j from the particle as well as the slot does
         const int32_t entry = (int32_t)((uint32_t)j | (mj == DV_MATERIAL_SOLID ? DV_NBR_SOLID : 0u));
-        bad |= mj != DV_MATERIAL_FLUID && mj != DV_MATERIAL_SOLID;
+        const bool odd = mj != DV_MATERIAL_FLUID && mj != DV_MATERIAL_SOLID;
+        if (__any_sync(0xffffffffu, odd)) {
+#pragma unroll 1
+          for (int t = 0; t < nt; ++t) {
+            const float* u = reinterpret_cast<const float*>(&s_t[w][t & ~1]) + (t & 1);
+            bad |= odd && rj != __float_as_int(u[6]) && sqnorm<3>(rel<3>(P, V3{u[0], u[2], u[4]}, xj)) < lim;
+          }
+        }
         const f2_t CX = f2_pack(xj.x, xj.x), CY = f2_pack(xj.y, xj.y), CZ = f2_pack(xj.z, xj.z);
 #pragma unroll
         for (int p = 0; p < kCsrGroup; p += 2) {
@@ -509,6 +516,7 @@ __global__ void __launch_bounds__(kCsrWarps * 32) k_csr_rows(dv_params P, DevGri
       __syncwarp();  // s_t is read
     } while (todo);
   }
+  if (bad) ok[0] = 0;  // of dead lanes too: they tested candidates
   if (!live) return;
   uint32_t at = (uint32_t)nbr_row0(i);
   if (mylen <= kNbrRow) {
@@ -522,12 +530,11 @@ __global__ void __launch_bounds__(kCsrWarps * 32) k_csr_rows(dv_params P, DevGri
                              [&](int j, V3, float, int mj) { out[e++] = nbr_entry(j, mj, ok); });
       while (e & 3) out[e++] = i;
     } else {
-      bad = true;  // no room: the sweeps scan cells
+      ok[0] = 0;  // no room: the sweeps scan cells
     }
   }
   off[i] = at;
   len[i] = mylen;
-  if (bad) ok[0] = 0;
 }
 
 // 2-D: a block scans the cells of its particles (a thread each) into rows of
