@@ -5,6 +5,8 @@
 // The Jacobi loops run on the device: every iteration kernel returns at once
 // when the solve's done flag is set, so the host launches iterations in
 // chunks and waits for their outcome once per chunk instead of once per iteration.
+#include <sched.h>
+
 #include <algorithm>
 
 #include "dv_internal.cuh"
@@ -899,10 +901,15 @@ DV_API int dv_pressure_iteration(dv_ctx* c, const dv_fields* f) {
 // Waits for the test after iteration `launched` of solve E (or an earlier one
 // that ended it).  The tests write their result to pinned memory, which the
 // host reads without a copy and a synchronisation of the stream; a stream that
-// has nothing left, or failed, ends the wait.
+// has nothing left, or failed, ends the wait.  Only where the device's flags
+// (cudaSetDeviceFlags) leave the host spinning: with blocking synchronisation
+// the thread sleeps in cudaStreamSynchronize, with yielding it yields.
 static int solve_poll(dv_ctx* c, const SolveEnd& E, int launched, bool* over) {
   const volatile unsigned long long* h = c->h_solve;
-  for (int spins = 0;; ++spins) {
+  unsigned flags = 0;
+  DV_CK(c, cudaGetDeviceFlags(&flags));
+  flags &= cudaDeviceScheduleMask;
+  for (int spins = 0; flags != cudaDeviceScheduleBlockingSync; ++spins) {
     const unsigned long long v = *h;
     if ((uint32_t)(v >> 32) == E.solve && ((v >> 31 & 1) || (int)(v & 0x7fffffff) >= launched)) {
       *over = v >> 31 & 1;
@@ -914,6 +921,7 @@ static int solve_poll(dv_ctx* c, const SolveEnd& E, int launched, bool* over) {
       if (e != cudaSuccess) return dv_cuda_check(c, e, "Jacobi loop");
       break;
     }
+    if (flags == cudaDeviceScheduleYield) sched_yield();
   }
   DV_CK(c, cudaMemcpyAsync(c->h_flag, E.done, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
   DV_CK(c, cudaStreamSynchronize(c->stream));
