@@ -118,10 +118,9 @@ DV_API void dv_destroy(dv_ctx* c) {
   void* ptrs[] = {c->d_cnt,   c->d_flag,    c->keys[0],   c->keys[1],   c->vals[0], c->vals[1],
                   c->mt[0],     c->mt[1],   c->mt[2],
                   c->look_state, c->dscan_part, c->red_part, c->ired_part, c->flags, c->offs,
-                  c->targets, c->cdf,       c->spos,      c->sw,        c->near_v,  c->near_S,
+                  c->targets, c->spos,      c->sw,        c->near_v,  c->near_S,
                   c->far_acc, c->mult,      c->nbr_off,   c->nbr_idx,   c->d_nbr_ok,
-                  c->srank,     c->sslot,   c->nbr_len,   c->pk_a,    c->pk_b,
-                  c->pk_k};
+                  c->srank,     c->sslot,   c->nbr_len};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (int k = 0; k < 2 * dv_ctx::kProfPool; ++k)
@@ -202,12 +201,18 @@ DV_API dv_ctx* dv_create(const dv_params* params, int64_t capacity, void* stream
   A(c->flags, cap + 1);
   A(c->offs, cap + 1);
   A(c->targets, cap);
-  A(c->cdf, cap);
   A(c->spos, cap);
   A(c->sw, cap);
   A(c->near_v, cap);
   A(c->near_S, cap);
   A(c->far_acc, cap * DV_MAX_FAR_CHUNKS);
+  // Made and read within a call, before or without the far field's sums: the
+  // packed copies and the CDF lie in the room of its chunks (their own 48 bytes
+  // a particle made contexts that had fitted the memory fail)
+  c->pk_a = c->far_acc;
+  c->pk_b = c->far_acc + cap;
+  c->pk_k = reinterpret_cast<float2*>(c->far_acc + 2 * cap);
+  c->cdf = reinterpret_cast<double*>(c->far_acc + 3 * cap);
   A(c->mult, cap);
   A(c->srank, cap + 1);
   A(c->sslot, cap);
@@ -219,9 +224,6 @@ DV_API dv_ctx* dv_create(const dv_params* params, int64_t capacity, void* stream
   A(c->nbr_off, cap + 1);
   if (params->dim == 3) {
     A(c->nbr_len, cap);
-    A(c->pk_a, cap);
-    A(c->pk_b, cap);
-    A(c->pk_k, cap);
   }
   A(c->nbr_idx, c->nbr_cap);
   A(c->d_nbr_ok, 2);  // [0]: lists valid, [1]: keys valid
@@ -243,11 +245,7 @@ DV_API dv_ctx* dv_create(const dv_params* params, int64_t capacity, void* stream
     dv_destroy(c);
     return nullptr;
   }
-  if (dv_farbox_create(c) != DV_OK) {
-    g_create_error = c->err;
-    dv_destroy(c);
-    return nullptr;
-  }
+  dv_farbox_create(c);
   return c;
 }
 

@@ -697,21 +697,42 @@ __global__ void k_box_pack(dv_params P, dv_fields F, dv_solver_fields S, DevGrid
 
 }  // namespace
 
-int dv_farbox_create(dv_ctx* c) {
-  dv_farbox& B = c->farbox;
+static void free_buffers(dv_farbox& B) {
+  void* ptrs[] = {B.meta, B.bt, B.bs, B.tbox, B.tcnt, B.tile0, B.sbox, B.scnt, B.nodes, B.coef, B.pos, B.w};
+  for (void* p : ptrs)
+    if (p) cudaFree(p);
+}
+
+// Contexts that can use the boxes get them if the buffers (about 92 bytes a
+// particle) take at most a quarter of the free memory: a context is created
+// wherever it was without them, and leaves room for the caller's own arrays.
+void dv_farbox_create(dv_ctx* c) {
+  dv_farbox B;
   const dv_params& P = c->p;
-  if (P.dim != 3 || P.n_scenes > 1 || c->cap < kMinTargets) return DV_OK;
+  if (P.dim != 3 || P.n_scenes > 1 || P.periodic || P.compensated || c->cap < kMinTargets) return;
   int total = 0, low = 0;
   for (int d = 0; d < 3; ++d) {
     total += c->axis_bits[d];
     low += std::min(kLeafLog, c->axis_bits[d]);
   }
   const int64_t nbox = (int64_t)1 << (total - low);
-  if (nbox * kMinPerBox > c->cap || nbox >= (1 << 20)) return DV_OK;
+  if (nbox * kMinPerBox > c->cap || nbox >= (1 << 20)) return;
   B.lowbits = low;
   B.nbox = (int)nbox;
   B.max_boxes = (int)std::min<int64_t>(nbox, std::max<int64_t>(64, c->cap / 1536));
-  cudaError_t e = cudaSuccess;
+  int g2 = 0;  // the farthest boxes of this grid
+  for (int d = 0; d < 3; ++d) {
+    const int gap = std::max((P.grid_num[d] + (1 << kLeafLog) - 1 >> kLeafLog) - 2, 0);
+    g2 += gap * gap;
+  }
+  B.sets = std::max(gap_class(g2) + 1, 1);
+  // few boxes: more stripes, so that the node sums fill the chip
+  B.stripe_mul = B.max_boxes <= 96 ? 4 : B.max_boxes <= 256 ? 2 : 1;
+  const size_t large = sizeof(float) * (size_t)B.max_boxes * kFloatsMax * B.stripe_mul +
+                       sizeof(float4) * ((size_t)B.max_boxes * kCoefMax + 2 * (size_t)c->cap);
+  size_t room = 0, total_mem = 0;
+  cudaError_t e = cudaMemGetInfo(&room, &total_mem);
+  if (e == cudaSuccess && large > room / 4) return;
   auto al = [&](auto** p, int64_t count) {
     if (e == cudaSuccess) e = cudaMalloc((void**)p, sizeof(**p) * (size_t)count);
   };
@@ -723,30 +744,21 @@ int dv_farbox_create(dv_ctx* c) {
   al(&B.tile0, B.max_boxes);
   al(&B.sbox, nbox);
   al(&B.scnt, nbox);
-  int g2 = 0;  // the farthest boxes of this grid
-  for (int d = 0; d < 3; ++d) {
-    const int gap = std::max((P.grid_num[d] + (1 << kLeafLog) - 1 >> kLeafLog) - 2, 0);
-    g2 += gap * gap;
-  }
-  B.sets = std::max(gap_class(g2) + 1, 1);
-  // few boxes: more stripes, so that the node sums fill the chip
-  B.stripe_mul = B.max_boxes <= 96 ? 4 : B.max_boxes <= 256 ? 2 : 1;
   al(&B.nodes, (int64_t)B.max_boxes * kFloatsMax * B.stripe_mul);
   al(&B.coef, (int64_t)B.max_boxes * kCoefMax);
   al(&B.pos, c->cap);
   al(&B.w, c->cap);
   if (e == cudaSuccess) e = cudaMemset(B.meta, 0, 16 * sizeof(uint32_t));
-  if (e != cudaSuccess) return dv_cuda_check(c, e, "far-field boxes");
+  if (e != cudaSuccess) {
+    free_buffers(B);
+    cudaGetLastError();  // the context does without
+    return;
+  }
   B.enabled = 1;
-  return DV_OK;
+  c->farbox = B;
 }
 
-void dv_farbox_free(dv_ctx* c) {
-  dv_farbox& B = c->farbox;
-  void* ptrs[] = {B.meta, B.bt, B.bs, B.tbox, B.tcnt, B.tile0, B.sbox, B.scnt, B.nodes, B.coef, B.pos, B.w};
-  for (void* p : ptrs)
-    if (p) cudaFree(p);
-}
+void dv_farbox_free(dv_ctx* c) { free_buffers(c->farbox); }
 
 // Whether this call may use the boxes: a grid and a size that they are built
 // for, plain sums, and enough pairs (the sample count is known here for the

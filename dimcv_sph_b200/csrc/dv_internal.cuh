@@ -90,7 +90,7 @@ struct dv_ctx {
   int64_t red_cap = 0;
 
   // 3-D: per-sweep copies of the fields a neighbour walk gathers, packed so
-  // that a neighbour costs one or two 16-byte loads (dv_pack)
+  // that a neighbour costs one or two 16-byte loads (dv_pack); in far_acc's room
   float4* pk_a = nullptr;  // cap: (x, m_V)
   float4* pk_b = nullptr;  // cap: (v, m), (Δω, KVN) or (smoothed Δω, kden)
   float2* pk_k = nullptr;  // cap: (k, m) of the Jacobi solves
@@ -99,7 +99,7 @@ struct dv_ctx {
   uint32_t* flags = nullptr;   // cap+1
   uint32_t* offs = nullptr;    // cap+1
   int32_t* targets = nullptr;  // cap
-  double* cdf = nullptr;       // cap
+  double* cdf = nullptr;       // cap, in far_acc's room
   float4* spos = nullptr;      // cap
   float4* sw = nullptr;        // cap
   float4* near_v = nullptr;    // cap
@@ -253,8 +253,9 @@ int dv_far_min_tile_width();  // the narrowest far-field tile (threads per CTA x
 int dv_build_targets(dv_ctx* c, const dv_fields* f, bool check = false);
 // dv_farbox.cu: the 3-D far field by interpolation on boxes.  wanted: host-side
 // rule; begin (before dv_build_targets), pack (instead of the slot list), plan,
-// run; the device decides with farbox_on whether the result is used
-int dv_farbox_create(dv_ctx* c);
+// run; the device decides with farbox_on whether the result is used.  create
+// leaves a context that has no use or no memory for the boxes without them
+void dv_farbox_create(dv_ctx* c);
 void dv_farbox_free(dv_ctx* c);
 bool dv_farbox_wanted(const dv_ctx* c);
 int dv_farbox_near_parts(const dv_ctx* c);
