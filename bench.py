@@ -396,6 +396,8 @@ def run_ours(args, rank, world, local):
     launches = lib.dv_launch_count(ctx) - launches0
     far_ms, far_launches, pairs = C.c_double(), C.c_int64(), C.c_double()
     lib.dv_profile_read(ctx, C.byref(far_ms), C.byref(far_launches), C.byref(pairs))
+    box_calls, all_pairs = C.c_int64(), C.c_double()
+    _lib.check(ctx, lib.dv_profile_far(ctx, C.byref(box_calls), C.byref(all_pairs)), "dv_profile_far")
     lib.dv_profile(ctx, 0)
     cnt1 = ps.counters()
     n_fluid = 0.5 * (cnt0["n_fluid"] + cnt1["n_fluid"])
@@ -408,8 +410,7 @@ def run_ours(args, rank, world, local):
     far_chunks = int(ps.lib.dv_get_far_chunks(ps.ctx))
     # the library evaluates fewer pairs than targets x samples where its boxes
     # carry the far field (3-D, large); the traffic records are of the direct loop
-    all_pairs = float(cnt1["n_targets"]) * cnt1["num_samples"] * args.steps
-    boxes = pairs.value < 0.95 * all_pairs
+    boxes = box_calls.value > 0
     tr = None if boxes else far_traffic(
         args.workload if args.scale == 1.0 else f"{args.workload}@{args.scale:g}", solver.far_tile, far_chunks,
         cnt1["n_targets"])
@@ -420,7 +421,8 @@ def run_ours(args, rank, world, local):
                 "traffic": tr["bytes_per_launch"] if tr else None,
                 "peak_source": "measured in this run: FP32 FMA chain kernel (dv_fp32_peak), an FMA counts 2",
                 "flops_per_pair": FLOPS_PER_PAIR[dim], "pairs_per_step": pairs.value / args.steps,
-                "targets_x_samples_per_step": all_pairs / args.steps,
+                "targets_x_samples_per_step": all_pairs.value / args.steps,
+                "calls_on_boxes": box_calls.value,
                 "kernel_ms_per_step": far_ms.value / args.steps,
                 "kernel_share_of_step": far_ms.value / ms_local}
     if tr:

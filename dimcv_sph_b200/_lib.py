@@ -94,6 +94,7 @@ PROTOTYPES = {
     "dv_vpm_smooth_bwd": (C.c_int, [_P, C.POINTER(DvVpmPlan), i32, _P, _P, _P, _P, _P]),
     "dv_vpm_velocity": (C.c_int, [_P, C.POINTER(DvVpmPlan), i32, _P, _P, _P, _P, i64]),
     "dv_vpm_velocity_bwd": (C.c_int, [_P, C.POINTER(DvVpmPlan), i32, _P, _P, _P, _P, _P, _P, i64]),
+    "dv_profile_far": (C.c_int, [_P, C.POINTER(i64), C.POINTER(f64)]),
     "dv_profile_read": (C.c_int, [_P, C.POINTER(f64), C.POINTER(i64), C.POINTER(f64)]),
 }
 

@@ -140,7 +140,7 @@ struct dv_ctx {
   int prof_used = 0;
   double prof_ms = 0.0;
   int64_t prof_launches = 0;
-  double* d_prof = nullptr;  // device: [0] pairs
+  double* d_prof = nullptr;  // device: [0] pairs evaluated, [1] targets x samples, [2] calls on boxes
 };
 
 int dv_fail(dv_ctx* c, int code, const char* fmt, ...);

@@ -785,8 +785,11 @@ static void launch_fix(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s,
 // pair evaluations of the far field: every target with every sample, or those
 // of the boxes
 __global__ void k_prof_pairs(const dv_counters* __restrict__ C, double* acc, dv_farbox B) {
-  acc[0] += farbox_on(B, C) ? (double)*reinterpret_cast<const unsigned long long*>(B.meta + 4)
-                            : (double)C->n_targets * (double)C->num_samples;
+  const double all = (double)C->n_targets * (double)C->num_samples;
+  const bool on = farbox_on(B, C);
+  acc[0] += on ? (double)*reinterpret_cast<const unsigned long long*>(B.meta + 4) : all;
+  acc[1] += all;
+  acc[2] += on ? 1.0 : 0.0;
 }
 
 static int prof_fold(dv_ctx* c) {
@@ -995,6 +998,16 @@ DV_API int dv_vvpe_mc(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s) 
     k_prof_pairs<<<1, 1, 0, c->stream>>>(c->d_cnt, c->d_prof, B);
     DV_LAUNCHED(c);
   }
+  return DV_OK;
+}
+
+DV_API int dv_profile_far(dv_ctx* c, int64_t* box_calls, double* all_pairs) {
+  if (!c) return DV_EINVAL;
+  double h[4];
+  DV_CK(c, cudaMemcpyAsync(h, c->d_prof, sizeof(double) * 4, cudaMemcpyDeviceToHost, c->stream));
+  DV_CK(c, cudaStreamSynchronize(c->stream));
+  if (box_calls) *box_calls = (int64_t)h[2];
+  if (all_pairs) *all_pairs = h[1];
   return DV_OK;
 }
 

@@ -439,6 +439,10 @@ DV_API int dv_bs_full(dv_ctx* ctx, const dv_fields* f, const float* omega, const
  * synchronises and returns the totals since the reset. */
 DV_API int dv_profile(dv_ctx* ctx, int32_t enable);
 DV_API int dv_profile_read(dv_ctx* ctx, double* far_ms, int64_t* launches, double* pairs);
+/* New: since the same reset, the calls whose far field the boxes carried and
+ * the sum of n_targets × num_samples over all calls (synchronises; either
+ * pointer may be NULL). */
+DV_API int dv_profile_far(dv_ctx* ctx, int64_t* box_calls, double* all_pairs);
 
 /* Allocation-free FP64 density error, for callers that cannot allocate
  * device memory: real-time step loops that forbid allocation after
