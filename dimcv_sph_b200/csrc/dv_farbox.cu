@@ -151,7 +151,7 @@ __global__ void k_box_ranges(const uint32_t* __restrict__ keys, const dv_counter
                              int lowbits, const uint32_t* __restrict__ toff, const uint32_t* __restrict__ srank,
                              const int32_t* __restrict__ keys_ok, int32_t* __restrict__ bt, int32_t* __restrict__ bs) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b > nbox) return;
+  if (b > nbox || !farbox_worth(C)) return;
   const int n = keys_ok[1] ? C->n : 0;
   int lo = 0, hi = n;
   if (b == nbox) lo = n;
@@ -187,9 +187,11 @@ __device__ __forceinline__ int4 box_coords(uint32_t key, int b0, int b1, int b2)
 // Lists of the boxes with targets (coordinates, first target; count; first
 // near tile) and with samples (coordinates, first sample; count).  One block.
 __global__ void __launch_bounds__(1024) k_box_lists(const int32_t* __restrict__ bt, const int32_t* __restrict__ bs,
-                                                    int nbox, int lowbits, int b0, int b1, int b2, dv_farbox B) {
+                                                    int nbox, int lowbits, int b0, int b1, int b2, dv_farbox B,
+                                                    const dv_counters* __restrict__ C) {
   __shared__ unsigned long long s_w[32];
   __shared__ unsigned long long s_tot;
+  if (!farbox_worth(C)) return;  // meta says no boxes
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   unsigned long long carry = 0;  // boxes with targets | boxes with samples << 20 | tiles << 40
   for (int base = 0; base < nbox; base += 1024) {
@@ -679,7 +681,8 @@ __global__ void __launch_bounds__(kNearT, 2) k_box_near(dv_params P, dv_farbox B
 // call to the direct loop.
 __global__ void k_box_pack(dv_params P, dv_fields F, dv_solver_fields S, DevGrid G, const uint32_t* __restrict__ keys,
                            const int32_t* __restrict__ mult, int nu, const uint32_t* __restrict__ rank, int lowbits,
-                           const int32_t* __restrict__ slot, dv_farbox B) {
+                           const int32_t* __restrict__ slot, dv_farbox B, const dv_counters* __restrict__ C) {
+  if (!farbox_worth(C)) return;
   const int ns = (int)rank[nu];
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < ns; r += gridDim.x * blockDim.x) {
     const int j = slot[r], m = mult[j];
@@ -728,6 +731,7 @@ void dv_farbox_create(dv_ctx* c) {
   B.sets = std::max(gap_class(g2) + 1, 1);
   // few boxes: more stripes, so that the node sums fill the chip
   B.stripe_mul = B.max_boxes <= 96 ? 4 : B.max_boxes <= 256 ? 2 : 1;
+  B.node_rows = B.stripe_mul * all_stripes(B.sets);
   const size_t large = sizeof(float) * (size_t)B.max_boxes * kFloatsMax * B.stripe_mul +
                        sizeof(float4) * ((size_t)B.max_boxes * kCoefMax + 2 * (size_t)c->cap);
   size_t room = 0, total_mem = 0;
@@ -768,7 +772,12 @@ bool dv_farbox_wanted(const dv_ctx* c) {
   const int64_t nu = std::min<int64_t>(c->n_upper, c->cap);
   if (!c->farbox.enabled || c->batch || c->p.periodic || c->p.compensated) return false;
   if (nu < kMinTargets || (int64_t)c->farbox.nbox * kMinPerBox > nu) return false;
-  return c->host_samples >= 0 ? (double)c->host_samples * (double)nu > 3.0e8 : nu >= 400000;
+  if (c->host_samples < 0) return nu >= 400000;
+  // farbox_on's cost without a pair, with a box for 4,096 slots, and what the
+  // planning of a call that then takes the direct loop may cost
+  const double base = (double)kBoxFixed + (double)kBoxPerTarget * (double)nu +
+                      (double)kBoxPerRow * c->farbox.node_rows * (double)nu / 4096.0;
+  return (double)c->host_samples * (double)nu > base + 3.5e8;
 }
 
 int dv_farbox_begin(dv_ctx* c) {
@@ -779,7 +788,7 @@ int dv_farbox_begin(dv_ctx* c) {
 int dv_farbox_pack(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s, int nu) {
   k_box_pack<<<c->num_sms * 4, DV_THREADS, 0, c->stream>>>(c->p, *f, *s, dv_grid_cells(c), c->keys[c->perm_buf],
                                                            c->mult, nu, c->srank, c->farbox.lowbits, c->sslot,
-                                                           c->farbox);
+                                                           c->farbox, c->d_cnt);
   DV_LAUNCHED(c);
   return DV_OK;
 }
@@ -799,7 +808,7 @@ int dv_farbox_plan(dv_ctx* c) {
                                                                   c->offs, c->srank, c->d_nbr_ok, B.bt, B.bs);
   DV_LAUNCHED(c);
   k_box_lists<<<1, 1024, 0, c->stream>>>(B.bt, B.bs, B.nbox, B.lowbits, c->axis_bits[0], c->axis_bits[1],
-                                         c->axis_bits[2], B);
+                                         c->axis_bits[2], B, c->d_cnt);
   DV_LAUNCHED(c);
   if (c->p.kernel_mode == DV_KERNEL_BLOB3D)
     k_box_cost<true><<<B.max_boxes, 128, 0, c->stream>>>(B);
@@ -813,7 +822,7 @@ template <bool BLOB>
 static int run(dv_ctx* c, const dv_fields* f) {
   dv_farbox& B = c->farbox;
   const Nodes nd = make_nodes<BLOB>();
-  const dim3 gn(B.max_boxes, B.stripe_mul * all_stripes(B.sets));
+  const dim3 gn(B.max_boxes, B.node_rows);
   k_box_nodes<BLOB><<<gn, Sets<BLOB>::WARPS * 32, 0, c->stream>>>(c->p, B, nd, c->d_cnt);
   DV_LAUNCHED(c);
   k_box_coefs<BLOB><<<dim3(B.max_boxes, 3), kProjT, 0, c->stream>>>(B, c->d_cnt);

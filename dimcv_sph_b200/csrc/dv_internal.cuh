@@ -26,6 +26,7 @@ struct dv_farbox {
   int enabled = 0;
   int nbox = 0, lowbits = 0, max_boxes = 0, stripe_mul = 1;
   int sets = 1;  // distance classes that the grid is large enough for
+  int node_rows = 0;  // blocks of the node sums per box
   // [0] a position or weight that needs the direct loop; [1] boxes with
   // targets, [2] boxes with samples, [3] near tiles; [4..5] pair evaluations (u64)
   uint32_t* meta = nullptr;
@@ -606,18 +607,29 @@ __device__ __forceinline__ void for_each_neighbor_p(const dv_params& P, const De
 
 // ------------------------------------------------- far field on boxes (3-D)
 // Whether the boxes carry this call's far field: every position in its sorted
-// box and every weight of ordinary size (meta[0]), and fewer pair evaluations
-// than the direct loop: the node sums and near pairs, 250 a target for reading
-// the polynomial, 5e7 (about 25 us) for the extra launches, and a tenth of
-// slack.  The same answer in every thread of every kernel that asks.
+// box and every weight of ordinary size (meta[0]), and a cost below the direct
+// loop's, in pair evaluations: the node sums and near pairs with a tenth more for
+// part-filled tiles, 400 a target for reading the polynomial and the near
+// parts, 34,000 (17 ns) a block of node sums, and 1.1e8 (55 us) for planning and
+// launches.  The terms are a fit to ten scenes of 70,000 to 2 million
+// particles (cubes, channels, plates) at 1.5e8 to 4e9 pairs; with 250 a
+// target and 5e7 alone, calls of few samples a box took the boxes and were up
+// to 1.4 times slower (420,000 in a channel, 738 samples: 353 us by the direct
+// loop, 483).  The same answer in every thread of every kernel that asks.
+constexpr unsigned long long kBoxFixed = 110000000ull, kBoxPerTarget = 400ull, kBoxPerRow = 34000ull;
+// Whether they can be: planning stops where even without a pair they would lose.
+__device__ __forceinline__ bool farbox_worth(const dv_counters* __restrict__ C) {
+  const unsigned long long nt = (unsigned long long)C->n_targets;
+  return kBoxFixed + kBoxPerTarget * nt < nt * (unsigned long long)C->num_samples;
+}
 __device__ __forceinline__ bool farbox_on(const dv_farbox& B, const dv_counters* __restrict__ C) {
   if (!B.enabled) return false;
   const uint32_t na = B.meta[1];
   if (B.meta[0] || na == 0 || na > (uint32_t)B.max_boxes) return false;
   const unsigned long long nt = (unsigned long long)C->n_targets, M = (unsigned long long)C->num_samples;
-  const unsigned long long cost =
-      *reinterpret_cast<const unsigned long long*>(B.meta + 4) + 250ull * nt + 50000000ull;
-  return cost < nt * M / 10ull * 9ull;
+  const unsigned long long cost = *reinterpret_cast<const unsigned long long*>(B.meta + 4) / 10ull * 11ull +
+                                  kBoxPerTarget * nt + kBoxPerRow * na * (unsigned)B.node_rows + kBoxFixed;
+  return cost < nt * M / 20ull * 19ull;
 }
 
 // x lies inside the cell grid and its box is that of the sorted cell `key`
