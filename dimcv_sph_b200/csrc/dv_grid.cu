@@ -376,6 +376,12 @@ constexpr int kCsrWarps = 8;  // of a block
 // `one` is 1: the squares are added by an fma with it, which rounds as the
 // reference's addition does.  ptxas turned mul.rn.f32x2 and add.rn.f32x2 into
 // one fma, so that a pair at the support radius was missed.
+// Cells of a warp's 32 slots beyond which each lane scans for its own particle:
+// with few particles a cell the cells are handled one after the other, each for
+// one or two particles (grid build of 750,000 particles at random, cell by cell
+// and by lanes: 0.1 a cell 462 and 303 us, 1 a cell 337 and 290, 2 a cell, about
+// 14 cells a warp, 318 and 355).
+constexpr int kCsrSparse = 18;
 constexpr int kCsrGroup = 12;  // particles of a cell tested together (8 a cell on a lattice)
 __global__ void __launch_bounds__(kCsrWarps * 32) k_csr_rows(dv_params P, DevGrid G, const float* __restrict__ x,
                                                              const int32_t* __restrict__ mat,
@@ -404,6 +410,8 @@ __global__ void __launch_bounds__(kCsrWarps * 32) k_csr_rows(dv_params P, DevGri
   const f2_t ONE = f2_pack(one, one);
   uint32_t mylen = 0;
   bool bad = false;
+  const bool sparse = __popc(heads) > kCsrSparse;
+  if (sparse) heads = 0;
   while (heads) {
     const int h = __ffs(heads) - 1;
     heads &= heads - 1;
@@ -519,20 +527,33 @@ __global__ void __launch_bounds__(kCsrWarps * 32) k_csr_rows(dv_params P, DevGri
   if (bad) ok[0] = 0;  // of dead lanes too: they tested candidates
   if (!live) return;
   uint32_t at = (uint32_t)nbr_row0(i);
-  if (mylen <= kNbrRow) {
-    for (uint32_t e = mylen; e & 3u; ++e) out[4 * ((int64_t)at + 32 * (e >> 2)) + (e & 3u)] = i;
-  } else {
-    const uint32_t room = (mylen + 3u) / 4u, a = atomicAdd(far_used, room);  // the sum may wrap: no a + room
-    if (room <= far_cap && a <= far_cap - room) {
-      at = far0 + a;
-      int64_t e = 4 * (int64_t)at;
-      for_each_neighbor_m<3>(P, G, x, mat, i, xi,
-                             [&](int j, V3, float, int mj) { out[e++] = nbr_entry(j, mj, ok); });
-      while (e & 3) out[e++] = i;
+  // a lane's own scans: its row in a sparse warp, a row longer than its place
+#pragma unroll 1
+  for (int pass = sparse ? 0 : 1; pass < 2; ++pass) {
+    uint32_t step = 124u, room = kNbrRow;
+    if (pass == 0) {
+      if (!((built >> lane) & 1u)) continue;
     } else {
-      ok[0] = 0;  // no room: the sweeps scan cells
+      if (mylen <= kNbrRow) break;
+      const uint32_t quads = (mylen + 3u) / 4u, a = atomicAdd(far_used, quads);  // the sum may wrap: no a + quads
+      if (quads > far_cap || a > far_cap - quads) {
+        ok[0] = 0;  // no room: the sweeps scan cells
+        break;
+      }
+      at = far0 + a;
+      step = 0u;
+      room = 0xffffffffu;
     }
+    int32_t* row = out + 4 * (int64_t)at;
+    uint32_t k = 0;
+    for_each_neighbor_m<3>(P, G, x, mat, i, xi, [&](int j, V3, float, int mj) {
+      if (k < room) row[k + step * (k >> 2)] = nbr_entry(j, mj, ok);
+      ++k;
+    });
+    mylen = k;
   }
+  for (uint32_t e = mylen; e & 3u; ++e)
+    out[4 * ((int64_t)at + nbr_stride(mylen) * (e >> 2)) + (e & 3u)] = i;
   off[i] = at;
   len[i] = mylen;
 }
@@ -540,8 +561,8 @@ __global__ void __launch_bounds__(kCsrWarps * 32) k_csr_rows(dv_params P, DevGri
 // 2-D: a block scans the cells of its particles (a thread each) into rows of
 // up to kCsrSlots entries in shared memory, scans the lengths (look-back over
 // the blocks before) and copies the rows out, eight lanes a row, the
-// neighbours' materials gathered on the way; a particle with more neighbours
-// (a settled lattice has at most 20) scans its cells again.  Counting, a scan
+// neighbours' materials gathered on the way; a thread whose particle has more
+// neighbours (a settled lattice has at most 20) scans its cells again.  Counting, a scan
 // and filling, with two more launches for the checks, before: 10,000 particles
 // 33 -> 21 us, a batch of 340,000 70 -> 66.
 constexpr int kCsrSlots = 32;
@@ -580,8 +601,14 @@ __global__ void __launch_bounds__(T) k_csr_build(dv_params P, DevGrid G, const f
   const uint32_t at = look_prefix<T>(K, tile, total) + before + inc - k;
   if (i < m) off[i] = at;
   __syncwarp();
+  if (k > (uint32_t)kCsrSlots && (int64_t)at + k <= cap) {  // a thread for each long row
+    uint32_t e = at;
+    for_each_neighbor_m<2>(P, G, x, mat, i, ldv<2>(x, i),
+                           [&](int j, V3, float, int mj) { out[e++] = nbr_entry(j, mj, ok); });
+  }
+  __syncwarp();
   for (int g = 0; g < 32; g += 4) {
-    const int r = g + (lane >> 3), ir = tile * T + 32 * w + r;
+    const int r = g + (lane >> 3);
     const uint32_t cnt = __shfl_sync(0xffffffffu, k, r), o = __shfl_sync(0xffffffffu, at, r);
     if (cnt == 0) continue;
     // too long for the buffer: the sweeps scan cells.  Asked of every row, as
@@ -590,35 +617,91 @@ __global__ void __launch_bounds__(T) k_csr_build(dv_params P, DevGrid G, const f
       ok[0] = 0;
       continue;
     }
+    if (cnt > (uint32_t)kCsrSlots) continue;
     const int32_t* row = s_rows + (32 * w + r) * ST;
-    if (cnt <= (uint32_t)kCsrSlots) {
-      for (uint32_t e = lane & 7; e < cnt; e += 8) out[o + e] = nbr_entry(row[e], __ldg(mat + row[e]), ok);
-    } else if ((lane & 7) == 0) {
-      uint32_t e = o;
-      for_each_neighbor_m<2>(P, G, x, mat, ir, ldv<2>(x, ir),
-                             [&](int j, V3, float, int mj) { out[e++] = nbr_entry(j, mj, ok); });
-    }
+    for (uint32_t e = lane & 7; e < cnt; e += 8) out[o + e] = nbr_entry(row[e], __ldg(mat + row[e]), ok);
   }
   if (look_end(K) && tid == 0 && look_failed(K.C)) ok[0] = 0;  // offsets that may decrease: the sweeps scan cells
+}
+
+// 2-D in two launches, for scenes too dense for the buffer (build_csr): lengths
+// and offsets, then, if the lists fit all the same, a thread for each row.
+template <int T>
+__global__ void __launch_bounds__(T) k_csr_count(dv_params P, DevGrid G, const float* __restrict__ x,
+                                                 const int32_t* __restrict__ mat, const uint8_t* __restrict__ dyn,
+                                                 int m, int64_t cap, DevLook K, uint32_t* __restrict__ off, int32_t* ok) {
+  constexpr int W = T / 32;
+  __shared__ uint32_t s_w[W];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int tile = look_tile(K.ctl), i = tile * T + tid;
+  uint32_t k = 0;
+  if (i < K.C->n && nbr_row_built(mat, dyn, i))
+    for_each_neighbor<2>(P, G, x, i, ldv<2>(x, i), [&](int, V3, float) { ++k; });
+  uint32_t inc = k;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
+  }
+  if (lane == 31) s_w[w] = inc;
+  __syncthreads();
+  uint32_t before = 0, total = 0;
+#pragma unroll
+  for (int q = 0; q < W; ++q) {
+    before += q < w ? s_w[q] : 0u;
+    total += s_w[q];
+  }
+  const uint32_t at = look_prefix<T>(K, tile, total) + before + inc - k;
+  if (i < m) off[i] = at;
+  if (k && (int64_t)at + k > cap) ok[0] = 0;
+  if (look_end(K) && tid == 0 && look_failed(K.C)) ok[0] = 0;
+}
+__global__ void __launch_bounds__(DV_THREADS) k_csr_fill(dv_params P, DevGrid G, const float* __restrict__ x,
+                                                         const int32_t* __restrict__ mat,
+                                                         const dv_counters* __restrict__ C,
+                                                         const uint32_t* __restrict__ off, const int32_t* fits,
+                                                         int32_t* ok,
+                                                         int32_t* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= C->n || *fits == 0) return;
+  uint32_t e = off[i];
+  if (e == off[i + 1]) return;
+  for_each_neighbor_m<2>(P, G, x, mat, i, ldv<2>(x, i),
+                         [&](int j, V3, float, int mj) { out[e++] = nbr_entry(j, mj, ok); });
 }
 
 static int build_csr(dv_ctx* c, const dv_fields* f) {
   const int m = (int)std::min<int64_t>(c->n_upper, c->cap) + 1;
   DevGrid G = dv_grid_cells(c);
-#define CSR2(T)                                                                                                     \
-  k_csr_build<T><<<dv_blocks(m, T), T, 0, c->stream>>>(c->p, G, f->x, f->material, f->is_dynamic, m, c->nbr_cap,     \
-                                                       dv_look(c), c->nbr_off, c->d_nbr_ok, c->nbr_idx)
-  if (c->p.dim == 3)
+  if (c->p.dim == 3) {
+    const uint32_t far0 = (uint32_t)nbr_row0(c->cap + 31 & ~(int64_t)31);
     k_csr_rows<<<dv_blocks(m, kCsrWarps * 32), kCsrWarps * 32, 0, c->stream>>>(
-        c->p, G, f->x, f->material, f->is_dynamic, c->d_cnt, 1.0f, (uint32_t)nbr_row0(c->cap + 31 & ~(int64_t)31),
-        (uint32_t)(c->nbr_cap / 4 - nbr_row0(c->cap + 31 & ~(int64_t)31)), c->look_ctl + 2, c->nbr_off, c->nbr_len,
-        c->d_nbr_ok, c->nbr_idx);
-  else if (m <= 256 * c->num_sms)
-    CSR2(64);
+        c->p, G, f->x, f->material, f->is_dynamic, c->d_cnt, 1.0f, far0, (uint32_t)(c->nbr_cap / 4 - far0),
+        c->look_ctl + 2, c->nbr_off, c->nbr_len, c->d_nbr_ok, c->nbr_idx);
+    DV_LAUNCHED(c);
+    return DV_OK;
+  }
+  // One launch where as many particles spread evenly over the grid would have
+  // lists that fit; where they would not, the lists are counted first, as rows
+  // made for nothing cost more than a second scan (grid build, one launch and
+  // two: 1.5M particles at 9.4 a cell 706 and 391 us, 340,000 at 7 a cell, whose
+  // lists fit, 193 and 198, at 4 a cell on a lattice 131 and 142).
+  const double cells = (double)c->p.grid_num[0] * c->p.grid_num[1] * std::max(c->p.n_scenes, 1);
+  const bool small = m <= 256 * c->num_sms, dense = 3.1416 * (m - 1) * ((m - 1) / cells) > (double)c->nbr_cap;
+#define CSR2(K, T, ...)                                                                                          \
+  K<T><<<dv_blocks(m, T), T, 0, c->stream>>>(c->p, G, f->x, f->material, f->is_dynamic, m, c->nbr_cap, dv_look(c), \
+                                             c->nbr_off, c->d_nbr_ok, ##__VA_ARGS__)
+  if (dense)
+    small ? CSR2(k_csr_count, 64) : CSR2(k_csr_count, 256);
   else
-    CSR2(256);
+    small ? CSR2(k_csr_build, 64, c->nbr_idx) : CSR2(k_csr_build, 256, c->nbr_idx);
 #undef CSR2
   DV_LAUNCHED(c);
+  if (dense) {
+    k_csr_fill<<<dv_blocks(m - 1), DV_THREADS, 0, c->stream>>>(c->p, G, f->x, f->material, c->d_cnt, c->nbr_off,
+                                                               c->d_nbr_ok, c->d_nbr_ok, c->nbr_idx);
+    DV_LAUNCHED(c);
+  }
   return DV_OK;
 }
 
