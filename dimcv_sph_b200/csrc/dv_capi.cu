@@ -198,7 +198,7 @@ DV_API dv_ctx* dv_create(const dv_params* params, int64_t capacity, void* stream
   A(c->dscan_part, c->scan_part_cap);
   A(c->red_part, c->red_cap);
   A(c->ired_part, c->red_cap);
-  A(c->flags, cap + 1);
+  A(c->flags, cap + 5);
   A(c->offs, cap + 1);
   A(c->targets, cap);
   A(c->spos, cap);
@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(T) k_scan_u32(const uint32_t* __restrict__ in,
     }
   }
   if (look_end(K) && look_failed(K.C))
-    for (int e = tid; e < m; e += T) out[e] = 0u;
+    for (int e = tid; e < m; e += T) out[e] = e < m - 1 ? 0u : 0xffffffffu;
 }
 
 // in and out start on 16 bytes (both are whole allocations here)

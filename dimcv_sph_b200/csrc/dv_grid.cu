@@ -940,7 +940,8 @@ DV_API int64_t dv_stored_lists(dv_ctx* c, uint32_t* dev_offsets, int32_t* dev_nb
   }
   DV_CK(c, cudaMemcpyAsync(&ok, c->d_nbr_ok, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
   DV_CK(c, cudaMemcpyAsync(&total32, off + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
-  if ((rc = dv_get_counters(c, &cnt))) return rc;  // of the scan too; synchronises
+  DV_CK(c, cudaStreamSynchronize(c->stream));
+  if (total32 == 0xffffffffu && (rc = dv_get_counters(c, &cnt))) return rc;  // a wait of the scan ran out
   if (!ok) return dv_fail(c, DV_EINVAL, "dv_stored_lists: no valid lists (positions changed since the grid build)");
   const int64_t total = total32;
   if (dev_offsets)
@@ -969,20 +970,22 @@ DV_API int64_t dv_neighbor_lists(dv_ctx* c, const dv_fields* f, int64_t* dev_off
   // always the cell scan: this entry point checks the lists the sweeps use
   DevGrid G = dv_grid_cells(c);
   int nb = dv_blocks(n);
-  // all pairs in 64 bits (scratch words): the offsets have 32
-  unsigned long long* sum = reinterpret_cast<unsigned long long*>(c->dscan_part);
-  DV_CK(c, cudaMemsetAsync(sum, 0, sizeof(*sum), c->stream));
+  // the last count of the scan and, behind it, all pairs in 64 bits: the offsets have 32
+  unsigned long long* sum = reinterpret_cast<unsigned long long*>(c->flags + ((n + 2) & ~1));
+  DV_CK(c, cudaMemsetAsync(c->flags + n, 0, 4 * sizeof(uint32_t), c->stream));
   if (c->p.dim == 2)
     k_nbr_count<2><<<nb, DV_THREADS, 0, c->stream>>>(c->p, G, f->x, c->d_cnt, c->flags, sum);
   else
     k_nbr_count<3><<<nb, DV_THREADS, 0, c->stream>>>(c->p, G, f->x, c->d_cnt, c->flags, sum);
   DV_LAUNCHED(c);
-  DV_CK(c, cudaMemsetAsync(c->flags + n, 0, sizeof(uint32_t), c->stream));
   rc = dv_scan_u32(c, c->flags, c->offs, (int64_t)n + 1);
   if (rc) return rc;
-  int64_t total = 0;
-  DV_CK(c, cudaMemcpyAsync(&total, sum, sizeof(total), cudaMemcpyDeviceToHost, c->stream));
-  if ((rc = dv_get_counters(c, &cnt))) return rc;  // of the scan too; synchronises
+  DV_CK(c, cudaMemcpyAsync(c->h_flag, sum, sizeof(*sum), cudaMemcpyDeviceToHost, c->stream));
+  DV_CK(c, cudaMemcpyAsync(c->h_flag + 2, c->offs + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
+  DV_CK(c, cudaStreamSynchronize(c->stream));
+  const int64_t total = *reinterpret_cast<const int64_t*>(c->h_flag);
+  // a wait of the scan that ran out
+  if ((uint32_t)c->h_flag[2] == 0xffffffffu && (rc = dv_get_counters(c, &cnt))) return rc;
   if (total > (int64_t)0xffffffff)
     return dv_fail(c, DV_ECAPACITY, "dv_neighbor_lists: %lld pairs, at most 2^32 - 1", (long long)total);
   if (dev_offsets) {

@@ -9,7 +9,8 @@
 // Every wait is bounded (DevLook::spins polls); a wait that runs out raises
 // DV_WARN_WAIT and goes on with what it has, so a kernel always ends.  What
 // it makes is then not to be used as indices: while the bit is set the last
-// block of a scan or compaction replaces its result by an empty one, the lists
+// block of a scan or compaction replaces its result by an empty one (a scan's
+// total by 2^32 - 1, which its host side asks about), the lists
 // are off, and k_permute keeps the order; the host gets DV_EWAIT from
 // its next synchronising call.  The last block to finish zeroes the state for
 // the next launch.

@@ -853,9 +853,9 @@ __global__ void k_farbox_on(dv_farbox B, const dv_counters* __restrict__ C, int3
   *out = farbox_on(B, C) ? 1 : 0;
 }
 
-// Times the far-field main loop for 2, 4, 6 and 8 targets per thread on the
-// current targets and samples (CUDA events, best of two launches after one
-// warm-up) and keeps the fastest for this context.
+// Times the far-field main loop for 2, 4, 6 and 8 targets per thread and 1 to 8
+// sample chunks on the current targets and samples (CUDA events, best of two
+// launches after a warm-up of each tile, 68 launches) and keeps the fastest for this context.
 DV_API int dv_autotune(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s, int32_t* best_tt,
                        float* best_ms) {
   if (!c || !f || !s || !s->sample_idx) return DV_EINVAL;
@@ -889,26 +889,33 @@ DV_API int dv_autotune(dv_ctx* c, const dv_fields* f, const dv_solver_fields* s,
   DV_CK(c, cudaEventCreate(&e0));
   DV_CK(c, cudaEventCreate(&e1));
   const int cand[4] = {2, 4, 6, 8};
+  auto launch = [&](int tt) {
+    if (c->p.dim == 2)
+      launch_main<2>(c, f, tt, none);
+    else
+      launch_main<3>(c, f, tt, none);
+  };
+  for (int tt : cand) {  // a warm-up of each tile's kernel
+    launch(tt);
+    DV_LAUNCHED(c);
+  }
   float best = 1e30f;
   int best_t = c->far_tt, best_c = c->far_chunks;
-  // every chunk count: a grid of two to four waves of blocks can waste most of its
-  // last one (62,500 targets: 41 tiles of 1,536 on 296 resident blocks are one
-  // wave with 7 chunks, 78 us, and 1.1 with 8; 1, 2, 3, 4, 6 and 8 alone gave 92)
+  // every chunk count: a grid of a few waves of blocks can waste most of its last
+  // one (62,500 targets: 41 tiles of 1,536 on 296 resident blocks are one wave
+  // with 7 chunks, 78 us, and 1.1 with 8; 1, 2, 3, 4, 6 and 8 alone gave 92)
   for (int nc = 1; nc <= DV_MAX_FAR_CHUNKS; ++nc) {
     c->far_chunks = nc;
     for (int tt : cand) {
-      for (int rep = 0; rep < 3; ++rep) {
+      for (int rep = 0; rep < 2; ++rep) {
         DV_CK(c, cudaEventRecord(e0, c->stream));
-        if (c->p.dim == 2)
-          launch_main<2>(c, f, tt, none);
-        else
-          launch_main<3>(c, f, tt, none);
+        launch(tt);
         DV_LAUNCHED(c);
         DV_CK(c, cudaEventRecord(e1, c->stream));
         DV_CK(c, cudaEventSynchronize(e1));
         float ms = 0.f;
         DV_CK(c, cudaEventElapsedTime(&ms, e0, e1));
-        if (rep > 0 && ms < best) {
+        if (ms < best) {
           best = ms;
           best_t = tt;
           best_c = nc;
