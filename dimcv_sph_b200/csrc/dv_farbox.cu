@@ -720,6 +720,8 @@ void dv_farbox_create(dv_ctx* c) {
   }
   const int64_t nbox = (int64_t)1 << (total - low);
   if (nbox * kMinPerBox > c->cap || nbox >= (1 << 20)) return;
+  for (int d = 0; d < 3; ++d)  // the squared gaps are 32-bit (2^15 boxes on one axis leave 2^5 on the others)
+    if (P.grid_num[d] > 1 << (15 + kLeafLog)) return;
   B.lowbits = low;
   B.nbox = (int)nbox;
   B.max_boxes = (int)std::min<int64_t>(nbox, std::max<int64_t>(64, c->cap / 1536));

@@ -54,3 +54,17 @@ def test_boxes_only_where_memory_allows(cuda):
     full, plain = used(ps, p, n), used(ps, params(compensated=True, **fine)[1], n)
     assert full > plain + 60 * n
     assert used(ps, p, n, keep=plain + (64 << 20)) <= plain + (16 << 20)
+
+
+def test_no_boxes_on_an_axis_too_long(cuda):
+    """Squared gaps of 46,341 boxes and more along an axis do not fit 32 bits
+    (a channel of 400,000 x 8 x 8 cells has 50,000): such grids have no boxes."""
+    n = 17_000_000  # enough slots for 256 in each of 65,536 boxes
+    h = 0.01
+    shape = {"domainEnd": [400_000 * h, 8 * h, 8 * h], "particleRadius": h / 4}
+    ps, p = params(**shape)
+    assert p.grid_num[0] >= 400_000
+    gap = p.grid_num[0] // 8 - 2
+    assert gap * gap > 2 ** 31
+    full, plain = used(ps, p, n), used(ps, params(compensated=True, **shape)[1], n)
+    assert full <= plain + (16 << 20)
