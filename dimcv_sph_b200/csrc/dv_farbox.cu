@@ -48,6 +48,7 @@
 // box centre before any rounding matters, so nodes carry no position error.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "dv_far.cuh"
 #include "dv_internal.cuh"
@@ -700,12 +701,6 @@ __global__ void k_box_pack(dv_params P, dv_fields F, dv_solver_fields S, DevGrid
 
 }  // namespace
 
-static void free_buffers(dv_farbox& B) {
-  void* ptrs[] = {B.meta, B.bt, B.bs, B.tbox, B.tcnt, B.tile0, B.sbox, B.scnt, B.nodes, B.coef, B.pos, B.w};
-  for (void* p : ptrs)
-    if (p) cudaFree(p);
-}
-
 // Contexts that can use the boxes get them if the buffers (about 92 bytes a
 // particle) take at most a quarter of the free memory: a context is created
 // wherever it was without them, and leaves room for the caller's own arrays.
@@ -734,29 +729,38 @@ void dv_farbox_create(dv_ctx* c) {
   // few boxes: more stripes, so that the node sums fill the chip
   B.stripe_mul = B.max_boxes <= 96 ? 4 : B.max_boxes <= 256 ? 2 : 1;
   B.node_rows = B.stripe_mul * all_stripes(B.sets);
-  const size_t large = sizeof(float) * (size_t)B.max_boxes * kFloatsMax * B.stripe_mul +
-                       sizeof(float4) * ((size_t)B.max_boxes * kCoefMax + 2 * (size_t)c->cap);
+  // one allocation, its parts on 256 bytes
+  size_t size = 0;
+  auto part = [&](auto** p, size_t count) {
+    if (B.buffer) *p = reinterpret_cast<std::remove_pointer_t<decltype(p)>>(static_cast<char*>(B.buffer) + size);
+    size += (sizeof(**p) * count + 255) & ~(size_t)255;
+  };
+  auto parts = [&] {
+    size = 0;
+    part(&B.meta, 16);
+    part(&B.bt, nbox + 1);
+    part(&B.bs, nbox + 1);
+    part(&B.tbox, B.max_boxes);
+    part(&B.tcnt, B.max_boxes);
+    part(&B.tile0, B.max_boxes);
+    part(&B.sbox, nbox);
+    part(&B.scnt, nbox);
+    part(&B.nodes, (size_t)B.max_boxes * kFloatsMax * B.stripe_mul);
+    part(&B.coef, (size_t)B.max_boxes * kCoefMax);
+    part(&B.pos, c->cap);
+    part(&B.w, c->cap);
+  };
+  parts();
   size_t room = 0, total_mem = 0;
   cudaError_t e = cudaMemGetInfo(&room, &total_mem);
-  if (e == cudaSuccess && large > room / 4) return;
-  auto al = [&](auto** p, int64_t count) {
-    if (e == cudaSuccess) e = cudaMalloc((void**)p, sizeof(**p) * (size_t)count);
-  };
-  al(&B.meta, 16);
-  al(&B.bt, nbox + 1);
-  al(&B.bs, nbox + 1);
-  al(&B.tbox, B.max_boxes);
-  al(&B.tcnt, B.max_boxes);
-  al(&B.tile0, B.max_boxes);
-  al(&B.sbox, nbox);
-  al(&B.scnt, nbox);
-  al(&B.nodes, (int64_t)B.max_boxes * kFloatsMax * B.stripe_mul);
-  al(&B.coef, (int64_t)B.max_boxes * kCoefMax);
-  al(&B.pos, c->cap);
-  al(&B.w, c->cap);
-  if (e == cudaSuccess) e = cudaMemset(B.meta, 0, 16 * sizeof(uint32_t));
+  if (e == cudaSuccess && size > room / 4) return;
+  if (e == cudaSuccess) e = cudaMalloc(&B.buffer, size);
+  if (e == cudaSuccess) {
+    parts();
+    e = cudaMemset(B.meta, 0, 16 * sizeof(uint32_t));
+  }
   if (e != cudaSuccess) {
-    free_buffers(B);
+    if (B.buffer) cudaFree(B.buffer);
     cudaGetLastError();  // the context does without
     return;
   }
@@ -764,7 +768,9 @@ void dv_farbox_create(dv_ctx* c) {
   c->farbox = B;
 }
 
-void dv_farbox_free(dv_ctx* c) { free_buffers(c->farbox); }
+void dv_farbox_free(dv_ctx* c) {
+  if (c->farbox.buffer) cudaFree(c->farbox.buffer);
+}
 
 // Whether this call may use the boxes: a grid and a size that they are built
 // for, plain sums, and enough pairs (the sample count is known here for the

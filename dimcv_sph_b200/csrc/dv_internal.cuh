@@ -27,6 +27,7 @@ struct dv_farbox {
   int nbox = 0, lowbits = 0, max_boxes = 0, stripe_mul = 1;
   int sets = 1;  // distance classes that the grid is large enough for
   int node_rows = 0;  // blocks of the node sums per box
+  void* buffer = nullptr;  // holds all arrays
   // [0] a position or weight that needs the direct loop; [1] boxes with
   // targets, [2] boxes with samples, [3] near tiles; [4..5] pair evaluations (u64)
   uint32_t* meta = nullptr;
