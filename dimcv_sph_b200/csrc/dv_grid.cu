@@ -90,7 +90,9 @@ __device__ __forceinline__ uint32_t cell_key(const dv_params& P, const dv_fields
 #define RS_TILE 2048  // elements of a block of the narrow form (8 rounds); the wide one takes 4,096
 #define RS_MAXP 4
 
-// rounds of 256 elements a block: 8, or 1 where that leaves most SMs idle
+// Rounds of 256 elements a block: 8 from 4 tiles an SM on, where the blocks'
+// atomic additions are the longer part (1.44M elements 17.9 us, with one round
+// 18.4), else 1 (0.81M 13.8 and 9.3, 10,000 9.9 and 2.8).
 template <int D, int R>
 __global__ void __launch_bounds__(RS_T) k_cell_keys(dv_params P, dv_fields F, DevGrid G, dv_counters* C,
                                                     uint32_t* __restrict__ keys, uint32_t invalid,
@@ -564,14 +566,14 @@ __global__ void __launch_bounds__(kCsrWarps * 32) k_csr_rows(dv_params P, DevGri
 // neighbours' materials gathered on the way; a thread whose particle has more
 // neighbours (a settled lattice has at most 20) scans its cells again.  Counting, a scan
 // and filling, with two more launches for the checks, before: 10,000 particles
-// 33 -> 21 us, a batch of 340,000 70 -> 66.
+// 33 -> 16 us, a batch of 340,000 70 -> 66.
 constexpr int kCsrSlots = 32;
-template <int T>
-__global__ void __launch_bounds__(T) k_csr_build(dv_params P, DevGrid G, const float* __restrict__ x,
+constexpr int kCsrT = 256;  // threads of a block; with 64, small scenes were slower too (10,000 particles 19.9 us, 16.2)
+__global__ void __launch_bounds__(kCsrT) k_csr_build(dv_params P, DevGrid G, const float* __restrict__ x,
                                                  const int32_t* __restrict__ mat, const uint8_t* __restrict__ dyn,
                                                  int m, int64_t cap, DevLook K, uint32_t* __restrict__ off, int32_t* ok,
                                                  int32_t* __restrict__ out) {
-  constexpr int ST = kCsrSlots + 1, W = T / 32;
+  constexpr int T = kCsrT, ST = kCsrSlots + 1, W = T / 32;
   __shared__ int32_t s_rows[T * ST];
   __shared__ uint32_t s_w[W];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -626,11 +628,10 @@ __global__ void __launch_bounds__(T) k_csr_build(dv_params P, DevGrid G, const f
 
 // 2-D in two launches, for scenes too dense for the buffer (build_csr): lengths
 // and offsets, then, if the lists fit all the same, a thread for each row.
-template <int T>
-__global__ void __launch_bounds__(T) k_csr_count(dv_params P, DevGrid G, const float* __restrict__ x,
+__global__ void __launch_bounds__(kCsrT) k_csr_count(dv_params P, DevGrid G, const float* __restrict__ x,
                                                  const int32_t* __restrict__ mat, const uint8_t* __restrict__ dyn,
                                                  int m, int64_t cap, DevLook K, uint32_t* __restrict__ off, int32_t* ok) {
-  constexpr int W = T / 32;
+  constexpr int T = kCsrT, W = T / 32;
   __shared__ uint32_t s_w[W];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int tile = look_tile(K.ctl), i = tile * T + tid;
@@ -687,15 +688,14 @@ static int build_csr(dv_ctx* c, const dv_fields* f) {
   // two: 1.5M particles at 9.4 a cell 706 and 391 us, 340,000 at 7 a cell, whose
   // lists fit, 193 and 198, at 4 a cell on a lattice 131 and 142).
   const double cells = (double)c->p.grid_num[0] * c->p.grid_num[1] * std::max(c->p.n_scenes, 1);
-  const bool small = m <= 256 * c->num_sms, dense = 3.1416 * (m - 1) * ((m - 1) / cells) > (double)c->nbr_cap;
-#define CSR2(K, T, ...)                                                                                          \
-  K<T><<<dv_blocks(m, T), T, 0, c->stream>>>(c->p, G, f->x, f->material, f->is_dynamic, m, c->nbr_cap, dv_look(c), \
-                                             c->nbr_off, c->d_nbr_ok, ##__VA_ARGS__)
+  const bool dense = 3.1416 * (m - 1) * ((m - 1) / cells) > (double)c->nbr_cap;
+  const int nb = dv_blocks(m, kCsrT);
   if (dense)
-    small ? CSR2(k_csr_count, 64) : CSR2(k_csr_count, 256);
+    k_csr_count<<<nb, kCsrT, 0, c->stream>>>(c->p, G, f->x, f->material, f->is_dynamic, m, c->nbr_cap, dv_look(c),
+                                             c->nbr_off, c->d_nbr_ok);
   else
-    small ? CSR2(k_csr_build, 64, c->nbr_idx) : CSR2(k_csr_build, 256, c->nbr_idx);
-#undef CSR2
+    k_csr_build<<<nb, kCsrT, 0, c->stream>>>(c->p, G, f->x, f->material, f->is_dynamic, m, c->nbr_cap, dv_look(c),
+                                             c->nbr_off, c->d_nbr_ok, c->nbr_idx);
   DV_LAUNCHED(c);
   if (dense) {
     k_csr_fill<<<dv_blocks(m - 1), DV_THREADS, 0, c->stream>>>(c->p, G, f->x, f->material, c->d_cnt, c->nbr_off,
@@ -752,7 +752,7 @@ DV_API int dv_grid_build(dv_ctx* c, const dv_fields* src, const dv_fields* dst) 
   const size_t zeroed =
       (size_t)c->look_words + 2 * (size_t)c->ncells + 256 * (size_t)c->npasses * (size_t)(tiles + 1) + 64;
   DV_CK(c, cudaMemsetAsync(c->look_state, 0, sizeof(uint32_t) * zeroed, c->stream));
-  const int kr = ntiles < 2 * c->num_sms ? 1 : 8;
+  const int kr = ntiles < 4 * c->num_sms ? 1 : 8;
 #define CK(DD, RR)                                                                                                  \
   k_cell_keys<DD, RR><<<dv_blocks(nu, RS_T * RR), RS_T, 0, c->stream>>>(c->p, *src, G, c->d_cnt, c->keys[0], invalid, \
                                                                         scn, c->scene_shift, c->npasses, count)
