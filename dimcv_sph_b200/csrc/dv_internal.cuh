@@ -628,9 +628,9 @@ __device__ __forceinline__ bool farbox_on(const dv_farbox& B, const dv_counters*
   const uint32_t na = B.meta[1];
   if (B.meta[0] || na == 0 || na > (uint32_t)B.max_boxes) return false;
   const unsigned long long nt = (unsigned long long)C->n_targets, M = (unsigned long long)C->num_samples;
-  const unsigned long long cost = *reinterpret_cast<const unsigned long long*>(B.meta + 4) / 10ull * 11ull +
-                                  kBoxPerTarget * nt + kBoxPerRow * na * (unsigned)B.node_rows + kBoxFixed;
-  return cost < nt * M / 20ull * 19ull;
+  const unsigned long long pairs = *reinterpret_cast<const unsigned long long*>(B.meta + 4);
+  const unsigned long long rest = kBoxPerTarget * nt + kBoxPerRow * na * (unsigned)B.node_rows + kBoxFixed;
+  return 22ull * pairs + 20ull * rest < 19ull * nt * M;  // 1.1 pairs + rest < 0.95 nt M
 }
 
 // x lies inside the cell grid and its box is that of the sorted cell `key`
