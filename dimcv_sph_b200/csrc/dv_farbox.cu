@@ -5,7 +5,7 @@
 // 0.82 of the FP32 peak, so only fewer pairs make it faster.  The targets of
 // a box of 8 x 8 x 8 cells (about 4,000 on an SPH lattice) see every sample
 // outside the 27 boxes around them as a smooth field: it is evaluated at a
-// few hundred nodes of the box, turned into a polynomial and read off at each
+// 54 to 855 nodes of the box, turned into a polynomial and read off at each
 // target.  The samples of the 27 boxes are summed pair by pair as before (the
 // samples within the support radius among them, which k_far_fix removes).
 //
@@ -35,11 +35,11 @@
 // blob kernel, 262,144 x 16,384).
 //
 // Far field on one B200, direct loop and boxes:
-//   2.02M targets x 63k samples, reference kernel   51.8 -> 6.9 ms
+//   2.02M targets x 63k samples, reference kernel   51.8 -> 7.0 ms
 //   262,144 x 16,384, blob kernel                   2.57 -> 1.07 ms
 //   205,379 x 6,418, reference kernel               0.60 -> 0.33 ms
 // The node sums and near pairs are bound by the FP32 pipe as the direct loop
-// is (two f32x2 lanes an instruction, far_x2_loop): 3.9 and 2.3 ms of the 6.9;
+// is (two f32x2 lanes an instruction, far_x2_loop): 3.9 and 2.3 ms of the 7.0;
 // reading the polynomial 0.3, staging the samples 0.2, the projection 0.1.
 // 16 cells on a side would make 8 times larger near parts, 4 cells (512
 // targets) no longer pay for 686 nodes.
@@ -726,7 +726,10 @@ void dv_farbox_create(dv_ctx* c) {
     g2 += gap * gap;
   }
   B.sets = std::max(gap_class(g2) + 1, 1);
-  // few boxes: more stripes, so that the node sums fill the chip
+  // Few boxes: more stripes, so that the node sums fill the chip.  Stage with 1,
+  // 2 and 4: 27 boxes (buffers for 64) 818, 758 and 699 us, 64 boxes 505, 488 and
+  // 503, a ring of 262,144 (buffers for 170) 1,273 and 1,258 with 1 and 2, a
+  // channel on 252 565, 608 and 706, a cube on 512 1,791, 1,888 and 2,143.
   B.stripe_mul = B.max_boxes <= 96 ? 4 : B.max_boxes <= 256 ? 2 : 1;
   B.node_rows = B.stripe_mul * all_stripes(B.sets);
   // one allocation, its parts on 256 bytes
@@ -773,9 +776,11 @@ void dv_farbox_free(dv_ctx* c) {
 }
 
 // Whether this call may use the boxes: a grid and a size that they are built
-// for, plain sums, and enough pairs (the sample count is known here for the
-// CDF and injected samplers; the birth/death sampler's lives on the device,
-// and only sizes where the planning kernels are below 1% of a step ask it).
+// for, plain sums, and enough pairs.  The sample count is known here for the
+// CDF and injected samplers; the birth/death sampler's lives on the device, and
+// only sizes where the planning kernels are below 1% of a step ask it.  Planning
+// a call that then takes the direct loop costs some 40 us (205,379 x 2,434:
+// 391 and 340 us with and without).
 bool dv_farbox_wanted(const dv_ctx* c) {
   const int64_t nu = std::min<int64_t>(c->n_upper, c->cap);
   if (!c->farbox.enabled || c->batch || c->p.periodic || c->p.compensated) return false;

@@ -267,9 +267,9 @@ int dv_farbox_plan(dv_ctx* c);
 int dv_farbox_run(dv_ctx* c, const dv_fields* f);
 
 // ------------------------------------------------------------- scan helpers
-// Exclusive scan of uint32 / double arrays on the context stream (uint32: one
-// launch, dv_lookback.cuh; double: deterministic three-phase block reduce,
-// scan of partials, block scan).
+// Exclusive scan of a uint32 array on the context stream (one launch,
+// dv_lookback.cuh) and of the draws' FP64 weights (two: tile sums with their
+// scan in the last block, then the tiles; the same order of additions always).
 int dv_scan_u32(dv_ctx* c, const uint32_t* in, uint32_t* out, int64_t m);
 // out[k] = sum of kden[targets[q]], q < k (0 past the target count), k < m
 int dv_scan_cdf(dv_ctx* c, const int32_t* targets, const float* kden, double* out, int64_t m);

@@ -41,9 +41,12 @@ namespace {
 constexpr int VT = 256;  // threads per block of the pair kernels
 constexpr int VTT = 2;   // targets per thread (FP64)
 constexpr int VTS = 128; // sources per shared-memory tile
-// targets per thread of the FP32 kernels: wide where there are targets enough
+// Targets per thread of the FP32 kernels: wide where there are targets enough
 // for it (the source side's warp reduction is shared by them), narrow for
-// small clouds, which need the blocks
+// small clouds, which need the blocks.  Both directions with wide and narrow
+// tiles, all particles as sources: 2,025 targets 104 and 100 us, 8,281 254 and
+// 259, 16,384 528 and 671; a sixteenth: 2,025 98 and 91, 10,000 102 and 101,
+// 16,384 118 and 127.
 constexpr int kWideN = 8192;
 __host__ inline int fwd_tt(int n) { return n >= kWideN ? 4 : 2; }
 __host__ inline int bwd_tt(int n) { return n >= kWideN ? 8 : 2; }
@@ -465,8 +468,8 @@ __device__ __forceinline__ void stage_sources(float4* s4, const float* __restric
 }
 
 // Targets 2p and 2p + 1 of a thread are the lanes of pair p.  Bound by the
-// FP32 pipe, 15 lane operations a pair with the periodic image; 65,536
-// targets x 4,096 sources: 245 -> 139 us (0.74 of the pipe).
+// FP32 pipe, 17 lane operations a pair with the periodic image; 65,536
+// targets x 4,096 sources: 245 -> 152 us (0.68 of the pipe).
 template <int IMG, int TT>
 __global__ void __launch_bounds__(VT) k_far_x2(Geo<float> g, dv_vpm_plan p, const float* __restrict__ x,
                                                const float* __restrict__ xb, const float* __restrict__ sp,
@@ -545,10 +548,10 @@ __device__ __forceinline__ float warp_sum5(float v0, float v1, float v2, float v
   return a;
 }
 
-// k_far_bwd for FP32, 25 lane operations a pair; the source side's five sums
+// k_far_bwd for FP32, 27 lane operations a pair; the source side's five sums
 // are added over the thread's targets before the warp reduction, so a wide
 // tile (8 targets) spends a tenth of its issue slots there instead of half.
-// 65,536 targets x 4,096 sources: 675 -> 281 us (6 targets: 310).
+// 65,536 targets x 4,096 sources: 675 -> 296 us.
 template <int IMG, int TT>
 __global__ void __launch_bounds__(VT) k_far_bwd_x2(Geo<float> g, dv_vpm_plan p, const float* __restrict__ x,
                                                    const float* __restrict__ xb, const float* __restrict__ sp,

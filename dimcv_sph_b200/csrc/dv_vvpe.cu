@@ -214,9 +214,10 @@ static bool fast_kernel_ok(const dv_params& P) {
 // adds a bounded term (|r_xy|/T·|ω̂| <= |ω̂|/h, the size of the largest far
 // terms).  A second kernel then finds, per target, the few samples with
 // |r| <= h — exactly, with the reference's non-FMA |r|² test — among the
-// particles of the target's cell window, subtracts their terms (recomputed
-// bit for bit as the main loop computed them) and removes them from the far
-// count.  Per pair this leaves ~14 issue slots instead of ~28.
+// particles of the target's cell window, subtracts their terms (recomputed by the
+// main loop's operations, to one rounding of each: the loop adds its products
+// unrounded, and the boxes' pair loop takes a sample drawn m times once with m
+// times its weight) and removes them from the far count.  Per pair this leaves ~14 issue slots instead of ~28.
 
 // coordinate difference, minimum image on a periodic box
 template <bool PER>

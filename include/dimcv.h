@@ -406,8 +406,9 @@ DV_API int dv_sample(dv_ctx* ctx, const dv_fields* f, const dv_solver_fields* s,
  * far field over sample_idx[0:num_samples], the ‖v_vort‖ < ‖v‖ gate.  In 3-D,
  * uncompensated, non-periodic and from 65,536 particles on, the far field of
  * targets and samples that lie in the boxes of the last grid build is
- * interpolated on those boxes where that takes fewer pair evaluations (chosen
- * on the device; same accuracy); every other call sums all pairs. */
+ * interpolated on those boxes where that costs less (chosen on the device;
+ * errors not above those of the sum of all pairs); every other call, and a
+ * context whose boxes found no memory, sums all pairs. */
 DV_API int dv_vvpe_mc(dv_ctx* ctx, const dv_fields* f, const dv_solver_fields* s);
 /* New (tuning): times the far-field main loop of dv_vvpe_mc for 2, 4, 6 and 8
  * targets per thread (6 runs as 8 where the loop is not the paired one) and
