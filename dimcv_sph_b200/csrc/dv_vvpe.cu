@@ -1313,14 +1313,27 @@ __global__ void k_bs_chunk_sum(const float4* __restrict__ acc, int nt, int nchun
   reinterpret_cast<float4*>(out)[t] = make_float4(a.x * coef, a.y * coef, a.z * coef, 0.0f);
 }
 
+// tiles of tt targets a thread, and source chunks: enough for about eight waves,
+// within the partial-sum buffer
+static int64_t bs_tiles(int nt, int tt) { return ((int64_t)nt + (int64_t)FT2 * tt - 1) / ((int64_t)FT2 * tt); }
+static int bs_chunks(const dv_ctx* c, int64_t tiles, int tt) {
+  const int64_t resident = (int64_t)c->num_sms * DV_FAR_MINB(tt) * 256 / FT2;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(DV_MAX_FAR_CHUNKS, (8 * resident + tiles - 1) / tiles));
+}
+// The work of the busiest SM (blocks x targets a thread x sources of a chunk, in
+// parts of all sources).  Up to a quarter million targets it decides: a grid is
+// one to seven blocks an SM, and 8 targets a thread give half as many blocks.
+static double bs_cost(const dv_ctx* c, int nt, int tt) {
+  const int64_t tiles = bs_tiles(nt, tt);
+  const int nchunk = bs_chunks(c, tiles, tt);
+  return (double)((tiles * nchunk + c->num_sms - 1) / c->num_sms) * tt / nchunk;
+}
+
 template <int TTV>
 static int launch_bs_x2(dv_ctx* c, const dv_fields* f, const int32_t* targets, int nt, const int32_t* ns,
                         float* out) {
-  const int64_t tiles = ((int64_t)nt + (int64_t)FT2 * TTV - 1) / ((int64_t)FT2 * TTV);
-  const int64_t resident = (int64_t)c->num_sms * DV_FAR_MINB(TTV) * 256 / FT2;
-  // enough chunks for about eight waves, within the partial-sum buffer
-  const int nchunk =
-      (int)std::max<int64_t>(1, std::min<int64_t>(DV_MAX_FAR_CHUNKS, (8 * resident + tiles - 1) / tiles));
+  const int64_t tiles = bs_tiles(nt, TTV);
+  const int nchunk = bs_chunks(c, tiles, TTV);
   const dim3 grid((unsigned)tiles, nchunk);
   k_bs_x2<TTV><<<grid, FT2, 0, c->stream>>>(c->p, f->x, targets, nt, c->spos, c->sw, ns, c->d_cnt, nchunk, c->cap,
                                             c->far_acc);
@@ -1337,11 +1350,12 @@ static int bs_dispatch(dv_ctx* c, const dv_fields* f, const int32_t* targets, in
   const bool blob = c->p.kernel_mode == DV_KERNEL_BLOB3D;
   const int32_t* ns = c->d_flag + 2;
   if (precision == 32 && blob && !c->p.periodic && !c->p.compensated && D == 3 && c->far_tt > 2) {
-    // the paired loop (a tile of 2 keeps the scalar loop below); while no tile
-    // has been chosen, 8 targets a thread unless rounding nt up to its tiles
-    // costs more than it gives (65,536 x 65,536: 2.84 ms with 4, 2.67 with 8)
-    auto padded = [&](int64_t tt) { return (nt + FT2 * tt - 1) / (FT2 * tt) * (FT2 * tt); };
-    const int tt = c->far_tt_set ? c->far_tt : 100 * padded(8) <= 109 * padded(4) ? 8 : 4;
+    // The paired loop (a tile of 2 keeps the scalar loop below).  While no tile
+    // has been chosen, 8 targets a thread, 6% faster a pair, unless the busiest SM
+    // has more to do with them.  n x n with 4 and 8: 17,000 233 and 376 us, 33,000
+    // 772 and 711, 37,000 861 and 1,533, 53,865 1,788 and 2,216, 65,536 2,853 and
+    // 2,685, 131,072 9.8 and 10.6 ms, 262,144 38.5 and 36.7.
+    const int tt = c->far_tt_set ? c->far_tt : bs_cost(c, nt, 8) <= 1.06 * bs_cost(c, nt, 4) ? 8 : 4;
     if (tt <= 4) return launch_bs_x2<4>(c, f, targets, nt, ns, (float*)out);
     if (tt <= 6) return launch_bs_x2<6>(c, f, targets, nt, ns, (float*)out);
     return launch_bs_x2<8>(c, f, targets, nt, ns, (float*)out);
