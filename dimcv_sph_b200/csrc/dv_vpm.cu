@@ -672,13 +672,17 @@ __global__ void k_vel_fin(Geo<T> g, dv_vpm_plan p, const T* __restrict__ x, cons
                           const T* __restrict__ wt, const T* __restrict__ part, int nch, T* __restrict__ u) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= p.n) return;
-  T fx = T(0), fy = T(0);
+  // The chunks' partial sums in FP64, here and in the backward pass: the FP32
+  // loops have up to a hundred short chunks, whose FP32 sum was in some sizes
+  // further off than the few long ones before (3,136 x 3,136: 2.1e-7 of the norm
+  // against 1.7e-7).
+  double fx = 0.0, fy = 0.0;
   for (int c = 0; c < nch; ++c) {
-    fx += part[2 * ((int64_t)c * p.n + i)];
-    fy += part[2 * ((int64_t)c * p.n + i) + 1];
+    fx += (double)part[2 * ((int64_t)c * p.n + i)];
+    fy += (double)part[2 * ((int64_t)c * p.n + i) + 1];
   }
   const T fi = (T)p.f[i];
-  T ux = fi * fx, uy = fi * fy;
+  T ux = fi * (T)fx, uy = fi * (T)fy;
   const int k1 = p.nbr_off[i + 1];
   for (int k = p.nbr_off[i]; k < k1; ++k) {
     const int j = p.nbr[k];
@@ -808,10 +812,11 @@ __global__ void k_src_fin(dv_vpm_plan p, const T* __restrict__ sp, const T* __re
   const int ns = *p.n_src;
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= ns) return;
-  T a[5] = {T(0), T(0), T(0), T(0), T(0)};
+  double d[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
   for (int b = 0; b < ntb; ++b)
 #pragma unroll
-    for (int e = 0; e < 5; ++e) a[e] += spart[((int64_t)b * p.src_cap + s) * 5 + e];
+    for (int e = 0; e < 5; ++e) d[e] += (double)spart[((int64_t)b * p.src_cap + s) * 5 + e];
+  const T a[5] = {(T)d[0], (T)d[1], (T)d[2], (T)d[3], (T)d[4]};
   const T bs = sp[3 * s + 2];
   // −b_s [(−Σ s ĝ_y, Σ s ĝ_x) − 2 Σ s² c r]
   sg[3 * s] = bs * (a[2] + T(2) * a[3]);
@@ -827,13 +832,14 @@ __global__ void k_vel_bwd_fin(Geo<T> g, dv_vpm_plan p, const T* __restrict__ x, 
   if (k >= p.n) return;
   const T fk = (T)p.f[k];
   const P2<T> gk{gu[2 * k], gu[2 * k + 1]};
-  T P = T(0), Qx = T(0), Qy = T(0);
+  double sp = 0.0, sx = 0.0, sy = 0.0;
   for (int c = 0; c < nch; ++c) {
     const T* t = tpart + 3 * ((int64_t)c * p.n + k);
-    P += t[0];
-    Qx += t[1];
-    Qy += t[2];
+    sp += (double)t[0];
+    sx += (double)t[1];
+    sy += (double)t[2];
   }
+  const T P = (T)sp, Qx = (T)sx, Qy = (T)sy;
   const T hx = fk * gk.x, hy = fk * gk.y;
   T ox = -hy * P - T(2) * Qx, oy = hx * P - T(2) * Qy;
   T ow = T(0);
