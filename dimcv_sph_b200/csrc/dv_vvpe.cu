@@ -438,11 +438,15 @@ __device__ __forceinline__ void far_fix_one(const dv_params& P, const DevGrid& G
   const float lim = P.far_r2_limit, d2 = P.blob_delta2;
   const float3 bx = make_float3(P.box[0], P.box[1], P.box[2]);
   float4 acc = far_acc[t];
-  for (int k = 1; k < nchunk; ++k) {  // sample-chunk partials, in chunk order
-    const float4 q = far_acc[k * stride + t];
-    acc.x = __fadd_rn(acc.x, q.x);
-    acc.y = __fadd_rn(acc.y, q.y);
-    acc.z = __fadd_rn(acc.z, q.z);
+  if (nchunk > 1) {  // sample-chunk partials, in chunk order; in FP64, so that more chunks never cost precision
+    double sx = acc.x, sy = acc.y, sz = acc.z;
+    for (int k = 1; k < nchunk; ++k) {
+      const float4 q = far_acc[k * stride + t];
+      sx += (double)q.x;
+      sy += (double)q.y;
+      sz += (double)q.z;
+    }
+    acc.x = (float)sx, acc.y = (float)sy, acc.z = (float)sz;
   }
   int near_cnt = 0;
   int lo0, hi0, lo1, hi1, lo2 = 0, hi2 = 0;
